@@ -53,6 +53,22 @@ DRB_DEV uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_sh
 // k-slice. The XOR keeps both patterns free of bank conflicts for slices of 4, 8 or 16 floats... per lane.
 DRB_DEV int swz4(int g) { return g ^ ((g >> 3) & 7); }
 
+// One lane of a converged warp, the same one every time. Code that issues tensor-core or tiled-copy instructions is
+// guarded by this and not by `lane == 0`: their descriptors live in uniform registers, and only behind elect.sync does
+// the compiler know that one lane runs and leave out the per-lane loops around the moves into them. Measured per
+// tcgen05.mma (M = 128, N = 16..64): 134-172 cycles of issue behind `lane == 0`, 39-48 (the unit itself) behind this.
+DRB_DEV bool elect_one() {
+  unsigned ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      :
+      : "memory");
+  return ok != 0;
+}
+
 // ------------------------------------------------------------------------------------------
 // programmatic dependent launch
 
@@ -104,10 +120,20 @@ DRB_DEV bool mbar_wait(uint64_t* bar, unsigned parity, unsigned err_code, unsign
 }
 
 // The same for a wait on a ring's step-to-step path: no sleep between polls (a sleeping waiter adds its wake-up time
-// to every hand-over of the ring), bounded all the same.
+// to every hand-over of the ring), and each poll may suspend the warp in hardware for up to 2 us: a warp that polls takes
+// issue slots from the ones that work (measured in the grouped GEMMs: half of all instructions issued). Bounded all the same.
 DRB_DEV bool mbar_wait_hot(uint64_t* bar, unsigned parity, unsigned err_code) {
-  for (unsigned it = 0; it < (1u << 24); ++it)
-    if (mbar_try_wait(bar, parity)) return true;
+  for (unsigned it = 0; it < (1u << 20); ++it) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(2000u)
+        : "memory");
+    if (ok) return true;
+  }
   atomicMax(&g_drb_error, err_code);
   return false;
 }

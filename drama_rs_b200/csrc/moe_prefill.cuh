@@ -1,5 +1,5 @@
 // Prefill-side kernels of the MoE path: per-row routing bookkeeping (count / permute / combine and the fused
-// grouping step), the launchers of the expert-grouped GEMMs (moe_prefill_mma.cuh), and the elementwise helpers the
+// grouping step), the launchers of the expert-grouped GEMMs (moe_prefill_tc.cuh), and the elementwise helpers the
 // reference's prefill calls around cuBLAS (dequant_q8, f32_to_bf16, swiglu_rows, rmsnorm).
 //
 // Replaces kernels/drama.cu:744-968 and 1114-1202 of the reference, same C signatures
@@ -7,6 +7,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "moe_prefill_tc.cuh"
 
 namespace pf {
 
@@ -360,7 +361,7 @@ __global__ void __launch_bounds__(256)
     const float v = xr[i] * inv * w[i];
     if (y) y[(size_t)blockIdx.x * D + i] = v;
     if (yb) {
-      if (F16) reinterpret_cast<__half*>(yb)[(size_t)blockIdx.x * D + i] = pfmma::f2h_sat(v);
+      if (F16) reinterpret_cast<__half*>(yb)[(size_t)blockIdx.x * D + i] = tc::f2h_sat(v);
       else yb[(size_t)blockIdx.x * D + i] = __float2bfloat16(v);
     }
   }
@@ -553,12 +554,10 @@ extern "C" int dr_moe_prefill(const uint8_t* gu_q, const __half2* gu_sm, const u
   if (E <= 0) return 0;
   const DrbDevice& dev = drb_device(st);
   if (!dev.ready) return -2;
-  const dim3 grid(pfmma::BLOCKS_PER_SM * dev.sms), block(pfmma::THREADS);
-  drb_launch(pfmma::k_grouped<0, 0, false>, grid, block, pfmma::SMEM_BYTES, st, false, gu_q, (const void*)gu_sm, (const void*)xp,
-             (void*)act, offsets, counts, E, pfmma::SharedExpert{}, (const int*)nullptr, 0, (const int*)nullptr);
-  drb_launch(pfmma::k_grouped<1, 0, false>, grid, block, pfmma::SMEM_BYTES, st, false, d_q, (const void*)d_sm, (const void*)act,
-             (void*)y, offsets, counts, E, pfmma::SharedExpert{}, (const int*)nullptr, 0, (const int*)nullptr);
-  return 0;
+  pft::Block b = {};
+  b.gu_w = gu_q, b.gu_s = gu_sm, b.d_w = d_q, b.d_s = d_sm, b.sgu_s = gu_sm, b.sd_s = d_sm, b.x = xp, b.x_bf16 = true;
+  b.offsets = offsets, b.counts = counts, b.act = act, b.y = y, b.E = E;
+  return pft::run_block<0>(b, dev, st);
 }
 
 // No counterpart in the reference. Count, exclusive scan and slot assignment of the (row, k) pairs in one launch:
@@ -666,8 +665,6 @@ extern "C" int drb_ep_wait(const unsigned* flags, int world, unsigned* step, uns
 // Every pointer of a part that runs must be a valid device address; with E = 0 or rows_sh = 0 the arrays of the part
 // that does not run are not used, but must still be valid addresses (any buffer will do, NULL will not): the compiler
 // may issue a load ahead of the branch that decides whether its value is needed. row_of and y_row_of may be NULL.
-// fp16 rows and E <= 256 take the kernels of moe_prefill_tma.cuh (and only they can store results to peers: peer_y);
-// bf16 rows, or more experts, the kernels of moe_prefill_mma.cuh.
 static int prefill_block_impl(const uint8_t* gu_q, const __half2* gu_sm, const uint8_t* d_q, const __half2* d_sm,
                                      const int8_t* sgu_q, const __half* sgu_s, const int8_t* sd_q, const __half* sd_s,
                                      const __nv_bfloat16* xb, const int* row_of, const int* offsets, const int* counts,
@@ -679,32 +676,12 @@ static int prefill_block_impl(const uint8_t* gu_q, const __half2* gu_sm, const u
     return -1;
   const DrbDevice& dev = drb_device(st);
   if (!dev.ready) return -2;
-  if (x_f16 && E <= pft::MAX_ITEM_SETS - 1) {
-    // fp16 rows: the kernels of moe_prefill_tma.cuh (weights by tiled TMA, token tiles by asynchronous copies)
-    const uint64_t ne = (uint64_t)(E > 0 ? E : 1);
-    CUtensorMap m_gu, m_d, m_sgu, m_sd;
-    if (pft::map_gate_up(&m_gu, gu_q, ne, I, H / 2) || pft::map_gate_up(&m_sgu, sgu_q, 1, I, H) ||
-        pft::map_rows(&m_d, d_q, ne * H, I / 2) || pft::map_rows(&m_sd, sd_q, H, I))
-      return -3;
-    const dim3 grid2(2 * dev.sms), block2(pft::THREADS);
-    const int ee = E > 0 ? E : 0, rs = rows_sh > 0 ? rows_sh : 0;
-    const __half* rows16 = reinterpret_cast<const __half*>(xb);
-    drb_launch(pft::k_grouped_tma<0>, grid2, block2, pft::SMEM_BYTES, st, false, m_gu, gu_sm, m_sgu, sgu_s, rows16, rows16, (void*)act,
-               (void*)sh_act, offsets, counts, ee, rs, row_of, (const int*)nullptr, (float* const*)nullptr, 0, 0);
-    drb_launch(pft::k_grouped_tma<1>, grid2, block2, pft::SMEM_BYTES, st, false, m_d, d_sm, m_sd, sd_s,
-               reinterpret_cast<const __half*>(act), reinterpret_cast<const __half*>(sh_act), (void*)y, (void*)sh_out, offsets, counts, ee, rs,
-               (const int*)nullptr, y_row_of, peer_y, peer_cap, peer_rank);
-    return 0;
-  }
-  if (peer_y) return -1;  // results to the peers: the TMA kernels only
-  const dim3 grid(pfmma::BLOCKS_PER_SM * dev.sms), block(pfmma::THREADS);
-  const pfmma::SharedExpert s0{sgu_q, sgu_s, (const void*)xb, (void*)sh_act, rows_sh};
-  const pfmma::SharedExpert s1{sd_q, sd_s, (const void*)sh_act, (void*)sh_out, rows_sh};
-  drb_launch(pfmma::k_grouped<0, 0, true>, grid, block, pfmma::SMEM_BYTES, st, false, gu_q, (const void*)gu_sm, (const void*)xb,
-             (void*)act, offsets, counts, E, s0, row_of, x_f16, (const int*)nullptr);
-  drb_launch(pfmma::k_grouped<1, 0, true>, grid, block, pfmma::SMEM_BYTES, st, false, d_q, (const void*)d_sm, (const void*)act,
-             (void*)y, offsets, counts, E, s1, (const int*)nullptr, 1, y_row_of);
-  return 0;
+  pft::Block b = {};
+  b.gu_w = gu_q, b.gu_s = gu_sm, b.d_w = d_q, b.d_s = d_sm, b.sgu_q = sgu_q, b.sgu_s = sgu_s, b.sd_q = sd_q, b.sd_s = sd_s;
+  b.x = xb, b.x_bf16 = !x_f16, b.row_of = row_of, b.offsets = offsets, b.counts = counts, b.y_row_of = y_row_of;
+  b.act = act, b.y = y, b.sh_act = sh_act, b.sh_out = sh_out, b.rows_sh = rows_sh > 0 ? rows_sh : 0, b.E = E > 0 ? E : 0;
+  b.peer_y = peer_y, b.peer_cap = peer_cap, b.peer_rank = peer_rank;
+  return pft::run_block<0>(b, dev, st);
 }
 
 extern "C" int drb_moe_prefill_block(const uint8_t* gu_q, const __half2* gu_sm, const uint8_t* d_q, const __half2* d_sm,
@@ -719,7 +696,7 @@ extern "C" int drb_moe_prefill_block(const uint8_t* gu_q, const __half2* gu_sm, 
 // buffers: y_row_of[slot] = s * cap + j names the token's source rank s and its slot j in this rank's receive
 // order; its result row goes to peer_y[s] (device array of every rank's result buffer [world * cap, h] f32) at row
 // rank * cap + j, over NVLink, from the down GEMM's epilogue. Follow with drb_ep_signal; the home rank's
-// drb_ep_wait then covers the results. fp16 rows and e <= 256 only (-1 otherwise). y is not written.
+// drb_ep_wait then covers the results. fp16 rows only. y is not written.
 extern "C" int drb_moe_prefill_block_peers(const uint8_t* gu_q, const __half2* gu_sm, const uint8_t* d_q, const __half2* d_sm,
                                            const int8_t* sgu_q, const __half* sgu_s, const int8_t* sd_q, const __half* sd_s,
                                            const __nv_bfloat16* xb, const int* row_of, const int* offsets, const int* counts,
@@ -739,29 +716,10 @@ extern "C" int dr_moe_prefill_fp8(const uint8_t* gu_w, const float* gu_s, const 
   if (E <= 0) return 0;
   const DrbDevice& dev = drb_device(st);
   if (!dev.ready) return -2;
-  // The weights reach the tensor cores as E4M3 (moe_prefill_fp8.cuh). DRB_FP8_DEQUANT=1 (read at every call) selects the
-  // earlier kernels, whose threads turn every weight into fp16 first: the route for more than 256 experts, kept
-  // selectable so that both can be compared and tested on the same inputs; same results within the parity bar.
-  const char* route = getenv("DRB_FP8_DEQUANT");
-  const bool dequant_route = route && route[0] == '1';
-  if (!dequant_route && E <= pf8::MAX_ITEM_SETS) {
-    CUtensorMap tm_gu, tm_d;
-    // 256-byte L2 promotion: a chunk's box brings the next chunk's 128 bytes of every row into L2 with it
-    if (pft::map_rows(&tm_gu, gu_w, (uint64_t)E * 2 * pf::I, pf::H, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) != 0) return -3;
-    if (pft::map_rows(&tm_d, d_w, (uint64_t)E * pf::H, pf::I, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) != 0) return -3;
-    const dim3 grid(2 * dev.sms), block(pf8::THREADS);
-    // y is written last (by the down kernel); until then its first floats hold every token row's largest magnitude
-    pf8::k_rowmax_bf16<<<2 * dev.sms, 256, 0, st>>>(xp, offsets, counts, E, y);
-    drb_launch(pf8::k_gate_up_fp8, grid, block, pf8::SMEM, st, false, tm_gu, gu_s, xp, (const float*)y, (__half*)act, offsets, counts, E);
-    drb_launch(pf8::down::k_down_fp8, grid, dim3(pf8::down::THREADS), pf8::down::SMEM, st, false, tm_d, d_s, (const __half*)act, y, offsets, counts, E);
-    return 0;
-  }
-  const dim3 grid(pfmma::BLOCKS_PER_SM * dev.sms), block(pfmma::THREADS);
-  drb_launch(pfmma::k_grouped<0, 1, false>, grid, block, pfmma::SMEM_BYTES, st, false, gu_w, (const void*)gu_s, (const void*)xp,
-             (void*)act, offsets, counts, E, pfmma::SharedExpert{}, (const int*)nullptr, 0, (const int*)nullptr);
-  drb_launch(pfmma::k_grouped<1, 1, false>, grid, block, pfmma::SMEM_BYTES, st, false, d_w, (const void*)d_s, (const void*)act,
-             (void*)y, offsets, counts, E, pfmma::SharedExpert{}, (const int*)nullptr, 0, (const int*)nullptr);
-  return 0;
+  pft::Block b = {};
+  b.gu_w = gu_w, b.gu_s = gu_s, b.d_w = d_w, b.d_s = d_s, b.x = xp, b.x_bf16 = true;
+  b.offsets = offsets, b.counts = counts, b.act = act, b.y = y, b.E = E;
+  return pft::run_block<1>(b, dev, st);
 }
 
 // Reference: kernels/drama.cu:1130-1134; src/ffi.rs:74. K a multiple of 128.

@@ -1,0 +1,886 @@
+// The expert-grouped prefill GEMMs (dr_moe_prefill, dr_moe_prefill_fp8, drb_moe_prefill_block and its peer-store form) on
+// the 5th-generation tensor cores, with the dequantised weights handed over in TENSOR memory.
+//
+//   gate/up:  for expert e with its tokens  D[128, nt] = W_tile[128, 2048] . X_e[nt, 2048]^T
+//             (the tile interleaves 64 gate rows with their 64 up rows), epilogue silu(g) * u -> act
+//   down:     D[128, nt] = Wd_tile[128, 512] . act_e[nt, 512]^T -> y
+//
+// The weight rows are the MMA's M = 128 dimension and the tokens its N dimension (16 .. 64): most experts see a handful
+// of tokens. Weights are int4 (scale and min per 64 inputs), block-FP8 (one f32 scale per 128 x 128 block) or, for the
+// shared expert, int8; every one becomes an fp16 operand with one rounding, accumulated in fp32.
+//
+// What bounds it. A weight is read once from HBM, so the floor is 1.77 MB (int4) or 3 MB (FP8) per expert hit at the copy
+// rate. Between HBM and the tensor core stands the conversion: 1.6 thread-instructions per int4 weight, 40 us for 256
+// experts on all issue slots. An A operand in SHARED memory would add its store, its read by the MMA and the raw bytes'
+// two passes, 5 bytes per weight through 128 B per cycle = 113 us, more than HBM takes; in tensor memory the same tile
+// costs one tcgen05.st (measured 700 B per cycle and multiprocessor), the MMA reads it there (14, 19, 32 cycles for
+// N = 16, 32, 64; from shared memory never below 39), and shared memory carries the raw bytes only.
+//
+// Roles, one block of 24 warps per multiprocessor, meeting only on mbarriers, every wait bounded (common.cuh):
+//   16 convert warps  a step is 256 inputs of 128 rows; two groups of eight warps take turns. A thread converts 128 inputs of
+//                 one row: four (int4) or eight (8-bit) 16-byte pieces out of the swizzled raw stage, two 32-column
+//                 tcgen05.st. Three stages: 128 columns each, with a token tile in shared memory.
+//   MMA warp      sixteen K = 16 instructions per step, one commit that frees the stage
+//   loader warp   tiled TMA: 128 rows x 128 bytes per request with the 128-byte swizzle; a gate/up tile arrives with gate
+//                 row j and up row j interleaved, which a 4-D view of the weight tensor expresses; the item's scales
+//                 ride on its first request
+//   token warp    the tokens' fp16 rows: groups of eight consecutive rows by one TMA request per step (4 KB: eight rows of
+//                 four 128-byte swizzled columns), scattered rows by tile::gather4 (512 bytes per request; it costs the copy
+//                 engine 19 cycles against 49 for the 4 KB box)
+//   table warp    the items' rows, result rows and row factors, ahead of everybody
+//   4 epilogue warps  drain an item's accumulator while the next item's MMAs fill the other one
+//
+// Work items: (shared expert or expert, group of up to 64 tokens, 128-row tile), enumerated from the device-side
+// counts by a prefix sum each block computes for itself, the shared expert's items first, walked round robin.
+// Replaces kernels/drama.cu:799-1109 of the reference (k_moe_pf_gate_up, k_moe_pf_down and their FP8 forms) together with
+// the cuBLAS shared expert of src/engine.rs:351-355, 560-562.
+#pragma once
+
+#include <cuda.h>  // CUtensorMap and the encode function's type only: the entry point is resolved at run time
+
+#include "common.cuh"
+#include "tcgen05.cuh"
+
+namespace pft {
+
+using namespace tc;
+
+constexpr int H = 2048, I = 512;
+constexpr int CONV_WARPS = 16, GROUP_WARPS = 8, EPI_WARPS = 4;
+constexpr int EPI_WARP0 = CONV_WARPS, MMA_WARP = EPI_WARP0 + EPI_WARPS, LOAD_WARP = MMA_WARP + 1, TOKEN_WARP = MMA_WARP + 2, TABLE_WARP = MMA_WARP + 3;
+constexpr int THREADS = (TABLE_WARP + 1) * 32;  // 768
+constexpr int TILE_M = 128;
+constexpr int STEP_K = 256;
+constexpr int MAX_NT = 64;                      // tokens per work item at most
+constexpr int NST = 3;                          // stages: an A tile in tensor memory with its token tile in shared memory
+constexpr int A_COLS = STEP_K / 2;              // 32-bit columns of one A tile
+constexpr int A_COL0 = 128;                     // ahead of them: the accumulators
+constexpr int TMEM_COLS = 512;
+static_assert(A_COL0 + NST * A_COLS <= TMEM_COLS, "tensor memory");
+constexpr int ROW_BYTES = 128;
+constexpr int RAW_BYTES = TILE_M * ROW_BYTES;   // 16 KB: 256 int4 or 128 8-bit inputs of the tile's 128 rows
+constexpr int NTAB = 4;
+constexpr int MAX_E = 1024;                     // experts per launch; more are taken by further launches
+constexpr int CTL_BYTES = 1024;
+constexpr int SET_BYTES = (MAX_E + 2) * 4 + 8;
+constexpr int TOKEN_STRIDE = 2 * H * 2;         // bytes between prepared token rows (k_prep_rows): fp16 row | factor
+
+struct Tab {  // one work item
+  int cols, mt, shared;         // accumulator columns (the MMA's N)
+  int full, srow, start;        // contiguous rows: so many boxes of eight from row srow on, and one more from row start (-1: none)
+  int quads, pad;               // rows fetched by number: so many fours of rows[], behind the boxes
+  __align__(16) int rows[MAX_NT];
+  __align__(16) int dst[MAX_NT];    // result row of each column, -1: none
+  __align__(16) float fac[MAX_NT];  // what the column's token row was divided by
+};
+struct Ctl {
+  uint64_t rawfull[10], rawempty[10];      // a raw stage has landed / has been read (one arrival per convert warp of a group)
+  uint64_t smfull[4];                      // an int4 item's scales have landed
+  uint64_t full[NST];                      // a stage is complete: the A tile (one arrival per convert warp of a group) and the token tile (TMA)
+  uint64_t done[NST];                      // the MMAs that read it have completed (tcgen05.commit)
+  uint64_t accfull[4], accfree[4];         // an accumulator is complete (tcgen05.commit) / has been drained (one arrival per epilogue warp)
+  uint64_t tabfull[NTAB], tabempty[NTAB];  // written / read for the last time (token, MMA and epilogue warps)
+  int wtot[THREADS / 32];                  // the prefix sum's warp totals
+  uint32_t tmem_base;
+};
+static_assert(sizeof(Ctl) <= CTL_BYTES, "control block");
+
+// Sizes of k_grouped<GEMM, FMT, .> and its shared memory: control block | raw stages | token tiles | int4 scales | tables | item prefix.
+template <int GEMM, int FMT>
+struct Smem {
+  static constexpr int NT = FMT == 1 ? 32 : 64;    // tokens per item
+  static constexpr int NACC = FMT == 1 ? 4 : 2;    // accumulators: int4: one per item; FP8: one per 128 inputs (see k_grouped)
+  static constexpr int B_BYTES = NT * STEP_K * 2;  // one token tile
+  static_assert(NT <= MAX_NT && NT * NACC <= A_COL0, "tensor memory");
+  static constexpr int NRAW = FMT == 1 ? 10 : GEMM == 0 ? 5 : 6;           // what fits; four are enough for the copy rate (a stream of such boxes alone: 6.2 TB/s with 4, 6.5 with 6)
+  static constexpr int NSM = FMT != 0 ? 0 : GEMM == 0 ? 2 : 4;             // slots for an int4 item's (scale, min) pairs: see the loader
+  static constexpr int SMB = TILE_M * ((GEMM == 0 ? H : I) / 64) * 4;      // bytes of one
+  static constexpr size_t BYTES = 1024 /* alignment slack */ + CTL_BYTES + NRAW * RAW_BYTES + NST * B_BYTES + NSM * SMB + NTAB * sizeof(Tab) + SET_BYTES;
+  static_assert(BYTES <= 232448, "shared memory");
+};
+
+// ---- weights -> fp16 ---------------------------------------------------------------------------------------------
+// A nibble in bits 0..3 of a 16-bit half, or-ed into 0x6400, is the half 1024 + q; a nibble in bits 4..7, or-ed into
+// 0x5400, is the half 64 + q (the unit in the last place of 64 is 1/16). Subtracting the offset is exact, the fused
+// multiply-add q*s + m rounds once.
+// The offsets live in registers the compiler cannot rebuild from immediates: it would, once per use.
+struct NibbleConst {
+  uint32_t k1024, k64, mixed;  // (1024, 1024), (64, 64), (1024, 64)
+  DRB_DEV NibbleConst() {
+    asm volatile("mov.b32 %0, 0x64006400;" : "=r"(k1024));
+    asm volatile("mov.b32 %0, 0x54005400;" : "=r"(k64));
+    asm volatile("mov.b32 %0, 0x54006400;" : "=r"(mixed));
+  }
+};
+template <uint32_t MASK>
+DRB_DEV uint32_t mask_or(uint32_t w, uint32_t c) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "n"(MASK), "r"(c));
+  return r;
+}
+DRB_DEV uint32_t sub_fma(uint32_t t, uint32_t off, __half2 s2, __half2 m2) {
+  const __half2 r = __hfma2(__hsub2(*reinterpret_cast<const __half2*>(&t), *reinterpret_cast<const __half2*>(&off)), s2, m2);
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+// Eight nibbles of one word in the order (0,4) (1,5) (2,6) (3,7): one shift serves both upper pairs, 13 instructions. The
+// token rows have to come in the same order.
+DRB_DEV void dequant8_perm(uint32_t w, __half2 s2, __half2 m2, const NibbleConst& c, uint32_t* o) {
+  const uint32_t w8 = w >> 8;
+  o[0] = sub_fma(mask_or<0x000F000Fu>(w, c.k1024), c.k1024, s2, m2);
+  o[1] = sub_fma(mask_or<0x00F000F0u>(w, c.k64), c.k64, s2, m2);
+  o[2] = sub_fma(mask_or<0x000F000Fu>(w8, c.k1024), c.k1024, s2, m2);
+  o[3] = sub_fma(mask_or<0x00F000F0u>(w8, c.k64), c.k64, s2, m2);
+}
+// The same in k order: a byte holds a consecutive pair, a permute puts it into both halves. 16 instructions.
+DRB_DEV void dequant8_nat(uint32_t w, __half2 s2, __half2 m2, const NibbleConst& c, uint32_t* o) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) o[i] = sub_fma(mask_or<0x00F0000Fu>(prmt(w, 0u, 0x1111u * i), c.mixed), c.mixed, s2, m2);
+}
+// Eight int8 weights (two words) times one fp16 scale, in k order or in the order of dequant8_perm. 0x6400 | (b ^ 0x80) is
+// the half 1024 + 128 + b; subtracting 1152 is exact, the product rounds once.
+template <bool PERM>
+DRB_DEV void dequant8_i8(uint32_t w0, uint32_t w1, __half2 s2, uint32_t* o) {
+  const __half2 k1152 = __half2half2(__ushort_as_half((unsigned short)0x6480));
+  const uint32_t u0 = w0 ^ 0x80808080u, u1 = w1 ^ 0x80808080u;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    uint32_t t;
+    if (PERM) t = lop3_and_or(prmt(u0, u1, (uint32_t)(i | (i << 4) | ((4 + i) << 8) | ((4 + i) << 12))), 0x00FF00FFu, 0x64006400u);
+    else t = prmt(i < 2 ? u0 : u1, 0x64646464u, (i & 1) ? 0x4342u : 0x4140u);
+    const __half2 r = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&t), k1152), s2);
+    o[i] = *reinterpret_cast<const uint32_t*>(&r);
+  }
+}
+// Four E4M3 weights, in k order: every one is an fp16 number. The block scales stay out of the operands (see k_grouped).
+DRB_DEV void dequant4_e4m3(uint32_t w, uint32_t* o) {
+  asm("{.reg .b16 lo, hi; mov.b32 {lo, hi}, %2; cvt.rn.f16x2.e4m3x2 %0, lo; cvt.rn.f16x2.e4m3x2 %1, hi;}" : "=r"(o[0]), "=r"(o[1]) : "r"(w));
+}
+// Position of input k within its eight in dequant8_perm's order.
+DRB_DEV int perm_pos(int k) { return (k & ~7) | ((k & 3) << 1) | ((k >> 2) & 1); }
+
+// ---- token rows ----------------------------------------------------------------------------------------------------
+// 16-bit rows -> fp16 rows in slot order at a stride of TOKEN_STRIDE bytes: routed slot s from row (row_of ? row_of[s] : s)
+// of x into dst, shared row r from row r of x into sh_dst; in the order of dequant8_perm when PERM. The down kernel's
+// outputs serve as the buffers (they are written after the gate/up kernel has read the rows), each row's factor sits behind its
+// 4 KB. bf16 rows carry a wider range than fp16: a row whose largest magnitude lies outside [2^-4, 2^15) is divided
+// by a power of two (the factor; the gate/up epilogue multiplies it back), every other row keeps its values.
+// One warp per row; L2 traffic only (8 KB per slot, 20 MB at 300 rows: 4 us).
+template <bool BF16, bool PERM>
+__global__ void __launch_bounds__(256)
+    k_prep_rows(const uint4* __restrict__ x, const int* __restrict__ row_of, const int* __restrict__ offsets, const int* __restrict__ counts, int E,
+                unsigned char* __restrict__ dst, int rows_sh, unsigned char* __restrict__ sh_dst) {
+  __shared__ int s_total;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) s_total = 0;
+  __syncthreads();
+  int end = 0;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    const int c = __ldg(counts + e);
+    if (c > 0) end = max(end, __ldg(offsets + e) + c);
+  }
+  end = __reduce_max_sync(0xffffffffu, end);
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_total, end);
+  __syncthreads();
+  const int total = s_total, lane = threadIdx.x & 31;
+  constexpr int PER = H / 8 / 32;
+  for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < total + rows_sh; i += gridDim.x * (blockDim.x >> 5)) {
+    const bool sh = i >= total;
+    const int row = sh ? i - total : (row_of ? __ldg(row_of + i) : i);
+    const uint4* p = x + (size_t)row * (H / 8);
+    unsigned char* out = sh ? sh_dst + (size_t)(i - total) * TOKEN_STRIDE : dst + (size_t)i * TOKEN_STRIDE;
+    uint4 v[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) v[j] = __ldcg(p + j * 32 + lane);
+    float inv = 1.f;
+    if (BF16) {
+      uint32_t m = 0u;  // bf16 with the sign bit cleared orders like an integer
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) m = max(m, max(w[q] & 0x7fffu, (w[q] >> 16) & 0x7fffu));
+      }
+      m = __reduce_max_sync(0xffffffffu, m);
+      const int e = (int)(m >> 7);  // biased exponent of the largest magnitude
+      float fac = 1.f;
+      if (m != 0u && e < 255 && (e < 127 - 4 || e >= 127 + 15)) {
+        const int ec = min(max(e, 2), 252);
+        fac = __uint_as_float((uint32_t)ec << 23), inv = __uint_as_float((uint32_t)(254 - ec) << 23);
+      }
+      if (lane == 0) *reinterpret_cast<float*>(out + H * 2) = fac;
+    }
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      uint4 o = v[j];
+      if (BF16) {
+        const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+        uint32_t* op = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) op[q] = f2h2_sat(__uint_as_float(w[q] << 16) * inv, __uint_as_float(w[q] & 0xffff0000u) * inv);
+      }
+      if (PERM) o = make_uint4(prmt(o.x, o.z, 0x5410u), prmt(o.x, o.z, 0x7632u), prmt(o.y, o.w, 0x5410u), prmt(o.y, o.w, 0x7632u));
+      reinterpret_cast<uint4*>(out)[j * 32 + lane] = o;
+    }
+  }
+}
+
+// ---- the grouped GEMM ----------------------------------------------------------------------------------------------
+// A position in a ring of N mbarriers and the parity its next completion has there, moved without a division: a convert
+// warp's step is 104 instructions of conversion, and index arithmetic had grown to 60 more.
+template <int N>
+struct Ring {
+  int i = 0;
+  uint32_t par = 0;
+  DRB_DEV void next(int k = 1) {  // k < N
+    i += k;
+    if (i >= N) i -= N, par ^= 1u;
+  }
+};
+// Bounded wait on barrier bars[r.i]; after one that ran out no later wait of the thread spins.
+template <int N>
+DRB_DEV void wait_at(uint64_t* bars, const Ring<N>& r, unsigned err, bool& dead) {
+  if (!dead) dead = !mbar_wait_hot(bars + r.i, r.par, err);
+}
+
+struct Maps {
+  CUtensorMap q;             // the routed experts' weights
+  CUtensorMap sm;            // int4 gate/up: their (scale, min) pairs, the same view
+  CUtensorMap sh;            // the shared expert's int8 weights
+  CUtensorMap tok8, tok1;    // routed token rows: boxes of eight rows x four 128-byte columns / single rows for gather4
+  CUtensorMap shtok8, shtok1;
+};
+struct Args {
+  const void* scales;        // int4: (scale, min) [E, R, K/64];  FP8: f32 [E, R/128, K/128]
+  const __half* shs;         // the shared expert's scales [R, K/128]
+  void *dst, *sh_dst;        // gate/up: act fp16 [., I];  down: y f32 [., H]
+  const int *offsets, *counts;
+  const int* row_of;         // gathered form (PREP = false) of gate/up: slot -> row
+  const int* dst_row_of;     // down: slot -> row of dst, or NULL
+  const unsigned char *fac, *sh_fac;  // prepared bf16 rows: where the factors lie (row i at i * TOKEN_STRIDE + 4096), or NULL
+  float* const* peer_y;      // down, routed results only: every rank's result buffer, or NULL. dst_row_of[slot] = s * cap + j
+  int peer_cap, peer_rank;   //   names the token's source rank s and its slot j there; the row is stored straight into
+                             //   rank s's buffer at row rank * cap + j over NVLink
+  int E, rows_sh;
+};
+
+// GEMM = 0: gate/up + SwiGLU; 1: down. FMT = 0: int4 experts; 1: block-FP8 experts.
+// FP8: a tile row's weights share one f32 scale over 128 inputs. Multiplied into the fp16 operand it would cost every weight
+// a rounding (measured 4.2e-4 per row against 2.1e-4); here the operands are exact, the MMAs of each 128 inputs have an
+// accumulator of their own (a ring of four), and the epilogue warps sum scale * accumulator in fp32 as they complete.
+// PREP (gate/up): the token rows are prepared (contiguous in slot order; int4: permuted); otherwise they are gathered
+// through row_of in k order. The down kernel's rows are the act array, contiguous, int4: permuted by the gate/up epilogue.
+template <int GEMM, int FMT, bool PREP>
+__global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ Maps maps, const Args a) {
+  constexpr int K = GEMM == 0 ? H : I;
+  constexpr int R = GEMM == 0 ? 2 * I : H;
+  constexpr int MT = R / TILE_M;         // tiles per expert: 8 / 16
+  constexpr int NSTEP = K / STEP_K;      // steps per item: 8 / 2
+  constexpr bool PERM = FMT == 0 && PREP;
+  using S = Smem<GEMM, FMT>;
+  constexpr int NRAW = S::NRAW, NSM = S::NSM, SMB = S::SMB, NT = S::NT, NACC = S::NACC, B_BYTES = S::B_BYTES;
+  extern __shared__ unsigned char dyn_raw[];
+  unsigned char* dyn = dyn_raw + (-smem_u32(dyn_raw) & 1023u);  // an offset, not a rounded address: loads stay shared-memory loads
+  Ctl& ctl = *reinterpret_cast<Ctl*>(dyn);
+  unsigned char* raw = dyn + CTL_BYTES;
+  unsigned char* bring = raw + NRAW * RAW_BYTES;
+  unsigned char* smbuf = bring + NST * B_BYTES;
+  Tab* tabs = reinterpret_cast<Tab*>(smbuf + NSM * SMB);
+  int* base = reinterpret_cast<int*>(tabs + NTAB);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NRAW; ++s) mbar_init(&ctl.rawfull[s], 1), mbar_init(&ctl.rawempty[s], GROUP_WARPS);
+    for (int s = 0; s < NSM; ++s) mbar_init(&ctl.smfull[s], 1);
+    for (int s = 0; s < NST; ++s) mbar_init(&ctl.full[s], GROUP_WARPS + 1), mbar_init(&ctl.done[s], 1);
+    for (int s = 0; s < NACC; ++s) mbar_init(&ctl.accfull[s], 1), mbar_init(&ctl.accfree[s], EPI_WARPS);
+    for (int s = 0; s < NTAB; ++s) mbar_init(&ctl.tabfull[s], 1), mbar_init(&ctl.tabempty[s], 2 + EPI_WARPS);
+    mbar_fence_init();
+  }
+  if (warp == MMA_WARP) tmem_alloc(&ctl.tmem_base, TMEM_COLS);
+  if (GEMM == 0) {
+    pdl_wait();  // counts, offsets and the token rows
+    pdl_launch_dependents();
+  }
+  // The down kernel follows the gate/up kernel, which lets its dependents start only after its own wait: counts and
+  // offsets are final by now, and so the weights can be requested while the last gate/up items still run.
+  // Items per set (set 0: the shared expert, set 1 + e: expert e), exclusive prefix in base[].
+  const int n_sets = a.E + 1;
+  {
+    constexpr int PER = (MAX_E + 1 + THREADS - 1) / THREADS;
+    int it[PER], sum = 0;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int s = threadIdx.x * PER + j;
+      const int cnt = s >= n_sets ? 0 : s == 0 ? a.rows_sh : __ldg(a.counts + s - 1);
+      it[j] = sum, sum += ((cnt + NT - 1) / NT) * MT;
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += u;
+    }
+    if (lane == 31) ctl.wtot[warp] = incl;
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    int before = incl - sum;
+    for (int w = 0; w < warp; ++w) before += ctl.wtot[w];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int s = threadIdx.x * PER + j;
+      if (s <= n_sets) base[s] = before + it[j];  // base[n_sets]: the total
+    }
+    __syncthreads();
+  }
+  const uint32_t tmem = ctl.tmem_base;
+  const int total_items = base[n_sets];
+
+  struct Item {
+    bool shared;
+    int e, mt, n0;
+  };
+  int cur = 0;  // the item's set: items come in ascending order, so the search goes on where it stood (whole warps)
+  auto decode = [&](int item) {
+    for (;;) {
+      const int s = cur + 1 + lane;
+      const int n = __popc(__ballot_sync(0xffffffffu, s < n_sets && base[s] <= item));
+      cur += n;
+      if (n < 32) break;
+    }
+    Item it;
+    it.shared = FMT == 0 && cur == 0;
+    it.e = cur - 1;
+    const int local = item - base[cur];
+    it.mt = local % MT;
+    it.n0 = (local / MT) * NT;
+    return it;
+  };
+  // weight row of tile row r: a gate/up tile interleaves gate j (even r) with up j (odd r)
+  auto weight_row = [&](int mt, int r) { return GEMM == 0 ? (r & 1) * I + mt * (TILE_M / 2) + (r >> 1) : mt * TILE_M + r; };
+
+  bool dead = false;    // a wait ran out once: stop waiting (the error word is set; results are void)
+
+  if (warp < CONV_WARPS) {
+    // ================= convert warps =================
+    // Two groups of eight take turns, group g the steps of parity g; within a group, warp (half h, lane quarter q4) converts
+    // inputs [128 h, +128) of the step's 256 for its 32 rows. The waits and arrivals of a step cost a warp as many instructions as
+    // 64 inputs of conversion do, so a thread takes 128 of every other step and not 64 of each (it measured 243 instructions
+    // per 64 inputs before, 104 of them conversion).
+    const int q4 = warp & 3, half = (warp >> 2) & 1, group = warp >> 3;
+    const int r = q4 * 32 + lane;  // tile row = tensor-memory lane
+    const NibbleConst nc;
+    const uint32_t acol = tmem + ((uint32_t)(q4 * 32) << 16) + A_COL0 + half * 64;
+    const unsigned char* xrow = raw + swz_off(r, 0);  // piece p of the row stands at xrow + piece(p)
+    auto piece = [&](int p) { return (((r & 7) ^ p) - (r & 7)) << 4; };
+    Ring<NRAW> rr;     // raw stages
+    Ring<NST> ra;      // stages; every one starts free
+    ra.par = 1;
+    ra.next(group);
+    auto a_wait = [&]() {  // the MMAs that read this stage's tiles must have completed
+      wait_at(ctl.done, ra, DRB_ERR_TMEM, dead);
+      tc_fence_after();
+    };
+    auto a_done = [&]() {
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl.full[ra.i]);
+      ra.next(2);
+    };
+    Ring<(NSM ? NSM : 1)> rs;  // int4 items' scales
+    for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
+      const Item it = decode(item);
+      if (FMT == 0 && !it.shared) {
+        // (scale, min) of this row's groups 4 step + 2 half, + 1
+        wait_at(ctl.smfull, rs, DRB_ERR_FULL_WAIT, dead);
+        const unsigned char* smp = smbuf + rs.i * SMB + (GEMM == 0 ? swz_off(r, 0) : r * 32) + 8 * half;
+        rs.next();
+        rr.next(group);
+#pragma unroll 1
+        for (int step = group; step < NSTEP; step += 2) {
+          wait_at(ctl.rawfull, rr, DRB_ERR_FULL_WAIT, dead);
+          const unsigned char* xp = xrow + rr.i * RAW_BYTES;
+          const unsigned char* gp = smp + (GEMM == 0 ? piece(step) : 16 * step);
+          a_wait();
+#pragma unroll 1
+          for (int g = 0; g < 2; ++g) {
+            const uint4 x0 = *reinterpret_cast<const uint4*>(xp + piece(4 * half + 2 * g)), x1 = *reinterpret_cast<const uint4*>(xp + piece(4 * half + 2 * g + 1));
+            const __half2 sm = *reinterpret_cast<const __half2*>(gp + 4 * g);
+            const __half2 s2 = __half2half2(__low2half(sm)), m2 = __half2half2(__high2half(sm));
+            const uint32_t w[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+            uint32_t o[32];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              if (PERM || GEMM == 1) dequant8_perm(w[j], s2, m2, nc, o + 4 * j);
+              else dequant8_nat(w[j], s2, m2, nc, o + 4 * j);
+            }
+            tmem_st32(acol + ra.i * A_COLS + g * 32, o);
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl.rawempty[rr.i]);
+          rr.next(step + 2 < NSTEP ? 2 : 2 - group);
+          a_done();
+        }
+      } else {  // 8-bit weights: a step is two raw stages, one per half
+        const int wrow = weight_row(it.mt, r);
+        const __half* ssrow = a.shs + (size_t)wrow * (K / 128) + half;
+        __half s_next = __half();  // shared expert: one scale per 128 inputs, fetched a step ahead
+        if (FMT == 0) s_next = __ldg(ssrow + 2 * group);
+        rr.next(2 * group);
+#pragma unroll 1
+        for (int step = group; step < NSTEP; step += 2) {
+          const __half2 s2 = __half2half2(s_next);
+          if (FMT == 0 && step + 2 < NSTEP) s_next = __ldg(ssrow + 2 * (step + 2));
+          // both stages are waited for although this warp reads one: an arrival must not run a ring's length ahead
+          const int sa = rr.i;
+          wait_at(ctl.rawfull, rr, DRB_ERR_FULL_WAIT, dead);
+          rr.next();
+          const int sb = rr.i;
+          wait_at(ctl.rawfull, rr, DRB_ERR_FULL_WAIT, dead);
+          rr.next(step + 2 < NSTEP ? 3 : 3 - 2 * group);
+          const unsigned char* xp = xrow + (half ? sb : sa) * RAW_BYTES;
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            uint32_t o[32];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint4 x = *reinterpret_cast<const uint4*>(xp + piece(4 * g + j));
+              const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+              if (FMT == 1) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) dequant4_e4m3(w[q], o + 8 * j + 2 * q);
+              } else {
+#pragma unroll
+                for (int q = 0; q < 2; ++q) dequant8_i8<FMT == 0 && (PREP || GEMM == 1)>(w[2 * q], w[2 * q + 1], s2, o + 8 * j + 4 * q);
+              }
+            }
+            if (g == 0) a_wait();
+            tmem_st32(acol + ra.i * A_COLS + g * 32, o);
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl.rawempty[sa]), mbar_arrive(&ctl.rawempty[sb]);
+          a_done();
+        }
+      }
+    }
+  } else if (warp == MMA_WARP) {
+    // ================= MMA warp =================
+    Ring<NTAB> rt;
+    Ring<NACC> rc;
+    Ring<NST> ra;
+    rc.par = 1;  // the accumulators start free
+    unsigned steps = 0;
+    const uint64_t bdesc0 = smem_desc(bring, 4096);  // eight-row groups lie 4 KB apart: four 1 KB columns each
+    for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
+      wait_at(ctl.tabfull, rt, DRB_ERR_FULL_WAIT, dead);
+      const uint32_t idesc = instr_desc_f16(tabs[rt.i].cols), d = tmem + (uint32_t)(rc.i * NT);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl.tabempty[rt.i]);
+      rt.next();
+      if (FMT == 0) wait_at(ctl.accfree, rc, DRB_ERR_TMEM, dead);
+#pragma unroll 1
+      for (int step = 0; step < NSTEP; ++step) {
+        wait_at(ctl.full, ra, DRB_ERR_TMEM, dead);
+        if (FMT == 0) {
+          tc_fence_after();
+          if (elect_one()) {
+            const uint32_t ac = tmem + A_COL0 + ra.i * A_COLS;
+            const uint64_t bd = bdesc0 + (uint32_t)(ra.i * (B_BYTES >> 4));
+            mma_f16_ts(d, ac, bd, idesc, step > 0);
+#pragma unroll
+            for (int k16 = 1; k16 < STEP_K / 16; ++k16) mma_f16_ts(d, ac + 8 * k16, bd + (uint64_t)((k16 >> 2) * 64 + (k16 & 3) * 2), idesc, true);
+            mma_commit(&ctl.done[ra.i]);
+            if (step == NSTEP - 1) mma_commit(&ctl.accfull[rc.i]);
+          }
+        } else {
+#pragma unroll
+          for (int kb = 0; kb < 2; ++kb) {
+            wait_at(ctl.accfree, rc, DRB_ERR_TMEM, dead);
+            tc_fence_after();
+            if (elect_one()) {
+              const uint32_t ac = tmem + A_COL0 + ra.i * A_COLS, dk = tmem + (uint32_t)(rc.i * NT);
+              const uint64_t bd = bdesc0 + (uint32_t)(ra.i * (B_BYTES >> 4));
+#pragma unroll
+              for (int k16 = 8 * kb; k16 < 8 * kb + 8; ++k16)
+                mma_f16_ts(dk, ac + 8 * k16, bd + (uint64_t)((k16 >> 2) * 64 + (k16 & 3) * 2), idesc, k16 > 8 * kb);
+              mma_commit(&ctl.accfull[rc.i]);
+              if (kb == 1) mma_commit(&ctl.done[ra.i]);
+            }
+            __syncwarp();
+            rc.next();
+          }
+        }
+        __syncwarp();
+        ra.next();
+      }
+      if (FMT == 0) rc.next();
+      steps += NSTEP;
+    }
+    // The block must not end before the completion arrivals it is owed have landed: the last one of every stage.
+    for (unsigned k = 0; k < NST && k < steps; ++k) {
+      const unsigned n = steps - 1 - k;
+      if (!dead) dead = !mbar_wait(&ctl.done[n % NST], (n / NST) & 1, DRB_ERR_TMEM);
+    }
+  } else if (warp == LOAD_WARP) {
+    // ================= loader =================
+    // The (scale, min) pairs of an int4 item go to one of NSM slots ahead of its first raw stage. By then the raw stage NRAW
+    // requests back has been read, so every item more than NSM - 1 items back is finished with its slot.
+    static_assert(NSM == 0 || (NSM - 1) * NSTEP >= NRAW, "scale slots");
+    Ring<NRAW> rr;
+    Ring<(NSM ? NSM : 1)> rs;
+    rr.par = 1;  // every raw stage starts free
+    for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
+      const Item it = decode(item);
+      const bool eight = FMT == 1 || it.shared;
+      const int nraw = NSTEP * (eight ? 2 : 1), unit0 = it.mt * (TILE_M / 2), e = it.shared ? 0 : it.e, row0 = e * R + it.mt * TILE_M;
+      const CUtensorMap* map = it.shared ? &maps.sh : &maps.q;
+#pragma unroll 1
+      for (int n = 0; n < nraw; ++n) {
+        wait_at(ctl.rawempty, rr, DRB_ERR_EMPTY_WAIT, dead);
+        __syncwarp();
+        if (elect_one()) {
+          uint64_t* bar = &ctl.rawfull[rr.i];
+          if (FMT == 0 && n == 0 && !it.shared) {
+            unsigned char* sp = smbuf + rs.i * SMB;
+            mbar_expect_tx(&ctl.smfull[rs.i], SMB);
+            if (GEMM == 0) tma_load_4d(sp, &maps.sm, 0, 0, unit0, e, &ctl.smfull[rs.i]);
+            else bulk_g2s(sp, static_cast<const unsigned char*>(a.scales) + (size_t)row0 * (K / 64) * 4, SMB, &ctl.smfull[rs.i]);
+          }
+          mbar_expect_tx(bar, RAW_BYTES);
+          if (GEMM == 0) tma_load_4d(raw + (size_t)rr.i * RAW_BYTES, map, n * ROW_BYTES, 0, unit0, e, bar);
+          else tma_load_2d(raw + (size_t)rr.i * RAW_BYTES, map, n * ROW_BYTES, row0, bar);
+        }
+        __syncwarp();
+        rr.next();
+      }
+      if (FMT == 0 && !it.shared) rs.next();
+    }
+  } else if (warp == TOKEN_WARP) {
+    // ================= token warp =================
+    if (GEMM == 1) pdl_wait();  // the gate/up kernel's activations
+    Ring<NTAB> rt;
+    Ring<NST> ra;
+    ra.par = 1;  // every stage starts free
+    for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
+      wait_at(ctl.tabfull, rt, DRB_ERR_FULL_WAIT, dead);
+      const Tab& tab = tabs[rt.i];
+      const int srow = tab.srow, full = tab.full, start = tab.start, quads = tab.quads;
+      const unsigned bytes = (full + (start >= 0)) * 4096 + quads * 2048;
+      const CUtensorMap *m8 = tab.shared ? &maps.shtok8 : &maps.tok8, *m1 = tab.shared ? &maps.shtok1 : &maps.tok1;
+#pragma unroll 1
+      for (int step = 0; step < NSTEP; ++step) {
+        wait_at(ctl.done, ra, DRB_ERR_EMPTY_WAIT, dead);
+        __syncwarp();
+        if (elect_one()) {
+          unsigned char* bp = bring + ra.i * B_BYTES;
+          uint64_t* bar = &ctl.full[ra.i];
+          mbar_expect_tx(bar, bytes);
+          if (start >= 0) tma_load_3d(bp + full * 4096, m8, 0, start, step * 4, bar);
+#pragma unroll 1
+          for (int g = 0; g < full; ++g) tma_load_3d(bp + g * 4096, m8, 0, srow + 8 * g, step * 4, bar);
+#pragma unroll 1
+          for (int q = 0; q < quads; ++q) {
+            const int4 row = *reinterpret_cast<const int4*>(&tab.rows[4 * q]);
+            unsigned char* qp = bp + (full + (q >> 1)) * 4096 + (q & 1) * 512;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) tma_gather4(qp + c * 1024, m1, step * STEP_K + c * 64, row.x, row.y, row.z, row.w, bar);
+          }
+        }
+        __syncwarp();
+        ra.next();
+      }
+      if (lane == 0) mbar_arrive(&ctl.tabempty[rt.i]);
+      rt.next();
+    }
+  } else if (warp == TABLE_WARP) {
+    // ================= table warp =================
+    Ring<NTAB> rt;
+    rt.par = 1;
+    for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
+      const Item it = decode(item);
+      if (!dead) dead = !mbar_wait(&ctl.tabempty[rt.i], rt.par, DRB_ERR_EMPTY_WAIT);
+      Tab& tab = tabs[rt.i];
+      const int cnt = it.shared ? a.rows_sh : __ldg(a.counts + it.e);
+      const int nt = min(NT, cnt - it.n0);
+      const int srow = (it.shared ? 0 : __ldg(a.offsets + it.e)) + it.n0, end = srow + nt, rest = nt & 7;
+      // Contiguous rows go by boxes of eight. What is left over takes one more box, of the last eight rows: no row beyond
+      // the item's end is touched, and the columns of rows that it repeats (or that are not the item's) have no result
+      // row. Among the array's first eight rows, and for scattered rows, gather4 fetches the rows by number.
+      const bool contig = GEMM == 1 || PREP || it.shared;
+      const int full = contig ? nt >> 3 : 0;
+      const int start = contig && rest && end >= 8 ? end - 8 : -1;
+      const int quads = start < 0 ? (nt - 8 * full + 3) >> 2 : 0;
+      const int cols = ((start >= 0 ? 8 * full + 8 : nt) + 15) & ~15;
+      const unsigned char* fac = it.shared ? a.sh_fac : a.fac;
+      for (int t = lane; t < cols; t += 32) {
+        const int slot = start >= 0 && t >= 8 * full ? start + (t - 8 * full) : srow + t;
+        const bool own = slot >= srow + (t >= 8 * full ? 8 * full : 0) && slot < end;
+        if (GEMM == 0) tab.fac[t] = own && fac ? __ldcg(reinterpret_cast<const float*>(fac + (size_t)slot * TOKEN_STRIDE + H * 2)) : 1.f;
+        tab.dst[t] = !own ? -1 : (GEMM == 1 && !it.shared && a.dst_row_of) ? __ldg(a.dst_row_of + slot) : slot;
+      }
+      for (int t = lane; t < 4 * quads; t += 32) {
+        const int slot = srow + min(8 * full + t, nt - 1);
+        tab.rows[t] = (GEMM == 0 && !PREP && !it.shared && a.row_of) ? __ldg(a.row_of + slot) : slot;
+      }
+      if (lane == 0) tab.cols = cols, tab.mt = it.mt, tab.shared = it.shared, tab.full = full, tab.srow = srow, tab.start = start, tab.quads = quads;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl.tabfull[rt.i]);
+      rt.next();
+    }
+  } else {
+    // ================= epilogue warps =================
+    if (GEMM == 1) pdl_wait();  // y may still be read as the gate/up kernel's token rows
+    const int q4 = warp & 3;
+    const int r = q4 * 32 + lane;  // tile row
+    Ring<NTAB> rt;
+    Ring<NACC> rc;
+    for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
+      wait_at(ctl.tabfull, rt, DRB_ERR_FULL_WAIT, dead);
+      const Tab& tab = tabs[rt.i];
+      const int cols = tab.cols, mt = tab.mt;
+      const bool sh = tab.shared != 0;
+      float sum[FMT == 1 ? NT : 1];  // FP8: the columns' sums over the accumulators
+      if (FMT == 1) {
+        // Lane l holds a scale: gate/up: input block l % 16 of the gate rows' (l < 16) or the up rows' block row; down: l % 4.
+        const Item it = decode(item);
+        const float* se = static_cast<const float*>(a.scales) + (size_t)it.e * (R / 128) * (K / 128);
+        const float sv = __ldg(se + (weight_row(mt, lane >> 4) >> 7) * (K / 128) + lane % (K / 128));
+#pragma unroll
+        for (int c = 0; c < NT; ++c) sum[c] = 0.f;
+#pragma unroll 1
+        for (int kb = 0; kb < K / 128; ++kb) {
+          const float s = __shfl_sync(0xffffffffu, sv, kb + (GEMM == 0 && (r & 1) ? 16 : 0));
+          wait_at(ctl.accfull, rc, DRB_ERR_TMEM, dead);
+          tc_fence_after();
+#pragma unroll
+          for (int c0 = 0; c0 < NT; c0 += 16)
+            if (c0 < cols) {
+              uint32_t v[16];
+              tmem_ld16(tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(rc.i * NT + c0), v);
+#pragma unroll
+              for (int i = 0; i < 16; ++i) sum[c0 + i] = fmaf(s, __uint_as_float(v[i]), sum[c0 + i]);
+            }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl.accfree[rc.i]);
+          rc.next();
+        }
+      } else {
+        wait_at(ctl.accfull, rc, DRB_ERR_TMEM, dead);
+        tc_fence_after();
+      }
+      const uint32_t acc = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(rc.i * NT);
+      // gate/up: unit j of act, in the order in which the down kernel's token rows want it. down: the row's column of y.
+      const int j = mt * (TILE_M / 2) + (r >> 1);
+      __half* const act = static_cast<__half*>(sh ? a.sh_dst : a.dst) + (FMT == 0 ? perm_pos(j) : j);
+      float* const y = static_cast<float*>(sh ? a.sh_dst : a.dst) + mt * TILE_M + r;
+      const bool odd = lane & 1;
+      auto columns = [&](int c0, const uint32_t(&v)[16]) {  // the results of sixteen columns
+#pragma unroll
+        for (int i4 = 0; i4 < 16; i4 += 4) {
+          const int4 d4 = *reinterpret_cast<const int4*>(&tab.dst[c0 + i4]);
+          const int dst[4] = {d4.x, d4.y, d4.z, d4.w};
+          if (GEMM == 0) {
+            // even lanes hold gate rows, odd lanes their up rows. Per pair of tokens the lanes swap what the other needs: the
+            // even lane finishes the first token, the odd lane the second.
+            const float4 f4 = *reinterpret_cast<const float4*>(&tab.fac[c0 + i4]);
+            const float fac[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+            for (int i = 0; i < 4; i += 2) {
+              const float v0 = __uint_as_float(v[i4 + i]), v1 = __uint_as_float(v[i4 + i + 1]);
+              const float got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
+              const int dt = odd ? dst[i + 1] : dst[i];
+              const float f = odd ? fac[i + 1] : fac[i];
+              if (dt >= 0) act[(size_t)dt * I] = f2h_sat(silu_f((odd ? got : v0) * f) * ((odd ? v1 : got) * f));
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float val = __uint_as_float(v[i4 + i]);
+              if (dst[i] < 0) continue;
+              if (a.peer_y && !sh) {
+                const int s = dst[i] / a.peer_cap;
+                a.peer_y[s][((size_t)a.peer_rank * a.peer_cap + (dst[i] - s * a.peer_cap)) * H + mt * TILE_M + r] = val;
+              } else {
+                y[(size_t)dst[i] * H] = val;
+              }
+            }
+          }
+        }
+      };
+      if (FMT == 1) {
+#pragma unroll
+        for (int c0 = 0; c0 < NT; c0 += 16)
+          if (c0 < cols) {
+            uint32_t v[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(sum[FMT == 1 ? c0 + i : 0]);
+            columns(c0, v);
+          }
+      } else {
+#pragma unroll 1
+        for (int c0 = 0; c0 < cols; c0 += 16) {
+          uint32_t v[16];
+          tmem_ld16(acc + (uint32_t)c0, v);
+          if (c0 + 16 >= cols) {  // everything is in registers: the accumulator is free
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ctl.accfree[rc.i]);
+          }
+          columns(c0, v);
+        }
+        rc.next();
+      }
+      if (GEMM == 1 && a.peer_y && !sh) __threadfence_system();  // before the flag that a later kernel writes to the peers
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl.tabempty[rt.i]);
+      rt.next();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == MMA_WARP) tmem_dealloc(tmem, TMEM_COLS);
+}
+
+// ---- host side ---------------------------------------------------------------------------------------------------
+// Tensor maps with the 128-byte swizzle. cuTensorMapEncodeTiled is a driver entry point: it is looked up through the
+// runtime once, so the library has no link-time dependency on the driver. The map functions return 0 or -3.
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static EncodeTiledFn g_encode = nullptr;
+
+static cudaError_t resolve_encode() {
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult status;
+  cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &status);
+  if (e != cudaSuccess) return e;
+  if (status != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
+  g_encode = reinterpret_cast<EncodeTiledFn>(fn);
+  return cudaSuccess;
+}
+
+static int encode(CUtensorMap* map, CUtensorMapDataType type, int rank, const void* p, const cuuint64_t* dims, const cuuint64_t* strides,
+                  const cuuint32_t* box) {
+  if (!g_encode) return -3;
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  return g_encode(map, type, rank, const_cast<void*>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
+             ? 0
+             : -3;
+}
+
+// Down projection: [rows, row_bytes] row-major, boxes of 128 rows x 128 bytes.
+static int map_rows(CUtensorMap* map, const void* p, uint64_t rows, uint64_t row_bytes) {
+  const cuuint64_t dims[2] = {row_bytes, rows}, strides[1] = {row_bytes};
+  const cuuint32_t box[2] = {ROW_BYTES, TILE_M};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, p, dims, strides, box);
+}
+
+// Gate/up: [experts][2 (gate | up)][units][row_bytes] seen as (row byte, gate|up, unit, expert); a box is 128 bytes of
+// 64 units' gate row and up row, interleaved.
+static int map_gate_up(CUtensorMap* map, const void* p, uint64_t experts, uint64_t units, uint64_t row_bytes) {
+  const cuuint64_t dims[4] = {row_bytes, 2, units, experts}, strides[3] = {units * row_bytes, row_bytes, 2 * units * row_bytes};
+  const cuuint32_t box[4] = {ROW_BYTES, 2, TILE_M / 2, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, p, dims, strides, box);
+}
+
+// fp16 token rows of k inputs at a stride of stride bytes. How many there are is known on the device only; the kernel asks
+// for rows that exist, and the maps' row extent is not a limit.
+static int map_tokens(CUtensorMap* m8, CUtensorMap* m1, const void* p, uint64_t k, uint64_t stride) {
+  const cuuint64_t rows = 1ull << 28;
+  const cuuint64_t dims3[3] = {64, rows, k / 64}, strides3[2] = {stride, 128};
+  const cuuint32_t box3[3] = {64, 8, STEP_K / 64};
+  const cuuint64_t dims2[2] = {k, rows}, strides2[1] = {stride};
+  const cuuint32_t box2[2] = {64, 1};
+  if (encode(m8, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, p, dims3, strides3, box3)) return -3;
+  return encode(m1, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p, dims2, strides2, box2);
+}
+
+// One grouped expert block: gate/up, then down.
+struct Block {
+  int fmt;                                  // 0: int4, 1: block FP8
+  const void *gu_w, *gu_s, *d_w, *d_s;      // routed experts
+  const void *sgu_q, *sgu_s, *sd_q, *sd_s;  // shared expert (rows_sh > 0)
+  const void* x;                            // 16-bit rows [., H]
+  bool x_bf16;
+  const int *row_of, *offsets, *counts, *y_row_of;
+  void *act, *y, *sh_act, *sh_out;
+  int rows_sh, E;
+  float* const* peer_y;
+  int peer_cap, peer_rank;
+};
+
+template <int FMT>
+static int run_block(const Block& b, const DrbDevice& dev, cudaStream_t st) {
+  constexpr int WB = FMT == 0 ? 2 : 1;  // weights per byte
+  // Rows are prepared wherever there is a buffer for them: y and sh_out, which are written last. With the results going to
+  // peers y is not this call's to write: the fp16 rows are gathered as they are.
+  const bool prep = b.peer_y == nullptr;
+  if (!prep && (b.x_bf16 || FMT != 0)) return -1;
+  unsigned char* tok = static_cast<unsigned char*>(b.y);
+  unsigned char* shtok = static_cast<unsigned char*>(b.sh_out);
+  if (prep) {
+    auto kp = b.x_bf16 ? k_prep_rows<true, FMT == 0> : k_prep_rows<false, FMT == 0>;
+    drb_launch(kp, dim3(2 * dev.sms), dim3(256), 0, st, false, static_cast<const uint4*>(b.x), b.row_of, b.offsets, b.counts, b.E, tok, b.rows_sh, shtok);
+  }
+  // Every gate/up launch before the first down launch: y holds the token rows until then.
+  const bool sh_on = b.rows_sh > 0;
+  for (int gemm = 0; gemm < 2; ++gemm) {
+    for (int e0 = 0; e0 == 0 || e0 < b.E; e0 += MAX_E) {
+      const int ne = b.E - e0 < MAX_E ? b.E - e0 : MAX_E;
+      const uint64_t em = ne > 0 ? ne : 1;
+      const bool sh = sh_on && e0 == 0;
+      const size_t row = (gemm == 0 ? H : I) / WB, rows = gemm == 0 ? 2 * I : H, cols = gemm == 0 ? H : I;
+      const size_t s_bytes = FMT == 0 ? rows * (cols / 64) * 4 : (rows / 128) * (cols / 128) * 4;  // scales per expert
+      const unsigned char* w = static_cast<const unsigned char*>(gemm == 0 ? b.gu_w : b.d_w) + rows * row * e0;
+      const unsigned char* sc = static_cast<const unsigned char*>(gemm == 0 ? b.gu_s : b.d_s) + s_bytes * e0;
+      Maps m = {};
+      Args a = {};
+      if (gemm == 0) {
+        if (map_gate_up(&m.q, w, em, I, row) || (FMT == 0 && map_gate_up(&m.sm, sc, em, I, (H / 64) * 4)) || (sh && map_gate_up(&m.sh, b.sgu_q, 1, I, H))) return -3;
+        if (map_tokens(&m.tok8, &m.tok1, prep ? tok : b.x, H, prep ? TOKEN_STRIDE : H * 2)) return -3;
+        if (sh && map_tokens(&m.shtok8, &m.shtok1, prep ? shtok : b.x, H, prep ? TOKEN_STRIDE : H * 2)) return -3;
+        a.dst = b.act, a.sh_dst = b.sh_act, a.row_of = b.row_of;
+        if (prep && b.x_bf16) a.fac = tok, a.sh_fac = shtok;
+      } else {
+        if (map_rows(&m.q, w, em * H, row) || (sh && map_rows(&m.sh, b.sd_q, H, I))) return -3;
+        if (map_tokens(&m.tok8, &m.tok1, b.act, I, I * 2) || (sh && map_tokens(&m.shtok8, &m.shtok1, b.sh_act, I, I * 2))) return -3;
+        a.dst = b.y, a.sh_dst = b.sh_out, a.dst_row_of = b.y_row_of;
+        a.peer_y = b.peer_y, a.peer_cap = b.peer_cap, a.peer_rank = b.peer_rank;
+      }
+      a.scales = sc, a.shs = static_cast<const __half*>(gemm == 0 ? b.sgu_s : b.sd_s);
+      a.offsets = b.offsets + e0, a.counts = b.counts + e0, a.E = ne > 0 ? ne : 0, a.rows_sh = sh ? b.rows_sh : 0;
+      if (gemm == 0)
+        drb_launch(prep ? k_grouped<0, FMT, true> : k_grouped<0, FMT, FMT != 0>, dim3(dev.sms), dim3(THREADS), Smem<0, FMT>::BYTES, st, false, m, a);
+      else  // only the first one follows the gate/up kernel
+        drb_launch(k_grouped<1, FMT, true>, dim3(dev.sms), dim3(THREADS), Smem<1, FMT>::BYTES, st, dev.pdl && b.E <= MAX_E, m, a);
+    }
+  }
+  return 0;
+}
+
+template <typename Kn>
+static cudaError_t configure_one(Kn kernel, size_t smem) {
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return e != cudaSuccess ? e : drb_carveout(kernel);
+}
+
+static cudaError_t configure_all() {
+  cudaError_t e;
+  if ((e = resolve_encode()) != cudaSuccess) return e;
+  if ((e = drb_carveout(k_prep_rows<false, false>)) != cudaSuccess) return e;
+  if ((e = drb_carveout(k_prep_rows<false, true>)) != cudaSuccess) return e;
+  if ((e = drb_carveout(k_prep_rows<true, false>)) != cudaSuccess) return e;
+  if ((e = drb_carveout(k_prep_rows<true, true>)) != cudaSuccess) return e;
+  if ((e = configure_one(k_grouped<0, 0, true>, Smem<0, 0>::BYTES)) != cudaSuccess) return e;
+  if ((e = configure_one(k_grouped<0, 0, false>, Smem<0, 0>::BYTES)) != cudaSuccess) return e;
+  if ((e = configure_one(k_grouped<1, 0, true>, Smem<1, 0>::BYTES)) != cudaSuccess) return e;
+  if ((e = configure_one(k_grouped<0, 1, true>, Smem<0, 1>::BYTES)) != cudaSuccess) return e;
+  return configure_one(k_grouped<1, 1, true>, Smem<1, 1>::BYTES);
+}
+
+}  // namespace pft

@@ -120,16 +120,16 @@ int dr_moe_count(const int* idx, int n, int* counts, dr_stream st); /* drama.cu:
 int dr_moe_permute(const int* idx, int rows, int topk, const int* offsets, int* fill, int* slot_of, const dr_bf16* x,
                    dr_bf16* xp, int h, dr_stream st);
 /* Rows of xp sorted by expert (offsets/counts). act: scratch, 16 bits per (slot, j), contents
- * unspecified. y[slot, :] = down_e(silu(gate_e . x) * (up_e . x)). h == 2048, i == 512.
+ * unspecified. y[slot, :] = down_e(silu(gate_e . x) * (up_e . x)). h == 2048, i == 512. The weights and the token rows are
+ * addressed through TMA tensor maps built from the pointers given: act and y 16-byte aligned, -3 when the driver
+ * refuses a map. Until its rows are written y is scratch: the token rows as the tensor cores want them.
  * drama.cu:799-968; ffi.rs:61-64 */
 int dr_moe_prefill(const uint8_t* gu_q, const dr_half* gu_sm, const uint8_t* d_q, const dr_half* d_sm,
                    const dr_bf16* xp, const int* offsets, const int* counts, dr_bf16* act, float* y, int e, int h, int i,
                    dr_stream st);
-/* dr_moe_prefill over block-FP8 experts (layouts as dr_moe_decode_fp8). The weight bytes reach the tensor cores as
- * E4M3 (tiled TMA, tcgen05 kind::f8f6f4); the block scales ride on the token operand. Until its rows are written, y is
- * scratch (its first floats hold every token row's largest magnitude), as act is. gu_w and d_w 16-byte aligned.
- * Returns -3 if a tensor map cannot be encoded. e > 256, or DRB_FP8_DEQUANT=1 in the environment: the kernels that turn
- * the weights into fp16 first. drama.cu:971-1109; ffi.rs:52-55 */
+/* dr_moe_prefill over block-FP8 experts (layouts as dr_moe_decode_fp8). The weights reach the tensor cores exactly (every
+ * E4M3 number is an fp16 number) and the block scales are applied in fp32 to sums over 128 inputs. gu_w and d_w 16-byte
+ * aligned. drama.cu:971-1109; ffi.rs:52-55 */
 int dr_moe_prefill_fp8(const uint8_t* gu_w, const float* gu_s, const uint8_t* d_w, const float* d_s, const dr_bf16* xp,
                        const int* offsets, const int* counts, dr_bf16* act, float* y, int e, int h, int i, dr_stream st);
 /* drama.cu:780-797; ffi.rs:70-73 */
@@ -205,8 +205,8 @@ int drb_moe_group(const int* idx, int rows, int topk, int e_lo, int e_n, int* co
  * y [slots, h] f32; y_row_of (or NULL): slot -> row of y. rows_sh = 0 skips the shared expert, e = 0 the routed
  * ones. Every pointer except row_of / y_row_of must be a valid device address even for a part that does not run
  * (any buffer will do): NULL returns -1. Intermediates are fp16: SwiGLU values beyond +-65504 are clamped.
- * h == 2048, i == 512, else -1. With x_f16 != 0 and e <= 256 the weights are addressed through TMA tensor maps built
- * from the pointers given (gu_q / d_q: e experts from the pointer on); -3 when the driver refuses a map. */
+ * h == 2048, i == 512, else -1. Tensor maps, alignment and the use of y (and of sh_out for the shared expert's rows) as
+ * scratch as in dr_moe_prefill (gu_q / d_q: e experts from the pointer on). */
 int drb_moe_prefill_block(const uint8_t* gu_q, const dr_half* gu_sm, const uint8_t* d_q, const dr_half* d_sm,
                           const int8_t* sgu_q, const dr_half* sgu_s, const int8_t* sd_q, const dr_half* sd_s,
                           const dr_bf16* xb, const int* row_of, const int* offsets, const int* counts, dr_bf16* act,
@@ -241,7 +241,7 @@ int drb_ep_group(const void* recv, int world, int cap, int row_bytes, int per, i
  * block_bytes % 16 == 0, world <= 64, else -1. */
 int drb_ep_put(const void* send, void* const* peer_recv, int world, int rank, size_t block_bytes, dr_stream st);
 /* drb_ep_pack with the blocks stored straight into the owners' receive buffers (this rank's block in peer o's buffer is
- * block `rank`; no local send buffer, no drb_ep_put), and drb_moe_prefill_block (fp16 rows, e <= 256) with the routed
+ * block `rank`; no local send buffer, no drb_ep_put), and drb_moe_prefill_block (fp16 rows) with the routed
  * results stored straight into the home ranks' result buffers from the down GEMM's epilogue: y_row_of[slot] = s * cap + j
  * names the token's source rank s and its slot j in this rank's receive order (drb_ep_group's pair_of); the row goes to
  * peer_y[s] ([world * cap, h] f32 on rank s) at row rank * cap + j. y must be a valid address and is not written.

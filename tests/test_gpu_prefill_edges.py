@@ -1,0 +1,132 @@
+"""The grouped prefill GEMMs at the edges of their tiles: token boxes of eight, MMA columns of sixteen, items of 64 (int4)
+and 32 (FP8) tokens, the array's first rows, more experts than one launch takes, and the gathered form behind the
+peer-store entry point."""
+
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from drama_rs_b200 import ffi, synth
+from drama_rs_b200.gpu import DevBuf, Stream, launched
+from drama_rs_b200.model import Fp8Experts, MoeLayer
+from oracle import moe_oracle as orc
+from tests.helpers import NULL, device_error_word
+
+pytestmark = pytest.mark.gpu
+
+EDGES = {
+    "boxes": [1, 2, 3, 4, 5, 7, 8, 9, 12, 15, 16, 17, 23, 24, 25, 0],
+    "items": [31, 32, 33, 63, 64, 65, 0, 127, 128, 129, 1, 0, 40, 47, 48, 49],
+    "first rows": [0, 3, 0, 2, 1, 0, 0, 9, 0, 0, 0, 0, 0, 0, 0, 6],
+    "one row": [0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 1, 0, 0, 0, 0],
+}
+
+
+@pytest.fixture(scope="module")
+def st():
+    return Stream()
+
+
+def check_rows(y, host, x, counts, offsets, experts, bar=8e-4):
+    assert device_error_word() == 0
+    for e, c, o in zip(experts, counts, offsets):
+        if c:
+            ref = orc.expert_forward(host, e, x[o : o + c], np.float64)
+            rel = np.linalg.norm(y[o : o + c] - ref, axis=1) / np.linalg.norm(ref, axis=1)
+            assert np.isfinite(rel).all() and rel.max() <= bar, (e, c, float(rel.max()))
+
+
+@pytest.mark.parametrize("fmt", ["int4", "fp8"])
+@pytest.mark.parametrize("edge", EDGES)
+def test_group_sizes(st, fmt, edge):
+    l, shape = ffi.lib(), synth.MoeShape(experts=16)
+    host = synth.make_layer(31, shape) if fmt == "int4" else synth.make_fp8_experts(31, shape)
+    counts = np.array(EDGES[edge], dtype=np.int32)
+    offsets = (np.cumsum(counts) - counts).astype(np.int32)
+    n = int(counts.sum())
+    xf = np.random.Generator(np.random.PCG64(n)).standard_normal((n, 2048), dtype=np.float32)
+    xf[0] *= 1e6  # a bf16 row beyond fp16's range, and one far below it: divided by a power of two on the way
+    xf[n - 1] *= 1e-6 if n > 1 else 1.0
+    xb = synth.f32_to_bf16_bits(xf)
+    dxp, dcnt, doff = DevBuf.from_array(xb, st), DevBuf.from_array(counts, st), DevBuf.from_array(offsets, st)
+    dact, dy = DevBuf(n * 1024), DevBuf(n * 8192)
+    dy.fill(0xFF, st)
+    if fmt == "int4":
+        dev = MoeLayer.upload(host, st)
+        w, call = (*dev.gate_up.expert(0), *dev.down.expert(0)), l.dr_moe_prefill
+    else:
+        f8 = Fp8Experts.upload(host, st)
+        w, call = (f8.gu_w.at(0), f8.gu_s.at(0), f8.d_w.at(0), f8.d_s.at(0)), l.dr_moe_prefill_fp8
+    launched(call(*w, dxp.at(0), doff.at(0), dcnt.at(0), dact.at(0), dy.at(0), 16, 2048, 512, st.raw), "prefill")
+    y = dy.download(np.float32, n * 2048, st).reshape(n, 2048)
+    x = synth.bf16_bits_to_f32(xb).astype(np.float64)
+    keep = np.ones(n, bool)
+    keep[[0, n - 1]] = False  # their activations leave fp16: finite is what is asked of them
+    assert np.isfinite(y).all()
+    for e in range(16):
+        rows = np.arange(offsets[e], offsets[e] + counts[e])[keep[offsets[e] : offsets[e] + counts[e]]]
+        if len(rows):
+            check_rows(y[rows], host, x[rows], [len(rows)], [0], [e])
+    assert device_error_word() == 0
+
+
+def test_more_experts_than_one_launch_takes(st):
+    import torch
+
+    l, e = ffi.lib(), 1027
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q = [torch.randint(0, 256, (e, n, k // 2), dtype=torch.uint8, device="cuda", generator=g) for n, k in ((1024, 2048), (2048, 512))]
+    s = [(torch.randn((e, n, k // 64), device="cuda", generator=g) * 0.01).abs().clamp_min(1e-4).half() for n, k in ((1024, 2048), (2048, 512))]
+    sm = [torch.stack((v, (v.float() * -8.0).half()), dim=-1).contiguous() for v in s]
+    hit = {0: 5, 511: 17, 1023: 3, 1024: 9, 1026: 66}
+    counts = np.zeros(e, dtype=np.int32)
+    counts[list(hit)] = list(hit.values())
+    offsets = (np.cumsum(counts) - counts).astype(np.int32)
+    n = int(counts.sum())
+    xb = synth.f32_to_bf16_bits(np.random.Generator(np.random.PCG64(8)).standard_normal((n, 2048), dtype=np.float32))
+    dxp, dcnt, doff = DevBuf.from_array(xb, st), DevBuf.from_array(counts, st), DevBuf.from_array(offsets, st)
+    dact, dy = DevBuf(n * 1024), DevBuf(n * 8192)
+    torch.cuda.synchronize()
+    p = lambda t: C.c_void_p(t.data_ptr())
+    launched(l.dr_moe_prefill(p(q[0]), p(sm[0]), p(q[1]), p(sm[1]), dxp.at(0), doff.at(0), dcnt.at(0), dact.at(0), dy.at(0), e, 2048, 512, st.raw), "prefill")
+    y = dy.download(np.float32, n * 2048, st).reshape(n, 2048)
+    x = synth.bf16_bits_to_f32(xb).astype(np.float64)
+    names = ("moe.gate_up.q4", "moe.down.q4", "moe.gate_up.sm", "moe.down.sm")
+    for ex in hit:
+        host = {k: t[ex : ex + 1].cpu().numpy() for k, t in zip(names, (*q, *sm))}
+        check_rows(y[offsets[ex] : offsets[ex] + counts[ex]], host, x[offsets[ex] : offsets[ex] + counts[ex]], [counts[ex]], [0], [0])
+
+
+@pytest.mark.parametrize("rows", [1, 5, 40])
+def test_gathered_rows_and_stored_results(st, rows):
+    """drb_moe_prefill_block_peers with one rank: its own buffer is the peer. Same results as drb_moe_prefill_block."""
+    l, shape = ffi.lib(), synth.MoeShape(experts=16)
+    dev = MoeLayer.upload(synth.make_layer(32, shape), st)
+    rng = np.random.Generator(np.random.PCG64(rows))
+    xh = rng.standard_normal((rows, 2048), dtype=np.float32).astype(np.float16)
+    idx = np.stack([rng.permutation(16)[:8] for _ in range(rows)]).astype(np.int32)
+    n = rows * 8
+    i32 = lambda m: DevBuf(m * 4)
+    dx, didx = DevBuf.from_array(xh, st), DevBuf.from_array(idx, st)
+    cnt, off, slot, row = i32(16), i32(16), i32(n), i32(n)
+    launched(l.drb_moe_group(didx.at(0), rows, 8, 0, 16, cnt.at(0), off.at(0), slot.at(0), row.at(0), st.raw), "group")
+    act, sh_act = DevBuf(n * 1024), DevBuf(rows * 1024)
+    out = {}
+    for name in ("block", "peers"):
+        y, sh, dst = DevBuf(n * 8192), DevBuf(rows * 8192), DevBuf.from_array(np.arange(n, dtype=np.int32), st)
+        w = (*dev.gate_up.expert(0), *dev.down.expert(0), *dev.shared_gate_up.rows(0), *dev.shared_down.rows(0))
+        bufs = (dx.at(0), row.at(0), off.at(0), cnt.at(0), act.at(0), y.at(0), sh_act.at(0), sh.at(0), rows, 16, 2048, 512)
+        if name == "block":
+            launched(l.drb_moe_prefill_block(*w, *bufs, 1, NULL, st.raw), name)
+            res = y
+        else:
+            res = DevBuf(n * 8192)
+            table = DevBuf.from_array(np.array([res.ptr], dtype=np.uint64), st)
+            launched(l.drb_moe_prefill_block_peers(*w, *bufs, dst.at(0), table.at(0), n, 0, st.raw), name)
+        out[name] = (res.download(np.float32, n * 2048, st), sh.download(np.float32, rows * 2048, st))
+    assert device_error_word() == 0
+    for a, b in zip(out["block"], out["peers"]):
+        assert np.linalg.norm(a - b) <= 2e-4 * np.linalg.norm(a)
