@@ -9,7 +9,7 @@
 // the last bit, its pick is not defined by its source.)
 //
 //   drb_quant_q4: tools/convert.py:44-89 (`quant_q4_groups`: 24-step clipping search, least-squares refit) and
-//                 92-101 (`quant_q4`: packing, low nibble = even k). One warp per group of 64 inputs.
+//                 92-101 (`quant_q4`: packing, low nibble = even k). Eight lanes per group of 64 inputs.
 //   drb_quant_q8: tools/convert.py:33-41 (`quant_q8`). One warp per group of 128 inputs.
 #pragma once
 
@@ -25,68 +25,178 @@ __constant__ float c_shrink[STEPS] = {1.0f,        0.97916669f, 0.95833331f, 0.9
 
 DRB_DEV float half_round(float v) { return __half2float(__float2half_rn(v)); }
 
-// Sum of the group's 64 values in the converter's order; lane l passes inputs 2l (a) and 2l + 1 (b), every lane
-// gets the total. Running sum j collects inputs j, 8 + j, 16 + j, ...: those of lanes j / 2, j / 2 + 4, ...
-DRB_DEV float sum64(float a, float b) {
-  const int p = threadIdx.x & 3;
-  float r0 = __shfl_sync(0xffffffffu, a, p), r1 = __shfl_sync(0xffffffffu, b, p);  // running sums 2p and 2p + 1
-#pragma unroll
-  for (int i = 1; i < 8; ++i) {
-    r0 = __fadd_rn(r0, __shfl_sync(0xffffffffu, a, p + 4 * i));
-    r1 = __fadd_rn(r1, __shfl_sync(0xffffffffu, b, p + 4 * i));
-  }
-  const float pr = __fadd_rn(r0, r1);                                       // r[2p] + r[2p + 1]
-  const float q = __fadd_rn(__shfl_sync(0xffffffffu, pr, 0), __shfl_sync(0xffffffffu, pr, 1));  // (r0 + r1) + (r2 + r3)
-  const float h = __fadd_rn(__shfl_sync(0xffffffffu, pr, 2), __shfl_sync(0xffffffffu, pr, 3));  // (r4 + r5) + (r6 + r7)
-  return __fadd_rn(q, h);
+// A team of eight lanes owns a group: lane j holds inputs j, 8 + j, ..., 56 + j, which are the terms of the converter's
+// running sum j in its order, so a 64-term sum is seven additions in the lane and three exchanges. (With two consecutive
+// inputs per lane, one warp per group, the same order took sixteen exchanges and fourteen additions for two inputs: 6.3 ms
+// for 134 M weights; now 1.48 ms.)
+struct Group {
+  unsigned long long v2[4];  // inputs 8 i + j as packed pairs (i = 0, 1), (2, 3), (4, 5), (6, 7)
+  unsigned long long n2[4];  // the same, negated
+};
+
+DRB_DEV unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+DRB_DEV unsigned long long dup2(float v) { return pack2(v, v); }
+DRB_DEV float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 
-// Lane l holds inputs 2l and 2l + 1 of the group.
-__global__ void __launch_bounds__(256) k_quant_q4(const float* __restrict__ w, size_t groups, uint8_t* __restrict__ q,
-                                                  __half2* __restrict__ sm) {
-  const size_t g = (size_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (g >= groups) return;
-  const float2 v = reinterpret_cast<const float2*>(w + g * 64)[lane];
-  float gmin = fminf(v.x, v.y), gmax = fmaxf(v.x, v.y);
+// The converter's sum of one packed value per input; every lane of the team gets the total.
+DRB_DEV float sum64(const unsigned long long (&t)[4]) {
+  float a, b, s;
+  unpack2(t[0], a, b);
+  s = __fadd_rn(a, b);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int i = 1; i < 4; ++i) {
+    unpack2(t[i], a, b);
+    s = __fadd_rn(__fadd_rn(s, a), b);
+  }
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));  // r0 + r1, (r0 + r1) + (r2 + r3), ...
+  return s;
+}
+
+// The eight codes of a lane: rint((v - lo) / scale) clamped to 0..15, as packed floats. The quotient is taken as a product with
+// the reciprocal, within 2^-22 of it, clamped before it is rounded. Where it lands within 1e-5 of an inner rounding boundary
+// the candidate n is settled exactly: with d = v - lo (a float, at least scale / 2 here) the remainder d - n scale is exact in
+// one fused operation, and it is compared with scale / 2; d's spacing is too coarse for the rounded quotient to reach a
+// boundary that the exact one misses. Weights on a bf16 grid make such boundaries common (one value in two thousand), nearly
+// all of them exact ties, which go to the even code.
+DRB_DEV void codes8(const Group& g, float lo, float scale, float rcp, unsigned long long (&q)[4]) {
+  const unsigned long long nlo = dup2(-lo), r2 = dup2(rcp), magic = dup2(12582912.f), nmagic = dup2(-12582912.f), neg1 = dup2(-1.f);
+  float worst = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float p0, p1, f0, f1;
+    unpack2(mul2(add2(g.v2[i], nlo), r2), p0, p1);
+    const unsigned long long p = pack2(fminf(fmaxf(p0, 0.f), 15.f), fminf(fmaxf(p1, 0.f), 15.f));
+    q[i] = add2(add2(p, magic), nmagic);  // the nearest integer
+    unpack2(fma2(q[i], neg1, p), f0, f1);
+    worst = max3(worst, fabsf(f0), fabsf(f1));
+  }
+  if (worst >= 0.49999f) {
+    const float half = 0.5f * scale;
+    auto settle = [&](float v, float n) {
+      const float e = __fmaf_rn(-n, scale, __fadd_rn(v, -lo));
+      const bool odd = ((int)n & 1) != 0;
+      const bool move = fabsf(e) > half || (fabsf(e) == half && odd);
+      return fminf(fmaxf(move ? (e > 0.f ? n + 1.f : n - 1.f) : n, 0.f), 15.f);
+    };
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float v0, v1, n0, n1;
+      unpack2(g.v2[i], v0, v1);
+      unpack2(q[i], n0, n1);
+      q[i] = pack2(settle(v0, n0), settle(v1, n1));
+    }
+  }
+}
+
+// sum of (q * scale + min - v)^2, every operation rounded
+DRB_DEV float error8(const Group& g, const unsigned long long (&q)[4], float scale, float lo) {
+  const unsigned long long s2 = dup2(scale), lo2 = dup2(lo);
+  unsigned long long t[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const unsigned long long d = add2(add2(mul2(q[i], s2), lo2), g.n2[i]);
+    t[i] = mul2(d, d);
+  }
+  return sum64(t);
+}
+
+constexpr int Q4_THREADS = 256, Q4_GROUPS = Q4_THREADS / 8;
+// What bounds it: fp32 issue (24 candidates x 9 fp32 operations and 3 comparisons per weight; the packed forms halve the issue
+// slots), not memory (4.6 bytes per weight). A candidate's scale, min and reciprocal are the same for the whole group:
+// each lane of the team prepares three of the 24 and hands them round.
+__global__ void __launch_bounds__(Q4_THREADS) k_quant_q4(const float* __restrict__ w, size_t groups, uint8_t* __restrict__ q,
+                                                         __half2* __restrict__ sm) {
+  const size_t gi = (size_t)blockIdx.x * Q4_GROUPS + (threadIdx.x >> 3);
+  const int j = threadIdx.x & 7;
+  const size_t gr = gi < groups ? gi : groups - 1;  // teams beyond the end redo the last group and write nothing
+  Group g;
+  float gmin = INFINITY, gmax = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float a = __ldg(w + gr * 64 + 16 * i + j), b = __ldg(w + gr * 64 + 16 * i + 8 + j);
+    gmin = fminf(gmin, fminf(a, b)), gmax = fmaxf(gmax, fmaxf(a, b));
+    g.v2[i] = pack2(a, b), g.n2[i] = pack2(-a, -b);
+  }
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
     gmin = fminf(gmin, __shfl_xor_sync(0xffffffffu, gmin, o));
     gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
   }
   const float center = __fmul_rn(__fadd_rn(gmin, gmax), 0.5f);
-  float best_err = 0.f, best_scale = 0.f, best_lo = 0.f, bq0 = 0.f, bq1 = 0.f;
-  for (int i = 0; i < STEPS; ++i) {
-    const float shrink = c_shrink[i];
+  float c_scale[STEPS / 8], c_lo[STEPS / 8], c_rcp[STEPS / 8];  // candidates j, 8 + j, 16 + j
+#pragma unroll
+  for (int t = 0; t < STEPS / 8; ++t) {
+    const float shrink = c_shrink[8 * t + j];
     const float lo_c = __fadd_rn(center, __fmul_rn(__fsub_rn(gmin, center), shrink));
     const float hi_c = __fadd_rn(center, __fmul_rn(__fsub_rn(gmax, center), shrink));
-    const float scale = fmaxf(__fdiv_rn(__fsub_rn(hi_c, lo_c), 15.0f), 1e-10f);
-    const float scale_h = fmaxf(half_round(scale), 1e-10f);
-    const float lo_h = half_round(lo_c);
-    const float q0 = fminf(fmaxf(rintf(__fdiv_rn(__fsub_rn(v.x, lo_h), scale_h)), 0.f), 15.f);
-    const float q1 = fminf(fmaxf(rintf(__fdiv_rn(__fsub_rn(v.y, lo_h), scale_h)), 0.f), 15.f);
-    const float d0 = __fsub_rn(__fadd_rn(__fmul_rn(q0, scale_h), lo_h), v.x);
-    const float d1 = __fsub_rn(__fadd_rn(__fmul_rn(q1, scale_h), lo_h), v.y);
-    const float err = sum64(__fmul_rn(d0, d0), __fmul_rn(d1, d1));
-    if (i == 0 || err < best_err) best_err = err, best_scale = scale_h, best_lo = lo_h, bq0 = q0, bq1 = q1;
+    c_scale[t] = fmaxf(half_round(fmaxf(__fdiv_rn(__fsub_rn(hi_c, lo_c), 15.0f), 1e-10f)), 1e-10f);
+    c_lo[t] = half_round(lo_c);
+    c_rcp[t] = __frcp_rn(c_scale[t]);
   }
+  float best_err = 0.f, best_scale = 0.f, best_lo = 0.f, best_rcp = 0.f;
+  unsigned long long bq[4];
+#pragma unroll
+  for (int t = 0; t < STEPS / 8; ++t)
+#pragma unroll 2
+    for (int i = 0; i < 8; ++i) {
+      const float scale = __shfl_sync(0xffffffffu, c_scale[t], i, 8), lo = __shfl_sync(0xffffffffu, c_lo[t], i, 8);
+      const float rcp = __shfl_sync(0xffffffffu, c_rcp[t], i, 8);
+      codes8(g, lo, scale, rcp, bq);
+      const float err = error8(g, bq, scale, lo);
+      if ((t == 0 && i == 0) || err < best_err) best_err = err, best_scale = scale, best_lo = lo, best_rcp = rcp;
+    }
+  codes8(g, best_lo, best_scale, best_rcp, bq);
   // One least-squares refinement of (scale, min) given the codes.
   const float n = 64.f;
-  const float sq = sum64(bq0, bq1);
-  const float sqq = sum64(__fmul_rn(bq0, bq0), __fmul_rn(bq1, bq1));
-  const float sw = sum64(v.x, v.y);
-  const float sqw = sum64(__fmul_rn(bq0, v.x), __fmul_rn(bq1, v.y));
+  unsigned long long t[4];
+  const float sq = sum64(bq);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) t[i] = mul2(bq[i], bq[i]);
+  const float sqq = sum64(t);
+  const float sw = sum64(g.v2);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) t[i] = mul2(bq[i], g.v2[i]);
+  const float sqw = sum64(t);
   const float det = __fsub_rn(__fmul_rn(n, sqq), __fmul_rn(sq, sq));
   const bool ok = fabsf(det) > 1e-6f;
   const float ls_scale = ok ? __fdiv_rn(__fsub_rn(__fmul_rn(n, sqw), __fmul_rn(sq, sw)), det) : best_scale;
   const float ls_min = ok ? __fdiv_rn(__fsub_rn(sw, __fmul_rn(ls_scale, sq)), n) : best_lo;
   const float ls_scale_h = half_round(ls_scale), ls_min_h = half_round(ls_min);
-  const float e0 = __fsub_rn(__fadd_rn(__fmul_rn(bq0, ls_scale_h), ls_min_h), v.x);
-  const float e1 = __fsub_rn(__fadd_rn(__fmul_rn(bq1, ls_scale_h), ls_min_h), v.y);
-  const float ls_err = sum64(__fmul_rn(e0, e0), __fmul_rn(e1, e1));
+  const float ls_err = error8(g, bq, ls_scale_h, ls_min_h);
   if (ls_err < best_err && ok && ls_scale_h > 0.f) best_scale = ls_scale_h, best_lo = ls_min_h;
-  q[g * 32 + lane] = (uint8_t)((unsigned)bq0 | ((unsigned)bq1 << 4));
-  if (lane == 0) sm[g] = __halves2half2(__float2half_rn(best_scale), __float2half_rn(best_lo));
+  // Packing: this lane's codes are nibble j of words 0..7; three exchanges transpose that to all nibbles of word j.
+  uint32_t m = 0u;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float a, b;
+    unpack2(bq[i], a, b);
+    m |= ((uint32_t)a << (8 * i)) | ((uint32_t)b << (8 * i + 4));
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    const uint32_t keep = o == 4 ? 0x0000FFFFu : o == 2 ? 0x00FF00FFu : 0x0F0F0F0Fu;  // nibbles whose index lacks bit o
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, m, o);
+    m = (j & o) ? ((m & ~keep) | ((got & ~keep) >> (4 * o))) : ((m & keep) | ((got & keep) << (4 * o)));
+  }
+  if (gi < groups) {
+    uint8_t* out = q + gi * 32 + 4 * j;
+    if ((reinterpret_cast<uintptr_t>(q) & 3) == 0) {
+      *reinterpret_cast<uint32_t*>(out) = m;
+    } else {
+#pragma unroll
+      for (int b = 0; b < 4; ++b) out[b] = (uint8_t)(m >> (8 * b));
+    }
+    if (j == 0) sm[gi] = __halves2half2(__float2half_rn(best_scale), __float2half_rn(best_lo));
+  }
 }
 
 // Lane l holds inputs 4l .. 4l + 3 of the group of 128.
@@ -114,7 +224,7 @@ __global__ void __launch_bounds__(256) k_quant_q8(const float* __restrict__ w, s
 // (its quantiser is the Python converter).
 extern "C" int drb_quant_q4(const float* w, size_t groups, uint8_t* q, __half2* sm, cudaStream_t st) {
   if (groups == 0) return 0;
-  quant::k_quant_q4<<<(unsigned)((groups + 7) / 8), 256, 0, st>>>(w, groups, q, sm);
+  quant::k_quant_q4<<<(unsigned)((groups + quant::Q4_GROUPS - 1) / quant::Q4_GROUPS), quant::Q4_THREADS, 0, st>>>(w, groups, q, sm);
   return 0;
 }
 
