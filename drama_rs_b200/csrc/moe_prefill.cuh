@@ -281,27 +281,40 @@ __global__ void __launch_bounds__(64)
 }
 
 // x[r] += sigmoid(sgate[r]) * shared[r] + sum_k w[r,k] * Y[slot_of[r,k]], k ascending (fixed order, so
-// the result does not depend on how slots were handed out).
+// the result does not depend on how slots were handed out). Block (r, c): 1024 columns of row r, one float4 per thread.
+// Bound by Y's bytes from L2 or HBM; all of a thread's rows are requested before the first is used (TK = 8: in a loop over a
+// runtime topk every row waited for the one before, 13 us at 300 rows instead of 5).
+template <int TK>
 __global__ void __launch_bounds__(256)
     k_combine(float* __restrict__ x, const float* __restrict__ Y, const int* __restrict__ slot_of,
               const float* __restrict__ wts, const float* __restrict__ sgate, const float* __restrict__ shared, int topk,
               int Hd) {
   pdl_wait();
-  const int r = blockIdx.x;
-  const float sg = sigmoid_f(sgate[r]);
-  for (int c = threadIdx.x * 4; c < Hd; c += blockDim.x * 4) {
-    const float4 sh = *reinterpret_cast<const float4*>(shared + (size_t)r * Hd + c);
-    float4 acc = make_float4(sg * sh.x, sg * sh.y, sg * sh.z, sg * sh.w);
-    for (int k = 0; k < topk; ++k) {
-      const float w = wts[r * topk + k];
-      const float4 v = *reinterpret_cast<const float4*>(Y + (size_t)slot_of[r * topk + k] * Hd + c);
-      acc.x += w * v.x, acc.y += w * v.y, acc.z += w * v.z, acc.w += w * v.w;
-    }
-    float4* xo = reinterpret_cast<float4*>(x + (size_t)r * Hd + c);
-    float4 o = *xo;
-    o.x += acc.x, o.y += acc.y, o.z += acc.z, o.w += acc.w;
-    *xo = o;
+  pdl_launch_dependents();
+  const int r = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+  if (c >= Hd) return;
+  float4* xo = reinterpret_cast<float4*>(x + (size_t)r * Hd + c);
+  const float gate = __ldcg(sgate + r);
+  const float4 sh = __ldcg(reinterpret_cast<const float4*>(shared + (size_t)r * Hd + c));
+  float4 o = __ldcg(xo), acc;
+  auto add = [&](float w, const float4& v) { acc.x += w * v.x, acc.y += w * v.y, acc.z += w * v.z, acc.w += w * v.w; };
+  auto row = [&](int k) { return __ldcg(reinterpret_cast<const float4*>(Y + (size_t)__ldcg(slot_of + (size_t)r * topk + k) * Hd + c)); };
+  if (TK > 0) {
+    float4 v[TK > 0 ? TK : 1];
+    float w[TK > 0 ? TK : 1];
+#pragma unroll
+    for (int k = 0; k < TK; ++k) v[k] = row(k), w[k] = __ldcg(wts + (size_t)r * TK + k);
+    const float sg = sigmoid_f(gate);
+    acc = make_float4(sg * sh.x, sg * sh.y, sg * sh.z, sg * sh.w);
+#pragma unroll
+    for (int k = 0; k < TK; ++k) add(w[k], v[k]);
+  } else {
+    const float sg = sigmoid_f(gate);
+    acc = make_float4(sg * sh.x, sg * sh.y, sg * sh.z, sg * sh.w);
+    for (int k = 0; k < topk; ++k) add(__ldcg(wts + (size_t)r * topk + k), row(k));
   }
+  o.x += acc.x, o.y += acc.y, o.z += acc.z, o.w += acc.w;
+  *xo = o;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -371,63 +384,236 @@ __global__ void __launch_bounds__(256)
 // pair is one warp's dot product in a fixed order (lane l takes the 16-byte chunks l, l + 32, ... of the K = 2048
 // inputs, products exact in fp32, one fixed butterfly). A library GEMM picks its kernel by the batch size (measured:
 // logits of the same row differ by 1.2e-6 between a batch of 300 and a batch of 38), which would let the routing of
-// a row depend on how the rows are spread over the GPUs. Block (x, y) = RB rows x the outputs y, y + gridDim.y, ...;
-// its warp w takes every 8th of those. The split over y only adds parallelism: it does not change any sum.
-// F16: the rows are fp16 instead of bf16 (the weights are bf16 either way).
-constexpr int RL_RB = 4, RL_K = 2048, RL_SPLIT = 9;
-template <bool F16>
-__global__ void __launch_bounds__(256)
-    k_router_logits(const __nv_bfloat16* __restrict__ xb, const __nv_bfloat16* __restrict__ w, float* __restrict__ logits,
-                    int rows, int e1, float beta) {
+// a row depend on how the rows are spread over the GPUs.
+// Block (x, y): rows [RB x, +RB), outputs in groups of OB; warp w takes groups y + gridDim.y * w, .... The rows stand in
+// shared memory as fp32, two rows interleaved (a packed fp32 FMA serves both), and a warp multiplies OB outputs with all RB
+// rows at once: four rows per block and one output per warp re-read the 1 MB of weights from L2 for every four rows and
+// converted every activation for every output (123 us for 2048 rows, 27 us for 300).
+// SRC: what the rows come from. LOGITS_NORM: fp32 rows, RMS-normalised here (sums in k_rmsnorm's order) and rounded to fp16;
+// blocks with y = 0 also store them. LOGITS_F16 / LOGITS_BF16: 16-bit rows as they are. The weights are bf16.
+constexpr int RL_K = 2048, RL_WARPS = 16;
+enum LogitsSrc { LOGITS_NORM, LOGITS_F16, LOGITS_BF16 };
+template <int RB>
+constexpr size_t logits_smem() { return (size_t)RB * RL_K * 4; }
+
+template <int SRC, int RB, int OB>
+__global__ void __launch_bounds__(RL_WARPS * 32, 1)
+    k_router_logits(const void* __restrict__ src, const float* __restrict__ nw, float eps, __half* __restrict__ rows16,
+                    const __nv_bfloat16* __restrict__ w, const float* bias, float* logits, int rows, int e1, float beta, int* __restrict__ zero, int n_zero) {
+  extern __shared__ __align__(16) float xs[];
+  pdl_launch_dependents();
   pdl_wait();
-  __shared__ __align__(16) __nv_bfloat16 xs[RL_RB][RL_K];
-  const int r0 = blockIdx.x * RL_RB;
-  const int nr = min(RL_RB, rows - r0);
-  for (int i = threadIdx.x; i < RL_RB * RL_K / 8; i += blockDim.x) {
-    const int r = i / (RL_K / 8), c = i % (RL_K / 8);
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (r < nr) v = __ldcg(reinterpret_cast<const uint4*>(xb + (size_t)(r0 + r) * RL_K) + c);
-    reinterpret_cast<uint4*>(&xs[r][0])[c] = v;
-  }
-  __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int o = blockIdx.y + gridDim.y * warp; o < e1; o += gridDim.y * 8) {
-    const uint4* wr = reinterpret_cast<const uint4*>(w + (size_t)o * RL_K);
-    uint4 wv8[RL_K / 8 / 32];
+  const int r0 = blockIdx.x * RB, nr = min(RB, rows - r0);
+  if (zero && blockIdx.x == 0 && blockIdx.y == 0)
+    for (int i = threadIdx.x; i < n_zero; i += blockDim.x) zero[i] = 0;
+  // where input k of row r stands: 16-byte pieces (two inputs of a row pair), permuted so that eight lanes reading
+  // consecutive chunks' piece p meet eight different bank groups
+  auto at = [](int r, int k) {
+    const int c = k >> 3, p = (k >> 1) & 3;
+    return (((r >> 1) * (RL_K / 2) + 4 * c + (p ^ ((c >> 1) & 3))) << 2) + 2 * (k & 1) + (r & 1);
+  };
+  for (int r = warp; r < RB; r += RL_WARPS) {
+    if (r >= nr) {
+      for (int k = lane; k < RL_K; k += 32) xs[at(r, k)] = 0.f;
+    } else if (SRC == LOGITS_NORM) {
+      // k_rmsnorm's sums: its thread t adds the squares of inputs t + 256 i in turn; each warp's 32 threads by butterfly, the
+      // eight warps in order
+      const float* xr = static_cast<const float*>(src) + (size_t)(r0 + r) * RL_K;
+      float v[RL_K / 32];
 #pragma unroll
-    for (int j = 0; j < RL_K / 8 / 32; ++j) wv8[j] = __ldg(wr + lane + 32 * j);  // all eight in flight at once
-    float acc[RL_RB];
+      for (int i = 0; i < RL_K / 32; ++i) v[i] = __ldcg(xr + 32 * i + lane);
+      float t = 0.f;
 #pragma unroll
-    for (int r = 0; r < RL_RB; ++r) acc[r] = 0.f;
+      for (int q = 0; q < 8; ++q) {
+        float ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < RL_K / 8 / 32; ++j) {
-      const uint4 wv = wv8[j];
-      const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
+        for (int i = 0; i < RL_K / 256; ++i) ss += v[8 * i + q] * v[8 * i + q];
+        t += warp_sum(ss);
+      }
+      const float inv = rsqrtf(t / RL_K + eps);
 #pragma unroll
-      for (int r = 0; r < RL_RB; ++r) {
-        const uint4 xv = reinterpret_cast<const uint4*>(&xs[r][0])[lane + 32 * j];
-        const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
+      for (int i = 0; i < RL_K / 32; ++i) {
+        const int k = 32 * i + lane;
+        const __half h = tc::f2h_sat(v[i] * inv * __ldg(nw + k));
+        if (blockIdx.y == 0) rows16[(size_t)(r0 + r) * RL_K + k] = h;
+        xs[at(r, k)] = __half2float(h);
+      }
+    } else {
+      const uint4* xr = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(src) + (size_t)(r0 + r) * RL_K);
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          float x0, x1;
-          if (F16) {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&xw[t]));
-            x0 = f.x, x1 = f.y;
-          } else {
-            x0 = __uint_as_float(xw[t] << 16), x1 = __uint_as_float(xw[t] & 0xffff0000u);
-          }
-          acc[r] = fmaf(__uint_as_float(ww[t] << 16), x0, acc[r]);
-          acc[r] = fmaf(__uint_as_float(ww[t] & 0xffff0000u), x1, acc[r]);
+      for (int i = 0; i < RL_K / 256; ++i) {
+        const uint4 v = __ldcg(xr + 32 * i + lane);
+        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          float2 f;
+          if (SRC == LOGITS_F16) f = __half22float2(*reinterpret_cast<const __half2*>(&u[q]));
+          else f = make_float2(__uint_as_float(u[q] << 16), __uint_as_float(u[q] & 0xffff0000u));
+          const int k = 8 * (32 * i + lane) + 2 * q;
+          xs[at(r, k)] = f.x, xs[at(r, k + 1)] = f.y;
         }
       }
     }
+  }
+  __syncthreads();
+  const ulonglong2* xs2 = reinterpret_cast<const ulonglong2*>(xs);
+  const int groups = (e1 + OB - 1) / OB;
+  for (int g = blockIdx.y + gridDim.y * warp; g < groups; g += gridDim.y * RL_WARPS) {
+    const uint4* wr[OB];
+    uint4 wn[OB];
 #pragma unroll
-    for (int r = 0; r < RL_RB; ++r) {
-      const float v = warp_sum(acc[r]);
-      if (lane == 0 && r < nr) {
-        float* out = logits + (size_t)(r0 + r) * e1 + o;
-        *out = beta != 0.f ? fmaf(beta, *out, v) : v;
+    for (int o = 0; o < OB; ++o) {
+      wr[o] = reinterpret_cast<const uint4*>(w + (size_t)min(OB * g + o, e1 - 1) * RL_K);
+      wn[o] = __ldg(wr[o] + lane);
+    }
+    unsigned long long acc[OB][RB / 2];
+#pragma unroll
+    for (int o = 0; o < OB; ++o)
+#pragma unroll
+      for (int q = 0; q < RB / 2; ++q) acc[o][q] = 0ull;
+#pragma unroll 1
+    for (int j = 0; j < RL_K / 256; ++j) {
+      const int c = lane + 32 * j, sw = (c >> 1) & 3;
+      uint32_t ww[OB][4];
+#pragma unroll
+      for (int o = 0; o < OB; ++o) {
+        ww[o][0] = wn[o].x, ww[o][1] = wn[o].y, ww[o][2] = wn[o].z, ww[o][3] = wn[o].w;
+        if (j + 1 < RL_K / 256) wn[o] = __ldg(wr[o] + c + 32);
       }
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        unsigned long long w0[OB], w1[OB];
+#pragma unroll
+        for (int o = 0; o < OB; ++o) {
+          const float lo = __uint_as_float(ww[o][p] << 16), hi = __uint_as_float(ww[o][p] & 0xffff0000u);
+          w0[o] = pack2(lo, lo), w1[o] = pack2(hi, hi);
+        }
+#pragma unroll
+        for (int q = 0; q < RB / 2; ++q) {
+          const ulonglong2 x2 = xs2[q * (RL_K / 2) + 4 * c + (p ^ sw)];
+#pragma unroll
+          for (int o = 0; o < OB; ++o) acc[o][q] = fma2(w1[o], x2.y, fma2(w0[o], x2.x, acc[o][q]));
+        }
+      }
+    }
+    // The butterfly over 32 lanes, for all sums at once: at each exchange a lane keeps half of them and hands the other
+    // half on, until one is left per lane group; every sum is formed from the same pairs in the same order as by itself.
+    constexpr int N = OB * RB;
+    float v[N];
+#pragma unroll
+    for (int o = 0; o < OB; ++o)
+#pragma unroll
+      for (int q = 0; q < RB / 2; ++q) unpack2(acc[o][q], v[o * RB + 2 * q], v[o * RB + 2 * q + 1]);
+    int n = N, id = 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      if (n > 1) {
+        n >>= 1;
+        const bool hi = lane & o;
+        id += hi ? n : 0;
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i)
+          if (i < n) {
+            const float keep = hi ? v[i + n] : v[i], send = hi ? v[i] : v[i + n];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+          }
+      } else {
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+      }
+    }
+    constexpr int LEFT = N > 32 ? N / 32 : 1, COPIES = N < 32 ? 32 / N : 1;  // sums per lane; lanes that hold the same one
+    if ((lane & (COPIES - 1)) == 0) {
+#pragma unroll
+      for (int i = 0; i < LEFT; ++i) {
+        const int o = OB * g + (id + i) / RB, r = (id + i) % RB;
+        if (o < e1 && r < nr) {
+          const size_t at_out = (size_t)(r0 + r) * e1 + o;
+          logits[at_out] = beta != 0.f ? fmaf(beta, bias[at_out], v[i]) : v[i];
+        }
+      }
+    }
+  }
+}
+
+// Shapes by the number of rows: up to eight rows, one output per warp over as many blocks as there are multiprocessors (the
+// weights' latency is all there is); up to 96, eight rows and four outputs; beyond that sixteen rows, so that the weights are
+// read from L2 once per sixteen rows.
+template <int SRC>
+static int launch_logits(const void* src, const float* nw, float eps, __half* rows16, const __nv_bfloat16* w, const float* bias, float* logits,
+                         int rows, int e1, float beta, int* zero, int n_zero, cudaStream_t st) {
+  const DrbDevice& dev = drb_device(st);
+  if (!dev.ready) return -2;
+  auto go = [&](auto kern, int rb, int ob) {
+    const int gx = (rows + rb - 1) / rb, groups = (e1 + ob - 1) / ob;
+    const int gy = min(groups, max(1, dev.sms / gx));
+    drb_launch(kern, dim3(gx, gy), dim3(RL_WARPS * 32), (size_t)rb * RL_K * 4, st, dev.pdl, src, nw, eps, rows16, w, bias, logits, rows, e1, beta, zero, n_zero);
+  };
+  if (rows <= 8) go(k_router_logits<SRC, 8, 1>, 8, 1);
+  else if (rows <= 96) go(k_router_logits<SRC, 8, 4>, 8, 4);
+  else go(k_router_logits<SRC, 16, 4>, 16, 4);
+  return 0;
+}
+
+template <int SRC>
+static cudaError_t configure_logits() {
+  auto one = [](auto kern, size_t smem) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return e != cudaSuccess ? e : drb_carveout(kern);
+  };
+  cudaError_t e;
+  if ((e = one(k_router_logits<SRC, 8, 1>, logits_smem<8>())) != cudaSuccess) return e;
+  if ((e = one(k_router_logits<SRC, 8, 4>, logits_smem<8>())) != cudaSuccess) return e;
+  return one(k_router_logits<SRC, 16, 4>, logits_smem<16>());
+}
+
+// One warp per row, behind the routing: the row's slots (the exclusive scan of the expert counts, which every block makes for
+// itself, plus the rank that router::k_moe_topk took with its count) and its copies for the grouped GEMMs: one per chosen
+// expert in slot order, one for the shared expert. Grouping and copying in one launch over the whole chip: as a launch
+// of one block and one of its own they took 7 + 6 us at 300 rows, 25 + 18 us at 2048.
+__global__ void __launch_bounds__(256)
+    k_scatter_rows(const __half* __restrict__ rows16, const int* __restrict__ idx, int rows, int topk, const int* __restrict__ counts, int E,
+                   int* __restrict__ offsets, int* __restrict__ slot_of, int* __restrict__ row_of, unsigned char* __restrict__ dst,
+                   unsigned char* __restrict__ sh_dst) {
+  __shared__ int offs[256], tot[8];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int c = t < E ? __ldcg(counts + t) : 0;
+  int incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  if (lane == 31) tot[warp] = incl;
+  __syncthreads();
+  int before = incl - c;
+  for (int q = 0; q < warp; ++q) before += tot[q];
+  offs[t] = before;
+  if (blockIdx.x == 0 && t < E) offsets[t] = before;
+  __syncthreads();
+  constexpr int PER = H / 8 / 32;
+  for (int r = blockIdx.x * 8 + warp; r < rows; r += gridDim.x * 8) {
+    const uint4* src = reinterpret_cast<const uint4*>(rows16 + (size_t)r * H);
+    uint4 v[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const uint4 u = __ldcg(src + 32 * j + lane);
+      v[j] = make_uint4(prmt(u.x, u.z, 0x5410u), prmt(u.x, u.z, 0x7632u), prmt(u.y, u.w, 0x5410u), prmt(u.y, u.w, 0x7632u));
+    }
+    int slot = 0;
+    if (lane < topk) {
+      const int p = r * topk + lane;
+      slot = offs[__ldcg(idx + p)] + __ldcg(slot_of + p);
+      slot_of[p] = slot;
+      row_of[slot] = r;
+    }
+    for (int k = 0; k <= topk; ++k) {
+      const int to = __shfl_sync(0xffffffffu, slot, k & 31);
+      uint4* out = reinterpret_cast<uint4*>(k < topk ? dst + (size_t)to * pft::TOKEN_STRIDE : sh_dst + (size_t)r * pft::TOKEN_STRIDE);
+#pragma unroll
+      for (int j = 0; j < PER; ++j) out[32 * j + lane] = v[j];
     }
   }
 }
@@ -464,11 +650,14 @@ __global__ void __launch_bounds__(256) k_offsets(const int* __restrict__ counts,
 static cudaError_t configure_all() {
   cudaError_t e;
   if ((e = drb_carveout(k_offsets)) != cudaSuccess) return e;
-  if ((e = drb_carveout(k_router_logits<false>)) != cudaSuccess) return e;
-  if ((e = drb_carveout(k_router_logits<true>)) != cudaSuccess) return e;
+  if ((e = configure_logits<LOGITS_NORM>()) != cudaSuccess) return e;
+  if ((e = configure_logits<LOGITS_F16>()) != cudaSuccess) return e;
+  if ((e = configure_logits<LOGITS_BF16>()) != cudaSuccess) return e;
+  if ((e = drb_carveout(k_scatter_rows)) != cudaSuccess) return e;
   if ((e = drb_carveout(k_count)) != cudaSuccess) return e;
   if ((e = drb_carveout(k_permute)) != cudaSuccess) return e;
-  if ((e = drb_carveout(k_combine)) != cudaSuccess) return e;
+  if ((e = drb_carveout(k_combine<8>)) != cudaSuccess) return e;
+  if ((e = drb_carveout(k_combine<0>)) != cudaSuccess) return e;
   if ((e = drb_carveout(k_group)) != cudaSuccess) return e;
   if ((e = drb_carveout(k_ep_plan)) != cudaSuccess) return e;
   if ((e = drb_carveout(k_ep_scatter)) != cudaSuccess) return e;
@@ -504,8 +693,7 @@ extern "C" int drb_router_logits(const __nv_bfloat16* xb, const __nv_bfloat16* w
                                  float beta, cudaStream_t st) {
   if (h != pf::RL_K) return -1;
   if (rows <= 0 || e1 <= 0) return 0;
-  pf::k_router_logits<false><<<dim3((rows + pf::RL_RB - 1) / pf::RL_RB, pf::RL_SPLIT), 256, 0, st>>>(xb, w, logits, rows, e1, beta);
-  return 0;
+  return pf::launch_logits<pf::LOGITS_BF16>(xb, nullptr, 0.f, nullptr, w, logits, logits, rows, e1, beta, nullptr, 0, st);
 }
 
 // The two calls above for rows kept in fp16 (no counterpart in the reference, whose prefill rounds the normalised rows
@@ -521,9 +709,7 @@ extern "C" int drb_router_logits_f16(const __half* xh, const __nv_bfloat16* w, f
                                      cudaStream_t st) {
   if (h != pf::RL_K) return -1;
   if (rows <= 0 || e1 <= 0) return 0;
-  pf::k_router_logits<true><<<dim3((rows + pf::RL_RB - 1) / pf::RL_RB, pf::RL_SPLIT), 256, 0, st>>>(
-      reinterpret_cast<const __nv_bfloat16*>(xh), w, logits, rows, e1, beta);
-  return 0;
+  return pf::launch_logits<pf::LOGITS_F16>(xh, nullptr, 0.f, nullptr, w, logits, logits, rows, e1, beta, nullptr, 0, st);
 }
 
 // Reference: kernels/drama.cu:774-778; src/ffi.rs:66-69. fill must be zeroed by the caller.
@@ -540,7 +726,9 @@ extern "C" int dr_moe_combine(float* x, const float* Y, const int* slot_of, cons
                               const float* shared, int rows, int topk, int H, cudaStream_t st) {
   if (H % 4 != 0) return -1;
   if (rows <= 0) return 0;
-  pf::k_combine<<<rows, 256, 0, st>>>(x, Y, slot_of, wts, sgate, shared, topk, H);
+  const DrbDevice& dev = drb_device(st);
+  drb_launch(topk == 8 ? pf::k_combine<8> : pf::k_combine<0>, dim3(rows, (H + 1023) / 1024), dim3(256), 0, st, dev.ready && dev.pdl, x, Y, slot_of,
+             wts, sgate, shared, topk, H);
   return 0;
 }
 
@@ -706,6 +894,47 @@ extern "C" int drb_moe_prefill_block_peers(const uint8_t* gu_q, const __half2* g
   if (!peer_y || !y_row_of || cap <= 0 || rank < 0) return -1;
   return prefill_block_impl(gu_q, gu_sm, d_q, d_sm, sgu_q, sgu_s, sd_q, sd_s, xb, row_of, offsets, counts, act, y, sh_act, sh_out, rows_sh, E,
                             H, I, 1, y_row_of, peer_y, cap, rank, st);
+}
+
+// One MoE block over `rows` rows in one call (include/dramakernels.h): what MoePrefill's own sequence of calls does, in six
+// launches, each started while the one before drains.
+struct drb_prefill_buffers {
+  float* x;
+  __half* rows16;
+  float* logits;
+  const float* logit_bias;
+  int* idx;
+  float *wts, *sgate;
+  int *counts, *offsets, *slot_of, *row_of;
+  __nv_bfloat16* act;
+  float* y;
+  __nv_bfloat16* sh_act;
+  float* sh_out;
+};
+extern "C" int drb_moe_prefill_layer(const drb_moe_layer* w, const drb_prefill_buffers* b, int rows, int e, int topk, int h, int i, float eps,
+                                     cudaStream_t st) {
+  if (!w || !b || h != pf::H || i != pf::I || e < 1 || e > 256 || topk < 1 || topk > e || topk > 31) return -1;
+  if (rows <= 0) return 0;
+  const DrbDevice& dev = drb_device(st);
+  if (!dev.ready) return -2;
+  const int r = pf::launch_logits<pf::LOGITS_NORM>(b->x, static_cast<const float*>(w->post_norm), eps, b->rows16,
+                                                   static_cast<const __nv_bfloat16*>(w->router), b->logit_bias, b->logits, rows, e + 1,
+                                                   b->logit_bias ? 1.f : 0.f, b->counts, e, st);
+  if (r != 0) return r;
+  drb_launch(router::k_moe_topk<true>, dim3(rows), dim3(router::THREADS), 0, st, dev.pdl, (const float*)b->logits, e, topk, e + 1, b->idx, b->wts,
+             b->sgate, b->counts, b->slot_of);
+  const int blocks = (rows + 7) / 8;
+  drb_launch(pf::k_scatter_rows, dim3(blocks < 2 * dev.sms ? blocks : 2 * dev.sms), dim3(256), 0, st, dev.pdl, (const __half*)b->rows16,
+             (const int*)b->idx, rows, topk, (const int*)b->counts, e, b->offsets, b->slot_of, b->row_of, reinterpret_cast<unsigned char*>(b->y),
+             reinterpret_cast<unsigned char*>(b->sh_out));
+  pft::Block k = {};
+  k.gu_w = w->gu_q, k.gu_s = w->gu_sm, k.d_w = w->d_q, k.d_s = w->d_sm;
+  k.sgu_q = w->sgu_q, k.sgu_s = w->sgu_s, k.sd_q = w->sd_q, k.sd_s = w->sd_s;
+  k.prepared = true, k.row_of = b->row_of, k.offsets = b->offsets, k.counts = b->counts;
+  k.act = b->act, k.y = b->y, k.sh_act = b->sh_act, k.sh_out = b->sh_out, k.rows_sh = rows, k.E = e;
+  const int g = pft::run_block<0>(k, dev, st);
+  if (g != 0) return g;
+  return dr_moe_combine(b->x, b->y, b->slot_of, b->wts, b->sgate, b->sh_out, rows, topk, h, st);
 }
 
 // dr_moe_prefill over block-FP8 experts (include/dramakernels.h). Reference: kernels/drama.cu:971-1109; src/ffi.rs:52-55.

@@ -807,6 +807,7 @@ struct Block {
   const void *sgu_q, *sgu_s, *sd_q, *sd_s;  // shared expert (rows_sh > 0)
   const void* x;                            // 16-bit rows [., H]
   bool x_bf16;
+  bool prepared;                            // y and sh_out hold the prepared rows already (x is not used)
   const int *row_of, *offsets, *counts, *y_row_of;
   void *act, *y, *sh_act, *sh_out;
   int rows_sh, E;
@@ -823,7 +824,7 @@ static int run_block(const Block& b, const DrbDevice& dev, cudaStream_t st) {
   if (!prep && (b.x_bf16 || FMT != 0)) return -1;
   unsigned char* tok = static_cast<unsigned char*>(b.y);
   unsigned char* shtok = static_cast<unsigned char*>(b.sh_out);
-  if (prep) {
+  if (prep && !b.prepared) {
     auto kp = b.x_bf16 ? k_prep_rows<true, FMT == 0> : k_prep_rows<false, FMT == 0>;
     drb_launch(kp, dim3(2 * dev.sms), dim3(256), 0, st, false, static_cast<const uint4*>(b.x), b.row_of, b.offsets, b.counts, b.E, tok, b.rows_sh, shtok);
   }
@@ -855,7 +856,7 @@ static int run_block(const Block& b, const DrbDevice& dev, cudaStream_t st) {
       a.scales = sc, a.shs = static_cast<const __half*>(gemm == 0 ? b.sgu_s : b.sd_s);
       a.offsets = b.offsets + e0, a.counts = b.counts + e0, a.E = ne > 0 ? ne : 0, a.rows_sh = sh ? b.rows_sh : 0;
       if (gemm == 0)
-        drb_launch(prep ? k_grouped<0, FMT, true> : k_grouped<0, FMT, FMT != 0>, dim3(dev.sms), dim3(THREADS), Smem<0, FMT>::BYTES, st, false, m, a);
+        drb_launch(prep ? k_grouped<0, FMT, true> : k_grouped<0, FMT, FMT != 0>, dim3(dev.sms), dim3(THREADS), Smem<0, FMT>::BYTES, st, dev.pdl && b.prepared && b.E <= MAX_E, m, a);
       else  // only the first one follows the gate/up kernel
         drb_launch(k_grouped<1, FMT, true>, dim3(dev.sms), dim3(THREADS), Smem<1, FMT>::BYTES, st, dev.pdl && b.E <= MAX_E, m, a);
     }

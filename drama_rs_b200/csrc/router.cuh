@@ -184,10 +184,12 @@ DRB_DEV void softmax_topk(float v, int E, int topk, int* __restrict__ idx, float
   else softmax_topk_impl<BAR_ID, 0>(v, E, topk, idx, wts, sm);
 }
 
-// grid = rows of logits; logits has E + 1 valid columns per row at the given stride.
+// grid = rows of logits; logits has E + 1 valid columns per row at the given stride. RANK: every chosen (row, expert) pair
+// also takes its place among the expert's pairs, rank[pair] = counts[expert]++ (the order is arbitrary; counts start at zero).
+template <bool RANK>
 __global__ void __launch_bounds__(THREADS)
     k_moe_topk(const float* __restrict__ logits, int E, int topk, int stride, int* __restrict__ idx,
-               float* __restrict__ wts, float* __restrict__ sgate) {
+               float* __restrict__ wts, float* __restrict__ sgate, int* __restrict__ counts, int* __restrict__ rank) {
   __shared__ TopkSmem sm;
   pdl_launch_dependents();
   pdl_wait();
@@ -196,6 +198,10 @@ __global__ void __launch_bounds__(THREADS)
   const float v = (int)threadIdx.x < E ? __ldcg(l + threadIdx.x) : -INFINITY;
   softmax_topk(v, E, topk, idx + (size_t)r * topk, wts + (size_t)r * topk, sm);
   if (threadIdx.x == 0) sgate[r] = __ldcg(l + E);
+  if (RANK && (int)threadIdx.x < topk) {  // warp 0, which wrote idx
+    const size_t p = (size_t)r * topk + threadIdx.x;
+    rank[p] = atomicAdd(counts + idx[p], 1);
+  }
 }
 
 constexpr int K = 2048;
@@ -351,7 +357,8 @@ static cudaError_t configure_all() {
   cudaError_t e = drb_carveout(cl::k_router_cluster);
   if (e != cudaSuccess) return e;
   if ((e = cudaFuncSetAttribute(cl::k_router_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cl::SMEM_BYTES)) != cudaSuccess) return e;
-  return drb_carveout(k_moe_topk);
+  if ((e = drb_carveout(k_moe_topk<true>)) != cudaSuccess) return e;
+  return drb_carveout(k_moe_topk<false>);
 }
 
 }  // namespace router
@@ -391,6 +398,7 @@ extern "C" int dr_moe_topk(const float* logits, int rows, int E, int topk, int s
   if (rows <= 0) return 0;
   const DrbDevice& dev = drb_device(st);
   if (!dev.ready) return -2;
-  drb_launch(router::k_moe_topk, dim3(rows), dim3(router::THREADS), 0, st, dev.pdl, logits, E, topk, stride, idx, wts, sgate);
+  drb_launch(router::k_moe_topk<false>, dim3(rows), dim3(router::THREADS), 0, st, dev.pdl, logits, E, topk, stride, idx, wts, sgate,
+             (int*)nullptr, (int*)nullptr);
   return 0;
 }

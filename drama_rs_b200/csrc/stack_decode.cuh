@@ -38,20 +38,6 @@
 #include "moe_decode.cuh"
 #include "router.cuh"
 
-// One layer's weights, device pointers in the reference's layouts (see include/dramakernels.h).
-struct drb_moe_layer {
-  const void* router;     // bf16 [E + 1, 2048]
-  const void* post_norm;  // f32 [2048]
-  const void* gu_q;       // u8  [E, 1024, 1024]
-  const void* gu_sm;      // f16 [E, 1024, 32, 2]
-  const void* d_q;        // u8  [E, 2048, 256]
-  const void* d_sm;       // f16 [E, 2048, 8, 2]
-  const void* sgu_q;      // i8  [1024, 2048]
-  const void* sgu_s;      // f16 [1024, 16]
-  const void* sd_q;       // i8  [2048, 512]
-  const void* sd_s;       // f16 [2048, 4]
-};
-
 namespace stack {
 
 using moe::H;

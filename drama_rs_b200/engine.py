@@ -8,9 +8,9 @@ into a graph that `step` replays — src/engine.rs:136-150 (`Op`), 674-708 (`rec
 Prefill: `MoePrefill` has two forms. `reference_calls=True` is src/engine.rs:544-604 call for call:
 cuBLAS router logits, dr_moe_topk, shared expert through dequant + cuBLAS, count, counts to the
 host, host exclusive scan, permute, grouped expert kernel, combine. The default is this library's
-own sequence of seven launches with no library GEMM and no host round trip: rmsnorm, router logits
-in a fixed order, top-k, one grouping kernel, the two grouped tensor-core GEMMs (which also run the
-int8 shared expert and read their rows in place), combine.
+own sequence in one call (drb_moe_prefill_layer) with no library GEMM and no host round trip: RMSNorm
+and router logits in a fixed order, top-k, row scatter, the two grouped tensor-core GEMMs (which also
+run the int8 shared expert), combine.
 """
 
 from __future__ import annotations
@@ -197,6 +197,7 @@ class MoePrefill:
         self.device_scan = False  # reference calls only: offsets by drb_moe_offsets on the device instead of the host scan
         self.invariant_router = not reference_calls  # router logits by drb_router_logits (independent of the batch size) instead of cuBLAS
         self.logit_bias: DevBuf | None = None  # [n, E + 1] f32 rows the router GEMM accumulates onto (not in the reference)
+        self._args = None
 
     def gemm_q8(self, a, w, c, m: int, beta: float) -> None:
         """C = A . dequant(W)^T + beta C for a q8 weight. src/engine.rs:351-355."""
@@ -240,6 +241,18 @@ class MoePrefill:
             check(l.dr_gemm(self.blas, self.hn_b.at(0), layer.router.at(0), self.rlog.at(0), n, e + 1, h, beta), "gemm")
         launched(l.dr_moe_topk(self.rlog.at(0), n, e, topk, e + 1, self.idx.at(0), self.wts.at(0), self.sgate.at(0), st), "moe_topk")
 
+    def _layer_args(self):
+        """The structs of drb_moe_prefill_layer for this object's buffers, kept until one of them is replaced."""
+        ly = self.layer
+        key = (ly, self.x, self.hn_b, self.rlog, self.logit_bias, self.idx, self.wts, self.sgate, self.counts, self.offsets, self.slot_of,
+               self.row_of, self.ap, self.yp, self.sh_act_b, self.sh_out)
+        if self._args is None or any(a is not b for a, b in zip(key, self._args[0])):
+            w = ffi.MoeLayerPtrs(*(b.ptr for b in (ly.router, ly.post_norm, ly.gate_up.q, ly.gate_up.sm, ly.down.q, ly.down.sm,
+                                                   ly.shared_gate_up.q, ly.shared_gate_up.s, ly.shared_down.q, ly.shared_down.s)))
+            b = ffi.PrefillBuffers(*(b.ptr if b is not None else None for b in key[1:]))
+            self._args = (key, C.byref(w), C.byref(b))
+        return self._args[1], self._args[2]
+
     def run_device(self, n: int) -> None:
         """The block on the n rows already in self.x (device), in place. With a logit bias the router logits are
         accumulated onto the bias rows (beta = 1) instead of overwriting them."""
@@ -247,6 +260,10 @@ class MoePrefill:
             return self.run_device_reference_calls(n)
         l, st, layer = self.l, self.st.raw, self.layer
         h, e, topk, i = layer.hidden, layer.experts, self.topk, layer.inter
+        if self.rows_f16 and e <= 256:
+            w, buf = self._layer_args()
+            launched(l.drb_moe_prefill_layer(w, buf, n, e, topk, h, i, self.eps, st), "moe_prefill_layer")
+            return
         self.route_device(n)
         launched(l.drb_moe_group(self.idx.at(0), n, topk, 0, e, self.counts.at(0), self.offsets.at(0), self.slot_of.at(0),
                                  self.row_of.at(0), st), "moe_group")

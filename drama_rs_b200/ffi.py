@@ -16,6 +16,21 @@ LIB_PATH = os.environ.get("DRAMA_KERNELS_LIB") or os.path.join(HERE, "libdramake
 
 P, I32, F32, SZ, U32 = C.c_void_p, C.c_int, C.c_float, C.c_size_t, C.c_uint
 
+
+
+class MoeLayerPtrs(C.Structure):
+    """drb_moe_layer: one layer's device pointers."""
+
+    _fields_ = [(n, P) for n in ("router", "post_norm", "gu_q", "gu_sm", "d_q", "d_sm", "sgu_q", "sgu_s", "sd_q", "sd_s")]
+
+
+class PrefillBuffers(C.Structure):
+    """drb_prefill_buffers."""
+
+    _fields_ = [(n, P) for n in ("x", "rows16", "logits", "logit_bias", "idx", "wts", "sgate", "counts", "offsets", "slot_of", "row_of", "act",
+                                 "y", "sh_act", "sh_out")]
+
+
 # name -> (restype, argtypes); the order within each tuple is the ABI.
 SIGNATURES: dict[str, tuple] = {
     "dr_error_string": (C.c_char_p, [I32]),
@@ -63,6 +78,7 @@ SIGNATURES: dict[str, tuple] = {
     "drb_moe_offsets": (I32, [P, I32, P, P]),
     "drb_moe_group": (I32, [P, I32, I32, I32, I32, P, P, P, P, P]),
     "drb_moe_prefill_block": (I32, [P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, I32, I32, I32, I32, I32, P, P]),
+    "drb_moe_prefill_layer": (I32, [P, P, I32, I32, I32, I32, I32, F32, P]),
     "drb_ep_block_rows": (I32, [I32, I32]),
     "drb_ep_pack": (I32, [P, P, I32, I32, I32, I32, I32, I32, P, P, P, P, P]),
     "drb_ep_group": (I32, [P, I32, I32, I32, I32, P, P, P, P, P, P]),

@@ -212,6 +212,28 @@ int drb_moe_prefill_block(const uint8_t* gu_q, const dr_half* gu_sm, const uint8
                           const dr_bf16* xb, const int* row_of, const int* offsets, const int* counts, dr_bf16* act,
                           float* y, dr_bf16* sh_act, float* sh_out, int rows_sh, int e, int h, int i, int x_f16,
                           const int* y_row_of, dr_stream st);
+/* One MoE block over `rows` rows in one call: x <- x + moe(rmsnorm(x, post_norm)) in place, the sequence drb_rmsnorm_f16,
+ * drb_router_logits_f16, dr_moe_topk, drb_moe_group, drb_moe_prefill_block, dr_moe_combine with the same results (bit for bit
+ * in the rows, logits, routing and x; slots inside an expert in arbitrary order) in six launches. w and buf are host
+ * structs of device pointers. buf: x f32 [rows, h]; rows16 fp16 [rows, h]; logits f32 [rows, e + 1]; logit_bias f32 [rows, e + 1]
+ * added to the logits, or NULL; idx, wts [rows, topk]; sgate [rows]; counts, offsets [e]; slot_of, row_of [rows * topk]; act,
+ * y, sh_act, sh_out as drb_moe_prefill_block. e <= 256, topk <= 31, h == 2048, i == 512, else -1; -3 when the driver refuses a
+ * tensor map. */
+typedef struct {
+  float* x;
+  dr_half* rows16;
+  float* logits;
+  const float* logit_bias;
+  int* idx;
+  float *wts, *sgate;
+  int *counts, *offsets, *slot_of, *row_of;
+  dr_bf16* act;
+  float* y;
+  dr_bf16* sh_act;
+  float* sh_out;
+} drb_prefill_buffers;
+int drb_moe_prefill_layer(const drb_moe_layer* w, const drb_prefill_buffers* buf, int rows, int e, int topk, int h, int i, float eps,
+                          dr_stream st);
 /* ---- expert parallelism (the reference is single-GPU) ---------------------------------------- */
 /* Rows travel between ranks in a buffer of `world` blocks; a block is drb_ep_block_rows(cap, row_bytes) rows of
  * row_bytes bytes: cap row slots, then the cap local expert ids of those rows (int32, `per` = empty slot), padded
