@@ -567,20 +567,32 @@ static cudaError_t configure_logits() {
   return one(k_router_logits<SRC, 16, 4>, logits_smem<16>());
 }
 
-// One warp per row, behind the routing: the row's slots (the exclusive scan of the expert counts, which every block makes for
+// Two warps per row, behind the routing: the row's slots (the exclusive scan of the expert counts, which every block makes for
 // itself, plus the rank that router::k_moe_topk took with its count) and its copies for the grouped GEMMs: one per chosen
 // expert in slot order, one for the shared expert. Grouping and copying in one launch over the whole chip: as a launch
 // of one block and one of its own they took 7 + 6 us at 300 rows, 25 + 18 us at 2048.
-__global__ void __launch_bounds__(256)
+constexpr int SC_ROWS = 2, SC_THREADS = SC_ROWS * 64;  // two warps per row, each half of it
+__global__ void __launch_bounds__(SC_THREADS)
     k_scatter_rows(const __half* __restrict__ rows16, const int* __restrict__ idx, int rows, int topk, const int* __restrict__ counts, int E,
-                   int* __restrict__ offsets, int* __restrict__ slot_of, int* __restrict__ row_of, unsigned char* __restrict__ dst,
-                   unsigned char* __restrict__ sh_dst) {
-  __shared__ int offs[256], tot[8];
+                   int* __restrict__ offsets, int* __restrict__ slot_of, const int* __restrict__ rank, int* __restrict__ row_of,
+                   unsigned char* __restrict__ dst, unsigned char* __restrict__ sh_dst) {
+  __shared__ int offs[256], tot[SC_THREADS / 32];
   pdl_launch_dependents();
   pdl_wait();
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int c = t < E ? __ldcg(counts + t) : 0;
-  int incl = c;
+  constexpr int CPT = 256 / SC_THREADS, PER = H / 8 / 64;
+  int r = blockIdx.x * SC_ROWS + (warp >> 1);
+  auto load = [&](int row, uint4(&v)[PER]) {
+    const uint4* src = reinterpret_cast<const uint4*>(rows16 + (size_t)row * H) + (warp & 1) * 32 * PER;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) v[j] = row < rows ? __ldcg(src + 32 * j + lane) : make_uint4(0u, 0u, 0u, 0u);
+  };
+  uint4 v[PER];
+  load(r, v);
+  int c[CPT], sum = 0;
+#pragma unroll
+  for (int j = 0; j < CPT; ++j) c[j] = sum, sum += CPT * t + j < E ? __ldcg(counts + CPT * t + j) : 0;
+  int incl = sum;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const int u = __shfl_up_sync(0xffffffffu, incl, o);
@@ -588,33 +600,34 @@ __global__ void __launch_bounds__(256)
   }
   if (lane == 31) tot[warp] = incl;
   __syncthreads();
-  int before = incl - c;
+  int before = incl - sum;
   for (int q = 0; q < warp; ++q) before += tot[q];
-  offs[t] = before;
-  if (blockIdx.x == 0 && t < E) offsets[t] = before;
-  __syncthreads();
-  constexpr int PER = H / 8 / 32;
-  for (int r = blockIdx.x * 8 + warp; r < rows; r += gridDim.x * 8) {
-    const uint4* src = reinterpret_cast<const uint4*>(rows16 + (size_t)r * H);
-    uint4 v[PER];
 #pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      const uint4 u = __ldcg(src + 32 * j + lane);
-      v[j] = make_uint4(prmt(u.x, u.z, 0x5410u), prmt(u.x, u.z, 0x7632u), prmt(u.y, u.w, 0x5410u), prmt(u.y, u.w, 0x7632u));
-    }
+  for (int j = 0; j < CPT; ++j) {
+    offs[CPT * t + j] = before + c[j];
+    if (blockIdx.x == 0 && CPT * t + j < E) offsets[CPT * t + j] = before + c[j];
+  }
+  __syncthreads();
+  for (; r < rows; r += gridDim.x * SC_ROWS) {
     int slot = 0;
     if (lane < topk) {
       const int p = r * topk + lane;
-      slot = offs[__ldcg(idx + p)] + __ldcg(slot_of + p);
-      slot_of[p] = slot;
-      row_of[slot] = r;
+      slot = offs[__ldcg(idx + p)] + __ldcg(rank + p);
+      if ((warp & 1) == 0) {
+        slot_of[p] = slot;
+        row_of[slot] = r;
+      }
     }
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+      v[j] = make_uint4(prmt(v[j].x, v[j].z, 0x5410u), prmt(v[j].x, v[j].z, 0x7632u), prmt(v[j].y, v[j].w, 0x5410u), prmt(v[j].y, v[j].w, 0x7632u));
     for (int k = 0; k <= topk; ++k) {
       const int to = __shfl_sync(0xffffffffu, slot, k & 31);
-      uint4* out = reinterpret_cast<uint4*>(k < topk ? dst + (size_t)to * pft::TOKEN_STRIDE : sh_dst + (size_t)r * pft::TOKEN_STRIDE);
+      uint4* out = reinterpret_cast<uint4*>(k < topk ? dst + (size_t)to * pft::TOKEN_STRIDE : sh_dst + (size_t)r * pft::TOKEN_STRIDE) + (warp & 1) * 32 * PER;
 #pragma unroll
       for (int j = 0; j < PER; ++j) out[32 * j + lane] = v[j];
     }
+    load(r + gridDim.x * SC_ROWS, v);
   }
 }
 
@@ -921,12 +934,14 @@ extern "C" int drb_moe_prefill_layer(const drb_moe_layer* w, const drb_prefill_b
                                                    static_cast<const __nv_bfloat16*>(w->router), b->logit_bias, b->logits, rows, e + 1,
                                                    b->logit_bias ? 1.f : 0.f, b->counts, e, st);
   if (r != 0) return r;
+  // The pairs' ranks: two warps read each, so they do not share slot_of's place; act is free until the gate/up kernel writes it.
+  int* rank = reinterpret_cast<int*>(b->act);
   drb_launch(router::k_moe_topk<true>, dim3(rows), dim3(router::THREADS), 0, st, dev.pdl, (const float*)b->logits, e, topk, e + 1, b->idx, b->wts,
-             b->sgate, b->counts, b->slot_of);
-  const int blocks = (rows + 7) / 8;
-  drb_launch(pf::k_scatter_rows, dim3(blocks < 2 * dev.sms ? blocks : 2 * dev.sms), dim3(256), 0, st, dev.pdl, (const __half*)b->rows16,
-             (const int*)b->idx, rows, topk, (const int*)b->counts, e, b->offsets, b->slot_of, b->row_of, reinterpret_cast<unsigned char*>(b->y),
-             reinterpret_cast<unsigned char*>(b->sh_out));
+             b->sgate, b->counts, rank);
+  const int blocks = (rows + pf::SC_ROWS - 1) / pf::SC_ROWS;
+  drb_launch(pf::k_scatter_rows, dim3(blocks < 8 * dev.sms ? blocks : 8 * dev.sms), dim3(pf::SC_THREADS), 0, st, dev.pdl, (const __half*)b->rows16,
+             (const int*)b->idx, rows, topk, (const int*)b->counts, e, b->offsets, b->slot_of, (const int*)rank, b->row_of,
+             reinterpret_cast<unsigned char*>(b->y), reinterpret_cast<unsigned char*>(b->sh_out));
   pft::Block k = {};
   k.gu_w = w->gu_q, k.gu_s = w->gu_sm, k.d_w = w->d_q, k.d_s = w->d_sm;
   k.sgu_q = w->sgu_q, k.sgu_s = w->sgu_s, k.sd_q = w->sd_q, k.sd_s = w->sd_s;

@@ -66,9 +66,9 @@ constexpr int SET_BYTES = (MAX_E + 2) * 4 + 8;
 constexpr int TOKEN_STRIDE = 2 * H * 2;         // bytes between prepared token rows (k_prep_rows): fp16 row | factor
 
 struct Tab {  // one work item
-  int cols, mt, shared;         // accumulator columns (the MMA's N)
+  int cols, used, mt, shared;   // accumulator columns (the MMA's N); those in use, in eights
   int full, srow, start;        // contiguous rows: so many boxes of eight from row srow on, and one more from row start (-1: none)
-  int quads, pad;               // rows fetched by number: so many fours of rows[], behind the boxes
+  int quads;                    // rows fetched by number: so many fours of rows[], behind the boxes
   __align__(16) int rows[MAX_NT];
   __align__(16) int dst[MAX_NT];    // result row of each column, -1: none
   __align__(16) float fac[MAX_NT];  // what the column's token row was divided by
@@ -103,6 +103,8 @@ struct Smem {
 // A nibble in bits 0..3 of a 16-bit half, or-ed into 0x6400, is the half 1024 + q; a nibble in bits 4..7, or-ed into
 // 0x5400, is the half 64 + q (the unit in the last place of 64 is 1/16). Subtracting the offset is exact, the fused
 // multiply-add q*s + m rounds once.
+// A nibble in bits 4..7 with nothing above it is the subnormal half q * 2^-20: with the scale times 2^20 (exact, while it stays
+// below 2^-4) the fused multiply-add needs no subtraction and rounds the same number.
 // The offsets live in registers the compiler cannot rebuild from immediates: it would, once per use.
 struct NibbleConst {
   uint32_t k1024, k64, mixed;  // (1024, 1024), (64, 64), (1024, 64)
@@ -122,14 +124,22 @@ DRB_DEV uint32_t sub_fma(uint32_t t, uint32_t off, __half2 s2, __half2 m2) {
   const __half2 r = __hfma2(__hsub2(*reinterpret_cast<const __half2*>(&t), *reinterpret_cast<const __half2*>(&off)), s2, m2);
   return *reinterpret_cast<const uint32_t*>(&r);
 }
-// Eight nibbles of one word in the order (0,4) (1,5) (2,6) (3,7): one shift serves both upper pairs, 13 instructions. The
-// token rows have to come in the same order.
-DRB_DEV void dequant8_perm(uint32_t w, __half2 s2, __half2 m2, const NibbleConst& c, uint32_t* o) {
+// Eight nibbles of one word in the order (0,4) (1,5) (2,6) (3,7): one shift serves both upper pairs; 13 instructions, SMALL
+// (every scale of the warp below 2^-4): 11. The token rows have to come in the same order. Issue slots are what the conversion
+// runs out of; the fp16 and the integer pipe take one instruction every other cycle each, and get six and five of the eleven.
+template <bool SMALL>
+DRB_DEV void dequant8_perm(uint32_t w, __half2 s2, __half2 m2, __half2 big, const NibbleConst& c, uint32_t* o) {
   const uint32_t w8 = w >> 8;
+  auto upper = [&](uint32_t v) {
+    if (!SMALL) return sub_fma(mask_or<0x00F000F0u>(v, c.k64), c.k64, s2, m2);
+    const uint32_t t = v & 0x00F000F0u;
+    const __half2 r = __hfma2(*reinterpret_cast<const __half2*>(&t), big, m2);
+    return *reinterpret_cast<const uint32_t*>(&r);
+  };
   o[0] = sub_fma(mask_or<0x000F000Fu>(w, c.k1024), c.k1024, s2, m2);
-  o[1] = sub_fma(mask_or<0x00F000F0u>(w, c.k64), c.k64, s2, m2);
+  o[1] = upper(w);
   o[2] = sub_fma(mask_or<0x000F000Fu>(w8, c.k1024), c.k1024, s2, m2);
-  o[3] = sub_fma(mask_or<0x00F000F0u>(w8, c.k64), c.k64, s2, m2);
+  o[3] = upper(w8);
 }
 // The same in k order: a byte holds a consecutive pair, a permute puts it into both halves. 16 instructions.
 DRB_DEV void dequant8_nat(uint32_t w, __half2 s2, __half2 m2, const NibbleConst& c, uint32_t* o) {
@@ -224,6 +234,9 @@ __global__ void __launch_bounds__(256)
     }
   }
 }
+
+// SiLU for a result that is rounded to fp16: the division within 2 units of the last fp32 place.
+DRB_DEV float silu_fast(float x) { return __fdividef(x, 1.f + expf(-x)); }
 
 // ---- the grouped GEMM ----------------------------------------------------------------------------------------------
 // A position in a ring of N mbarriers and the parity its next completion has there, moved without a division: a convert
@@ -411,12 +424,23 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
             const __half2 s2 = __half2half2(__low2half(sm)), m2 = __half2half2(__high2half(sm));
             const uint32_t w[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
             uint32_t o[32];
+            if (!PERM && GEMM == 0) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              if (PERM || GEMM == 1) dequant8_perm(w[j], s2, m2, nc, o + 4 * j);
-              else dequant8_nat(w[j], s2, m2, nc, o + 4 * j);
+              for (int j = 0; j < 8; ++j) dequant8_nat(w[j], s2, m2, nc, o + 4 * j);
+              tmem_st32(acol + ra.i * A_COLS + g * 32, o);
+            } else {
+              const __half2 k1024 = __half2half2(__ushort_as_half((unsigned short)0x6400));
+              const __half2 big = __hmul2(__hmul2(s2, k1024), k1024);
+              if (__all_sync(0xffffffffu, __hlt(__habs(__low2half(sm)), __ushort_as_half((unsigned short)0x2C00)))) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) dequant8_perm<true>(w[j], s2, m2, big, nc, o + 4 * j);
+                tmem_st32(acol + ra.i * A_COLS + g * 32, o);
+              } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) dequant8_perm<false>(w[j], s2, m2, big, nc, o + 4 * j);
+                tmem_st32(acol + ra.i * A_COLS + g * 32, o);
+              }
             }
-            tmem_st32(acol + ra.i * A_COLS + g * 32, o);
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(&ctl.rawempty[rr.i]);
@@ -624,7 +648,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
         const int slot = srow + min(8 * full + t, nt - 1);
         tab.rows[t] = (GEMM == 0 && !PREP && !it.shared && a.row_of) ? __ldg(a.row_of + slot) : slot;
       }
-      if (lane == 0) tab.cols = cols, tab.mt = it.mt, tab.shared = it.shared, tab.full = full, tab.srow = srow, tab.start = start, tab.quads = quads;
+      if (lane == 0) tab.cols = cols, tab.used = (start >= 0 ? 8 * full + 8 : nt + 7) & ~7, tab.mt = it.mt, tab.shared = it.shared, tab.full = full, tab.srow = srow, tab.start = start, tab.quads = quads;
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl.tabfull[rt.i]);
       rt.next();
@@ -639,7 +663,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
     for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
       wait_at(ctl.tabfull, rt, DRB_ERR_FULL_WAIT, dead);
       const Tab& tab = tabs[rt.i];
-      const int cols = tab.cols, mt = tab.mt;
+      const int cols = FMT == 1 ? tab.cols : tab.used, mt = tab.mt;
       const bool sh = tab.shared != 0;
       float sum[FMT == 1 ? NT : 1];  // FP8: the columns' sums over the accumulators
       if (FMT == 1) {
@@ -677,9 +701,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
       __half* const act = static_cast<__half*>(sh ? a.sh_dst : a.dst) + (FMT == 0 ? perm_pos(j) : j);
       float* const y = static_cast<float*>(sh ? a.sh_dst : a.dst) + mt * TILE_M + r;
       const bool odd = lane & 1;
-      auto columns = [&](int c0, const uint32_t(&v)[16]) {  // the results of sixteen columns
+      auto columns = [&](int c0, const uint32_t(&v)[8]) {  // the results of eight columns
 #pragma unroll
-        for (int i4 = 0; i4 < 16; i4 += 4) {
+        for (int i4 = 0; i4 < 8; i4 += 4) {
           const int4 d4 = *reinterpret_cast<const int4*>(&tab.dst[c0 + i4]);
           const int dst[4] = {d4.x, d4.y, d4.z, d4.w};
           if (GEMM == 0) {
@@ -693,7 +717,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
               const float got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
               const int dt = odd ? dst[i + 1] : dst[i];
               const float f = odd ? fac[i + 1] : fac[i];
-              if (dt >= 0) act[(size_t)dt * I] = f2h_sat(silu_f((odd ? got : v0) * f) * ((odd ? v1 : got) * f));
+              if (dt >= 0) act[(size_t)dt * I] = f2h_sat(silu_fast((odd ? got : v0) * f) * ((odd ? v1 : got) * f));
             }
           } else {
 #pragma unroll
@@ -712,19 +736,19 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
       };
       if (FMT == 1) {
 #pragma unroll
-        for (int c0 = 0; c0 < NT; c0 += 16)
+        for (int c0 = 0; c0 < NT; c0 += 8)
           if (c0 < cols) {
-            uint32_t v[16];
+            uint32_t v[8];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(sum[FMT == 1 ? c0 + i : 0]);
+            for (int i = 0; i < 8; ++i) v[i] = __float_as_uint(sum[FMT == 1 ? c0 + i : 0]);
             columns(c0, v);
           }
       } else {
 #pragma unroll 1
-        for (int c0 = 0; c0 < cols; c0 += 16) {
-          uint32_t v[16];
-          tmem_ld16(acc + (uint32_t)c0, v);
-          if (c0 + 16 >= cols) {  // everything is in registers: the accumulator is free
+        for (int c0 = 0; c0 < cols; c0 += 8) {
+          uint32_t v[8];
+          tmem_ld8(acc + (uint32_t)c0, v);
+          if (c0 + 8 >= cols) {  // everything is in registers: the accumulator is free
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&ctl.accfree[rc.i]);
