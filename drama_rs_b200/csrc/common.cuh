@@ -123,17 +123,23 @@ DRB_DEV bool mbar_wait(uint64_t* bar, unsigned parity, unsigned err_code, unsign
 // to every hand-over of the ring), and each poll may suspend the warp in hardware for up to 2 us: a warp that polls takes
 // issue slots from the ones that work (measured in the grouped GEMMs: half of all instructions issued). Bounded all the same.
 DRB_DEV bool mbar_wait_hot(uint64_t* bar, unsigned parity, unsigned err_code) {
-  for (unsigned it = 0; it < (1u << 20); ++it) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(2000u)
-        : "memory");
-    if (ok) return true;
-  }
+  unsigned ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .u32 n;\n\t"
+      "mov.u32 n, 0;\n"
+      "WAIT_AGAIN:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "@p bra WAIT_OVER;\n\t"
+      "add.u32 n, n, 1;\n\t"
+      "setp.lt.u32 p, n, 1048576;\n\t"
+      "@p bra WAIT_AGAIN;\n\t"
+      "setp.ne.u32 p, n, n;\n"
+      "WAIT_OVER:\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(2000u)
+      : "memory");
+  if (ok) return true;
   atomicMax(&g_drb_error, err_code);
   return false;
 }

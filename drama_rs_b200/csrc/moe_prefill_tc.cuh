@@ -238,6 +238,21 @@ __global__ void __launch_bounds__(256)
 // SiLU for a result that is rounded to fp16: the division within 2 units of the last fp32 place.
 DRB_DEV float silu_fast(float x) { return __fdividef(x, 1.f + expf(-x)); }
 
+DRB_DEV void lds128(uint32_t addr, uint32_t* v) {
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
+}
+DRB_DEV void lds64(uint32_t addr, uint32_t& a, uint32_t& b) {
+  asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "r"(addr) : "memory");
+}
+DRB_DEV __half2 dup_low(uint32_t v) {
+  const uint32_t r = prmt(v, 0u, 0x1010u);
+  return *reinterpret_cast<const __half2*>(&r);
+}
+DRB_DEV __half2 dup_high(uint32_t v) {
+  const uint32_t r = prmt(v, 0u, 0x3232u);
+  return *reinterpret_cast<const __half2*>(&r);
+}
+
 // ---- the grouped GEMM ----------------------------------------------------------------------------------------------
 // A position in a ring of N mbarriers and the parity its next completion has there, moved without a division: a convert
 // warp's step is 104 instructions of conversion, and index arithmetic had grown to 60 more.
@@ -387,6 +402,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
     const uint32_t acol = tmem + ((uint32_t)(q4 * 32) << 16) + A_COL0 + half * 64;
     const unsigned char* xrow = raw + swz_off(r, 0);  // piece p of the row stands at xrow + piece(p)
     auto piece = [&](int p) { return (((r & 7) ^ p) - (r & 7)) << 4; };
+    const uint32_t x_row = smem_u32(raw) + swz_off(r, 4 * half);  // int4: this thread's first piece
     Ring<NRAW> rr;     // raw stages
     Ring<NST> ra;      // stages; every one starts free
     ra.par = 1;
@@ -406,41 +422,45 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
     for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
       const Item it = decode(item);
       if (FMT == 0 && !it.shared) {
-        // (scale, min) of this row's groups 4 step + 2 half, + 1
         wait_at(ctl.smfull, rs, DRB_ERR_FULL_WAIT, dead);
-        const unsigned char* smp = smbuf + rs.i * SMB + (GEMM == 0 ? swz_off(r, 0) : r * 32) + 8 * half;
+        // (scale, min) of this row's groups 4 step + 2 half, + 1: gate/up: piece `step` of a swizzled row; down: 16 bytes a step
+        const uint32_t sm_a = smem_u32(smbuf) + rs.i * SMB + (GEMM == 0 ? swz_off(r, 0) : r * 32) + 8 * half;
         rs.next();
         rr.next(group);
 #pragma unroll 1
         for (int step = group; step < NSTEP; step += 2) {
           wait_at(ctl.rawfull, rr, DRB_ERR_FULL_WAIT, dead);
-          const unsigned char* xp = xrow + rr.i * RAW_BYTES;
-          const unsigned char* gp = smp + (GEMM == 0 ? piece(step) : 16 * step);
+          // piece 4 half + j of the row stands at xa ^ 16 j: in the swizzled row the piece's number is xor-ed into the address
+          uint32_t xa = x_row + rr.i * RAW_BYTES;
+          uint32_t sm[2];
+          lds64(GEMM == 0 ? sm_a ^ (step << 4) : sm_a + 16 * step, sm[0], sm[1]);
+          const bool small = __all_sync(0xffffffffu, max(sm[0] & 0x7fffu, sm[1] & 0x7fffu) < 0x2C00u);  // both scales below 2^-4
           a_wait();
+          uint32_t to = acol + ra.i * A_COLS;
 #pragma unroll 1
           for (int g = 0; g < 2; ++g) {
-            const uint4 x0 = *reinterpret_cast<const uint4*>(xp + piece(4 * half + 2 * g)), x1 = *reinterpret_cast<const uint4*>(xp + piece(4 * half + 2 * g + 1));
-            const __half2 sm = *reinterpret_cast<const __half2*>(gp + 4 * g);
-            const __half2 s2 = __half2half2(__low2half(sm)), m2 = __half2half2(__high2half(sm));
-            const uint32_t w[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+            uint32_t w[8];
+            lds128(xa, w), lds128(xa ^ 16u, w + 4);
+            xa ^= 32u;
+            const __half2 s2 = dup_low(sm[0]), m2 = dup_high(sm[0]);
+            sm[0] = sm[1];
             uint32_t o[32];
             if (!PERM && GEMM == 0) {
 #pragma unroll
               for (int j = 0; j < 8; ++j) dequant8_nat(w[j], s2, m2, nc, o + 4 * j);
-              tmem_st32(acol + ra.i * A_COLS + g * 32, o);
-            } else {
-              const __half2 k1024 = __half2half2(__ushort_as_half((unsigned short)0x6400));
+              tmem_st32(to, o);
+            } else if (small) {
+              const __half2 k1024 = *reinterpret_cast<const __half2*>(&nc.k1024);
               const __half2 big = __hmul2(__hmul2(s2, k1024), k1024);
-              if (__all_sync(0xffffffffu, __hlt(__habs(__low2half(sm)), __ushort_as_half((unsigned short)0x2C00)))) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) dequant8_perm<true>(w[j], s2, m2, big, nc, o + 4 * j);
-                tmem_st32(acol + ra.i * A_COLS + g * 32, o);
-              } else {
+              for (int j = 0; j < 8; ++j) dequant8_perm<true>(w[j], s2, m2, big, nc, o + 4 * j);
+              tmem_st32(to, o);
+            } else {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) dequant8_perm<false>(w[j], s2, m2, big, nc, o + 4 * j);
-                tmem_st32(acol + ra.i * A_COLS + g * 32, o);
-              }
+              for (int j = 0; j < 8; ++j) dequant8_perm<false>(w[j], s2, m2, s2, nc, o + 4 * j);
+              tmem_st32(to, o);
             }
+            to += 32;
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(&ctl.rawempty[rr.i]);
