@@ -15,16 +15,21 @@
 
 namespace gemv {
 
-constexpr int RING_BYTES = 128 * 1024;
+// Two blocks per multiprocessor: a kernel launched behind another (programmatic dependent launch) then becomes resident while
+// its predecessor still runs and fills its ring, up to 15 MB chip-wide, before its input exists. With one block of
+// 128 KB per multiprocessor every launch began with an idle memory system (a chain of 33 projections of 7 MB to 25 MB each
+// took 258 us, against 68 us for its bytes).
+constexpr int BLOCK_BYTES = 113 * 1024;
 constexpr int MAX_STAGES = 8;
+constexpr int PART_ROWS = 64;  // at most so many outputs whose partial sums wait for the other warps' parts of K
 
 enum Mode { Q8_PLAIN = 0, Q8_SWIGLU = 1, BF16_PLAIN = 2 };
 
-struct Smem {
+struct alignas(128) Smem {
   uint64_t full[MAX_STAGES];
   uint64_t empty[MAX_STAGES];
-  float red[64];      // cross-warp partials (K split over several warps, or the norm's sum of squares)
-  float inv_rms;
+  float red[16];      // the norm's sum of squares
+  float part[PART_ROWS * 4 * 2];  // K split over several warps: [output][segment][weight row]
 };
 
 // Named barrier over the consumer warps only (the producer warp never joins).
@@ -33,7 +38,7 @@ DRB_DEV void consumer_sync(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(t
 // KSEG: elements of K one warp covers (512 or 2048). NSEG: warps that share a row (K = KSEG * NSEG).
 // RPW: rows a warp handles per stage. CW: consumer warps.
 template <int KSEG, int NSEG, int RPW, int CW, int MODE>
-__global__ void __launch_bounds__((CW + 1) * 32, 1)
+__global__ void __launch_bounds__((CW + 1) * 32, 2)
     k_gemv(const void* __restrict__ Wv, const __half* __restrict__ S, const float* __restrict__ x, const float* res,
            float* y, int N, const float* __restrict__ nw, float eps, const char* pf, size_t pf_bytes) {
   constexpr int K = KSEG * NSEG;
@@ -47,15 +52,18 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1)
   constexpr int SROW = MODE == BF16_PLAIN ? 0 : (K / 128) * 2;  // bytes of group scales per weight row
   constexpr bool S_IN_STAGE = SROW >= 16;                     // bulk copies need 16-byte granules
   constexpr int STAGE_BYTES = RB * U * (ROW_BYTES + (S_IN_STAGE ? SROW : 0));
+  constexpr int RING_BYTES = BLOCK_BYTES - (int)sizeof(Smem) - K * 4;
   constexpr int STAGES = RING_BYTES / STAGE_BYTES < MAX_STAGES ? RING_BYTES / STAGE_BYTES : MAX_STAGES;
   constexpr int NT = CW * 32;
+  constexpr int PR = PART_ROWS / RB * RB;                    // whole stages of partial sums
+  constexpr int XV = (K / 4 + NT - 1) / NT;                  // float4s of the input per consumer thread
   static_assert(STAGES >= 2, "ring too small");
   static_assert(NCH >= 1, "segment too small");
 
   extern __shared__ __align__(128) unsigned char dyn[];
   Smem& sm = *reinterpret_cast<Smem*>(dyn);
-  float4* xs4 = reinterpret_cast<float4*>(dyn + 1024);
-  unsigned char* ring = dyn + 1024 + K * 4;
+  float4* xs4 = reinterpret_cast<float4*>(dyn + sizeof(Smem));
+  unsigned char* ring = dyn + sizeof(Smem) + K * 4;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned G = gridDim.x, b = blockIdx.x;
@@ -98,36 +106,46 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1)
   }
 
   // ---------------- consumers
+  // The norm weights are constants: requested before the input may be read. Whole warps own a float4 index or skip it.
+  float4 wv[XV], xv[XV];
+#pragma unroll
+  for (int j = 0; j < XV; ++j) {
+    const int i = threadIdx.x + j * NT;
+    wv[j] = nw && i < K / 4 ? __ldg(reinterpret_cast<const float4*>(nw) + i) : make_float4(1.f, 1.f, 1.f, 1.f);
+  }
   pdl_wait();  // x and res come from the previous kernel
+#pragma unroll
+  for (int j = 0; j < XV; ++j) {
+    const int i = threadIdx.x + j * NT;
+    xv[j] = i < K / 4 ? __ldcg(reinterpret_cast<const float4*>(x) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
   const int seg = warp % NSEG, rg = warp / NSEG;
   float inv = 1.f;
   if (nw) {
     float ss = 0.f;
-    const float4* x4 = reinterpret_cast<const float4*>(x);
-    for (int i = threadIdx.x; i < K / 4; i += NT) {
-      const float4 v = __ldcg(x4 + i);
-      ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-    }
+#pragma unroll
+    for (int j = 0; j < XV; ++j) ss += xv[j].x * xv[j].x + xv[j].y * xv[j].y + xv[j].z * xv[j].z + xv[j].w * xv[j].w;
     ss = warp_sum(ss);
-    if (lane == 0) sm.red[32 + warp] = ss;
+    if (lane == 0) sm.red[warp] = ss;
     consumer_sync(NT);
     float t = 0.f;
 #pragma unroll
-    for (int w = 0; w < CW; ++w) t += sm.red[32 + w];
+    for (int w = 0; w < CW; ++w) t += sm.red[w];
     inv = rsqrtf(t / K + eps);
   }
-  // Stage the (normalised) activations once per block: coalesced read, then either a swizzled float4 store
-  // (bf16 weights keep fp32 activations) or conversion to limb blocks of 16 values (int8 weights, dp4a).
-  // Chunk c = lane + 32*i of the segment covers k = seg*KSEG + EPC*c ...; whole warps enter or skip the loop.
+  // Stage the (normalised) activations once per block: a swizzled float4 store (bf16 weights keep fp32 activations) or
+  // conversion to limb blocks of 16 values (int8 weights, dp4a).
+  // Chunk c = lane + 32*i of the segment covers k = seg*KSEG + EPC*c ....
   unsigned char* qb = reinterpret_cast<unsigned char*>(xs4);
-  for (int i = threadIdx.x; i < K / 4; i += NT) {
-    float4 v = __ldcg(reinterpret_cast<const float4*>(x) + i);
-    if (nw) {
-      const float4 w = reinterpret_cast<const float4*>(nw)[i];
-      v = make_float4(v.x * inv * w.x, v.y * inv * w.y, v.z * inv * w.z, v.w * inv * w.w);
+#pragma unroll
+  for (int j = 0; j < XV; ++j) {
+    const int i = threadIdx.x + j * NT;
+    if (i < K / 4) {
+      float4 v = xv[j];
+      if (nw) v = make_float4(v.x * inv * wv[j].x, v.y * inv * wv[j].y, v.z * inv * wv[j].z, v.w * inv * wv[j].w);
+      if (MODE == BF16_PLAIN) xs4[swz4(i)] = v;
+      else quant_store_nat(qb, i, v, true);
     }
-    if (MODE == BF16_PLAIN) xs4[swz4(i)] = v;
-    else quant_store_nat(qb, i, v, true);
   }
   consumer_sync(NT);
   unsigned long long xp[MODE == BF16_PLAIN ? NCH * EPC / 2 : 1];
@@ -153,6 +171,9 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1)
     const int r0 = u0 + c * RB;
     const int nr = min(RB, u1 - r0);
     const unsigned char* st = ring + (size_t)s * STAGE_BYTES;
+    float rv[RPW];  // the residual, requested before the wait as well
+#pragma unroll
+    for (int p = 0; p < RPW; ++p) rv[p] = (res && NSEG == 1 && p * RG + rg < nr) ? __ldcg(res + r0 + p * RG + rg) : 0.f;
     // Group scales come straight from global memory; issue them before waiting on the copy.
     float sc[RPW][U][NCH];
     if (MODE != BF16_PLAIN) {
@@ -214,30 +235,36 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1)
       if (NSEG == 1) {
         if (lane == 0 && lr < nr) {
           const int row = r0 + lr;
-          y[row] = U == 2 ? silu_f(d[0]) * d[U - 1] : d[0] + (res ? __ldcg(res + row) : 0.f);
+          y[row] = U == 2 ? silu_f(d[0]) * d[U - 1] : d[0] + rv[p];
         }
-      } else {
-        // K is split over NSEG warps: combine their partial sums in segment order.
-        if (lane == 0) {
-          sm.red[(rg * NSEG + seg) * 2] = d[0];
-          sm.red[(rg * NSEG + seg) * 2 + 1] = d[U - 1];
-        }
-        consumer_sync(CW * 32);
-        if (seg == 0 && lane == 0 && lr < nr) {
-          float t0 = 0.f, t1 = 0.f;
-#pragma unroll
-          for (int q = 0; q < NSEG; ++q) {
-            t0 += sm.red[(rg * NSEG + q) * 2];
-            t1 += sm.red[(rg * NSEG + q) * 2 + 1];
-          }
-          const int row = r0 + lr;
-          y[row] = U == 2 ? silu_f(t0) * t1 : t0 + (res ? __ldcg(res + row) : 0.f);
-        }
-        consumer_sync(CW * 32);
+      } else if (lane == 0 && lr < nr) {  // K is split over NSEG warps: their partial sums meet in shared memory
+        float* pp = sm.part + ((r0 + lr - u0) % PR * NSEG + seg) * U;
+        pp[0] = d[0];
+        if (U == 2) pp[1] = d[1];
       }
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(&sm.empty[s]);
+    if (NSEG > 1) {
+      static_assert(NSEG <= 4 && PART_ROWS <= NT, "one thread per output");
+      const int done = r0 + nr - u0;  // outputs so far: added up and written every PR, in segment order
+      if (done % PR == 0 || c == nchunks - 1) {
+        const int first = (done - 1) / PR * PR, n = done - first;
+        float add = 0.f;
+        if (res && (int)threadIdx.x < n) add = __ldcg(res + u0 + first + threadIdx.x);
+        consumer_sync(NT);
+        if ((int)threadIdx.x < n) {
+          float t0 = 0.f, t1 = 0.f;
+#pragma unroll
+          for (int q = 0; q < NSEG; ++q) {
+            t0 += sm.part[(threadIdx.x * NSEG + q) * U];
+            if (U == 2) t1 += sm.part[(threadIdx.x * NSEG + q) * U + 1];
+          }
+          y[u0 + first + threadIdx.x] = U == 2 ? silu_f(t0) * t1 : t0 + add;
+        }
+        consumer_sync(NT);
+      }
+    }
   }
 }
 
@@ -248,8 +275,9 @@ constexpr size_t smem_bytes() {
   constexpr int U = MODE == Q8_SWIGLU ? 2 : 1;
   constexpr int SROW = MODE == BF16_PLAIN ? 0 : (K / 128) * 2;
   constexpr int STAGE = (CW / NSEG) * RPW * U * (K * ESZ + (SROW >= 16 ? SROW : 0));
+  constexpr int RING_BYTES = BLOCK_BYTES - (int)sizeof(Smem) - K * 4;
   constexpr int STAGES = RING_BYTES / STAGE < MAX_STAGES ? RING_BYTES / STAGE : MAX_STAGES;
-  return 1024 + (size_t)K * 4 + (size_t)STAGES * STAGE;
+  return sizeof(Smem) + (size_t)K * 4 + (size_t)STAGES * STAGE;
 }
 
 template <int KSEG, int NSEG, int RPW, int CW, int MODE>
