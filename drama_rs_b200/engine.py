@@ -22,7 +22,7 @@ from typing import Callable, Optional
 import numpy as np
 
 from . import ffi
-from .gpu import DevBuf, Graph, Stream, check, launched
+from .gpu import DevBuf, Graph, HostRow, Stream, check, launched
 from .model import MoeLayer
 
 NULL = C.c_void_p(0)
@@ -60,6 +60,7 @@ class MoeDecoder:
         f32 = 4
         self.idx_trace = DevBuf(len(layers) * topk * 4) if trace_routing else None
         self.x = DevBuf((h) * f32)
+        self.row = HostRow(h, self.st)
         self.rlog = DevBuf((e + 1) * f32)
         self.idx = DevBuf(topk * 4)
         self.wts = DevBuf(topk * f32)
@@ -132,17 +133,17 @@ class MoeDecoder:
         self.graph = Graph(self.st, self.record_step)
 
     def set_x(self, x: np.ndarray) -> None:
-        self.x.upload(x.astype(np.float32), self.st)
+        self.row.put(self.x, x)
 
     def step(self) -> np.ndarray:
         """Replays the captured step on the current x and returns the new hidden state."""
         assert self.graph is not None, "capture first"
         self.graph.launch(self.st)
-        return self.x.download(np.float32, self.hidden, self.st)
+        return self.row.get(self.x)
 
     def step_eager(self) -> np.ndarray:
         self.record_step()
-        return self.x.download(np.float32, self.hidden, self.st)
+        return self.row.get(self.x)
 
     def routing_trace(self) -> np.ndarray:
         assert self.idx_trace is not None
@@ -325,6 +326,7 @@ class MoeStackDecoder:
                         ly.shared_gate_up.q.ptr, ly.shared_gate_up.s.ptr, ly.shared_down.q.ptr, ly.shared_down.s.ptr]
         self.table = DevBuf.from_array(table, self.st)
         self.x = DevBuf(self.hidden * 4)
+        self.row = HostRow(self.hidden, self.st)
         self.ws = DevBuf.zeros(self.l.drb_moe_stack_workspace_bytes(), self.st)
         self.idx_trace = DevBuf(len(layers) * topk * 4)
         self.wts_trace = DevBuf(len(layers) * topk * 4)
@@ -340,14 +342,14 @@ class MoeStackDecoder:
         self.graph = Graph(self.st, self.launch)
 
     def set_x(self, x: np.ndarray) -> None:
-        self.x.upload(x.astype(np.float32), self.st)
+        self.row.put(self.x, x)
 
     def step(self) -> np.ndarray:
         if self.graph is not None:
             self.graph.launch(self.st)
         else:
             self.launch()
-        return self.x.download(np.float32, self.hidden, self.st)
+        return self.row.get(self.x)
 
     def routing(self) -> tuple[np.ndarray, np.ndarray]:
         n = len(self.layers) * self.topk

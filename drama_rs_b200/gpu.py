@@ -127,6 +127,47 @@ class Graph:
             self.exec = C.c_void_p()
 
 
+class HostRow:
+    """A row of floats that crosses between the host and the front of a device buffer on every step. Both directions go
+    through pinned memory of the row's own, so that the copies are queued behind one another and the host waits once, for the
+    result (pageable memory made every step two staged copies with a wait each: 146 us a step of 112 us of kernels, 133 so).
+    Copies by a kernel of one block, in a graph or beside it, and a word in pinned memory that the host watches instead of
+    the stream measured the same or slower."""
+
+    def __init__(self, count: int, st: Stream) -> None:
+        self._l, self._st = ffi.lib(), st
+        self._p = C.c_void_p()
+        check(self._l.dr_host_alloc(C.byref(self._p), 8 * count), "host_alloc")
+        both = np.frombuffer((C.c_float * (2 * count)).from_address(self._p.value), dtype=np.float32)
+        self._in, self._out, self._out_p = both[:count], both[count:], C.c_void_p(self._p.value + 4 * count)
+        self._queued = False  # a copy out of _in may still be under way
+
+    def put(self, dev, x: np.ndarray) -> None:
+        n = x.size
+        assert n <= self._in.size and 4 * n <= dev.nbytes
+        if self._queued:
+            self._st.sync()
+        np.copyto(self._in if n == self._in.size else self._in[:n], x.reshape(-1))
+        self._queued = True
+        check(self._l.dr_h2d(dev.ptr, self._p, 4 * n, self._st.raw), "h2d")
+
+    def get(self, dev) -> np.ndarray:
+        check(self._l.dr_d2h(self._out_p, dev.ptr, 4 * self._out.size, self._st.raw), "d2h")
+        self._st.sync()
+        self._queued = False
+        return self._out.copy()
+
+    def __del__(self) -> None:
+        try:
+            if self._p:
+                if self._queued:
+                    self._st.sync()
+                self._l.dr_host_free(self._p)
+                self._p = C.c_void_p()
+        except Exception:
+            pass
+
+
 class ExtBuf:
     """Device memory owned by someone else (for example a torch tensor), seen through DevBuf's interface."""
 
