@@ -27,6 +27,17 @@ namespace gemv {
 
 constexpr int BLOCK_BYTES = 112 * 1024;  // two blocks per multiprocessor
 
+// The caller's prefetch hint. With overlapping launches a successor fills its rings itself as soon as its blocks are resident
+// (about `skip` bytes of each block's share); asked for here as well, the same lines twice, it slowed both (a chain of 33
+// projections 135 us instead of 129). So what lies behind them is prefetched, and no more than 128 KB per block: a
+// vocabulary-sized region would only push out what the running kernels still read.
+DRB_DEV void prefetch_hint(const char* pf, size_t pf_bytes, unsigned skip, unsigned block, unsigned blocks) {
+  if (skip == 0) return prefetch_share(pf, pf_bytes, block, blocks);
+  const size_t per = pf_bytes / blocks;
+  if (pf && per > skip) prefetch_share(pf + block * per + skip, per - skip < 131072 ? per - skip : 131072, 0, 1);
+}
+constexpr unsigned HINT_SKIP = 96 * 1024;
+
 // ---- int8 weights -----------------------------------------------------------------------------------------------------
 namespace q8 {
 
@@ -71,7 +82,7 @@ DRB_DEV void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t
 template <int K, int U>
 __global__ void __launch_bounds__(THREADS, 2)
     k_gemv(const int8_t* __restrict__ W, const __half* __restrict__ S, const float* __restrict__ x, const float* res, float* y, int N,
-           const float* __restrict__ nw, float eps, const char* pf, size_t pf_bytes) {
+           const float* __restrict__ nw, float eps, const char* pf, size_t pf_bytes, unsigned pf_skip) {
   using P = Shape<K, U>;
   constexpr int STAGES = P::STAGES, NSEG = P::NSEG, KW = P::KW, RS = P::RS, ROWS = P::ROWS, SEG = P::SEG, PITCH = P::PITCH, SROW = P::SROW;
   constexpr int SLOTS = P::S_SLOTS ? P::S_SLOTS : 1;
@@ -119,7 +130,7 @@ __global__ void __launch_bounds__(THREADS, 2)
           if (++s == STAGES) s = 0, par ^= 1u;
         }
       }
-      prefetch_share(pf, pf_bytes, b, G);
+      prefetch_hint(pf, pf_bytes, pf_skip, b, G);
     }
     return;
   }
@@ -136,6 +147,12 @@ __global__ void __launch_bounds__(THREADS, 2)
   uint32_t par = 0;
   uint4 v0, v1, w0, w1;  // rows g and g + 8 of the tile, two pieces each
   __half sc0 = __half(), sc1 = __half();
+  auto release = [&]() {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&ctl.empty[s]);
+    if (++s == STAGES) s = 0, par ^= 1u;
+  };
+  auto operand = [&]() { return ring + s * P::STAGE_BYTES + (sub * 16 + g) * PITCH + kw * GROUP + 16 * t4; };
   auto load = [&](int t, int q) {
     if (!P::S_COPY) {
       const int row = u0 + t * OUT + sub * 16 + g;
@@ -143,21 +160,19 @@ __global__ void __launch_bounds__(THREADS, 2)
       sc1 = row + 8 < u1 ? __ldg(S + (size_t)(row + 8) * (K / GROUP) + kw) : __half();
     }
     if (!dead) dead = !mbar_wait_hot(&ctl.full[s], par, DRB_ERR_FULL_WAIT);
-    const unsigned char* rp = ring + s * P::STAGE_BYTES + (sub * 16 + g) * PITCH + kw * GROUP + 16 * t4;
-    v0 = *reinterpret_cast<const uint4*>(rp), v1 = *reinterpret_cast<const uint4*>(rp + 64);
-    w0 = *reinterpret_cast<const uint4*>(rp + 8 * PITCH), w1 = *reinterpret_cast<const uint4*>(rp + 8 * PITCH + 64);
+    const unsigned char* rp = operand();
+    v0 = *reinterpret_cast<const uint4*>(rp), w0 = *reinterpret_cast<const uint4*>(rp + 8 * PITCH);
+    if (EARLY) v1 = *reinterpret_cast<const uint4*>(rp + 64), w1 = *reinterpret_cast<const uint4*>(rp + 8 * PITCH + 64);
     if (P::S_COPY) {
       const unsigned char* sp = scales + (t % SLOTS * ROWS + sub * 16 + g) * SROW + 2 * (q * KW + kw);
       sc0 = *reinterpret_cast<const __half*>(sp), sc1 = *reinterpret_cast<const __half*>(sp + 8 * SROW);
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&ctl.empty[s]);
-    if (++s == STAGES) s = 0, par ^= 1u;
+    if (EARLY) release();
   };
   // The norm weights are constants: requested before the input may be read.
   float4 wv[NSEG], xv[NSEG];
 #pragma unroll
-  for (int q = 0; q < NSEG; ++q) wv[q] = nw ? __ldg(reinterpret_cast<const float4*>(nw + q * SEG + kw * GROUP) + lane) : make_float4(1.f, 1.f, 1.f, 1.f);
+  for (int q = 0; q < NSEG; ++q) wv[q] = nw && EARLY ? __ldg(reinterpret_cast<const float4*>(nw + q * SEG + kw * GROUP) + lane) : make_float4(1.f, 1.f, 1.f, 1.f);
   if (EARLY) load(0, 0);
   pdl_wait();  // x and res come from the previous kernel
 #pragma unroll
@@ -182,8 +197,10 @@ __global__ void __launch_bounds__(THREADS, 2)
     }
     const float inv = rsqrtf(tot / K + eps);
 #pragma unroll
-    for (int q = 0; q < NSEG; ++q)
+    for (int q = 0; q < NSEG; ++q) {
+      if (!EARLY) wv[q] = __ldg(reinterpret_cast<const float4*>(nw + q * SEG + kw * GROUP) + lane);
       xv[q] = make_float4(xv[q].x * inv * wv[q].x, xv[q].y * inv * wv[q].y, xv[q].z * inv * wv[q].z, xv[q].w * inv * wv[q].w);
+    }
   }
   // Limbs. Lane l holds inputs 4 l .. 4 l + 3 of the 128; the operand wants, in lane (g, t4), limb g of inputs 16 t4 + 4 i and
   // 64 + 16 t4 + 4 i: the order in which a lane's two 16-byte pieces of a weight row come (any order serves a sum).
@@ -220,22 +237,33 @@ __global__ void __launch_bounds__(THREADS, 2)
     delta[q] = t4 == 0 ? d : t4 == 1 ? d * 16384.f : 0.f;
   }
   __syncwarp();  // before partial sums overwrite the limbs
-  if (!EARLY) load(0, 0);
 
   for (int t = 0; t < ntiles; ++t) {
     float a0 = 0.f, a1 = 0.f;  // rows g and g + 8 of the tile
 #pragma unroll
     for (int q = 0; q < NSEG; ++q) {
+      if (!EARLY) load(t, q);
       int c[4] = {0, 0, 0, 0}, e[4] = {0, 0, 0, 0};
       mma_s8(c, v0.x, w0.x, v0.y, w0.y, bf[q][0], bf[q][1]);
-      mma_s8(e, v1.x, w1.x, v1.y, w1.y, bf[q][4], bf[q][5]);
-      mma_s8(c, v0.z, w0.z, v0.w, w0.w, bf[q][2], bf[q][3]);
-      mma_s8(e, v1.z, w1.z, v1.w, w1.w, bf[q][6], bf[q][7]);
+      if (EARLY) {
+        mma_s8(e, v1.x, w1.x, v1.y, w1.y, bf[q][4], bf[q][5]);
+        mma_s8(c, v0.z, w0.z, v0.w, w0.w, bf[q][2], bf[q][3]);
+        mma_s8(e, v1.z, w1.z, v1.w, w1.w, bf[q][6], bf[q][7]);
+      } else {  // the second pieces in the registers of the first
+        mma_s8(c, v0.z, w0.z, v0.w, w0.w, bf[q][2], bf[q][3]);
+        const unsigned char* rp = operand() + 64;
+        v0 = *reinterpret_cast<const uint4*>(rp), w0 = *reinterpret_cast<const uint4*>(rp + 8 * PITCH);
+        release();
+        mma_s8(c, v0.x, w0.x, v0.y, w0.y, bf[q][4], bf[q][5]);
+        mma_s8(c, v0.z, w0.z, v0.w, w0.w, bf[q][6], bf[q][7]);
+      }
       // |a limb's sum| <= 128 * 128 * 64 = 2^20: limb + 128 * next limb stays an exact integer
       a0 = fmaf(__half2float(sc0) * delta[q], (float)((c[0] + e[0]) + ((c[1] + e[1]) << 7)), a0);
       a1 = fmaf(__half2float(sc1) * delta[q], (float)((c[2] + e[2]) + ((c[3] + e[3]) << 7)), a1);
-      if (q + 1 < NSEG) load(t, q + 1);
-      else if (t + 1 < ntiles) load(t + 1, 0);
+      if (EARLY) {
+        if (q + 1 < NSEG) load(t, q + 1);
+        else if (t + 1 < ntiles) load(t + 1, 0);
+      }
     }
     a0 += __shfl_xor_sync(0xffffffffu, a0, 1);
     a1 += __shfl_xor_sync(0xffffffffu, a1, 1);
@@ -269,7 +297,8 @@ int launch(const int8_t* W, const __half* S, const float* x, const float* res, f
   const DrbDevice& dev = drb_device(st);
   if (!dev.ready) return -2;
   if (N <= 0) return 0;
-  drb_launch(k_gemv<K, U>, dim3(N < dev.sms ? N : dev.sms), dim3(THREADS), Shape<K, U>::BYTES, st, dev.pdl, W, S, x, res, y, N, nw, eps, pf, pf_bytes);
+  drb_launch(k_gemv<K, U>, dim3(N < dev.sms ? N : dev.sms), dim3(THREADS), Shape<K, U>::BYTES, st, dev.pdl, W, S, x, res, y, N, nw, eps, pf, pf_bytes,
+             dev.pdl ? HINT_SKIP : 0u);
   return 0;
 }
 
@@ -300,7 +329,7 @@ DRB_DEV void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memor
 
 __global__ void __launch_bounds__(THREADS, 2)
     k_gemv(const __nv_bfloat16* __restrict__ W, const float* __restrict__ x, float* __restrict__ y, int N, const float* __restrict__ nw, float eps,
-           const char* pf, size_t pf_bytes) {
+           const char* pf, size_t pf_bytes, unsigned pf_skip) {
   extern __shared__ __align__(128) unsigned char dyn[];
   Ctl& ctl = *reinterpret_cast<Ctl*>(dyn);
   float4* xs4 = reinterpret_cast<float4*>(dyn + 512);
@@ -327,7 +356,7 @@ __global__ void __launch_bounds__(THREADS, 2)
         mbar_expect_tx(&ctl.full[s], bytes);
         bulk_g2s(ring + s * STAGE_BYTES, W + (size_t)r0 * K, bytes, &ctl.full[s]);
       }
-      prefetch_share(pf, pf_bytes, b, G);
+      prefetch_hint(pf, pf_bytes, pf_skip, b, G);
     }
     return;
   }
@@ -441,6 +470,7 @@ extern "C" int dr_gemv_bf16(const __nv_bfloat16* W, const float* x, float* y, in
   const DrbDevice& dev = drb_device(st);
   if (!dev.ready) return -2;
   if (N <= 0) return 0;
-  drb_launch(k_gemv, dim3(N < dev.sms ? N : dev.sms), dim3(THREADS), BYTES, st, dev.pdl, W, x, y, N, nw, eps, pf, pf_bytes);
+  drb_launch(k_gemv, dim3(N < dev.sms ? N : dev.sms), dim3(THREADS), BYTES, st, dev.pdl, W, x, y, N, nw, eps, pf, pf_bytes,
+             dev.pdl ? gemv::HINT_SKIP : 0u);
   return 0;
 }

@@ -128,3 +128,22 @@ def test_gemv_q8_extreme_codes_against_a_constant_slice(st):
     ref = orc.gemv_q8(q, s, x, dtype=np.float64)
     assert np.abs(y - ref).max() <= 1e-5 * np.abs(ref).max(), (y[:4], ref[:4])
     assert device_error_word() == 0
+
+
+@pytest.mark.parametrize("k", [512, 2048, 4096, 6144, 8192])
+@pytest.mark.parametrize("n", [1, 15, 17, 148 * 16 + 5, 148 * 64 + 77])
+def test_gemv_q8_tile_edges(st, n, k):
+    """Row counts around the sixteen-row tiles, the 64-row batches and the ring of stages, with norm and aliased residual."""
+    if n * k > 40_000_000:
+        n = 148 * 17 + 9
+    q, s = synth.make_q8(n + k, n, k)
+    rng = np.random.Generator(np.random.PCG64(n * k))
+    x = synth.make_x(n + 3 * k, 1, k)[0]
+    x[rng.integers(0, k, 8)] *= 300.0  # outliers share their group of 128 with ordinary inputs
+    nw = (1.0 + 0.1 * rng.standard_normal(k)).astype(np.float32)
+    res = rng.standard_normal(n).astype(np.float32)
+    y = run_q8(st, q, s, x, res=res, nw=nw, alias=True)
+    xn = orc.rmsnorm(x[None].astype(np.float64), nw, 1e-6, np.float64)[0]
+    ref = orc.gemv_q8(q, s, xn, dtype=np.float64) + res
+    assert np.abs(y - ref).max() <= 1e-5 * np.abs(ref).max() + 5e-6, (n, k)
+    assert device_error_word() == 0
