@@ -144,6 +144,30 @@ DRB_DEV bool mbar_wait_hot(uint64_t* bar, unsigned parity, unsigned err_code) {
   return false;
 }
 
+// mbar_wait_hot for a ring's innermost waits: two instructions when the barrier is complete. `spent` starts at zero; after a
+// wait that ran out (the error word is set, results are void) it stands at the limit, and no later wait retries.
+constexpr unsigned WAIT_SPENT = 1u << 20;
+template <unsigned ERR>
+DRB_DEV void mbar_wait_ring(uint32_t bar, unsigned parity, unsigned& spent) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .u32 n;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 2000;\n\t"
+      "@p bra RING_OVER;\n\t"
+      "mov.u32 n, %0;\n"
+      "RING_AGAIN:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 2000;\n\t"
+      "@p bra RING_OVER;\n\t"
+      "add.u32 n, n, 1;\n\t"
+      "setp.lt.u32 p, n, 1048576;\n\t"
+      "@p bra RING_AGAIN;\n\t"
+      "mov.u32 %0, 1048576;\n\t"
+      "red.relaxed.gpu.global.max.u32 [g_drb_error], %3;\n"
+      "RING_OVER:\n\t}"
+      : "+r"(spent)
+      : "r"(bar), "r"(parity), "n"(ERR)
+      : "memory");
+}
+
 // Global -> shared bulk copy. dst, src 16-byte aligned; bytes a multiple of 16.
 DRB_DEV void bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(

@@ -266,9 +266,9 @@ struct Ring {
   }
 };
 // Bounded wait on barrier bars[r.i]; after one that ran out no later wait of the thread spins.
-template <int N>
-DRB_DEV void wait_at(uint64_t* bars, const Ring<N>& r, unsigned err, bool& dead) {
-  if (!dead) dead = !mbar_wait_hot(bars + r.i, r.par, err);
+template <unsigned ERR, int N>
+DRB_DEV void wait_at(uint64_t* bars, const Ring<N>& r, unsigned& spent) {
+  mbar_wait_ring<ERR>(smem_u32(bars) + 8 * r.i, r.par, spent);
 }
 
 struct Maps {
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
   // weight row of tile row r: a gate/up tile interleaves gate j (even r) with up j (odd r)
   auto weight_row = [&](int mt, int r) { return GEMM == 0 ? (r & 1) * I + mt * (TILE_M / 2) + (r >> 1) : mt * TILE_M + r; };
 
-  bool dead = false;    // a wait ran out once: stop waiting (the error word is set; results are void)
+  unsigned spent = 0;  // see mbar_wait_ring
 
   if (warp < CONV_WARPS) {
     // ================= convert warps =================
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
     ra.par = 1;
     ra.next(group);
     auto a_wait = [&]() {  // the MMAs that read this stage's tiles must have completed
-      wait_at(ctl.done, ra, DRB_ERR_TMEM, dead);
+      wait_at<DRB_ERR_TMEM>(ctl.done, ra, spent);
       tc_fence_after();
     };
     auto a_done = [&]() {
@@ -422,14 +422,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
     for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
       const Item it = decode(item);
       if (FMT == 0 && !it.shared) {
-        wait_at(ctl.smfull, rs, DRB_ERR_FULL_WAIT, dead);
+        wait_at<DRB_ERR_FULL_WAIT>(ctl.smfull, rs, spent);
         // (scale, min) of this row's groups 4 step + 2 half, + 1: gate/up: piece `step` of a swizzled row; down: 16 bytes a step
         const uint32_t sm_a = smem_u32(smbuf) + rs.i * SMB + (GEMM == 0 ? swz_off(r, 0) : r * 32) + 8 * half;
         rs.next();
         rr.next(group);
 #pragma unroll 1
         for (int step = group; step < NSTEP; step += 2) {
-          wait_at(ctl.rawfull, rr, DRB_ERR_FULL_WAIT, dead);
+          wait_at<DRB_ERR_FULL_WAIT>(ctl.rawfull, rr, spent);
           // piece 4 half + j of the row stands at xa ^ 16 j: in the swizzled row the piece's number is xor-ed into the address
           uint32_t xa = x_row + rr.i * RAW_BYTES;
           uint32_t sm[2];
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
           const bool small = __all_sync(0xffffffffu, max(sm[0] & 0x7fffu, sm[1] & 0x7fffu) < 0x2C00u);  // both scales below 2^-4
           a_wait();
           uint32_t to = acol + ra.i * A_COLS;
-#pragma unroll 1
+#pragma unroll
           for (int g = 0; g < 2; ++g) {
             uint32_t w[8];
             lds128(xa, w), lds128(xa ^ 16u, w + 4);
@@ -479,10 +479,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
           if (FMT == 0 && step + 2 < NSTEP) s_next = __ldg(ssrow + 2 * (step + 2));
           // both stages are waited for although this warp reads one: an arrival must not run a ring's length ahead
           const int sa = rr.i;
-          wait_at(ctl.rawfull, rr, DRB_ERR_FULL_WAIT, dead);
+          wait_at<DRB_ERR_FULL_WAIT>(ctl.rawfull, rr, spent);
           rr.next();
           const int sb = rr.i;
-          wait_at(ctl.rawfull, rr, DRB_ERR_FULL_WAIT, dead);
+          wait_at<DRB_ERR_FULL_WAIT>(ctl.rawfull, rr, spent);
           rr.next(step + 2 < NSTEP ? 3 : 3 - 2 * group);
           const unsigned char* xp = xrow + (half ? sb : sa) * RAW_BYTES;
 #pragma unroll
@@ -518,15 +518,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
     unsigned steps = 0;
     const uint64_t bdesc0 = smem_desc(bring, 4096);  // eight-row groups lie 4 KB apart: four 1 KB columns each
     for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
-      wait_at(ctl.tabfull, rt, DRB_ERR_FULL_WAIT, dead);
+      wait_at<DRB_ERR_FULL_WAIT>(ctl.tabfull, rt, spent);
       const uint32_t idesc = instr_desc_f16(tabs[rt.i].cols), d = tmem + (uint32_t)(rc.i * NT);
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl.tabempty[rt.i]);
       rt.next();
-      if (FMT == 0) wait_at(ctl.accfree, rc, DRB_ERR_TMEM, dead);
+      if (FMT == 0) wait_at<DRB_ERR_TMEM>(ctl.accfree, rc, spent);
 #pragma unroll 1
       for (int step = 0; step < NSTEP; ++step) {
-        wait_at(ctl.full, ra, DRB_ERR_TMEM, dead);
+        wait_at<DRB_ERR_TMEM>(ctl.full, ra, spent);
         if (FMT == 0) {
           tc_fence_after();
           if (elect_one()) {
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
         } else {
 #pragma unroll
           for (int kb = 0; kb < 2; ++kb) {
-            wait_at(ctl.accfree, rc, DRB_ERR_TMEM, dead);
+            wait_at<DRB_ERR_TMEM>(ctl.accfree, rc, spent);
             tc_fence_after();
             if (elect_one()) {
               const uint32_t ac = tmem + A_COL0 + ra.i * A_COLS, dk = tmem + (uint32_t)(rc.i * NT);
@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
     // The block must not end before the completion arrivals it is owed have landed: the last one of every stage.
     for (unsigned k = 0; k < NST && k < steps; ++k) {
       const unsigned n = steps - 1 - k;
-      if (!dead) dead = !mbar_wait(&ctl.done[n % NST], (n / NST) & 1, DRB_ERR_TMEM);
+      mbar_wait_ring<DRB_ERR_TMEM>(smem_u32(&ctl.done[n % NST]), (n / NST) & 1, spent);
     }
   } else if (warp == LOAD_WARP) {
     // ================= loader =================
@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
       const CUtensorMap* map = it.shared ? &maps.sh : &maps.q;
 #pragma unroll 1
       for (int n = 0; n < nraw; ++n) {
-        wait_at(ctl.rawempty, rr, DRB_ERR_EMPTY_WAIT, dead);
+        wait_at<DRB_ERR_EMPTY_WAIT>(ctl.rawempty, rr, spent);
         __syncwarp();
         if (elect_one()) {
           uint64_t* bar = &ctl.rawfull[rr.i];
@@ -608,14 +608,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
     Ring<NST> ra;
     ra.par = 1;  // every stage starts free
     for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
-      wait_at(ctl.tabfull, rt, DRB_ERR_FULL_WAIT, dead);
+      wait_at<DRB_ERR_FULL_WAIT>(ctl.tabfull, rt, spent);
       const Tab& tab = tabs[rt.i];
       const int srow = tab.srow, full = tab.full, start = tab.start, quads = tab.quads;
       const unsigned bytes = (full + (start >= 0)) * 4096 + quads * 2048;
       const CUtensorMap *m8 = tab.shared ? &maps.shtok8 : &maps.tok8, *m1 = tab.shared ? &maps.shtok1 : &maps.tok1;
 #pragma unroll 1
       for (int step = 0; step < NSTEP; ++step) {
-        wait_at(ctl.done, ra, DRB_ERR_EMPTY_WAIT, dead);
+        wait_at<DRB_ERR_EMPTY_WAIT>(ctl.done, ra, spent);
         __syncwarp();
         if (elect_one()) {
           unsigned char* bp = bring + ra.i * B_BYTES;
@@ -644,7 +644,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
     rt.par = 1;
     for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
       const Item it = decode(item);
-      if (!dead) dead = !mbar_wait(&ctl.tabempty[rt.i], rt.par, DRB_ERR_EMPTY_WAIT);
+      wait_at<DRB_ERR_EMPTY_WAIT>(ctl.tabempty, rt, spent);
       Tab& tab = tabs[rt.i];
       const int cnt = it.shared ? a.rows_sh : __ldg(a.counts + it.e);
       const int nt = min(NT, cnt - it.n0);
@@ -681,7 +681,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
     Ring<NTAB> rt;
     Ring<NACC> rc;
     for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
-      wait_at(ctl.tabfull, rt, DRB_ERR_FULL_WAIT, dead);
+      wait_at<DRB_ERR_FULL_WAIT>(ctl.tabfull, rt, spent);
       const Tab& tab = tabs[rt.i];
       const int cols = FMT == 1 ? tab.cols : tab.used, mt = tab.mt;
       const bool sh = tab.shared != 0;
@@ -696,7 +696,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
 #pragma unroll 1
         for (int kb = 0; kb < K / 128; ++kb) {
           const float s = __shfl_sync(0xffffffffu, sv, kb + (GEMM == 0 && (r & 1) ? 16 : 0));
-          wait_at(ctl.accfull, rc, DRB_ERR_TMEM, dead);
+          wait_at<DRB_ERR_TMEM>(ctl.accfull, rc, spent);
           tc_fence_after();
 #pragma unroll
           for (int c0 = 0; c0 < NT; c0 += 16)
@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
           rc.next();
         }
       } else {
-        wait_at(ctl.accfull, rc, DRB_ERR_TMEM, dead);
+        wait_at<DRB_ERR_TMEM>(ctl.accfull, rc, spent);
         tc_fence_after();
       }
       const uint32_t acc = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(rc.i * NT);
