@@ -16,8 +16,8 @@
 // costs one tcgen05.st (measured 700 B per cycle and multiprocessor), the MMA reads it there (14, 19, 32 cycles for
 // N = 16, 32, 64; from shared memory never below 39), and shared memory carries the raw bytes only.
 //
-// Roles, one block of 24 warps per multiprocessor, meeting only on mbarriers, every wait bounded (common.cuh):
-//   16 convert warps  a step is 256 inputs of 128 rows; two groups of eight warps take turns. A thread converts 128 inputs of
+// Roles, one block of 24 warps (FP8: 20) per multiprocessor, meeting only on mbarriers, every wait bounded (common.cuh):
+//   16 convert warps (FP8: 8)  a step is 256 inputs of 128 rows; groups of eight warps take turns. A thread converts 128 inputs of
 //                 one row: four (int4) or eight (8-bit) 16-byte pieces out of the swizzled raw stage, two 32-column
 //                 tcgen05.st. Three stages: 128 columns each, with a token tile in shared memory.
 //   MMA warp      sixteen K = 16 instructions per step, one commit that frees the stage
@@ -28,7 +28,7 @@
 //                 four 128-byte swizzled columns), scattered rows by tile::gather4 (512 bytes per request; it costs the copy
 //                 engine 19 cycles against 49 for the 4 KB box)
 //   table warp    the items' rows, result rows and row factors, ahead of everybody
-//   4 epilogue warps  drain an item's accumulator while the next item's MMAs fill the other one
+//   4 epilogue warps (FP8: 8)  drain an item's accumulator while the next item's MMAs fill the other one
 //
 // Work items: (shared expert or expert, group of up to 64 tokens, 128-row tile), enumerated from the device-side
 // counts by a prefix sum each block computes for itself, the shared expert's items first, walked round robin.
@@ -46,9 +46,8 @@ namespace pft {
 using namespace tc;
 
 constexpr int H = 2048, I = 512;
-constexpr int CONV_WARPS = 16, GROUP_WARPS = 8, EPI_WARPS = 4;
-constexpr int EPI_WARP0 = CONV_WARPS, MMA_WARP = EPI_WARP0 + EPI_WARPS, LOAD_WARP = MMA_WARP + 1, TOKEN_WARP = MMA_WARP + 2, TABLE_WARP = MMA_WARP + 3;
-constexpr int THREADS = (TABLE_WARP + 1) * 32;  // 768
+constexpr int GROUP_WARPS = 8, EPI_WARPS = 4;   // warps of a convert group / of an epilogue set
+constexpr int MAX_WARPS = 24;
 constexpr int TILE_M = 128;
 constexpr int STEP_K = 256;
 constexpr int MAX_NT = 64;                      // tokens per work item at most
@@ -80,7 +79,7 @@ struct Ctl {
   uint64_t done[NST];                      // the MMAs that read it have completed (tcgen05.commit)
   uint64_t accfull[4], accfree[4];         // an accumulator is complete (tcgen05.commit) / has been drained (one arrival per epilogue warp)
   uint64_t tabfull[NTAB], tabempty[NTAB];  // written / read for the last time (token, MMA and epilogue warps)
-  int wtot[THREADS / 32];                  // the prefix sum's warp totals
+  int wtot[MAX_WARPS];                     // the prefix sum's warp totals
   uint32_t tmem_base;
 };
 static_assert(sizeof(Ctl) <= CTL_BYTES, "control block");
@@ -92,6 +91,14 @@ struct Smem {
   static constexpr int NACC = FMT == 1 ? 4 : 2;    // accumulators: int4: one per item; FP8: one per 128 inputs (see k_grouped)
   static constexpr int B_BYTES = NT * STEP_K * 2;  // one token tile
   static_assert(NT <= MAX_NT && NT * NACC <= A_COL0, "tensor memory");
+  // int4: conversion is the work, two groups take turns at the steps and one set of epilogue warps follows. FP8: a weight takes half
+  // an instruction to convert, but every 128 inputs have an accumulator to drain: one group, two sets that take
+  // turns at the items, each with two accumulators of its own (with one set the MMAs waited for it a third of the time).
+  static constexpr int GROUPS = FMT == 1 ? 1 : 2, SETS = FMT == 1 ? 2 : 1;
+  static constexpr int CONV_WARPS = GROUPS * GROUP_WARPS;
+  static constexpr int MMA_WARP = CONV_WARPS + SETS * EPI_WARPS, LOAD_WARP = MMA_WARP + 1, TOKEN_WARP = MMA_WARP + 2, TABLE_WARP = MMA_WARP + 3;
+  static constexpr int THREADS = (TABLE_WARP + 1) * 32;  // 768 / 640
+  static_assert(TABLE_WARP < MAX_WARPS, "warps");
   static constexpr int NRAW = FMT == 1 ? 10 : GEMM == 0 ? 5 : 6;           // what fits; four are enough for the copy rate (a stream of such boxes alone: 6.2 TB/s with 4, 6.5 with 6)
   static constexpr int NSM = FMT != 0 ? 0 : GEMM == 0 ? 2 : 4;             // slots for an int4 item's (scale, min) pairs: see the loader
   static constexpr int SMB = TILE_M * ((GEMM == 0 ? H : I) / 64) * 4;      // bytes of one
@@ -299,7 +306,7 @@ struct Args {
 // PREP (gate/up): the token rows are prepared (contiguous in slot order; int4: permuted); otherwise they are gathered
 // through row_of in k order. The down kernel's rows are the act array, contiguous, int4: permuted by the gate/up epilogue.
 template <int GEMM, int FMT, bool PREP>
-__global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ Maps maps, const Args a) {
+__global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const __grid_constant__ Maps maps, const Args a) {
   constexpr int K = GEMM == 0 ? H : I;
   constexpr int R = GEMM == 0 ? 2 * I : H;
   constexpr int MT = R / TILE_M;         // tiles per expert: 8 / 16
@@ -307,6 +314,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
   constexpr bool PERM = FMT == 0 && PREP;
   using S = Smem<GEMM, FMT>;
   constexpr int NRAW = S::NRAW, NSM = S::NSM, SMB = S::SMB, NT = S::NT, NACC = S::NACC, B_BYTES = S::B_BYTES;
+  constexpr int GROUPS = S::GROUPS, SETS = S::SETS, CONV_WARPS = S::CONV_WARPS, THREADS = S::THREADS;
+  constexpr int MMA_WARP = S::MMA_WARP, LOAD_WARP = S::LOAD_WARP, TOKEN_WARP = S::TOKEN_WARP, TABLE_WARP = S::TABLE_WARP;
+  constexpr int SET_ACC = NACC / SETS;  // accumulators of an epilogue set
   extern __shared__ unsigned char dyn_raw[];
   unsigned char* dyn = dyn_raw + (-smem_u32(dyn_raw) & 1023u);  // an offset, not a rounded address: loads stay shared-memory loads
   Ctl& ctl = *reinterpret_cast<Ctl*>(dyn);
@@ -392,7 +402,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
 
   if (warp < CONV_WARPS) {
     // ================= convert warps =================
-    // Two groups of eight take turns, group g the steps of parity g; within a group, warp (half h, lane quarter q4) converts
+    // The groups of eight take turns at the steps; within a group, warp (half h, lane quarter q4) converts
     // inputs [128 h, +128) of the step's 256 for its 32 rows. The waits and arrivals of a step cost a warp as many instructions as
     // 64 inputs of conversion do, so a thread takes 128 of every other step and not 64 of each (it measured 243 instructions
     // per 64 inputs before, 104 of them conversion).
@@ -416,7 +426,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl.full[ra.i]);
-      ra.next(2);
+      ra.next(GROUPS);
     };
     Ring<(NSM ? NSM : 1)> rs;  // int4 items' scales
     for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
@@ -428,7 +438,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
         rs.next();
         rr.next(group);
 #pragma unroll 1
-        for (int step = group; step < NSTEP; step += 2) {
+        for (int step = group; step < NSTEP; step += GROUPS) {
           wait_at<DRB_ERR_FULL_WAIT>(ctl.rawfull, rr, spent);
           // piece 4 half + j of the row stands at xa ^ 16 j: in the swizzled row the piece's number is xor-ed into the address
           uint32_t xa = x_row + rr.i * RAW_BYTES;
@@ -464,7 +474,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(&ctl.rawempty[rr.i]);
-          rr.next(step + 2 < NSTEP ? 2 : 2 - group);
+          rr.next(step + GROUPS < NSTEP ? GROUPS : GROUPS - group);
           a_done();
         }
       } else {  // 8-bit weights: a step is two raw stages, one per half
@@ -474,16 +484,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
         if (FMT == 0) s_next = __ldg(ssrow + 2 * group);
         rr.next(2 * group);
 #pragma unroll 1
-        for (int step = group; step < NSTEP; step += 2) {
+        for (int step = group; step < NSTEP; step += GROUPS) {
           const __half2 s2 = __half2half2(s_next);
-          if (FMT == 0 && step + 2 < NSTEP) s_next = __ldg(ssrow + 2 * (step + 2));
+          if (FMT == 0 && step + GROUPS < NSTEP) s_next = __ldg(ssrow + 2 * (step + GROUPS));
           // both stages are waited for although this warp reads one: an arrival must not run a ring's length ahead
           const int sa = rr.i;
           wait_at<DRB_ERR_FULL_WAIT>(ctl.rawfull, rr, spent);
           rr.next();
           const int sb = rr.i;
           wait_at<DRB_ERR_FULL_WAIT>(ctl.rawfull, rr, spent);
-          rr.next(step + 2 < NSTEP ? 3 : 3 - 2 * group);
+          rr.next(2 * (step + GROUPS < NSTEP ? GROUPS : GROUPS - group) - 1);
           const unsigned char* xp = xrow + (half ? sb : sa) * RAW_BYTES;
 #pragma unroll
           for (int g = 0; g < 2; ++g) {
@@ -512,14 +522,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
   } else if (warp == MMA_WARP) {
     // ================= MMA warp =================
     Ring<NTAB> rt;
-    Ring<NACC> rc;
+    Ring<SET_ACC> rc;  // FP8: an item takes an even number of turns of its set's two accumulators, so the next item finds it as it was
     Ring<NST> ra;
     rc.par = 1;  // the accumulators start free
     unsigned steps = 0;
+    int acc0 = 0;  // the item's first accumulator: 0, FP8: of the set whose turn it is
+    static_assert(FMT == 0 || (K / 128 / SET_ACC) % 2 == 0, "even turns");
     const uint64_t bdesc0 = smem_desc(bring, 4096);  // eight-row groups lie 4 KB apart: four 1 KB columns each
     for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
       wait_at<DRB_ERR_FULL_WAIT>(ctl.tabfull, rt, spent);
-      const uint32_t idesc = instr_desc_f16(tabs[rt.i].cols), d = tmem + (uint32_t)(rc.i * NT);
+      const uint32_t idesc = instr_desc_f16(tabs[rt.i].cols), d = tmem + (uint32_t)((acc0 + rc.i) * NT);
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl.tabempty[rt.i]);
       rt.next();
@@ -541,15 +553,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
         } else {
 #pragma unroll
           for (int kb = 0; kb < 2; ++kb) {
-            wait_at<DRB_ERR_TMEM>(ctl.accfree, rc, spent);
+            wait_at<DRB_ERR_TMEM>(ctl.accfree + acc0, rc, spent);
             tc_fence_after();
             if (elect_one()) {
-              const uint32_t ac = tmem + A_COL0 + ra.i * A_COLS, dk = tmem + (uint32_t)(rc.i * NT);
+              const uint32_t ac = tmem + A_COL0 + ra.i * A_COLS, dk = tmem + (uint32_t)((acc0 + rc.i) * NT);
               const uint64_t bd = bdesc0 + (uint32_t)(ra.i * (B_BYTES >> 4));
 #pragma unroll
               for (int k16 = 8 * kb; k16 < 8 * kb + 8; ++k16)
                 mma_f16_ts(dk, ac + 8 * k16, bd + (uint64_t)((k16 >> 2) * 64 + (k16 & 3) * 2), idesc, k16 > 8 * kb);
-              mma_commit(&ctl.accfull[rc.i]);
+              mma_commit(&ctl.accfull[acc0 + rc.i]);
               if (kb == 1) mma_commit(&ctl.done[ra.i]);
             }
             __syncwarp();
@@ -560,6 +572,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
         ra.next();
       }
       if (FMT == 0) rc.next();
+      if (SETS > 1) acc0 ^= SET_ACC;
       steps += NSTEP;
     }
     // The block must not end before the completion arrivals it is owed have landed: the last one of every stage.
@@ -676,11 +689,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
   } else {
     // ================= epilogue warps =================
     if (GEMM == 1) pdl_wait();  // y may still be read as the gate/up kernel's token rows
-    const int q4 = warp & 3;
+    const int q4 = warp & 3, set = SETS > 1 ? (warp - CONV_WARPS) / EPI_WARPS : 0;
     const int r = q4 * 32 + lane;  // tile row
+    const int acc0 = set * SET_ACC;
     Ring<NTAB> rt;
-    Ring<NACC> rc;
-    for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
+    Ring<SET_ACC> rc;
+    if (SETS > 1) rt.next(set);  // a table slot serves one set only: NTAB is a multiple of SETS
+    for (int item = blockIdx.x + set * gridDim.x; item < total_items; item += SETS * gridDim.x) {
       wait_at<DRB_ERR_FULL_WAIT>(ctl.tabfull, rt, spent);
       const Tab& tab = tabs[rt.i];
       const int cols = FMT == 1 ? tab.cols : tab.used, mt = tab.mt;
@@ -696,19 +711,19 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
 #pragma unroll 1
         for (int kb = 0; kb < K / 128; ++kb) {
           const float s = __shfl_sync(0xffffffffu, sv, kb + (GEMM == 0 && (r & 1) ? 16 : 0));
-          wait_at<DRB_ERR_TMEM>(ctl.accfull, rc, spent);
+          wait_at<DRB_ERR_TMEM>(ctl.accfull + acc0, rc, spent);
           tc_fence_after();
 #pragma unroll
           for (int c0 = 0; c0 < NT; c0 += 16)
             if (c0 < cols) {
               uint32_t v[16];
-              tmem_ld16(tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(rc.i * NT + c0), v);
+              tmem_ld16(tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)((acc0 + rc.i) * NT + c0), v);
 #pragma unroll
               for (int i = 0; i < 16; ++i) sum[c0 + i] = fmaf(s, __uint_as_float(v[i]), sum[c0 + i]);
             }
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&ctl.accfree[rc.i]);
+          if (lane == 0) mbar_arrive(&ctl.accfree[acc0 + rc.i]);
           rc.next();
         }
       } else {
@@ -780,7 +795,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_grouped(const __grid_constant__ 
       if (GEMM == 1 && a.peer_y && !sh) __threadfence_system();  // before the flag that a later kernel writes to the peers
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl.tabempty[rt.i]);
-      rt.next();
+      rt.next(SETS);
     }
   }
   tc_fence_before();
@@ -900,9 +915,9 @@ static int run_block(const Block& b, const DrbDevice& dev, cudaStream_t st) {
       a.scales = sc, a.shs = static_cast<const __half*>(gemm == 0 ? b.sgu_s : b.sd_s);
       a.offsets = b.offsets + e0, a.counts = b.counts + e0, a.E = ne > 0 ? ne : 0, a.rows_sh = sh ? b.rows_sh : 0;
       if (gemm == 0)
-        drb_launch(prep ? k_grouped<0, FMT, true> : k_grouped<0, FMT, FMT != 0>, dim3(dev.sms), dim3(THREADS), Smem<0, FMT>::BYTES, st, dev.pdl && b.prepared && b.E <= MAX_E, m, a);
+        drb_launch(prep ? k_grouped<0, FMT, true> : k_grouped<0, FMT, FMT != 0>, dim3(dev.sms), dim3(Smem<0, FMT>::THREADS), Smem<0, FMT>::BYTES, st, dev.pdl && b.prepared && b.E <= MAX_E, m, a);
       else  // only the first one follows the gate/up kernel
-        drb_launch(k_grouped<1, FMT, true>, dim3(dev.sms), dim3(THREADS), Smem<1, FMT>::BYTES, st, dev.pdl && b.E <= MAX_E, m, a);
+        drb_launch(k_grouped<1, FMT, true>, dim3(dev.sms), dim3(Smem<1, FMT>::THREADS), Smem<1, FMT>::BYTES, st, dev.pdl && b.E <= MAX_E, m, a);
     }
   }
   return 0;
