@@ -380,191 +380,201 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Router logits whose value for a row does not depend on how many rows are computed together: every (row, output)
-// pair is one warp's dot product in a fixed order (lane l takes the 16-byte chunks l, l + 32, ... of the K = 2048
-// inputs, products exact in fp32, one fixed butterfly). A library GEMM picks its kernel by the batch size (measured:
+// Router logits whose value for a row does not depend on how many rows are computed together: every (row, output) sum is
+// formed in one fixed order whatever the launch's shape. A library GEMM picks its kernel by the batch size (measured:
 // logits of the same row differ by 1.2e-6 between a batch of 300 and a batch of 38), which would let the routing of
 // a row depend on how the rows are spread over the GPUs.
-// Block (x, y): rows [RB x, +RB), outputs in groups of OB; warp w takes groups y + gridDim.y * w, .... The rows stand in
-// shared memory as fp32, two rows interleaved (a packed fp32 FMA serves both), and a warp multiplies OB outputs with all RB
-// rows at once: four rows per block and one output per warp re-read the 1 MB of weights from L2 for every four rows and
-// converted every activation for every output (123 us for 2048 rows, 27 us for 300).
+//
+// A block takes 16 rows and the 8-output tiles blockIdx.y, blockIdx.y + gridDim.y, ...; warp w takes inputs [256 w, +256) of
+// all of them on mma.sync m16n8k16 bf16, with the rows as the A operand in its registers for the whole launch. The weights are
+// bf16 already; an fp16 row value (eleven bits) is the exact sum of two bf16 values, and the low part's products are the
+// addend of the high part's. Every instruction starts from zero and its sixteen products join the running sum by an fp32
+// addition, so nothing is lost to the tensor core's own accumulation over long sums; the eight warps' sums are added in order.
+// Which input a lane takes as which of an instruction's sixteen is the same permutation on both sides, chosen so that a lane's
+// share of two instructions is one 16-byte load.
+// Bound by the weights' way from L2 (1 MB per 16 rows, 64 bytes per clock at the instruction rate); at few rows by latency.
 // SRC: what the rows come from. LOGITS_NORM: fp32 rows, RMS-normalised here (sums in k_rmsnorm's order) and rounded to fp16;
-// blocks with y = 0 also store them. LOGITS_F16 / LOGITS_BF16: 16-bit rows as they are. The weights are bf16.
-constexpr int RL_K = 2048, RL_WARPS = 16;
+// blocks with y = 0 also store them. LOGITS_F16 / LOGITS_BF16: 16-bit rows as they are.
+constexpr int RL_K = 2048, RL_WARPS = 8, RL_ROWS = 16, RL_TILE = 8;
+constexpr int RL_SEG = RL_K / RL_WARPS;                 // inputs per warp
+constexpr int RL_STRIDE = RL_K * 2 + 64;                // bytes per staged row: the fragments' loads meet no bank twice
+constexpr int RL_STAGE = RL_ROWS * RL_STRIDE;
+constexpr int RL_PART = RL_ROWS * RL_TILE;              // floats per warp and tile
 enum LogitsSrc { LOGITS_NORM, LOGITS_F16, LOGITS_BF16 };
-template <int RB>
-constexpr size_t logits_smem() { return (size_t)RB * RL_K * 4; }
+constexpr size_t logits_smem(int tiles) { return RL_STAGE + (size_t)tiles * RL_WARPS * RL_PART * 4; }
+constexpr int RL_MAX_TILES = (232448 - RL_STAGE) / (RL_WARPS * RL_PART * 4);  // tiles of one block
 
-template <int SRC, int RB, int OB>
+DRB_DEV void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, const float (&c)[4]) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %11, %12, %13};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
+}
+
+// Two fp16 values as the sum of two pairs of bf16 values; exact.
+DRB_DEV void split_f16x2(uint32_t v, uint32_t& hi, uint32_t& lo) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
+  const __nv_bfloat162 h = __floats2bfloat162_rn(f.x, f.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  const __nv_bfloat162 l = __floats2bfloat162_rn(f.x - __uint_as_float(hi << 16), f.y - __uint_as_float(hi & 0xffff0000u));
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+template <int SRC>
 __global__ void __launch_bounds__(RL_WARPS * 32, 1)
     k_router_logits(const void* __restrict__ src, const float* __restrict__ nw, float eps, __half* __restrict__ rows16,
                     const __nv_bfloat16* __restrict__ w, const float* bias, float* logits, int rows, int e1, float beta, int* __restrict__ zero, int n_zero) {
-  extern __shared__ __align__(16) float xs[];
+  extern __shared__ __align__(16) unsigned char dyn[];
+  float* part = reinterpret_cast<float*>(dyn + RL_STAGE);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+  const int r0 = blockIdx.x * RL_ROWS, nr = min(RL_ROWS, rows - r0);
+  const int tiles = (e1 + RL_TILE - 1) / RL_TILE;
+  constexpr int LOADS = RL_SEG / 32;  // 16-byte loads of a lane per row and segment
+  const int k0 = warp * RL_SEG + 8 * q;
+  uint4 b[LOADS];
+  auto fetch = [&](int tile) {
+    const uint4* p = reinterpret_cast<const uint4*>(w + (size_t)min(tile * RL_TILE + g, e1 - 1) * RL_K + k0);
+#pragma unroll
+    for (int j = 0; j < LOADS; ++j) b[j] = __ldg(p + 4 * j);
+  };
+  // the row groups start at different tiles: in step, all of them would ask L2 for the same lines at once
+  const int mine = (tiles - (int)blockIdx.y + (int)gridDim.y - 1) / (int)gridDim.y;  // tiles of this block, at least one
+  int t = (int)(blockIdx.x % (unsigned)mine);
+  fetch(blockIdx.y + t * gridDim.y);
   pdl_launch_dependents();
   pdl_wait();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r0 = blockIdx.x * RB, nr = min(RB, rows - r0);
   if (zero && blockIdx.x == 0 && blockIdx.y == 0)
     for (int i = threadIdx.x; i < n_zero; i += blockDim.x) zero[i] = 0;
-  // where input k of row r stands: 16-byte pieces (two inputs of a row pair), permuted so that eight lanes reading
-  // consecutive chunks' piece p meet eight different bank groups
-  auto at = [](int r, int k) {
-    const int c = k >> 3, p = (k >> 1) & 3;
-    return (((r >> 1) * (RL_K / 2) + 4 * c + (p ^ ((c >> 1) & 3))) << 2) + 2 * (k & 1) + (r & 1);
-  };
-  for (int r = warp; r < RB; r += RL_WARPS) {
-    if (r >= nr) {
-      for (int k = lane; k < RL_K; k += 32) xs[at(r, k)] = 0.f;
-    } else if (SRC == LOGITS_NORM) {
-      // k_rmsnorm's sums: its thread t adds the squares of inputs t + 256 i in turn; each warp's 32 threads by butterfly, the
-      // eight warps in order
-      const float* xr = static_cast<const float*>(src) + (size_t)(r0 + r) * RL_K;
-      float v[RL_K / 32];
+  constexpr int RPW = RL_ROWS / RL_WARPS;  // rows warp + RL_WARPS p; all requested before the first is used
+  if (SRC == LOGITS_NORM) {
+    // k_rmsnorm's sums: its thread t adds the squares of inputs t + 256 i in turn; each warp's 32 threads by butterfly, the
+    // eight warps in order
+    float v[RPW][RL_K / 32];
 #pragma unroll
-      for (int i = 0; i < RL_K / 32; ++i) v[i] = __ldcg(xr + 32 * i + lane);
+    for (int p = 0; p < RPW; ++p) {
+      const float* xr = static_cast<const float*>(src) + (size_t)(r0 + warp + RL_WARPS * p) * RL_K;
+      const bool in = warp + RL_WARPS * p < nr;
+#pragma unroll
+      for (int i = 0; i < RL_K / 32; ++i) v[p][i] = in ? __ldcg(xr + 32 * i + lane) : 0.f;
+    }
+    float inv[RPW];
+#pragma unroll
+    for (int p = 0; p < RPW; ++p) {
       float t = 0.f;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
+      for (int s = 0; s < 8; ++s) {
         float ss = 0.f;
 #pragma unroll
-        for (int i = 0; i < RL_K / 256; ++i) ss += v[8 * i + q] * v[8 * i + q];
+        for (int i = 0; i < RL_K / 256; ++i) ss += v[p][8 * i + s] * v[p][8 * i + s];
         t += warp_sum(ss);
       }
-      const float inv = rsqrtf(t / RL_K + eps);
+      inv[p] = rsqrtf(t / RL_K + eps);
+    }
 #pragma unroll
-      for (int i = 0; i < RL_K / 32; ++i) {
-        const int k = 32 * i + lane;
-        const __half h = tc::f2h_sat(v[i] * inv * __ldg(nw + k));
-        if (blockIdx.y == 0) rows16[(size_t)(r0 + r) * RL_K + k] = h;
-        xs[at(r, k)] = __half2float(h);
-      }
-    } else {
+    for (int i = 0; i < RL_K / 32; ++i) {
+      const int k = 32 * i + lane;
+      const float f = __ldg(nw + k);
+#pragma unroll
+      for (int p = 0; p < RPW; ++p)
+        reinterpret_cast<__half*>(dyn + (warp + RL_WARPS * p) * RL_STRIDE)[k] =
+            warp + RL_WARPS * p < nr ? tc::f2h_sat(v[p][i] * inv[p] * f) : __half(0.f);
+    }
+  } else {
+#pragma unroll
+    for (int p = 0; p < RPW; ++p) {
+      const int r = warp + RL_WARPS * p;
       const uint4* xr = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(src) + (size_t)(r0 + r) * RL_K);
 #pragma unroll
-      for (int i = 0; i < RL_K / 256; ++i) {
-        const uint4 v = __ldcg(xr + 32 * i + lane);
-        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+      for (int i = 0; i < RL_K / 256; ++i)
+        reinterpret_cast<uint4*>(dyn + r * RL_STRIDE)[32 * i + lane] = r < nr ? __ldcg(xr + 32 * i + lane) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
+  if (SRC == LOGITS_NORM && blockIdx.y == 0) {
+    __syncwarp();
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float2 f;
-          if (SRC == LOGITS_F16) f = __half22float2(*reinterpret_cast<const __half2*>(&u[q]));
-          else f = make_float2(__uint_as_float(u[q] << 16), __uint_as_float(u[q] & 0xffff0000u));
-          const int k = 8 * (32 * i + lane) + 2 * q;
-          xs[at(r, k)] = f.x, xs[at(r, k + 1)] = f.y;
-        }
-      }
+    for (int p = 0; p < RPW; ++p) {
+      const int r = warp + RL_WARPS * p;
+      uint4* out = reinterpret_cast<uint4*>(rows16 + (size_t)(r0 + r) * RL_K);
+      if (r < nr)
+#pragma unroll
+        for (int i = 0; i < RL_K / 256; ++i) out[32 * i + lane] = reinterpret_cast<const uint4*>(dyn + r * RL_STRIDE)[32 * i + lane];
     }
   }
   __syncthreads();
-  const ulonglong2* xs2 = reinterpret_cast<const ulonglong2*>(xs);
-  const int groups = (e1 + OB - 1) / OB;
-  for (int g = blockIdx.y + gridDim.y * warp; g < groups; g += gridDim.y * RL_WARPS) {
-    const uint4* wr[OB];
-    uint4 wn[OB];
+  // this warp's A fragments, two instructions per 16-byte piece: rows g and g + 8
+  uint32_t ah[2 * LOADS][4], al[2 * LOADS][4];
 #pragma unroll
-    for (int o = 0; o < OB; ++o) {
-      wr[o] = reinterpret_cast<const uint4*>(w + (size_t)min(OB * g + o, e1 - 1) * RL_K);
-      wn[o] = __ldg(wr[o] + lane);
-    }
-    unsigned long long acc[OB][RB / 2];
+  for (int j = 0; j < LOADS; ++j) {
+    const uint4 u = *reinterpret_cast<const uint4*>(dyn + g * RL_STRIDE + 2 * (k0 + 32 * j));
+    const uint4 v = *reinterpret_cast<const uint4*>(dyn + (g + 8) * RL_STRIDE + 2 * (k0 + 32 * j));
+    const uint32_t f[2][4] = {{u.x, v.x, u.y, v.y}, {u.z, v.z, u.w, v.w}};
 #pragma unroll
-    for (int o = 0; o < OB; ++o)
+    for (int s = 0; s < 2; ++s)
 #pragma unroll
-      for (int q = 0; q < RB / 2; ++q) acc[o][q] = 0ull;
-#pragma unroll 1
-    for (int j = 0; j < RL_K / 256; ++j) {
-      const int c = lane + 32 * j, sw = (c >> 1) & 3;
-      uint32_t ww[OB][4];
-#pragma unroll
-      for (int o = 0; o < OB; ++o) {
-        ww[o][0] = wn[o].x, ww[o][1] = wn[o].y, ww[o][2] = wn[o].z, ww[o][3] = wn[o].w;
-        if (j + 1 < RL_K / 256) wn[o] = __ldg(wr[o] + c + 32);
+      for (int i = 0; i < 4; ++i) {
+        if (SRC == LOGITS_BF16) ah[2 * j + s][i] = f[s][i];
+        else split_f16x2(f[s][i], ah[2 * j + s][i], al[2 * j + s][i]);
       }
+  }
+  for (int n = 0; n < mine; ++n) {
+    uint4 c[LOADS];
 #pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        unsigned long long w0[OB], w1[OB];
+    for (int j = 0; j < LOADS; ++j) c[j] = b[j];
+    const int now = t;
+    if (++t == mine) t = 0;
+    if (n + 1 < mine) fetch(blockIdx.y + t * gridDim.y);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int o = 0; o < OB; ++o) {
-          const float lo = __uint_as_float(ww[o][p] << 16), hi = __uint_as_float(ww[o][p] & 0xffff0000u);
-          w0[o] = pack2(lo, lo), w1[o] = pack2(hi, hi);
+    for (int j = 0; j < LOADS; ++j) {
+      const uint32_t f[4] = {c[j].x, c[j].y, c[j].z, c[j].w};
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const float z[4] = {0.f, 0.f, 0.f, 0.f};
+        float d[4];
+        if (SRC == LOGITS_BF16) {
+          mma_bf16(d, ah[2 * j + s], f[2 * s], f[2 * s + 1], z);
+        } else {
+          float l[4];
+          mma_bf16(l, al[2 * j + s], f[2 * s], f[2 * s + 1], z);
+          mma_bf16(d, ah[2 * j + s], f[2 * s], f[2 * s + 1], l);
         }
 #pragma unroll
-        for (int q = 0; q < RB / 2; ++q) {
-          const ulonglong2 x2 = xs2[q * (RL_K / 2) + 4 * c + (p ^ sw)];
-#pragma unroll
-          for (int o = 0; o < OB; ++o) acc[o][q] = fma2(w1[o], x2.y, fma2(w0[o], x2.x, acc[o][q]));
-        }
+        for (int i = 0; i < 4; ++i) acc[i] += d[i];
       }
     }
-    // The butterfly over 32 lanes, for all sums at once: at each exchange a lane keeps half of them and hands the other
-    // half on, until one is left per lane group; every sum is formed from the same pairs in the same order as by itself.
-    constexpr int N = OB * RB;
-    float v[N];
+    float* p = part + (now * RL_WARPS + warp) * RL_PART + g * RL_TILE + 2 * q;
+    *reinterpret_cast<float2*>(p) = make_float2(acc[0], acc[1]);
+    *reinterpret_cast<float2*>(p + 8 * RL_TILE) = make_float2(acc[2], acc[3]);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < mine * RL_PART; i += RL_WARPS * 32) {
+    const int m = i / RL_PART, at = i % RL_PART, r = at / RL_TILE, o = (blockIdx.y + m * gridDim.y) * RL_TILE + at % RL_TILE;
+    if (o >= e1 || r >= nr) continue;
+    float v = 0.f;
 #pragma unroll
-    for (int o = 0; o < OB; ++o)
-#pragma unroll
-      for (int q = 0; q < RB / 2; ++q) unpack2(acc[o][q], v[o * RB + 2 * q], v[o * RB + 2 * q + 1]);
-    int n = N, id = 0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      if (n > 1) {
-        n >>= 1;
-        const bool hi = lane & o;
-        id += hi ? n : 0;
-#pragma unroll
-        for (int i = 0; i < N / 2; ++i)
-          if (i < n) {
-            const float keep = hi ? v[i + n] : v[i], send = hi ? v[i] : v[i + n];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-          }
-      } else {
-        v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-      }
-    }
-    constexpr int LEFT = N > 32 ? N / 32 : 1, COPIES = N < 32 ? 32 / N : 1;  // sums per lane; lanes that hold the same one
-    if ((lane & (COPIES - 1)) == 0) {
-#pragma unroll
-      for (int i = 0; i < LEFT; ++i) {
-        const int o = OB * g + (id + i) / RB, r = (id + i) % RB;
-        if (o < e1 && r < nr) {
-          const size_t at_out = (size_t)(r0 + r) * e1 + o;
-          logits[at_out] = beta != 0.f ? fmaf(beta, bias[at_out], v[i]) : v[i];
-        }
-      }
-    }
+    for (int s = 0; s < RL_WARPS; ++s) v += part[(m * RL_WARPS + s) * RL_PART + at];
+    const size_t at_out = (size_t)(r0 + r) * e1 + o;
+    logits[at_out] = beta != 0.f ? fmaf(beta, bias[at_out], v) : v;
   }
 }
 
-// Shapes by the number of rows: up to eight rows, one output per warp over as many blocks as there are multiprocessors (the
-// weights' latency is all there is); up to 96, eight rows and four outputs; beyond that sixteen rows, so that the weights are
-// read from L2 once per sixteen rows.
+// As many blocks side by side as share out the tiles of all the row groups over the multiprocessors, at least as many as the
+// partial sums of a block's tiles need to fit into its shared memory.
 template <int SRC>
 static int launch_logits(const void* src, const float* nw, float eps, __half* rows16, const __nv_bfloat16* w, const float* bias, float* logits,
                          int rows, int e1, float beta, int* zero, int n_zero, cudaStream_t st) {
   const DrbDevice& dev = drb_device(st);
   if (!dev.ready) return -2;
-  auto go = [&](auto kern, int rb, int ob) {
-    const int gx = (rows + rb - 1) / rb, groups = (e1 + ob - 1) / ob;
-    const int gy = min(groups, max(1, dev.sms / gx));
-    drb_launch(kern, dim3(gx, gy), dim3(RL_WARPS * 32), (size_t)rb * RL_K * 4, st, dev.pdl, src, nw, eps, rows16, w, bias, logits, rows, e1, beta, zero, n_zero);
-  };
-  if (rows <= 8) go(k_router_logits<SRC, 8, 1>, 8, 1);
-  else if (rows <= 96) go(k_router_logits<SRC, 8, 4>, 8, 4);
-  else go(k_router_logits<SRC, 16, 4>, 16, 4);
+  const int gx = (rows + RL_ROWS - 1) / RL_ROWS, tiles = (e1 + RL_TILE - 1) / RL_TILE;
+  const int gy = min(tiles, max((tiles + RL_MAX_TILES - 1) / RL_MAX_TILES, dev.sms / gx));
+  drb_launch(k_router_logits<SRC>, dim3(gx, gy), dim3(RL_WARPS * 32), logits_smem((tiles + gy - 1) / gy), st, dev.pdl, src, nw, eps, rows16, w, bias,
+             logits, rows, e1, beta, zero, n_zero);
   return 0;
 }
 
 template <int SRC>
 static cudaError_t configure_logits() {
-  auto one = [](auto kern, size_t smem) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return e != cudaSuccess ? e : drb_carveout(kern);
-  };
-  cudaError_t e;
-  if ((e = one(k_router_logits<SRC, 8, 1>, logits_smem<8>())) != cudaSuccess) return e;
-  if ((e = one(k_router_logits<SRC, 8, 4>, logits_smem<8>())) != cudaSuccess) return e;
-  return one(k_router_logits<SRC, 16, 4>, logits_smem<16>());
+  const cudaError_t e = cudaFuncSetAttribute(k_router_logits<SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)logits_smem(RL_MAX_TILES));
+  return e != cudaSuccess ? e : drb_carveout(k_router_logits<SRC>);
 }
 
 // Two warps per row, behind the routing: the row's slots (the exclusive scan of the expert counts, which every block makes for

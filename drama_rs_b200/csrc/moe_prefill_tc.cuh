@@ -193,8 +193,8 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   int end = 0;
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    const int c = __ldg(counts + e);
-    if (c > 0) end = max(end, __ldg(offsets + e) + c);
+    const int c = __ldcg(counts + e);
+    if (c > 0) end = max(end, __ldcg(offsets + e) + c);
   }
   end = __reduce_max_sync(0xffffffffu, end);
   if ((threadIdx.x & 31) == 0) atomicMax(&s_total, end);
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(256)
   constexpr int PER = H / 8 / 32;
   for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < total + rows_sh; i += gridDim.x * (blockDim.x >> 5)) {
     const bool sh = i >= total;
-    const int row = sh ? i - total : (row_of ? __ldg(row_of + i) : i);
+    const int row = sh ? i - total : (row_of ? __ldcg(row_of + i) : i);
     const uint4* p = x + (size_t)row * (H / 8);
     unsigned char* out = sh ? sh_dst + (size_t)(i - total) * TOKEN_STRIDE : dst + (size_t)i * TOKEN_STRIDE;
     uint4 v[PER];
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
       const int s = threadIdx.x * PER + j;
-      const int cnt = s >= n_sets ? 0 : s == 0 ? a.rows_sh : __ldg(a.counts + s - 1);
+      const int cnt = s >= n_sets ? 0 : s == 0 ? a.rows_sh : __ldcg(a.counts + s - 1);
       it[j] = sum, sum += ((cnt + NT - 1) / NT) * MT;
     }
     int incl = sum;
@@ -659,9 +659,9 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
       const Item it = decode(item);
       wait_at<DRB_ERR_EMPTY_WAIT>(ctl.tabempty, rt, spent);
       Tab& tab = tabs[rt.i];
-      const int cnt = it.shared ? a.rows_sh : __ldg(a.counts + it.e);
+      const int cnt = it.shared ? a.rows_sh : __ldcg(a.counts + it.e);
       const int nt = min(NT, cnt - it.n0);
-      const int srow = (it.shared ? 0 : __ldg(a.offsets + it.e)) + it.n0, end = srow + nt, rest = nt & 7;
+      const int srow = (it.shared ? 0 : __ldcg(a.offsets + it.e)) + it.n0, end = srow + nt, rest = nt & 7;
       // Contiguous rows go by boxes of eight. What is left over takes one more box, of the last eight rows: no row beyond
       // the item's end is touched, and the columns of rows that it repeats (or that are not the item's) have no result
       // row. Among the array's first eight rows, and for scattered rows, gather4 fetches the rows by number.
@@ -675,11 +675,11 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
         const int slot = start >= 0 && t >= 8 * full ? start + (t - 8 * full) : srow + t;
         const bool own = slot >= srow + (t >= 8 * full ? 8 * full : 0) && slot < end;
         if (GEMM == 0) tab.fac[t] = own && fac ? __ldcg(reinterpret_cast<const float*>(fac + (size_t)slot * TOKEN_STRIDE + H * 2)) : 1.f;
-        tab.dst[t] = !own ? -1 : (GEMM == 1 && !it.shared && a.dst_row_of) ? __ldg(a.dst_row_of + slot) : slot;
+        tab.dst[t] = !own ? -1 : (GEMM == 1 && !it.shared && a.dst_row_of) ? __ldcg(a.dst_row_of + slot) : slot;
       }
       for (int t = lane; t < 4 * quads; t += 32) {
         const int slot = srow + min(8 * full + t, nt - 1);
-        tab.rows[t] = (GEMM == 0 && !PREP && !it.shared && a.row_of) ? __ldg(a.row_of + slot) : slot;
+        tab.rows[t] = (GEMM == 0 && !PREP && !it.shared && a.row_of) ? __ldcg(a.row_of + slot) : slot;
       }
       if (lane == 0) tab.cols = cols, tab.used = (start >= 0 ? 8 * full + 8 : nt + 7) & ~7, tab.mt = it.mt, tab.shared = it.shared, tab.full = full, tab.srow = srow, tab.start = start, tab.quads = quads;
       __syncwarp();
