@@ -245,6 +245,14 @@ __global__ void __launch_bounds__(256)
 // SiLU for a result that is rounded to fp16: the division within 2 units of the last fp32 place.
 DRB_DEV float silu_fast(float x) { return __fdividef(x, 1.f + expf(-x)); }
 
+// *p = v unless at < 0.
+DRB_DEV void store_valid(__half* p, __half v, int at) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %2, 0;\n\t@p st.global.b16 [%0], %1;\n\t}" ::"l"(p), "h"(__half_as_ushort(v)), "r"(at) : "memory");
+}
+DRB_DEV void store_valid(float* p, float v, int at) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %2, 0;\n\t@p st.global.f32 [%0], %1;\n\t}" ::"l"(p), "f"(v), "r"(at) : "memory");
+}
+
 DRB_DEV void lds128(uint32_t addr, uint32_t* v) {
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
 }
@@ -735,36 +743,40 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
       const int j = mt * (TILE_M / 2) + (r >> 1);
       __half* const act = static_cast<__half*>(sh ? a.sh_dst : a.dst) + (FMT == 0 ? perm_pos(j) : j);
       float* const y = static_cast<float*>(sh ? a.sh_dst : a.dst) + mt * TILE_M + r;
-      const bool odd = lane & 1;
-      auto columns = [&](int c0, const uint32_t(&v)[8]) {  // the results of eight columns
+      const bool odd = lane & 1, peers = GEMM == 1 && a.peer_y && !sh;
+      // The results of eight columns. The stores carry their own predicate: behind a branch on it the arithmetic of one column
+      // waited for the store of the one before (gate/up, 64 columns: 7000 cycles per item).
+      auto columns = [&](int c0, const uint32_t(&v)[8]) {
+        if (GEMM == 0) {
+          // even lanes hold gate rows, odd lanes their up rows. Per pair of tokens the lanes swap what the other needs: the
+          // even lane finishes the first token, the odd lane the second.
+          float got[4];
 #pragma unroll
-        for (int i4 = 0; i4 < 8; i4 += 4) {
-          const int4 d4 = *reinterpret_cast<const int4*>(&tab.dst[c0 + i4]);
-          const int dst[4] = {d4.x, d4.y, d4.z, d4.w};
-          if (GEMM == 0) {
-            // even lanes hold gate rows, odd lanes their up rows. Per pair of tokens the lanes swap what the other needs: the
-            // even lane finishes the first token, the odd lane the second.
-            const float4 f4 = *reinterpret_cast<const float4*>(&tab.fac[c0 + i4]);
-            const float fac[4] = {f4.x, f4.y, f4.z, f4.w};
+          for (int i = 0; i < 4; ++i) got[i] = __shfl_xor_sync(0xffffffffu, __uint_as_float(odd ? v[2 * i] : v[2 * i + 1]), 1);
 #pragma unroll
-            for (int i = 0; i < 4; i += 2) {
-              const float v0 = __uint_as_float(v[i4 + i]), v1 = __uint_as_float(v[i4 + i + 1]);
-              const float got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
-              const int dt = odd ? dst[i + 1] : dst[i];
-              const float f = odd ? fac[i + 1] : fac[i];
-              if (dt >= 0) act[(size_t)dt * I] = f2h_sat(silu_fast((odd ? got : v0) * f) * ((odd ? v1 : got) * f));
-            }
-          } else {
+          for (int i = 0; i < 4; ++i) {
+            const int2 d2 = *reinterpret_cast<const int2*>(&tab.dst[c0 + 2 * i]);
+            const float2 f2 = *reinterpret_cast<const float2*>(&tab.fac[c0 + 2 * i]);
+            const int dt = odd ? d2.y : d2.x;
+            const float f = odd ? f2.y : f2.x;
+            const float own = __uint_as_float(odd ? v[2 * i + 1] : v[2 * i]);
+            store_valid(act + (ptrdiff_t)dt * I, f2h_sat(silu_fast((odd ? got[i] : own) * f) * ((odd ? own : got[i]) * f)), dt);
+          }
+        } else {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float val = __uint_as_float(v[i4 + i]);
-              if (dst[i] < 0) continue;
-              if (a.peer_y && !sh) {
+          for (int i4 = 0; i4 < 8; i4 += 4) {
+            const int4 d4 = *reinterpret_cast<const int4*>(&tab.dst[c0 + i4]);
+            const int dst[4] = {d4.x, d4.y, d4.z, d4.w};
+            if (peers) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                if (dst[i] < 0) continue;
                 const int s = dst[i] / a.peer_cap;
-                a.peer_y[s][((size_t)a.peer_rank * a.peer_cap + (dst[i] - s * a.peer_cap)) * H + mt * TILE_M + r] = val;
-              } else {
-                y[(size_t)dst[i] * H] = val;
+                a.peer_y[s][((size_t)a.peer_rank * a.peer_cap + (dst[i] - s * a.peer_cap)) * H + mt * TILE_M + r] = __uint_as_float(v[i4 + i]);
               }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) store_valid(y + (ptrdiff_t)dst[i] * H, __uint_as_float(v[i4 + i]), dst[i]);
             }
           }
         }
@@ -780,19 +792,20 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
           }
       } else {
 #pragma unroll 1
-        for (int c0 = 0; c0 < cols; c0 += 8) {
-          uint32_t v[8];
-          tmem_ld8(acc + (uint32_t)c0, v);
-          if (c0 + 8 >= cols) {  // everything is in registers: the accumulator is free
+        for (int c0 = 0; c0 < cols; c0 += 16) {
+          uint32_t v[2][8];
+          tmem_ld16(acc + (uint32_t)c0, v);
+          if (c0 + 16 >= cols) {  // everything is in registers: the accumulator is free
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&ctl.accfree[rc.i]);
           }
-          columns(c0, v);
+          columns(c0, v[0]);
+          if (c0 + 8 < cols) columns(c0 + 8, v[1]);
         }
         rc.next();
       }
-      if (GEMM == 1 && a.peer_y && !sh) __threadfence_system();  // before the flag that a later kernel writes to the peers
+      if (peers) __threadfence_system();  // before the flag that a later kernel writes to the peers
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl.tabempty[rt.i]);
       rt.next(SETS);

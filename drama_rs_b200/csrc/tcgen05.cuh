@@ -67,14 +67,7 @@ DRB_DEV void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// Eight of them.
-DRB_DEV void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "r"(taddr)
-               : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
+DRB_DEV void tmem_ld16(uint32_t taddr, uint32_t (&v)[2][8]) { tmem_ld16(taddr, reinterpret_cast<uint32_t(&)[16]>(v)); }
 
 // Byte offset of 16-byte chunk c (0..7) of row r inside a K-major 128-byte-swizzled tile.
 DRB_DEV uint32_t swz_off(int r, int c) { return (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((c ^ (r & 7)) << 4)); }
