@@ -130,3 +130,21 @@ def test_gathered_rows_and_stored_results(st, rows):
     assert device_error_word() == 0
     for a, b in zip(out["block"], out["peers"]):
         assert np.linalg.norm(a - b) <= 2e-4 * np.linalg.norm(a)
+
+
+@pytest.mark.parametrize("f16", [True, False], ids=["f16", "bf16"])
+@pytest.mark.parametrize("rows,e1", [(1, 257), (15, 1), (16, 8), (17, 9), (40, 257), (2400, 257), (2400, 401)])
+def test_router_logits_tiles(st, rows, e1, f16):
+    """Row groups of 16, output tiles of 8, and more row groups than multiprocessors (all the tiles in one block, or in two)."""
+    rng = np.random.Generator(np.random.PCG64(rows + e1))
+    x = rng.standard_normal((rows, 2048), dtype=np.float32) * rng.choice([1e-3, 1.0, 30.0], (rows, 1)).astype(np.float32)
+    xb = x.astype(np.float16) if f16 else synth.f32_to_bf16_bits(x)
+    wb = synth.f32_to_bf16_bits(rng.standard_normal((e1, 2048), dtype=np.float32) * 0.02)
+    bias = rng.standard_normal((rows, e1), dtype=np.float32)
+    dx, dw, dl = DevBuf.from_array(xb, st), DevBuf.from_array(wb, st), DevBuf.from_array(bias, st)
+    call = ffi.lib().drb_router_logits_f16 if f16 else ffi.lib().drb_router_logits
+    launched(call(dx.at(0), dw.at(0), dl.at(0), rows, e1, 2048, 2.0, st.raw), "router_logits")
+    wide = lambda bits: (bits.astype(np.uint32) << 16).view(np.float32).astype(np.float64)  # noqa: E731
+    xv, wv = xb.astype(np.float64) if f16 else wide(xb), wide(wb)
+    err = np.abs(dl.download(np.float32, rows * e1, st).reshape(rows, e1) - (xv @ wv.T + 2.0 * bias))
+    assert (err <= 3e-7 * (np.abs(xv) @ np.abs(wv).T + 2.0 * np.abs(bias)) + 1e-9).all()
