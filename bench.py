@@ -288,7 +288,7 @@ def parity_check(st) -> dict:
 
 def prefill_extra(torch, layers, st, ext_stream) -> dict:
     """Benchmark configuration 3 on this GPU: 300 rows through one MoE layer, Zipf(1.1) expert popularity. The library's
-    own sequence (seven launches, no library GEMM) from a graph, its two grouped tensor-core GEMMs alone, and the
+    own sequence (one call, six launches, no library GEMM) from a graph, its two grouped tensor-core GEMMs alone, and the
     reference's call sequence (src/engine.rs:544-604) with host rows in. Four layers are rotated so the expert weights
     come from HBM."""
     from drama_rs_b200.engine import MoePrefill
