@@ -641,6 +641,99 @@ __global__ void __launch_bounds__(SC_THREADS)
   }
 }
 
+// router::k_moe_topk and k_scatter_rows in one launch for up to sixteen rows, where a launch's way costs more than its work. Block r
+// copies row r; every block forms the routing of all the rows for itself, a warp per row, so nothing crosses blocks: the experts'
+// rows are sixteen-bit masks, a pair's rank is the number of rows before it in its expert's mask. Weights and order have the same bits as
+// k_moe_topk's (the same sums in the same order; larger probability, then lower index).
+constexpr int FEW_ROWS = 16, FEW_THREADS = FEW_ROWS * 32;
+__global__ void __launch_bounds__(FEW_THREADS)
+    k_route_few(const float* __restrict__ logits, const __half* __restrict__ rows16, int rows, int E, int topk, int* __restrict__ idx,
+                float* __restrict__ wts, float* __restrict__ sgate, int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ slot_of,
+                int* __restrict__ row_of, unsigned char* __restrict__ dst, unsigned char* __restrict__ sh_dst) {
+  __shared__ unsigned mask[256];
+  __shared__ int offs[256], tot[8], to[32];
+  pdl_launch_dependents();
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, row = blockIdx.x;
+  if (t < 256) mask[t] = 0u;
+  __syncthreads();
+  pdl_wait();
+  constexpr int PIECES = H / 8;  // 16-byte pieces of a row; threads t and t + 256 hold piece t and share out the copies
+  uint4 v = __ldcg(reinterpret_cast<const uint4*>(rows16 + (size_t)row * H) + (t & (PIECES - 1)));
+  static_assert(FEW_THREADS == 2 * PIECES, "two threads per piece");
+  int mine = 0;  // lane k < topk of warp r: the k-th expert of row r
+  if (warp < rows) {
+    const float* l = logits + (size_t)warp * (E + 1);
+    float x[8], m = -INFINITY, ws[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      x[j] = lane + 32 * j < E ? __ldcg(l + lane + 32 * j) : -INFINITY;
+    }
+    // the maximum on order-preserving integer keys, as router::softmax_topk takes it
+    unsigned ord = 0u;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const unsigned b = __float_as_uint(x[j]);
+      ord = max(ord, (b & 0x80000000u) ? ~b : (b | 0x80000000u));
+    }
+    m = router::ord_to_float(__reduce_max_sync(0xffffffffu, ord));
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      x[j] = lane + 32 * j < E ? expf(x[j] - m) : 0.f;
+      ws[j] = warp_sum(x[j]);
+    }
+    const float z = ((ws[0] + ws[4]) + (ws[2] + ws[6])) + ((ws[1] + ws[5]) + (ws[3] + ws[7]));
+    unsigned key[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) key[j] = lane + 32 * j < E ? __float_as_uint(x[j] / z) + 1u : 0u;
+    float top = 0.f, total = 0.f;
+    for (int k = 0; k < topk; ++k) {
+      unsigned best = key[0];
+#pragma unroll
+      for (int j = 1; j < 8; ++j) best = max(best, key[j]);
+      best = __reduce_max_sync(0xffffffffu, best);
+      int e = 256;
+#pragma unroll
+      for (int j = 7; j >= 0; --j) e = key[j] == best ? lane + 32 * j : e;
+      e = __reduce_min_sync(0xffffffffu, e);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) key[j] = e == lane + 32 * j ? 0u : key[j];
+      const float p = __uint_as_float(best - 1u);
+      total += p;  // rank order, as the reference accumulates
+      if (lane == k) mine = e, top = p;
+    }
+    if (lane < topk) {
+      atomicOr(&mask[mine], 1u << warp);
+      if (warp == row) idx[row * topk + lane] = mine, wts[row * topk + lane] = top / total;
+    }
+    if (warp == row && lane == 0) sgate[row] = __ldcg(l + E);
+  }
+  __syncthreads();
+  const int c = t < 256 ? __popc(mask[t]) : 0;
+  int incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  if (lane == 31 && warp < 8) tot[warp] = incl;
+  __syncthreads();
+  if (t < 256) {
+    int before = incl - c;
+    for (int q = 0; q < warp; ++q) before += tot[q];
+    offs[t] = before;
+    if (row == 0 && t < E) offsets[t] = before, counts[t] = c;
+  }
+  __syncthreads();
+  if (warp == row && lane < topk) {
+    const int slot = offs[mine] + __popc(mask[mine] & ((1u << row) - 1u));
+    to[lane] = slot, slot_of[row * topk + lane] = slot, row_of[slot] = row;
+  }
+  __syncthreads();
+  v = make_uint4(prmt(v.x, v.z, 0x5410u), prmt(v.x, v.z, 0x7632u), prmt(v.y, v.w, 0x5410u), prmt(v.y, v.w, 0x7632u));
+  for (int k = t / PIECES; k <= topk; k += 2)
+    reinterpret_cast<uint4*>(k < topk ? dst + (size_t)to[k] * pft::TOKEN_STRIDE : sh_dst + (size_t)row * pft::TOKEN_STRIDE)[t & (PIECES - 1)] = v;
+}
+
 // offsets[e] = sum of counts[0..e): the exclusive scan the reference does on the host between two launches
 // (src/engine.rs:567-574). One block, any number of experts.
 __global__ void __launch_bounds__(256) k_offsets(const int* __restrict__ counts, int E, int* __restrict__ offsets) {
@@ -677,6 +770,7 @@ static cudaError_t configure_all() {
   if ((e = configure_logits<LOGITS_F16>()) != cudaSuccess) return e;
   if ((e = configure_logits<LOGITS_BF16>()) != cudaSuccess) return e;
   if ((e = drb_carveout(k_scatter_rows)) != cudaSuccess) return e;
+  if ((e = drb_carveout(k_route_few)) != cudaSuccess) return e;
   if ((e = drb_carveout(k_count)) != cudaSuccess) return e;
   if ((e = drb_carveout(k_permute)) != cudaSuccess) return e;
   if ((e = drb_carveout(k_combine<8>)) != cudaSuccess) return e;
@@ -944,14 +1038,19 @@ extern "C" int drb_moe_prefill_layer(const drb_moe_layer* w, const drb_prefill_b
                                                    static_cast<const __nv_bfloat16*>(w->router), b->logit_bias, b->logits, rows, e + 1,
                                                    b->logit_bias ? 1.f : 0.f, b->counts, e, st);
   if (r != 0) return r;
-  // The pairs' ranks: two warps read each, so they do not share slot_of's place; act is free until the gate/up kernel writes it.
-  int* rank = reinterpret_cast<int*>(b->act);
-  drb_launch(router::k_moe_topk<true>, dim3(rows), dim3(router::THREADS), 0, st, dev.pdl, (const float*)b->logits, e, topk, e + 1, b->idx, b->wts,
-             b->sgate, b->counts, rank);
-  const int blocks = (rows + pf::SC_ROWS - 1) / pf::SC_ROWS;
-  drb_launch(pf::k_scatter_rows, dim3(blocks < 8 * dev.sms ? blocks : 8 * dev.sms), dim3(pf::SC_THREADS), 0, st, dev.pdl, (const __half*)b->rows16,
-             (const int*)b->idx, rows, topk, (const int*)b->counts, e, b->offsets, b->slot_of, (const int*)rank, b->row_of,
-             reinterpret_cast<unsigned char*>(b->y), reinterpret_cast<unsigned char*>(b->sh_out));
+  if (rows <= pf::FEW_ROWS) {
+    drb_launch(pf::k_route_few, dim3(rows), dim3(pf::FEW_THREADS), 0, st, dev.pdl, (const float*)b->logits, (const __half*)b->rows16, rows, e, topk, b->idx,
+               b->wts, b->sgate, b->counts, b->offsets, b->slot_of, b->row_of, reinterpret_cast<unsigned char*>(b->y), reinterpret_cast<unsigned char*>(b->sh_out));
+  } else {
+    // The pairs' ranks: two warps read each, so they do not share slot_of's place; act is free until the gate/up kernel writes it.
+    int* rank = reinterpret_cast<int*>(b->act);
+    drb_launch(router::k_moe_topk<true>, dim3(rows), dim3(router::THREADS), 0, st, dev.pdl, (const float*)b->logits, e, topk, e + 1, b->idx, b->wts,
+               b->sgate, b->counts, rank);
+    const int blocks = (rows + pf::SC_ROWS - 1) / pf::SC_ROWS;
+    drb_launch(pf::k_scatter_rows, dim3(blocks < 8 * dev.sms ? blocks : 8 * dev.sms), dim3(pf::SC_THREADS), 0, st, dev.pdl, (const __half*)b->rows16,
+               (const int*)b->idx, rows, topk, (const int*)b->counts, e, b->offsets, b->slot_of, (const int*)rank, b->row_of,
+               reinterpret_cast<unsigned char*>(b->y), reinterpret_cast<unsigned char*>(b->sh_out));
+  }
   pft::Block k = {};
   k.gu_w = w->gu_q, k.gu_s = w->gu_sm, k.d_w = w->d_q, k.d_s = w->d_sm;
   k.sgu_q = w->sgu_q, k.sgu_s = w->sgu_s, k.sd_q = w->sd_q, k.sd_s = w->sd_s;

@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 from drama_rs_b200 import ffi, synth
+from drama_rs_b200.engine import MoePrefill
 from drama_rs_b200.gpu import DevBuf, Stream, launched
 from drama_rs_b200.model import Fp8Experts, MoeLayer
 from oracle import moe_oracle as orc
@@ -148,3 +149,25 @@ def test_router_logits_tiles(st, rows, e1, f16):
     xv, wv = xb.astype(np.float64) if f16 else wide(xb), wide(wb)
     err = np.abs(dl.download(np.float32, rows * e1, st).reshape(rows, e1) - (xv @ wv.T + 2.0 * bias))
     assert (err <= 3e-7 * (np.abs(xv) @ np.abs(wv).T + 2.0 * np.abs(bias)) + 1e-9).all()
+
+
+@pytest.mark.parametrize("experts,topk", [(256, 8), (40, 3), (8, 8)])
+@pytest.mark.parametrize("rows", [1, 2, 16])
+def test_few_rows_route_like_many(st, experts, topk, rows):
+    """Up to sixteen rows take one routing launch, more take two: weights, experts and results of a row are the same."""
+    host = synth.make_layer(35, synth.MoeShape(experts=experts))
+    dev = MoeLayer.upload(host, st)
+    x = synth.make_x(36, 17, 2048)
+    x[3] = x[2]  # equal rows, and ties between experts' logits in a row of zeros
+    x[4] = 0.0
+    few, many = MoePrefill(dev, rows, topk, st=st), MoePrefill(dev, 17, topk, st=st)
+    y, ref = few.run(x[:rows]), many.run(x)
+    assert device_error_word() == 0
+    for name in ("idx", "wts"):
+        a, b = (getattr(p, name).download(np.uint32, rows * topk, st) for p in (few, many))
+        assert np.array_equal(a, b), name
+    assert np.array_equal(few.sgate.download(np.uint32, rows, st), many.sgate.download(np.uint32, rows, st))
+    idx = few.idx.download(np.int32, rows * topk, st)
+    assert np.array_equal(few.counts.download(np.int32, experts, st), np.bincount(idx, minlength=experts))
+    assert sorted(few.slot_of.download(np.int32, rows * topk, st)) == list(range(rows * topk))
+    assert np.abs(y - ref[:rows]).max() <= 1e-6 * np.abs(ref).max()
