@@ -641,12 +641,14 @@ __global__ void __launch_bounds__(SC_THREADS)
   }
 }
 
-// router::k_moe_topk and k_scatter_rows in one launch for up to sixteen rows, where a launch's way costs more than its work. Block r
+// router::k_moe_topk and k_scatter_rows in one launch for up to 32 rows, where a launch's way costs more than its work. Block r
 // copies row r; every block forms the routing of all the rows for itself, a warp per row, so nothing crosses blocks: the experts'
-// rows are sixteen-bit masks, a pair's rank is the number of rows before it in its expert's mask. Weights and order have the same bits as
+// rows are bit masks, a pair's rank is the number of rows before it in its expert's mask. Weights and order have the same bits as
 // k_moe_topk's (the same sums in the same order; larger probability, then lower index).
-constexpr int FEW_ROWS = 16, FEW_THREADS = FEW_ROWS * 32;
-__global__ void __launch_bounds__(FEW_THREADS)
+// A whole call: 49.3 -> 46.5 us at 5 rows, 73.6 -> 68.8 at 16, 77.8 -> 75.7 at 20, 91.8 -> 90.6 at 32; the redundant part grows with the
+// rows, and beyond 32 a block has no warp per row.
+constexpr int FEW_ROWS = 32, FEW_MIN_THREADS = 512;  // blocks of 32 threads per row, but at least so many for the copies
+__global__ void __launch_bounds__(FEW_ROWS * 32)
     k_route_few(const float* __restrict__ logits, const __half* __restrict__ rows16, int rows, int E, int topk, int* __restrict__ idx,
                 float* __restrict__ wts, float* __restrict__ sgate, int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ slot_of,
                 int* __restrict__ row_of, unsigned char* __restrict__ dst, unsigned char* __restrict__ sh_dst) {
@@ -657,9 +659,8 @@ __global__ void __launch_bounds__(FEW_THREADS)
   if (t < 256) mask[t] = 0u;
   __syncthreads();
   pdl_wait();
-  constexpr int PIECES = H / 8;  // 16-byte pieces of a row; threads t and t + 256 hold piece t and share out the copies
+  constexpr int PIECES = H / 8;  // 16-byte pieces of a row; threads t, t + 256, ... hold piece t and share out the copies
   uint4 v = __ldcg(reinterpret_cast<const uint4*>(rows16 + (size_t)row * H) + (t & (PIECES - 1)));
-  static_assert(FEW_THREADS == 2 * PIECES, "two threads per piece");
   int mine = 0;  // lane k < topk of warp r: the k-th expert of row r
   if (warp < rows) {
     const float* l = logits + (size_t)warp * (E + 1);
@@ -730,7 +731,7 @@ __global__ void __launch_bounds__(FEW_THREADS)
   }
   __syncthreads();
   v = make_uint4(prmt(v.x, v.z, 0x5410u), prmt(v.x, v.z, 0x7632u), prmt(v.y, v.w, 0x5410u), prmt(v.y, v.w, 0x7632u));
-  for (int k = t / PIECES; k <= topk; k += 2)
+  for (int k = t / PIECES; k <= topk; k += blockDim.x / PIECES)
     reinterpret_cast<uint4*>(k < topk ? dst + (size_t)to[k] * pft::TOKEN_STRIDE : sh_dst + (size_t)row * pft::TOKEN_STRIDE)[t & (PIECES - 1)] = v;
 }
 
@@ -1014,7 +1015,7 @@ extern "C" int drb_moe_prefill_block_peers(const uint8_t* gu_q, const __half2* g
 }
 
 // One MoE block over `rows` rows in one call (include/dramakernels.h): what MoePrefill's own sequence of calls does, in six
-// launches, each started while the one before drains.
+// launches (five up to 32 rows), each started while the one before drains.
 struct drb_prefill_buffers {
   float* x;
   __half* rows16;
@@ -1039,7 +1040,7 @@ extern "C" int drb_moe_prefill_layer(const drb_moe_layer* w, const drb_prefill_b
                                                    b->logit_bias ? 1.f : 0.f, b->counts, e, st);
   if (r != 0) return r;
   if (rows <= pf::FEW_ROWS) {
-    drb_launch(pf::k_route_few, dim3(rows), dim3(pf::FEW_THREADS), 0, st, dev.pdl, (const float*)b->logits, (const __half*)b->rows16, rows, e, topk, b->idx,
+    drb_launch(pf::k_route_few, dim3(rows), dim3(rows * 32 <= pf::FEW_MIN_THREADS ? pf::FEW_MIN_THREADS : pf::FEW_ROWS * 32), 0, st, dev.pdl, (const float*)b->logits, (const __half*)b->rows16, rows, e, topk, b->idx,
                b->wts, b->sgate, b->counts, b->offsets, b->slot_of, b->row_of, reinterpret_cast<unsigned char*>(b->y), reinterpret_cast<unsigned char*>(b->sh_out));
   } else {
     // The pairs' ranks: two warps read each, so they do not share slot_of's place; act is free until the gate/up kernel writes it.

@@ -152,15 +152,15 @@ def test_router_logits_tiles(st, rows, e1, f16):
 
 
 @pytest.mark.parametrize("experts,topk", [(256, 8), (40, 3), (8, 8)])
-@pytest.mark.parametrize("rows", [1, 2, 16])
+@pytest.mark.parametrize("rows", [1, 2, 16, 17, 32])
 def test_few_rows_route_like_many(st, experts, topk, rows):
-    """Up to sixteen rows take one routing launch, more take two: weights, experts and results of a row are the same."""
+    """Up to 32 rows take one routing launch, more take two: weights, experts and results of a row are the same."""
     host = synth.make_layer(35, synth.MoeShape(experts=experts))
     dev = MoeLayer.upload(host, st)
-    x = synth.make_x(36, 17, 2048)
+    x = synth.make_x(36, 33, 2048)
     x[3] = x[2]  # equal rows, and ties between experts' logits in a row of zeros
     x[4] = 0.0
-    few, many = MoePrefill(dev, rows, topk, st=st), MoePrefill(dev, 17, topk, st=st)
+    few, many = MoePrefill(dev, rows, topk, st=st), MoePrefill(dev, 33, topk, st=st)
     y, ref = few.run(x[:rows]), many.run(x)
     assert device_error_word() == 0
     for name in ("idx", "wts"):
