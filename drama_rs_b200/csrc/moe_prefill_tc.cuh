@@ -447,13 +447,13 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
         rr.next(group);
 #pragma unroll 1
         for (int step = group; step < NSTEP; step += GROUPS) {
-          wait_at<DRB_ERR_FULL_WAIT>(ctl.rawfull, rr, spent);
-          // piece 4 half + j of the row stands at xa ^ 16 j: in the swizzled row the piece's number is xor-ed into the address
-          uint32_t xa = x_row + rr.i * RAW_BYTES;
           uint32_t sm[2];
           lds64(GEMM == 0 ? sm_a ^ (step << 4) : sm_a + 16 * step, sm[0], sm[1]);
+          a_wait();  // ahead of the raw stage: see the loader
+          wait_at<DRB_ERR_FULL_WAIT>(ctl.rawfull, rr, spent);
           const bool small = __all_sync(0xffffffffu, max(sm[0] & 0x7fffu, sm[1] & 0x7fffu) < 0x2C00u);  // both scales below 2^-4
-          a_wait();
+          // piece 4 half + j of the row stands at xa ^ 16 j: in the swizzled row the piece's number is xor-ed into the address
+          uint32_t xa = x_row + rr.i * RAW_BYTES;
           uint32_t to = acol + ra.i * A_COLS;
 #pragma unroll
           for (int g = 0; g < 2; ++g) {
@@ -496,6 +496,7 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
           const __half2 s2 = __half2half2(s_next);
           if (FMT == 0 && step + GROUPS < NSTEP) s_next = __ldg(ssrow + 2 * (step + GROUPS));
           // both stages are waited for although this warp reads one: an arrival must not run a ring's length ahead
+          if (GROUPS > 1) a_wait();  // ahead of the raw stages: see the loader
           const int sa = rr.i;
           wait_at<DRB_ERR_FULL_WAIT>(ctl.rawfull, rr, spent);
           rr.next();
@@ -518,7 +519,7 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
                 for (int q = 0; q < 2; ++q) dequant8_i8<FMT == 0 && (PREP || GEMM == 1)>(w[2 * q], w[2 * q + 1], s2, o + 8 * j + 4 * q);
               }
             }
-            if (g == 0) a_wait();
+            if (GROUPS == 1 && g == 0) a_wait();  // one group: the first conversion needs no tensor memory yet
             tmem_st32(acol + ra.i * A_COLS + g * 32, o);
           }
           __syncwarp();
@@ -593,6 +594,12 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
     // The (scale, min) pairs of an int4 item go to one of NSM slots ahead of its first raw stage. By then the raw stage NRAW
     // requests back has been read, so every item more than NSM - 1 items back is finished with its slot.
     static_assert(NSM == 0 || (NSM - 1) * NSTEP >= NRAW, "scale slots");
+    // A wait for a raw stage tests one bit of its phase, so it tells "landed" from "in flight" only once the stage's use before
+    // this one is known to have landed; boxes land in any order. A group's own uses it has waited for itself. With two groups a
+    // stage also passes from one to the other, and there the stage's MMAs vouch: after a_wait() of step s everything up to step s - NST
+    // has been converted. A step takes one raw stage or two, so the use NRAW requests back lies at least NRAW / 2 steps back: NST or more,
+    // or two, which is the group's own. Hence NRAW, and a_wait() in front of the raw stages in either branch.
+    static_assert(GROUPS == 1 || (GROUPS == 2 && NST == 3 && NRAW >= 5), "raw stages");
     Ring<NRAW> rr;
     Ring<(NSM ? NSM : 1)> rs;
     rr.par = 1;  // every raw stage starts free
