@@ -1033,6 +1033,10 @@ extern "C" int drb_moe_prefill_layer(const drb_moe_layer* w, const drb_prefill_b
                                      cudaStream_t st) {
   if (!w || !b || h != pf::H || i != pf::I || e < 1 || e > 256 || topk < 1 || topk > e || topk > 31) return -1;
   if (rows <= 0) return 0;
+  // what is read or written in 16-byte pieces, before anything is launched
+  for (const void* p : {(const void*)b->x, (const void*)b->rows16, (const void*)b->y, (const void*)b->sh_out, (const void*)b->act, (const void*)b->sh_act, w->router,
+                        w->gu_q, w->gu_sm, w->d_q, w->d_sm, w->sgu_q, w->sd_q})
+    if (reinterpret_cast<uintptr_t>(p) & 15) return -3;
   const DrbDevice& dev = drb_device(st);
   if (!dev.ready) return -2;
   const int r = pf::launch_logits<pf::LOGITS_NORM>(b->x, static_cast<const float*>(w->post_norm), eps, b->rows16,

@@ -901,8 +901,16 @@ static int run_block(const Block& b, const DrbDevice& dev, cudaStream_t st) {
   // peers y is not this call's to write: the fp16 rows are gathered as they are.
   const bool prep = b.peer_y == nullptr;
   if (!prep && (b.x_bf16 || FMT != 0)) return -1;
-  unsigned char* tok = static_cast<unsigned char*>(b.y);
-  unsigned char* shtok = static_cast<unsigned char*>(b.sh_out);
+  // Results are stored float by float, so y and sh_out may start at any float. Prepared rows start at the next 16-byte boundary: the
+  // 4 KB and the factor fill half of a row's stride, so the last one still ends inside the buffer.
+  auto align16 = [](void* p) { return reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15); };
+  unsigned char* tok = align16(b.y);
+  unsigned char* shtok = align16(b.sh_out);
+  // What the kernels read in 16-byte pieces, before anything is launched.
+  auto odd = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
+  if ((!b.prepared && odd(b.x)) || (b.E > 0 && (odd(b.gu_w) || odd(b.d_w) || odd(b.act) || (FMT == 0 && (odd(b.gu_s) || odd(b.d_s))))) ||
+      (b.rows_sh > 0 && (odd(b.sgu_q) || odd(b.sd_q) || odd(b.sh_act))))
+    return -3;
   if (prep && !b.prepared) {
     auto kp = b.x_bf16 ? k_prep_rows<true, FMT == 0> : k_prep_rows<false, FMT == 0>;
     drb_launch(kp, dim3(2 * dev.sms), dim3(256), 0, st, false, static_cast<const uint4*>(b.x), b.row_of, b.offsets, b.counts, b.E, tok, b.rows_sh, shtok);
@@ -912,7 +920,6 @@ static int run_block(const Block& b, const DrbDevice& dev, cudaStream_t st) {
   for (int gemm = 0; gemm < 2; ++gemm) {
     for (int e0 = 0; e0 == 0 || e0 < b.E; e0 += MAX_E) {
       const int ne = b.E - e0 < MAX_E ? b.E - e0 : MAX_E;
-      const uint64_t em = ne > 0 ? ne : 1;
       const bool sh = sh_on && e0 == 0;
       const size_t row = (gemm == 0 ? H : I) / WB, rows = gemm == 0 ? 2 * I : H, cols = gemm == 0 ? H : I;
       const size_t s_bytes = FMT == 0 ? rows * (cols / 64) * 4 : (rows / 128) * (cols / 128) * 4;  // scales per expert
@@ -921,14 +928,15 @@ static int run_block(const Block& b, const DrbDevice& dev, cudaStream_t st) {
       Maps m = {};
       Args a = {};
       if (gemm == 0) {
-        if (map_gate_up(&m.q, w, em, I, row) || (FMT == 0 && map_gate_up(&m.sm, sc, em, I, (H / 64) * 4)) || (sh && map_gate_up(&m.sh, b.sgu_q, 1, I, H))) return -3;
-        if (map_tokens(&m.tok8, &m.tok1, prep ? tok : b.x, H, prep ? TOKEN_STRIDE : H * 2)) return -3;
+        if (ne > 0 && (map_gate_up(&m.q, w, ne, I, row) || (FMT == 0 && map_gate_up(&m.sm, sc, ne, I, (H / 64) * 4)))) return -3;
+        if (ne > 0 && map_tokens(&m.tok8, &m.tok1, prep ? tok : b.x, H, prep ? TOKEN_STRIDE : H * 2)) return -3;
+        if (sh && map_gate_up(&m.sh, b.sgu_q, 1, I, H)) return -3;
         if (sh && map_tokens(&m.shtok8, &m.shtok1, prep ? shtok : b.x, H, prep ? TOKEN_STRIDE : H * 2)) return -3;
         a.dst = b.act, a.sh_dst = b.sh_act, a.row_of = b.row_of;
         if (prep && b.x_bf16) a.fac = tok, a.sh_fac = shtok;
       } else {
-        if (map_rows(&m.q, w, em * H, row) || (sh && map_rows(&m.sh, b.sd_q, H, I))) return -3;
-        if (map_tokens(&m.tok8, &m.tok1, b.act, I, I * 2) || (sh && map_tokens(&m.shtok8, &m.shtok1, b.sh_act, I, I * 2))) return -3;
+        if (ne > 0 && (map_rows(&m.q, w, (uint64_t)ne * H, row) || map_tokens(&m.tok8, &m.tok1, b.act, I, I * 2))) return -3;
+        if (sh && (map_rows(&m.sh, b.sd_q, H, I) || map_tokens(&m.shtok8, &m.shtok1, b.sh_act, I, I * 2))) return -3;
         a.dst = b.y, a.sh_dst = b.sh_out, a.dst_row_of = b.y_row_of;
         a.peer_y = b.peer_y, a.peer_cap = b.peer_cap, a.peer_rank = b.peer_rank;
       }

@@ -121,8 +121,9 @@ int dr_moe_permute(const int* idx, int rows, int topk, const int* offsets, int* 
                    dr_bf16* xp, int h, dr_stream st);
 /* Rows of xp sorted by expert (offsets/counts). act: scratch, 16 bits per (slot, j), contents
  * unspecified. y[slot, :] = down_e(silu(gate_e . x) * (up_e . x)). h == 2048, i == 512. The weights and the token rows are
- * addressed through TMA tensor maps built from the pointers given: act and y 16-byte aligned, -3 when the driver
- * refuses a map. Until its rows are written y is scratch: the token rows as the tensor cores want them.
+ * addressed through TMA tensor maps built from the pointers given: weights, xp and act 16-byte aligned, else -3 and nothing is
+ * launched; -3 also when the driver refuses a map. y may start at any float. Until its rows are written y is scratch: the token
+ * rows as the tensor cores want them.
  * drama.cu:799-968; ffi.rs:61-64 */
 int dr_moe_prefill(const uint8_t* gu_q, const dr_half* gu_sm, const uint8_t* d_q, const dr_half* d_sm,
                    const dr_bf16* xp, const int* offsets, const int* counts, dr_bf16* act, float* y, int e, int h, int i,
@@ -217,8 +218,8 @@ int drb_moe_prefill_block(const uint8_t* gu_q, const dr_half* gu_sm, const uint8
  * in the rows, logits, routing and x; slots inside an expert in arbitrary order) in six launches. w and buf are host
  * structs of device pointers. buf: x f32 [rows, h]; rows16 fp16 [rows, h]; logits f32 [rows, e + 1]; logit_bias f32 [rows, e + 1]
  * added to the logits, or NULL; idx, wts [rows, topk]; sgate [rows]; counts, offsets [e]; slot_of, row_of [rows * topk]; act,
- * y, sh_act, sh_out as drb_moe_prefill_block. e <= 256, topk <= 31, h == 2048, i == 512, else -1; -3 when the driver refuses a
- * tensor map. */
+ * y, sh_act, sh_out as drb_moe_prefill_block. e <= 256, topk <= 31, h == 2048, i == 512, else -1; x, rows16, act, y, sh_act, sh_out
+ * and the weights 16-byte aligned, else -3 and nothing is launched. */
 typedef struct {
   float* x;
   dr_half* rows16;

@@ -171,3 +171,60 @@ def test_few_rows_route_like_many(st, experts, topk, rows):
     assert np.array_equal(few.counts.download(np.int32, experts, st), np.bincount(idx, minlength=experts))
     assert sorted(few.slot_of.download(np.int32, rows * topk, st)) == list(range(rows * topk))
     assert np.abs(y - ref[:rows]).max() <= 1e-6 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("fmt", ["int4", "fp8"])
+def test_results_at_any_float_and_refused_addresses(st, fmt):
+    """y and sh_out may start at any float: same bits as at an aligned address, nothing written beside them. Rows, act and weights
+    are read in 16-byte pieces: other addresses are refused before anything is launched."""
+    l, shape = ffi.lib(), synth.MoeShape(experts=16)
+    counts = np.array([1, 9, 0, 3, 17, 0, 2, 8, 0, 0, 5, 33, 1, 0, 4, 7], dtype=np.int32)
+    offsets = (np.cumsum(counts) - counts).astype(np.int32)
+    n = int(counts.sum())
+    xb = synth.f32_to_bf16_bits(np.random.Generator(np.random.PCG64(4)).standard_normal((n, 2048), dtype=np.float32))
+    dxp, dcnt, doff = DevBuf(n * 4096 + 16), DevBuf.from_array(counts, st), DevBuf.from_array(offsets, st)
+    dxp.upload(xb, st)
+    dact, shact = DevBuf(n * 1024 + 16), DevBuf(n * 1024 + 16)
+    dev = MoeLayer.upload(synth.make_layer(33, shape), st)
+    if fmt == "int4":
+        shared = (*dev.shared_gate_up.rows(0), *dev.shared_down.rows(0))
+
+        def call(y, sh=None, xp=dxp.at(0), act=dact.at(0), off=0):
+            w = (C.c_void_p(dev.gate_up.q.ptr + off), dev.gate_up.sm.at(0), *dev.down.expert(0), *shared)
+            return l.drb_moe_prefill_block(*w, xp, NULL, doff.at(0), dcnt.at(0), act, y, shact.at(0), sh, n, 16, 2048, 512, 0, NULL, st.raw)
+    else:
+        f8 = Fp8Experts.upload(synth.make_fp8_experts(33, shape), st)
+
+        def call(y, sh=None, xp=dxp.at(0), act=dact.at(0), off=0):
+            return l.dr_moe_prefill_fp8(f8.gu_w.at(off), f8.gu_s.at(0), f8.d_w.at(0), f8.d_s.at(0), xp, doff.at(0), dcnt.at(0), act, y, 16, 2048, 512, st.raw)
+
+    words, got = n * 2048, {}
+    dy, dsh = DevBuf(words * 4 + 32), DevBuf(words * 4 + 32)
+    for at in (16, 4, 8, 12):
+        dy.fill(0x55, st), dsh.fill(0x55, st)
+        launched(call(dy.at(at), dsh.at(at)), "prefill")
+        for name, buf in (("y", dy), ("shared", dsh)):
+            raw = buf.download(np.uint32, words + 8, st)
+            assert (raw[: at // 4] == 0x55555555).all() and (raw[at // 4 + words :] == 0x55555555).all(), (name, at)
+            got.setdefault(name, raw[at // 4 : at // 4 + words])
+            assert np.array_equal(raw[at // 4 : at // 4 + words], got[name]), (name, at)
+    assert np.isfinite(got["y"].view(np.float32)).all() and device_error_word() == 0
+    dy.fill(0x55, st)
+    for bad in ({"xp": dxp.at(2)}, {"xp": dxp.at(8)}, {"act": dact.at(8)}, {"off": 8}):
+        assert call(dy.at(0), dsh.at(0), **bad) == -3
+    assert (dy.download(np.uint32, words, st) == 0x55555555).all() and l.dr_last_error() == 0
+
+
+def test_layer_call_refuses_addresses_it_cannot_use(st):
+    dev = MoeLayer.upload(synth.make_layer(34, synth.MoeShape(experts=16)), st)
+    pre = MoePrefill(dev, 4, st=st)
+    x = synth.make_x(37, 4, 2048)
+    pre.x.upload(x, st)
+    w, b = (a._obj for a in pre._layer_args())
+    for struct, names in ((b, ("x", "rows16", "y", "sh_out", "act", "sh_act")), (w, ("router", "gu_q", "gu_sm", "d_q", "d_sm", "sgu_q", "sd_q"))):
+        for name in names:
+            p = getattr(struct, name)
+            setattr(struct, name, p + 8)
+            assert ffi.lib().drb_moe_prefill_layer(C.byref(w), C.byref(b), 4, 16, 8, 2048, 512, 1e-6, st.raw) == -3, name
+            setattr(struct, name, p)
+    assert np.array_equal(pre.x.download(np.float32, 4 * 2048, st).reshape(4, 2048), x) and ffi.lib().dr_last_error() == 0
