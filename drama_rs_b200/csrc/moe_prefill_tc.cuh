@@ -181,31 +181,54 @@ DRB_DEV int perm_pos(int k) { return (k & ~7) | ((k & 3) << 1) | ((k >> 2) & 1);
 // outputs serve as the buffers (they are written after the gate/up kernel has read the rows), each row's factor sits behind its
 // 4 KB. bf16 rows carry a wider range than fp16: a row whose largest magnitude lies outside [2^-4, 2^15) is divided
 // by a power of two (the factor; the gate/up epilogue multiplies it back), every other row keeps its values.
+// Only the experts' own slots are read and written: offsets may leave gaps, whose row_of says nothing and whose rows of y are the
+// caller's. Every block makes the prefix sum of the counts for itself and looks a row's expert up in it.
 // One warp per row; L2 traffic only (8 KB per slot, 20 MB at 300 rows: 4 us).
+constexpr int PREP_THREADS = 256;
 template <bool BF16, bool PERM>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(PREP_THREADS)
     k_prep_rows(const uint4* __restrict__ x, const int* __restrict__ row_of, const int* __restrict__ offsets, const int* __restrict__ counts, int E,
                 unsigned char* __restrict__ dst, int rows_sh, unsigned char* __restrict__ sh_dst) {
-  __shared__ int s_total;
+  __shared__ int first[MAX_E], offs[MAX_E], wtot[PREP_THREADS / 32];  // rows of the experts before e; e's first slot
   pdl_wait();
   pdl_launch_dependents();
-  if (threadIdx.x == 0) s_total = 0;
-  __syncthreads();
-  int end = 0;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    const int c = __ldcg(counts + e);
-    if (c > 0) end = max(end, __ldcg(offsets + e) + c);
+  constexpr int PER_T = MAX_E / PREP_THREADS;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int c[PER_T], sum = 0;
+#pragma unroll
+  for (int j = 0; j < PER_T; ++j) {
+    const int e = threadIdx.x * PER_T + j;
+    c[j] = sum;
+    if (e < E) sum += max(__ldcg(counts + e), 0), offs[e] = __ldcg(offsets + e);
   }
-  end = __reduce_max_sync(0xffffffffu, end);
-  if ((threadIdx.x & 31) == 0) atomicMax(&s_total, end);
+  int incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  if (lane == 31) wtot[warp] = incl;
   __syncthreads();
-  const int total = s_total, lane = threadIdx.x & 31;
+  int before = incl - sum, total = 0;
+#pragma unroll
+  for (int w = 0; w < PREP_THREADS / 32; ++w) before += w < warp ? wtot[w] : 0, total += wtot[w];
+#pragma unroll
+  for (int j = 0; j < PER_T; ++j) first[threadIdx.x * PER_T + j] = before + c[j];
+  __syncthreads();
   constexpr int PER = H / 8 / 32;
-  for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < total + rows_sh; i += gridDim.x * (blockDim.x >> 5)) {
+  for (int i = blockIdx.x * (PREP_THREADS / 32) + warp; i < total + rows_sh; i += gridDim.x * (PREP_THREADS / 32)) {
     const bool sh = i >= total;
-    const int row = sh ? i - total : (row_of ? __ldcg(row_of + i) : i);
+    int row = i - total, slot = row;  // the shared expert's
+    if (!sh) {
+      int e = 0;  // the last expert with first[e] <= i, and so the one that owns row i
+#pragma unroll
+      for (int step = MAX_E / 2; step > 0; step >>= 1)
+        if (e + step < E && first[e + step] <= i) e += step;
+      slot = offs[e] + (i - first[e]);
+      row = row_of ? __ldcg(row_of + slot) : slot;
+    }
     const uint4* p = x + (size_t)row * (H / 8);
-    unsigned char* out = sh ? sh_dst + (size_t)(i - total) * TOKEN_STRIDE : dst + (size_t)i * TOKEN_STRIDE;
+    unsigned char* out = (sh ? sh_dst : dst) + (size_t)slot * TOKEN_STRIDE;
     uint4 v[PER];
 #pragma unroll
     for (int j = 0; j < PER; ++j) v[j] = __ldcg(p + j * 32 + lane);
@@ -913,7 +936,9 @@ static int run_block(const Block& b, const DrbDevice& dev, cudaStream_t st) {
     return -3;
   if (prep && !b.prepared) {
     auto kp = b.x_bf16 ? k_prep_rows<true, FMT == 0> : k_prep_rows<false, FMT == 0>;
-    drb_launch(kp, dim3(2 * dev.sms), dim3(256), 0, st, false, static_cast<const uint4*>(b.x), b.row_of, b.offsets, b.counts, b.E, tok, b.rows_sh, shtok);
+    for (int e0 = 0; e0 == 0 || e0 < b.E; e0 += MAX_E)  // the shared expert's rows with the first experts
+      drb_launch(kp, dim3(2 * dev.sms), dim3(PREP_THREADS), 0, st, false, static_cast<const uint4*>(b.x), b.row_of, b.offsets + e0, b.counts + e0,
+                 b.E - e0 < MAX_E ? b.E - e0 : MAX_E, tok, e0 == 0 ? b.rows_sh : 0, shtok);
   }
   // Every gate/up launch before the first down launch: y holds the token rows until then.
   const bool sh_on = b.rows_sh > 0;

@@ -228,3 +228,38 @@ def test_layer_call_refuses_addresses_it_cannot_use(st):
             assert ffi.lib().drb_moe_prefill_layer(C.byref(w), C.byref(b), 4, 16, 8, 2048, 512, 1e-6, st.raw) == -3, name
             setattr(struct, name, p)
     assert np.array_equal(pre.x.download(np.float32, 4 * 2048, st).reshape(4, 2048), x) and ffi.lib().dr_last_error() == 0
+
+
+@pytest.mark.parametrize("gathered", [False, True])
+def test_gaps_between_the_experts_slots(st, gathered):
+    """Offsets that leave gaps, and more experts than one preparing launch takes: the slots between the experts are nobody's. Their
+    row_of is not looked at (it names a row of NaN here) and their rows of y keep what the caller had there."""
+    l, e = ffi.lib(), 1026
+    host = synth.make_layer(38, synth.MoeShape(experts=2))
+    dev = MoeLayer.upload(host, st)
+    counts, offsets = np.zeros(e, dtype=np.int32), np.zeros(e, dtype=np.int32)
+    counts[[0, 1]], offsets[[0, 1]] = [3, 12], [2, 11]  # slots 0, 1, 5 .. 10 and from 23 on belong to no expert
+    n, slots = 16, 30
+    rng = np.random.Generator(np.random.PCG64(6))
+    xf = rng.standard_normal((n, 2048), dtype=np.float32)
+    xf[0] = np.nan
+    row_of = np.zeros(slots, dtype=np.int32)
+    own = np.r_[2:5, 11:23]
+    row_of[own] = rng.permutation(15) + 1
+    if not gathered:
+        xf = np.where(np.isin(np.arange(slots), own)[:, None], xf[row_of], np.float32(np.nan))
+    xb = synth.f32_to_bf16_bits(xf)
+    dx, drow, dcnt, doff = (DevBuf.from_array(a, st) for a in (xb, row_of, counts, offsets))
+    dact, dy, dsh = DevBuf(slots * 1024), DevBuf(slots * 8192), DevBuf(16)
+    dy.fill(0x55, st)
+    w = (*dev.gate_up.expert(0), *dev.down.expert(0))
+    if gathered:
+        rc = l.drb_moe_prefill_block(*w, *dev.shared_gate_up.rows(0), *dev.shared_down.rows(0), dx.at(0), drow.at(0), doff.at(0), dcnt.at(0), dact.at(0),
+                                     dy.at(0), dact.at(0), dsh.at(0), 0, e, 2048, 512, 0, NULL, st.raw)
+    else:
+        rc = l.dr_moe_prefill(*w, dx.at(0), doff.at(0), dcnt.at(0), dact.at(0), dy.at(0), e, 2048, 512, st.raw)
+    launched(rc, "prefill")
+    raw = dy.download(np.uint32, slots * 2048, st).reshape(slots, 2048)
+    assert device_error_word() == 0 and (np.delete(raw, own, axis=0) == 0x55555555).all()
+    x = synth.bf16_bits_to_f32(xb).astype(np.float64)
+    check_rows(raw.view(np.float32), host, x[row_of] if gathered else x, counts[:2], offsets[:2], [0, 1])
