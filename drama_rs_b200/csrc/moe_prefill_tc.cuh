@@ -177,9 +177,9 @@ DRB_DEV int perm_pos(int k) { return (k & ~7) | ((k & 3) << 1) | ((k >> 2) & 1);
 
 // ---- token rows ----------------------------------------------------------------------------------------------------
 // 16-bit rows -> fp16 rows in slot order at a stride of TOKEN_STRIDE bytes: routed slot s from row (row_of ? row_of[s] : s)
-// of x into dst, shared row r from row r of x into sh_dst; in the order of dequant8_perm when PERM. The down kernel's
-// outputs serve as the buffers (they are written after the gate/up kernel has read the rows), each row's factor sits behind its
-// 4 KB. bf16 rows carry a wider range than fp16: a row whose largest magnitude lies outside [2^-4, 2^15) is divided
+// of x into row (dst_row_of ? dst_row_of[s] : s) of dst, shared row r from row r of x into sh_dst; in the order of dequant8_perm
+// when PERM. The down kernel's outputs serve as the buffers (they are written after the gate/up kernel has read the rows), each
+// slot's row in the place of its result, so that no other row of y is touched; a row's factor sits behind its 4 KB. bf16 rows carry a wider range than fp16: a row whose largest magnitude lies outside [2^-4, 2^15) is divided
 // by a power of two (the factor; the gate/up epilogue multiplies it back), every other row keeps its values.
 // Only the experts' own slots are read and written: offsets may leave gaps, whose row_of says nothing and whose rows of y are the
 // caller's. Every block makes the prefix sum of the counts for itself and looks a row's expert up in it.
@@ -188,7 +188,7 @@ constexpr int PREP_THREADS = 256;
 template <bool BF16, bool PERM>
 __global__ void __launch_bounds__(PREP_THREADS)
     k_prep_rows(const uint4* __restrict__ x, const int* __restrict__ row_of, const int* __restrict__ offsets, const int* __restrict__ counts, int E,
-                unsigned char* __restrict__ dst, int rows_sh, unsigned char* __restrict__ sh_dst) {
+                const int* __restrict__ dst_row_of, unsigned char* __restrict__ dst, int rows_sh, unsigned char* __restrict__ sh_dst) {
   __shared__ int first[MAX_E], offs[MAX_E], wtot[PREP_THREADS / 32];  // rows of the experts before e; e's first slot
   pdl_wait();
   pdl_launch_dependents();
@@ -218,17 +218,18 @@ __global__ void __launch_bounds__(PREP_THREADS)
   constexpr int PER = H / 8 / 32;
   for (int i = blockIdx.x * (PREP_THREADS / 32) + warp; i < total + rows_sh; i += gridDim.x * (PREP_THREADS / 32)) {
     const bool sh = i >= total;
-    int row = i - total, slot = row;  // the shared expert's
+    int row = i - total, to = row;  // the shared expert's
     if (!sh) {
       int e = 0;  // the last expert with first[e] <= i, and so the one that owns row i
 #pragma unroll
       for (int step = MAX_E / 2; step > 0; step >>= 1)
         if (e + step < E && first[e + step] <= i) e += step;
-      slot = offs[e] + (i - first[e]);
+      const int slot = offs[e] + (i - first[e]);
       row = row_of ? __ldcg(row_of + slot) : slot;
+      to = dst_row_of ? __ldcg(dst_row_of + slot) : slot;
     }
     const uint4* p = x + (size_t)row * (H / 8);
-    unsigned char* out = (sh ? sh_dst : dst) + (size_t)slot * TOKEN_STRIDE;
+    unsigned char* out = (sh ? sh_dst : dst) + (size_t)to * TOKEN_STRIDE;
     uint4 v[PER];
 #pragma unroll
     for (int j = 0; j < PER; ++j) v[j] = __ldcg(p + j * 32 + lane);
@@ -321,7 +322,7 @@ struct Args {
   const __half* shs;         // the shared expert's scales [R, K/128]
   void *dst, *sh_dst;        // gate/up: act fp16 [., I];  down: y f32 [., H]
   const int *offsets, *counts;
-  const int* row_of;         // gathered form (PREP = false) of gate/up: slot -> row
+  const int* row_of;         // gate/up: slot -> row of the token rows (PREP = false: of x; true: of y, where they are prepared), or NULL
   const int* dst_row_of;     // down: slot -> row of dst, or NULL
   const unsigned char *fac, *sh_fac;  // prepared bf16 rows: where the factors lie (row i at i * TOKEN_STRIDE + 4096), or NULL
   float* const* peer_y;      // down, routed results only: every rank's result buffer, or NULL. dst_row_of[slot] = s * cap + j
@@ -334,8 +335,8 @@ struct Args {
 // FP8: a tile row's weights share one f32 scale over 128 inputs. Multiplied into the fp16 operand it would cost every weight
 // a rounding (measured 4.2e-4 per row against 2.1e-4); here the operands are exact, the MMAs of each 128 inputs have an
 // accumulator of their own (a ring of four), and the epilogue warps sum scale * accumulator in fp32 as they complete.
-// PREP (gate/up): the token rows are prepared (contiguous in slot order; int4: permuted); otherwise they are gathered
-// through row_of in k order. The down kernel's rows are the act array, contiguous, int4: permuted by the gate/up epilogue.
+// PREP (gate/up): the token rows are prepared (contiguous in slot order, or through row_of; int4: permuted); otherwise they are
+// gathered through row_of in k order. The down kernel's rows are the act array, contiguous, int4: permuted by the gate/up epilogue.
 template <int GEMM, int FMT, bool PREP>
 __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const __grid_constant__ Maps maps, const Args a) {
   constexpr int K = GEMM == 0 ? H : I;
@@ -703,7 +704,7 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
       // Contiguous rows go by boxes of eight. What is left over takes one more box, of the last eight rows: no row beyond
       // the item's end is touched, and the columns of rows that it repeats (or that are not the item's) have no result
       // row. Among the array's first eight rows, and for scattered rows, gather4 fetches the rows by number.
-      const bool contig = GEMM == 1 || PREP || it.shared;
+      const bool contig = GEMM == 1 || it.shared || (PREP && !a.row_of);
       const int full = contig ? nt >> 3 : 0;
       const int start = contig && rest && end >= 8 ? end - 8 : -1;
       const int quads = start < 0 ? (nt - 8 * full + 3) >> 2 : 0;
@@ -712,12 +713,16 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
       for (int t = lane; t < cols; t += 32) {
         const int slot = start >= 0 && t >= 8 * full ? start + (t - 8 * full) : srow + t;
         const bool own = slot >= srow + (t >= 8 * full ? 8 * full : 0) && slot < end;
-        if (GEMM == 0) tab.fac[t] = own && fac ? __ldcg(reinterpret_cast<const float*>(fac + (size_t)slot * TOKEN_STRIDE + H * 2)) : 1.f;
+        if (GEMM == 0) {
+          float f = 1.f;
+          if (own && fac) f = __ldcg(reinterpret_cast<const float*>(fac + (size_t)(a.row_of && !it.shared ? __ldcg(a.row_of + slot) : slot) * TOKEN_STRIDE + H * 2));
+          tab.fac[t] = f;
+        }
         tab.dst[t] = !own ? -1 : (GEMM == 1 && !it.shared && a.dst_row_of) ? __ldcg(a.dst_row_of + slot) : slot;
       }
       for (int t = lane; t < 4 * quads; t += 32) {
         const int slot = srow + min(8 * full + t, nt - 1);
-        tab.rows[t] = (GEMM == 0 && !PREP && !it.shared && a.row_of) ? __ldcg(a.row_of + slot) : slot;
+        tab.rows[t] = (GEMM == 0 && !it.shared && a.row_of) ? __ldcg(a.row_of + slot) : slot;
       }
       if (lane == 0) tab.cols = cols, tab.used = (start >= 0 ? 8 * full + 8 : nt + 7) & ~7, tab.mt = it.mt, tab.shared = it.shared, tab.full = full, tab.srow = srow, tab.start = start, tab.quads = quads;
       __syncwarp();
@@ -938,7 +943,7 @@ static int run_block(const Block& b, const DrbDevice& dev, cudaStream_t st) {
     auto kp = b.x_bf16 ? k_prep_rows<true, FMT == 0> : k_prep_rows<false, FMT == 0>;
     for (int e0 = 0; e0 == 0 || e0 < b.E; e0 += MAX_E)  // the shared expert's rows with the first experts
       drb_launch(kp, dim3(2 * dev.sms), dim3(PREP_THREADS), 0, st, false, static_cast<const uint4*>(b.x), b.row_of, b.offsets + e0, b.counts + e0,
-                 b.E - e0 < MAX_E ? b.E - e0 : MAX_E, tok, e0 == 0 ? b.rows_sh : 0, shtok);
+                 b.E - e0 < MAX_E ? b.E - e0 : MAX_E, b.y_row_of, tok, e0 == 0 ? b.rows_sh : 0, shtok);
   }
   // Every gate/up launch before the first down launch: y holds the token rows until then.
   const bool sh_on = b.rows_sh > 0;
@@ -957,7 +962,7 @@ static int run_block(const Block& b, const DrbDevice& dev, cudaStream_t st) {
         if (ne > 0 && map_tokens(&m.tok8, &m.tok1, prep ? tok : b.x, H, prep ? TOKEN_STRIDE : H * 2)) return -3;
         if (sh && map_gate_up(&m.sh, b.sgu_q, 1, I, H)) return -3;
         if (sh && map_tokens(&m.shtok8, &m.shtok1, prep ? shtok : b.x, H, prep ? TOKEN_STRIDE : H * 2)) return -3;
-        a.dst = b.act, a.sh_dst = b.sh_act, a.row_of = b.row_of;
+        a.dst = b.act, a.sh_dst = b.sh_act, a.row_of = prep ? b.y_row_of : b.row_of;
         if (prep && b.x_bf16) a.fac = tok, a.sh_fac = shtok;
       } else {
         if (ne > 0 && (map_rows(&m.q, w, (uint64_t)ne * H, row) || map_tokens(&m.tok8, &m.tok1, b.act, I, I * 2))) return -3;

@@ -123,7 +123,7 @@ int dr_moe_permute(const int* idx, int rows, int topk, const int* offsets, int* 
  * unspecified. y[slot, :] = down_e(silu(gate_e . x) * (up_e . x)). h == 2048, i == 512. The weights and the token rows are
  * addressed through TMA tensor maps built from the pointers given: weights, xp and act 16-byte aligned, else -3 and nothing is
  * launched; -3 also when the driver refuses a map. y may start at any float. Until its rows are written y is scratch: the token
- * rows as the tensor cores want them.
+ * rows as the tensor cores want them, each in the place of its result; rows of y that no slot names are not touched.
  * drama.cu:799-968; ffi.rs:61-64 */
 int dr_moe_prefill(const uint8_t* gu_q, const dr_half* gu_sm, const uint8_t* d_q, const dr_half* d_sm,
                    const dr_bf16* xp, const int* offsets, const int* counts, dr_bf16* act, float* y, int e, int h, int i,

@@ -263,3 +263,30 @@ def test_gaps_between_the_experts_slots(st, gathered):
     assert device_error_word() == 0 and (np.delete(raw, own, axis=0) == 0x55555555).all()
     x = synth.bf16_bits_to_f32(xb).astype(np.float64)
     check_rows(raw.view(np.float32), host, x[row_of] if gathered else x, counts[:2], offsets[:2], [0, 1])
+
+
+@pytest.mark.parametrize("f16", [True, False], ids=["f16", "bf16"])
+def test_results_scattered_through_y_row_of(st, f16):
+    """With y_row_of the results go to rows of the caller's choosing: the same bits as in slot order, and no other row of y is touched."""
+    l = ffi.lib()
+    dev = MoeLayer.upload(synth.make_layer(39, synth.MoeShape(experts=16)), st)
+    counts = np.array([0, 3, 0, 2, 1, 40, 0, 9, 0, 70, 8, 16, 17, 5, 0, 1], dtype=np.int32)
+    offsets = (np.cumsum(counts) - counts).astype(np.int32)
+    n, rows, rng = int(counts.sum()), int(counts.sum()) + 37, np.random.Generator(np.random.PCG64(9))
+    xf = rng.standard_normal((n, 2048), dtype=np.float32)
+    xf[::3] *= 0.004  # bf16: rows that are divided by a power of two on the way
+    to = rng.permutation(rows)[:n].astype(np.int32)
+    dx = DevBuf.from_array(xf.astype(np.float16) if f16 else synth.f32_to_bf16_bits(xf), st)
+    dcnt, doff, dto = (DevBuf.from_array(a, st) for a in (counts, offsets, to))
+    dact, dsh = DevBuf(n * 1024), DevBuf(16)
+    w = (*dev.gate_up.expert(0), *dev.down.expert(0), *dev.shared_gate_up.rows(0), *dev.shared_down.rows(0))
+    got = []
+    for y_row_of in (NULL, dto.at(0)):
+        dy = DevBuf(rows * 8192)
+        dy.fill(0x55, st)
+        launched(l.drb_moe_prefill_block(*w, dx.at(0), NULL, doff.at(0), dcnt.at(0), dact.at(0), dy.at(0), dact.at(0), dsh.at(0), 0, 16, 2048, 512,
+                                         int(f16), y_row_of, st.raw), "block")
+        got.append(dy.download(np.uint32, rows * 2048, st).reshape(rows, 2048))
+    assert device_error_word() == 0 and np.isfinite(got[0][:n].view(np.float32)).all()
+    assert np.array_equal(got[1][to], got[0][:n])
+    assert (np.delete(got[1], to, axis=0) == 0x55555555).all() and (got[0][n:] == 0x55555555).all()
