@@ -198,7 +198,6 @@ class MoePrefill:
         self.device_scan = False  # reference calls only: offsets by drb_moe_offsets on the device instead of the host scan
         self.invariant_router = not reference_calls  # router logits by drb_router_logits (independent of the batch size) instead of cuBLAS
         self.logit_bias: DevBuf | None = None  # [n, E + 1] f32 rows the router GEMM accumulates onto (not in the reference)
-        self._args = None
 
     def gemm_q8(self, a, w, c, m: int, beta: float) -> None:
         """C = A . dequant(W)^T + beta C for a q8 weight. src/engine.rs:351-355."""
@@ -243,16 +242,14 @@ class MoePrefill:
         launched(l.dr_moe_topk(self.rlog.at(0), n, e, topk, e + 1, self.idx.at(0), self.wts.at(0), self.sgate.at(0), st), "moe_topk")
 
     def _layer_args(self):
-        """The structs of drb_moe_prefill_layer for this object's buffers, kept until one of them is replaced."""
+        """The structs of drb_moe_prefill_layer for this object's weights and buffers as they are now."""
         ly = self.layer
-        key = (ly, self.x, self.hn_b, self.rlog, self.logit_bias, self.idx, self.wts, self.sgate, self.counts, self.offsets, self.slot_of,
-               self.row_of, self.ap, self.yp, self.sh_act_b, self.sh_out)
-        if self._args is None or any(a is not b for a, b in zip(key, self._args[0])):
-            w = ffi.MoeLayerPtrs(*(b.ptr for b in (ly.router, ly.post_norm, ly.gate_up.q, ly.gate_up.sm, ly.down.q, ly.down.sm,
-                                                   ly.shared_gate_up.q, ly.shared_gate_up.s, ly.shared_down.q, ly.shared_down.s)))
-            b = ffi.PrefillBuffers(*(b.ptr if b is not None else None for b in key[1:]))
-            self._args = (key, C.byref(w), C.byref(b))
-        return self._args[1], self._args[2]
+        weights = (ly.router, ly.post_norm, ly.gate_up.q, ly.gate_up.sm, ly.down.q, ly.down.sm, ly.shared_gate_up.q, ly.shared_gate_up.s,
+                   ly.shared_down.q, ly.shared_down.s)
+        bufs = (self.x, self.hn_b, self.rlog, self.logit_bias, self.idx, self.wts, self.sgate, self.counts, self.offsets, self.slot_of,
+                self.row_of, self.ap, self.yp, self.sh_act_b, self.sh_out)
+        w, b = ffi.MoeLayerPtrs(*[t.ptr for t in weights]), ffi.PrefillBuffers(*[t.ptr if t is not None else None for t in bufs])
+        return C.byref(w), C.byref(b)
 
     def run_device(self, n: int) -> None:
         """The block on the n rows already in self.x (device), in place. With a logit bias the router logits are
