@@ -1031,7 +1031,7 @@ struct drb_prefill_buffers {
 };
 extern "C" int drb_moe_prefill_layer(const drb_moe_layer* w, const drb_prefill_buffers* b, int rows, int e, int topk, int h, int i, float eps,
                                      cudaStream_t st) {
-  if (!w || !b || h != pf::H || i != pf::I || e < 1 || e > 256 || topk < 1 || topk > e || topk > 31) return -1;
+  if (!w || !b || h != pf::H || i != pf::I || e < 1 || e > 256 || topk < 1 || topk > e || topk > 32) return -1;
   if (rows <= 0) return 0;
   // what is read or written in 16-byte pieces, before anything is launched
   for (const void* p : {(const void*)b->x, (const void*)b->rows16, (const void*)b->y, (const void*)b->sh_out, (const void*)b->act, (const void*)b->sh_act, w->router,

@@ -290,3 +290,30 @@ def test_results_scattered_through_y_row_of(st, f16):
     assert device_error_word() == 0 and np.isfinite(got[0][:n].view(np.float32)).all()
     assert np.array_equal(got[1][to], got[0][:n])
     assert (np.delete(got[1], to, axis=0) == 0x55555555).all() and (got[0][n:] == 0x55555555).all()
+
+
+@pytest.mark.parametrize("experts,topk", [(256, 8), (64, 32), (32, 32), (40, 1)])
+@pytest.mark.parametrize("rows", [1, 7, 32, 33, 150])
+def test_layer_call_equals_the_separate_calls(st, experts, topk, rows):
+    """drb_moe_prefill_layer against the calls that it stands for, with a logit bias: the same bits in rows, logits, routing and x. top-k up
+    to 32, as dr_moe_topk takes it."""
+    l = ffi.lib()
+    dev = MoeLayer.upload(synth.make_layer(40, synth.MoeShape(experts=experts)), st)
+    x = synth.make_x(41, rows, 2048)
+    bias = DevBuf.from_array(np.random.Generator(np.random.PCG64(7)).standard_normal((rows, experts + 1), dtype=np.float32), st)
+    one, sep = MoePrefill(dev, rows, topk, st=st), MoePrefill(dev, rows, topk, st=st)
+    for p in (one, sep):
+        p.logit_bias = bias
+        p.x.upload(x, st)
+    one.run_device(rows)
+    sep.route_device(rows)
+    launched(l.drb_moe_group(sep.idx.at(0), rows, topk, 0, experts, sep.counts.at(0), sep.offsets.at(0), sep.slot_of.at(0), sep.row_of.at(0), st.raw), "group")
+    w = (*dev.gate_up.expert(0), *dev.down.expert(0), *dev.shared_gate_up.rows(0), *dev.shared_down.rows(0))
+    launched(l.drb_moe_prefill_block(*w, sep.hn_b.at(0), sep.row_of.at(0), sep.offsets.at(0), sep.counts.at(0), sep.ap.at(0), sep.yp.at(0), sep.sh_act_b.at(0),
+                                     sep.sh_out.at(0), rows, experts, 2048, 512, 1, NULL, st.raw), "block")
+    launched(l.dr_moe_combine(sep.x.at(0), sep.yp.at(0), sep.slot_of.at(0), sep.wts.at(0), sep.sgate.at(0), sep.sh_out.at(0), rows, topk, 2048, st.raw), "combine")
+    for name, count in (("hn_b", rows * 1024), ("rlog", rows * (experts + 1)), ("idx", rows * topk), ("wts", rows * topk), ("sgate", rows),
+                        ("counts", experts), ("offsets", experts), ("x", rows * 2048)):
+        a, b = (getattr(p, name).download(np.uint32, count, st) for p in (one, sep))
+        assert np.array_equal(a, b), name
+    assert np.isfinite(one.x.download(np.float32, rows * 2048, st)).all() and device_error_word() == 0
