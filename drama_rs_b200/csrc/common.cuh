@@ -182,6 +182,9 @@ DRB_DEV void bulk_prefetch_l2(const void* p, unsigned bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
+// One line into L2. What a kernel reads of it comes after its dependency wait, so that a tensor which the launch before wrote is seen.
+DRB_DEV void prefetch_line_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Prefetches this block's share of [pf, pf + pf_bytes) into L2 (the next kernel's weights).
 // Called by one thread per block. The region is cut into 16-byte aligned pieces of at most 64 KB.
 DRB_DEV void prefetch_share(const char* pf, size_t pf_bytes, unsigned block, unsigned blocks) {

@@ -169,14 +169,18 @@ __global__ void __launch_bounds__(THREADS, 2)
     }
     if (EARLY) release();
   };
-  // The norm weights are constants: requested before the input may be read.
+  // The norm weights are brought as far as L2 before the input may be read (they may be the work of the launch before).
   float4 wv[NSEG], xv[NSEG];
+  if (nw && sub == 0 && (lane & 7) == 0)
 #pragma unroll
-  for (int q = 0; q < NSEG; ++q) wv[q] = nw && EARLY ? __ldg(reinterpret_cast<const float4*>(nw + q * SEG + kw * GROUP) + lane) : make_float4(1.f, 1.f, 1.f, 1.f);
+    for (int q = 0; q < NSEG; ++q) prefetch_line_l2(nw + q * SEG + kw * GROUP + 4 * lane);
   if (EARLY) load(0, 0);
   pdl_wait();  // x and res come from the previous kernel
 #pragma unroll
-  for (int q = 0; q < NSEG; ++q) xv[q] = __ldcg(reinterpret_cast<const float4*>(x + q * SEG + kw * GROUP) + lane);
+  for (int q = 0; q < NSEG; ++q) {
+    xv[q] = __ldcg(reinterpret_cast<const float4*>(x + q * SEG + kw * GROUP) + lane);
+    if (EARLY && nw) wv[q] = __ldcg(reinterpret_cast<const float4*>(nw + q * SEG + kw * GROUP) + lane);
+  }
   // Thread o < bo writes output o of every batch; the first batch's residual is requested now.
   constexpr int bo = BATCH / U;
   const bool writer = (int)threadIdx.x < bo;
@@ -198,7 +202,7 @@ __global__ void __launch_bounds__(THREADS, 2)
     const float inv = rsqrtf(tot / K + eps);
 #pragma unroll
     for (int q = 0; q < NSEG; ++q) {
-      if (!EARLY) wv[q] = __ldg(reinterpret_cast<const float4*>(nw + q * SEG + kw * GROUP) + lane);
+      if (!EARLY) wv[q] = __ldcg(reinterpret_cast<const float4*>(nw + q * SEG + kw * GROUP) + lane);
       xv[q] = make_float4(xv[q].x * inv * wv[q].x, xv[q].y * inv * wv[q].y, xv[q].z * inv * wv[q].z, xv[q].w * inv * wv[q].w);
     }
   }
@@ -363,11 +367,15 @@ __global__ void __launch_bounds__(THREADS, 2)
 
   // ---------------- consumers
   float4 wv[2], xv[2];
+  if (nw && (lane & 7) == 0)
 #pragma unroll
-  for (int j = 0; j < 2; ++j) wv[j] = nw ? __ldg(reinterpret_cast<const float4*>(nw) + threadIdx.x + j * NT) : make_float4(1.f, 1.f, 1.f, 1.f);
+    for (int j = 0; j < 2; ++j) prefetch_line_l2(nw + 4 * (threadIdx.x + j * NT));
   pdl_wait();  // x comes from the previous kernel
 #pragma unroll
-  for (int j = 0; j < 2; ++j) xv[j] = __ldcg(reinterpret_cast<const float4*>(x) + threadIdx.x + j * NT);
+  for (int j = 0; j < 2; ++j) {
+    xv[j] = __ldcg(reinterpret_cast<const float4*>(x) + threadIdx.x + j * NT);
+    wv[j] = nw ? __ldcg(reinterpret_cast<const float4*>(nw) + threadIdx.x + j * NT) : make_float4(1.f, 1.f, 1.f, 1.f);
+  }
   float inv = 1.f;
   if (nw) {
     float ss = 0.f;

@@ -439,9 +439,11 @@ __global__ void __launch_bounds__(RL_WARPS * 32, 1)
   // the row groups start at different tiles: in step, all of them would ask L2 for the same lines at once
   const int mine = (tiles - (int)blockIdx.y + (int)gridDim.y - 1) / (int)gridDim.y;  // tiles of this block, at least one
   int t = (int)(blockIdx.x % (unsigned)mine);
-  fetch(blockIdx.y + t * gridDim.y);
+  // the first tile's weights as far as L2: they too may be the work of the launch before
+  prefetch_line_l2(w + (size_t)min((int)(blockIdx.y + t * gridDim.y) * RL_TILE + g, e1 - 1) * RL_K + warp * RL_SEG + 64 * q);
   pdl_launch_dependents();
   pdl_wait();
+  fetch(blockIdx.y + t * gridDim.y);
   if (zero && blockIdx.x == 0 && blockIdx.y == 0)
     for (int i = threadIdx.x; i < n_zero; i += blockDim.x) zero[i] = 0;
   constexpr int RPW = RL_ROWS / RL_WARPS;  // rows warp + RL_WARPS p; all requested before the first is used
