@@ -27,14 +27,19 @@ namespace gemv {
 
 constexpr int BLOCK_BYTES = 112 * 1024;  // two blocks per multiprocessor
 
-// The caller's prefetch hint. With overlapping launches a successor fills its rings itself as soon as its blocks are resident
-// (about `skip` bytes of each block's share); asked for here as well, the same lines twice, it slowed both (a chain of 33
-// projections 135 us instead of 129). So what lies behind them is prefetched, and no more than 128 KB per block: a
-// vocabulary-sized region would only push out what the running kernels still read.
-DRB_DEV void prefetch_hint(const char* pf, size_t pf_bytes, unsigned skip, unsigned block, unsigned blocks) {
-  if (skip == 0) return prefetch_share(pf, pf_bytes, block, blocks);
-  const size_t per = pf_bytes / blocks;
-  if (pf && per > skip) prefetch_share(pf + block * per + skip, per - skip < 131072 ? per - skip : 131072, 0, 1);
+// The caller's prefetch hint. A following GEMV of this library fills its rings itself as soon as its blocks are resident, about `skip`
+// bytes per multiprocessor from the start of each block's share of the rows; asked for here as well, the same lines twice, it
+// slowed both (a chain of 33 projections 135 us instead of 129). So of a region that size what lies behind them is prefetched, and no more
+// than 128 KB per multiprocessor: a vocabulary-sized region would only push out what the running kernels still read. This launch's
+// blocks, when they are fewer, go over all of the successor's shares. A region of at most 2 MB (a router's, a short projection's) is
+// prefetched whole, whoever reads it: chains of GEMVs of 0.5, 1 and 2 MB take the same with the hint as without (1.785, 1.815,
+// 1.87 us a launch); at 4 MB the lines asked for twice begin to show (1.90 -> 1.97).
+constexpr size_t HINT_WHOLE = 2 << 20;
+DRB_DEV void prefetch_hint(const char* pf, size_t pf_bytes, unsigned skip, unsigned sms, unsigned block, unsigned blocks) {
+  if (skip == 0 || pf_bytes <= HINT_WHOLE) return prefetch_share(pf, pf_bytes, block, blocks);
+  const size_t per = pf_bytes / sms;
+  if (!pf || per <= skip) return;
+  for (unsigned i = block; i < sms; i += blocks) prefetch_share(pf + i * per + skip, per - skip < 131072 ? per - skip : 131072, 0, 1);
 }
 constexpr unsigned HINT_SKIP = 96 * 1024;
 
@@ -82,7 +87,7 @@ DRB_DEV void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t
 template <int K, int U>
 __global__ void __launch_bounds__(THREADS, 2)
     k_gemv(const int8_t* __restrict__ W, const __half* __restrict__ S, const float* __restrict__ x, const float* res, float* y, int N,
-           const float* __restrict__ nw, float eps, const char* pf, size_t pf_bytes, unsigned pf_skip) {
+           const float* __restrict__ nw, float eps, const char* pf, size_t pf_bytes, unsigned pf_skip, unsigned sms) {
   using P = Shape<K, U>;
   constexpr int STAGES = P::STAGES, NSEG = P::NSEG, KW = P::KW, RS = P::RS, ROWS = P::ROWS, SEG = P::SEG, PITCH = P::PITCH, SROW = P::SROW;
   constexpr int SLOTS = P::S_SLOTS ? P::S_SLOTS : 1;
@@ -130,7 +135,7 @@ __global__ void __launch_bounds__(THREADS, 2)
           if (++s == STAGES) s = 0, par ^= 1u;
         }
       }
-      prefetch_hint(pf, pf_bytes, pf_skip, b, G);
+      prefetch_hint(pf, pf_bytes, pf_skip, sms, b, G);
     }
     return;
   }
@@ -302,7 +307,7 @@ int launch(const int8_t* W, const __half* S, const float* x, const float* res, f
   if (!dev.ready) return -2;
   if (N <= 0) return 0;
   drb_launch(k_gemv<K, U>, dim3(N < dev.sms ? N : dev.sms), dim3(THREADS), Shape<K, U>::BYTES, st, dev.pdl, W, S, x, res, y, N, nw, eps, pf, pf_bytes,
-             dev.pdl ? HINT_SKIP : 0u);
+             dev.pdl ? HINT_SKIP : 0u, (unsigned)dev.sms);
   return 0;
 }
 
@@ -333,7 +338,7 @@ DRB_DEV void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memor
 
 __global__ void __launch_bounds__(THREADS, 2)
     k_gemv(const __nv_bfloat16* __restrict__ W, const float* __restrict__ x, float* __restrict__ y, int N, const float* __restrict__ nw, float eps,
-           const char* pf, size_t pf_bytes, unsigned pf_skip) {
+           const char* pf, size_t pf_bytes, unsigned pf_skip, unsigned sms) {
   extern __shared__ __align__(128) unsigned char dyn[];
   Ctl& ctl = *reinterpret_cast<Ctl*>(dyn);
   float4* xs4 = reinterpret_cast<float4*>(dyn + 512);
@@ -360,7 +365,7 @@ __global__ void __launch_bounds__(THREADS, 2)
         mbar_expect_tx(&ctl.full[s], bytes);
         bulk_g2s(ring + s * STAGE_BYTES, W + (size_t)r0 * K, bytes, &ctl.full[s]);
       }
-      prefetch_hint(pf, pf_bytes, pf_skip, b, G);
+      prefetch_hint(pf, pf_bytes, pf_skip, sms, b, G);
     }
     return;
   }
@@ -479,6 +484,6 @@ extern "C" int dr_gemv_bf16(const __nv_bfloat16* W, const float* x, float* y, in
   if (!dev.ready) return -2;
   if (N <= 0) return 0;
   drb_launch(k_gemv, dim3(N < dev.sms ? N : dev.sms), dim3(THREADS), BYTES, st, dev.pdl, W, x, y, N, nw, eps, pf, pf_bytes,
-             dev.pdl ? gemv::HINT_SKIP : 0u);
+             dev.pdl ? gemv::HINT_SKIP : 0u, (unsigned)dev.sms);
   return 0;
 }

@@ -64,7 +64,10 @@ int dr_gemm(void* h, const dr_bf16* a, const dr_bf16* w, float* c, int m, int n,
 
 /* y[n] = W[n] . x' (+ res[n]);  x' = rmsnorm(x, nw, eps) when nw != NULL, else x. y may alias res.
  * K in {512, 2048, 4096, 6144, 8192}. pf/pf_bytes: a region to prefetch into L2 (the next kernel's
- * weights), or NULL. drama.cu:222-240, 283-294; ffi.rs:33-36 */
+ * weights), or NULL. A region above 2 MB is taken for the weights of a following GEMV of this library, which requests the first
+ * 96 KB of each multiprocessor's share of the rows itself while this kernel still runs: what lies behind them is prefetched, up to
+ * 128 KB per multiprocessor (everything with DRB_PDL=0). Weight matrices are read ahead of the launch before: they must not
+ * be that launch's work. Norm weights may be. drama.cu:222-240, 283-294; ffi.rs:33-36 */
 int dr_gemv_q8(const int8_t* w, const dr_half* s, const float* x, const float* res, float* y, int n, int k,
                const float* nw, float eps, const char* pf, size_t pf_bytes, dr_stream st);
 
