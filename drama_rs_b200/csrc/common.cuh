@@ -122,6 +122,8 @@ DRB_DEV bool mbar_wait(uint64_t* bar, unsigned parity, unsigned err_code, unsign
 // The same for a wait on a ring's step-to-step path: no sleep between polls (a sleeping waiter adds its wake-up time
 // to every hand-over of the ring), and each poll may suspend the warp in hardware for up to 2 us: a warp that polls takes
 // issue slots from the ones that work (measured in the grouped GEMMs: half of all instructions issued). Bounded all the same.
+constexpr unsigned RING_POLLS = 1u << 20;  // about two seconds of waiting
+template <unsigned LIMIT = RING_POLLS>
 DRB_DEV bool mbar_wait_hot(uint64_t* bar, unsigned parity, unsigned err_code) {
   unsigned ok;
   asm volatile(
@@ -131,13 +133,13 @@ DRB_DEV bool mbar_wait_hot(uint64_t* bar, unsigned parity, unsigned err_code) {
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "@p bra WAIT_OVER;\n\t"
       "add.u32 n, n, 1;\n\t"
-      "setp.lt.u32 p, n, 1048576;\n\t"
+      "setp.lt.u32 p, n, %4;\n\t"
       "@p bra WAIT_AGAIN;\n\t"
       "setp.ne.u32 p, n, n;\n"
       "WAIT_OVER:\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(2000u)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(2000u), "n"(LIMIT)
       : "memory");
   if (ok) return true;
   atomicMax(&g_drb_error, err_code);
@@ -146,8 +148,7 @@ DRB_DEV bool mbar_wait_hot(uint64_t* bar, unsigned parity, unsigned err_code) {
 
 // mbar_wait_hot for a ring's innermost waits: two instructions when the barrier is complete. `spent` starts at zero; after a
 // wait that ran out (the error word is set, results are void) it stands at the limit, and no later wait retries.
-constexpr unsigned WAIT_SPENT = 1u << 20;
-template <unsigned ERR>
+template <unsigned ERR, unsigned LIMIT = RING_POLLS>
 DRB_DEV void mbar_wait_ring(uint32_t bar, unsigned parity, unsigned& spent) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t.reg .u32 n;\n\t"
@@ -158,13 +159,13 @@ DRB_DEV void mbar_wait_ring(uint32_t bar, unsigned parity, unsigned& spent) {
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 2000;\n\t"
       "@p bra RING_OVER;\n\t"
       "add.u32 n, n, 1;\n\t"
-      "setp.lt.u32 p, n, 1048576;\n\t"
+      "setp.lt.u32 p, n, %4;\n\t"
       "@p bra RING_AGAIN;\n\t"
-      "mov.u32 %0, 1048576;\n\t"
+      "mov.u32 %0, %4;\n\t"
       "red.relaxed.gpu.global.max.u32 [g_drb_error], %3;\n"
       "RING_OVER:\n\t}"
       : "+r"(spent)
-      : "r"(bar), "r"(parity), "n"(ERR)
+      : "r"(bar), "r"(parity), "n"(ERR), "n"(LIMIT)
       : "memory");
 }
 

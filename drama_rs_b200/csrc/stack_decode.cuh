@@ -795,7 +795,9 @@ static cudaError_t configure_all() {
 // wait gives up after `limit` polls, records its code and lets the kernel run to its end, which is what the host
 // observes through drb_device_error(). which = 1: the copy wait of the per-layer kernels (mbar_wait); 2: the copy wait
 // of the persistent kernel (wait_full); 3: its tagged-word polls, by one thread and then by whole warps, the later
-// ones returning at once because the block has already given up.
+// ones returning at once because the block has already given up; 4 and 5: the ring waits of the GEMVs (mbar_wait_hot) and of the
+// grouped prefill GEMMs (mbar_wait_ring, then once more: a spent wait does not retry), whose limit is compiled in, RING_TEST_POLLS here.
+constexpr unsigned RING_TEST_POLLS = 2000;
 __global__ void __launch_bounds__(64, 1) k_test_waits(int which, unsigned limit, const unsigned long long* word, unsigned* polls_after) {
   __shared__ uint64_t bar;
   __shared__ int abort_word;
@@ -814,6 +816,16 @@ __global__ void __launch_bounds__(64, 1) k_test_waits(int which, unsigned limit,
     if (threadIdx.x == 0) wait_full(&bar, 0, limit, abort_flag);
     __syncthreads();
     wait_full(&bar, 0, limit, abort_flag);  // every thread: returns at once, the block has given up
+  } else if (which == 4) {
+    if (threadIdx.x == 0) mbar_wait_hot<RING_TEST_POLLS>(&bar, 0, DRB_ERR_FULL_WAIT);
+  } else if (which == 5) {
+    unsigned spent = 0;
+    if (threadIdx.x == 0) {
+      mbar_wait_ring<DRB_ERR_FULL_WAIT, RING_TEST_POLLS>(smem_u32(&bar), 0, spent);
+      const long long t0 = clock64();
+      mbar_wait_ring<DRB_ERR_FULL_WAIT, RING_TEST_POLLS>(smem_u32(&bar), 0, spent);
+      if (polls_after) *polls_after = spent == RING_TEST_POLLS ? (unsigned)(clock64() - t0) : 0xffffffffu;
+    }
   } else {
     if (threadIdx.x == 0) ll_poll1(word, 1u, limit, abort_flag);
     __syncthreads();
@@ -855,11 +867,11 @@ extern "C" int drb_moe_stack_decode(const drb_moe_layer* layers, int n_layers, f
 }
 
 // Test hook (no counterpart in the reference): launches one block whose bounded wait runs out after `limit` polls
-// (which: 1 = mbar_wait, 2 = wait_full, 3 = tagged-word polls; word: 512 zeroed bytes of device memory; clocks: a
-// device word receiving the clocks the later polls of case 3 took, or NULL). The launch completes normally; the
+// (which: 1 = mbar_wait, 2 = wait_full, 3 = tagged-word polls, 4 = mbar_wait_hot, 5 = mbar_wait_ring; word: 512 zeroed bytes of
+// device memory; clocks: a device word receiving the clocks that the later polls of cases 3 and 5 took, or NULL). The launch completes normally; the
 // code is then read with drb_device_error(). limit <= 65536 (a few milliseconds), else -1.
 extern "C" int drb_test_wait_runs_out(int which, unsigned limit, const void* word, unsigned* clocks, cudaStream_t st) {
-  if (which < 1 || which > 3 || limit == 0 || limit > 65536u || !word) return -1;
+  if (which < 1 || which > 5 || limit == 0 || limit > 65536u || !word) return -1;
   const DrbDevice& dev = drb_device(st);
   if (!dev.ready) return -2;
   stack::k_test_waits<<<1, 64, 0, st>>>(which, limit, static_cast<const unsigned long long*>(word), clocks);

@@ -296,7 +296,8 @@ int drb_init(void);                    /* per-device setup; also run by the pre-
 int drb_device_error(unsigned* out);   /* reads and clears the bounded-wait error word; synchronises */
 int drb_grid_blocks(void);             /* blocks of the persistent kernels on the current device */
 /* Test hook: one block whose bounded wait runs out after `limit` polls (which: 1 = copy wait of the per-layer
- * kernels, 2 = copy wait of the persistent kernel, 3 = its tagged-word polls; word: 512 zeroed device bytes; clocks:
+ * kernels, 2 = copy wait of the persistent kernel, 3 = its tagged-word polls, 4 / 5 = ring waits of the GEMVs / of the
+ * grouped prefill GEMMs (their limit: 2000 polls); word: 512 zeroed device bytes; clocks:
  * device word or NULL). The launch completes normally and the code is read with drb_device_error().
  * limit <= 65536 (milliseconds at most), else -1. */
 int drb_test_wait_runs_out(int which, unsigned limit, const void* word, unsigned* clocks, dr_stream st);

@@ -21,7 +21,7 @@ pytestmark = pytest.mark.gpu
 FULL_WAIT, GRID_WAIT = 1, 3  # DrbError in csrc/common.cuh
 
 
-@pytest.mark.parametrize("which,code", [(1, FULL_WAIT), (2, FULL_WAIT), (3, GRID_WAIT)])
+@pytest.mark.parametrize("which,code", [(1, FULL_WAIT), (2, FULL_WAIT), (3, GRID_WAIT), (4, FULL_WAIT), (5, FULL_WAIT)])
 def test_wait_that_runs_out_is_reported_and_the_context_stays_usable(which, code):
     lib = ffi.lib()
     st = Stream()
@@ -34,7 +34,7 @@ def test_wait_that_runs_out_is_reported_and_the_context_stays_usable(which, code
     assert time.perf_counter() - t0 < 0.5, "a wait of 2000 polls ends within milliseconds"
     assert device_error_word() == code
     assert device_error_word() == 0, "reading the word clears it"
-    if which == 3:
+    if which in (3, 5):
         # once the block has given up, its later polls return at once instead of spinning to their own limit
         assert int(clocks.download(np.uint32, 1, st)[0]) < 20000
     # the same context then runs the real kernels, and they are exact
