@@ -850,7 +850,7 @@ extern "C" int dr_moe_permute(const int* idx, int rows, int topk, const int* off
 extern "C" int dr_moe_combine(float* x, const float* Y, const int* slot_of, const float* wts, const float* sgate,
                               const float* shared, int rows, int topk, int H, cudaStream_t st) {
   if (H % 4 != 0) return -1;
-  if (rows <= 0) return 0;
+  if (rows <= 0 || H <= 0) return 0;
   const DrbDevice& dev = drb_device(st);
   drb_launch(topk == 8 ? pf::k_combine<8> : pf::k_combine<0>, dim3(rows, (H + 1023) / 1024), dim3(256), 0, st, dev.ready && dev.pdl, x, Y, slot_of,
              wts, sgate, shared, topk, H);

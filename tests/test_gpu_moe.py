@@ -468,3 +468,11 @@ def test_moe_prefill_zipf_300(st, layers):
     assert counts.sum() == 2400 and np.array_equal(counts, orc.moe_count(got_idx, 256))
     assert_parity((y - x)[safe], out[safe], "prefill zipf 300", **prefill_bar(out[safe]))
     assert device_error_word() == 0
+
+
+def test_combine_of_nothing_launches_nothing(st):
+    """No rows, or rows of no columns: nothing to do, and no launch of an empty grid that the next call would report."""
+    l, x = ffi.lib(), DevBuf.zeros(256, Stream())
+    for rows, h in ((0, 2048), (3, 0)):
+        assert l.dr_moe_combine(*[x.at(0)] * 6, rows, 8, h, NULL) == 0 and l.dr_last_error() == 0
+    assert l.dr_moe_combine(*[x.at(0)] * 6, 3, 8, 6, NULL) == -1
