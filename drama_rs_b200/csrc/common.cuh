@@ -246,69 +246,6 @@ DRB_DEV uint32_t lop3_and_or(uint32_t a, uint32_t b, uint32_t c) {  // (a & b) |
   return r;
 }
 
-// ------------------------------------------------------------------------------------------
-// int4: eight nibbles of one 32-bit word against eight activations.
-//
-// Nibble q (0..15) is placed in mantissa bits 19..22 of 0x41800000, which is the float 16 + q,
-// exactly. A byte permute builds that float from a pre-shifted copy of the word, so each weight
-// costs 1.5 integer instructions and half a packed FMA and never touches the conversion unit.
-// The dot product accumulates sum((16 + q) * x); callers remove the offset with the chunk's
-// sum of x:  sum(q * x) = acc - 16 * sum(x), folded into the group's min term.
-//
-// xp[0..3] hold (x0,x1), (x2,x3), (x4,x5), (x6,x7) for the word's nibbles in k order.
-DRB_DEV unsigned long long dot8_q4(uint32_t w, const unsigned long long* xp, unsigned long long acc) {
-  const uint32_t ev = lop3_and_or(w << 3, 0x78787878u, 0x80808080u);  // nibbles 0,2,4,6 as 0x80|q<<3
-  const uint32_t od = lop3_and_or(w >> 1, 0x78787878u, 0x80808080u);  // nibbles 1,3,5,7
-  const uint32_t hi = 0x00000041u;                                    // byte 4 = 0x41, byte 5 = 0x00
-  acc = fma2(pack2(__uint_as_float(prmt(ev, hi, 0x4055u)), __uint_as_float(prmt(od, hi, 0x4055u))), xp[0], acc);
-  acc = fma2(pack2(__uint_as_float(prmt(ev, hi, 0x4155u)), __uint_as_float(prmt(od, hi, 0x4155u))), xp[1], acc);
-  acc = fma2(pack2(__uint_as_float(prmt(ev, hi, 0x4255u)), __uint_as_float(prmt(od, hi, 0x4255u))), xp[2], acc);
-  acc = fma2(pack2(__uint_as_float(prmt(ev, hi, 0x4355u)), __uint_as_float(prmt(od, hi, 0x4355u))), xp[3], acc);
-  return acc;
-}
-
-// One 16-byte chunk (32 nibbles, k ascending) against xp[0..15]; returns sum((16 + q) * x).
-DRB_DEV float dot32_q4(const uint4& v, const unsigned long long* xp) {
-  unsigned long long a = 0ull, b = 0ull;
-  a = dot8_q4(v.x, xp + 0, a);
-  b = dot8_q4(v.y, xp + 4, b);
-  a = dot8_q4(v.z, xp + 8, a);
-  b = dot8_q4(v.w, xp + 12, b);
-  float a0, a1, b0, b1;
-  unpack2(a, a0, a1);
-  unpack2(b, b0, b1);
-  return (a0 + a1) + (b0 + b1);
-}
-
-// ------------------------------------------------------------------------------------------
-// int8: four signed bytes of one word against four activations.
-//
-// Flipping the sign bit gives u = b + 128 in 0..255; a byte permute builds 0x4B0000uu, the float
-// 2^23 + u; one packed add removes 2^23 + 128 exactly. 2.25 instructions per weight.
-DRB_DEV unsigned long long dot4_q8(uint32_t w, const unsigned long long* xp, unsigned long long acc) {
-  const uint32_t u = w ^ 0x80808080u;
-  const uint32_t hi = 0x0000004Bu;
-  const unsigned long long off = pack2(-8388736.f, -8388736.f);  // -(2^23 + 128)
-  const unsigned long long p0 = add2(pack2(__uint_as_float(prmt(u, hi, 0x4550u)), __uint_as_float(prmt(u, hi, 0x4551u))), off);
-  const unsigned long long p1 = add2(pack2(__uint_as_float(prmt(u, hi, 0x4552u)), __uint_as_float(prmt(u, hi, 0x4553u))), off);
-  acc = fma2(p0, xp[0], acc);
-  acc = fma2(p1, xp[1], acc);
-  return acc;
-}
-
-// One 16-byte chunk (16 int8, k ascending) against xp[0..7]; returns sum(w * x).
-DRB_DEV float dot16_q8(const uint4& v, const unsigned long long* xp) {
-  unsigned long long a = 0ull, b = 0ull;
-  a = dot4_q8(v.x, xp + 0, a);
-  b = dot4_q8(v.y, xp + 2, b);
-  a = dot4_q8(v.z, xp + 4, a);
-  b = dot4_q8(v.w, xp + 6, b);
-  float a0, a1, b0, b1;
-  unpack2(a, a0, a1);
-  unpack2(b, b0, b1);
-  return (a0 + a1) + (b0 + b1);
-}
-
 // One 16-byte chunk of bf16 (8 weights) against xp[0..3].
 DRB_DEV unsigned long long dot8_bf16(const uint4& v, const unsigned long long* xp, unsigned long long acc) {
   acc = fma2(pack2(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u)), xp[0], acc);
@@ -354,32 +291,11 @@ template <int N, bool EO>
 struct QAct {
   uint32_t l[3][N / 4];
   float delta;
-  DRB_DEV void quantize(const float* x) {
-    float m = 0.f;
-#pragma unroll
-    for (int k = 0; k < N; ++k) m = fmaxf(m, fabsf(x[k]));
-    delta = m > 0.f ? m * (1.f / 1048576.f) : 1.f;
-    const float inv = 1.f / delta;
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-#pragma unroll
-      for (int i = 0; i < N / 4; ++i) l[j][i] = 0u;
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-      int l0, l1, l2;
-      limbs3(__float2int_rn(x[k] * inv), l0, l1, l2);
-      const int word = EO ? 2 * (k / 8) + (k & 1) : k / 4;
-      const int byte = EO ? (k & 7) >> 1 : k & 3;
-      l[0][word] |= (uint32_t)(l0 & 0xff) << (8 * byte);
-      l[1][word] |= (uint32_t)(l1 & 0xff) << (8 * byte);
-      l[2][word] |= (uint32_t)(l2 & 0xff) << (8 * byte);
-    }
-  }
 };
 
 // Cooperative quantisation: instead of every lane converting its own slice (hundreds of
 // instructions, repeated by every warp that owns the same slice), each thread converts the float4
-// it loaded, the threads of one block of 16 or 32 values agree on max|x| with shuffles, and the
+// it loaded, the threads of one block of 32 values agree on max|x| with shuffles, and the
 // packed limb words go to shared memory, from where the owning lanes pick them up with a few
 // 128-bit loads. Must be called by whole warps (it shuffles); threads with nothing to convert pass
 // valid = false. g4 is the float4's index in the vector: consecutive lanes hold consecutive g4.
@@ -416,27 +332,8 @@ DRB_DEV void quant_store_eo(unsigned char* blocks, int g4, float4 v, bool valid)
   }
 }
 
-// Natural packing, 16 values per block, 64 bytes per block: 3 limbs x 4 words, delta, pad.
+// Natural packing, 16 values per block, 64 bytes per block: 3 limbs x 4 words, delta, pad (the SwiGLU outputs of the shared expert).
 constexpr int QB16_BYTES = 64;
-DRB_DEV void quant_store_nat(unsigned char* blocks, int g4, float4 v, bool valid) {
-  float m = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-  if (!valid) return;
-  const float delta = m > 0.f ? m * (1.f / 1048576.f) : 1.f;
-  const float inv = 1.f / delta;
-  int l[4][3];
-  limbs3(__float2int_rn(v.x * inv), l[0][0], l[0][1], l[0][2]);
-  limbs3(__float2int_rn(v.y * inv), l[1][0], l[1][1], l[1][2]);
-  limbs3(__float2int_rn(v.z * inv), l[2][0], l[2][1], l[2][2]);
-  limbs3(__float2int_rn(v.w * inv), l[3][0], l[3][1], l[3][2]);
-  unsigned char* blk = blocks + (size_t)(g4 >> 2) * QB16_BYTES;
-#pragma unroll
-  for (int j = 0; j < 3; ++j)
-    *reinterpret_cast<uint32_t*>(blk + (j * 4 + (g4 & 3)) * 4) =
-        (uint32_t)(l[0][j] & 0xff) | ((uint32_t)(l[1][j] & 0xff) << 8) | ((uint32_t)(l[2][j] & 0xff) << 16) | ((uint32_t)(l[3][j] & 0xff) << 24);
-  if ((g4 & 3) == 0) *reinterpret_cast<float*>(blk + 48) = delta;
-}
 
 DRB_DEV void qact_load(QAct<32, true>& a, float& sum, const unsigned char* blk) {
 #pragma unroll

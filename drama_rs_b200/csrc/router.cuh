@@ -17,9 +17,6 @@ namespace router {
 constexpr int THREADS = 256;  // one probability per thread in the tail: E <= 256
 constexpr int MAX_TOPK = 32;
 
-// a ranks before b: larger probability, or equal probability and lower index.
-DRB_DEV bool before(float pa, int ia, float pb, int ib) { return pa > pb || (pa == pb && ia < ib); }
-
 struct TopkSmem {
   float red[8];
   unsigned ured[8];
@@ -28,26 +25,6 @@ struct TopkSmem {
   __align__(16) unsigned long long comp[8 * MAX_TOPK];
   float top[MAX_TOPK];
 };
-
-// Sum over a 256-thread block with the reference's tree: xor-butterfly inside each warp, then the
-// same butterfly over the eight warp totals (kernels/drama.cu:39-47). Every thread gets the total.
-DRB_DEV float block_sum_256(float v, float* red) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  v = warp_sum(v);
-  __syncthreads();
-  if (lane == 0) red[w] = v;
-  __syncthreads();
-  return warp_sum(lane < 8 ? red[lane] : 0.f);
-}
-
-DRB_DEV float block_max_256(float v, float* red) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  v = warp_max(v);
-  __syncthreads();
-  if (lane == 0) red[w] = v;
-  __syncthreads();
-  return warp_max(lane < 8 ? red[lane] : -INFINITY);
-}
 
 // Softmax + top-k of one row of logits by a 256-thread block. Thread e holds logit e (or -inf).
 //
