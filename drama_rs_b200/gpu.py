@@ -147,7 +147,7 @@ class HostRow:
         assert n <= self._in.size and 4 * n <= dev.nbytes
         if self._queued:
             self._st.sync()
-        np.copyto(self._in if n == self._in.size else self._in[:n], x.reshape(-1))
+        np.copyto(self._in if n == self._in.size else self._in[:n], x.reshape(-1), casting="unsafe")  # as astype(np.float32) takes it
         self._queued = True
         check(self._l.dr_h2d(dev.ptr, self._p, 4 * n, self._st.raw), "h2d")
 
