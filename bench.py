@@ -344,8 +344,8 @@ def prefill_extra(torch, layers, st, ext_stream) -> dict:
     return {
         "workload": "prefill_300rows_zipf1.1_one_layer", "rows": rows, "experts_hit": hit, "max_group": int(counts.max()),
         "output_sum": float(y0.astype(np.float64).sum()),
-        "rows_per_s": rows / us_graph * 1e6, "us_layer_device_graph": us_graph, "launches_per_layer": 7,
-        "sequence": "rmsnorm_f16, router_logits_f16, moe_topk, moe_group, 2 x grouped tcgen05 GEMM (routed int4 + shared int8), combine",
+        "rows_per_s": rows / us_graph * 1e6, "us_layer_device_graph": us_graph, "launches_per_layer": 6,
+        "sequence": "one call: RMSNorm + router logits, top-k with ranks, row scatter, 2 x grouped tcgen05 GEMM (routed int4 + shared int8), combine",
         "rows_per_s_reference_call_sequence": rows / us_full * 1e6, "us_layer_reference_call_sequence_host_rows_in": us_full,
         "grouped_gemm_us": us_grouped, "grouped_gemm_rows_per_s": rows / us_grouped * 1e6,
         "grouped_gemm_includes": "8 routed experts per row and the shared expert (both GEMMs)",

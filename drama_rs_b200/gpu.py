@@ -130,7 +130,7 @@ class Graph:
 class HostRow:
     """A row of floats that crosses between the host and the front of a device buffer on every step. Both directions go
     through pinned memory of the row's own, so that the copies are queued behind one another and the host waits once, for the
-    result (pageable memory made every step two staged copies with a wait each: 146 us a step of 112 us of kernels, 133 so).
+    result (pageable memory made every step two staged copies with a wait each: 146 us a step of 112 us of kernels, 130 so).
     Copies by a kernel of one block, in a graph or beside it, and a word in pinned memory that the host watches instead of
     the stream measured the same or slower."""
 
