@@ -1040,9 +1040,14 @@ extern "C" int drb_moe_prefill_layer(const drb_moe_layer* w, const drb_prefill_b
                                      cudaStream_t st) {
   if (!w || !b || h != pf::H || i != pf::I || e < 1 || e > 256 || topk < 1 || topk > e || topk > 32) return -1;
   if (rows <= 0) return 0;
-  // what is read or written in 16-byte pieces, before anything is launched
-  for (const void* p : {(const void*)b->x, (const void*)b->rows16, (const void*)b->y, (const void*)b->sh_out, (const void*)b->act, (const void*)b->sh_act, w->router,
-                        w->gu_q, w->gu_sm, w->d_q, w->d_sm, w->sgu_q, w->sd_q})
+  // every pointer but logit_bias, before anything is launched; those that are read or written in 16-byte pieces on 16 bytes
+  const void* vec[] = {b->x, b->rows16, b->y, b->sh_out, b->act, b->sh_act, w->router, w->gu_q, w->gu_sm, w->d_q, w->d_sm, w->sgu_q, w->sd_q};
+  const void* word[] = {b->logits, b->idx, b->wts, b->sgate, b->counts, b->offsets, b->slot_of, b->row_of, w->post_norm, w->sgu_s, w->sd_s};
+  for (const void* p : vec)
+    if (!p) return -1;
+  for (const void* p : word)
+    if (!p) return -1;
+  for (const void* p : vec)
     if (reinterpret_cast<uintptr_t>(p) & 15) return -3;
   const DrbDevice& dev = drb_device(st);
   if (!dev.ready) return -2;

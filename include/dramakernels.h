@@ -221,8 +221,8 @@ int drb_moe_prefill_block(const uint8_t* gu_q, const dr_half* gu_sm, const uint8
  * in the rows, logits, routing and x; slots inside an expert in arbitrary order) in six launches. w and buf are host
  * structs of device pointers. buf: x f32 [rows, h]; rows16 fp16 [rows, h]; logits f32 [rows, e + 1]; logit_bias f32 [rows, e + 1]
  * added to the logits, or NULL; idx, wts [rows, topk]; sgate [rows]; counts, offsets [e]; slot_of, row_of [rows * topk]; act,
- * y, sh_act, sh_out as drb_moe_prefill_block. e <= 256, topk <= 32, h == 2048, i == 512, else -1; x, rows16, act, y, sh_act, sh_out
- * and the weights 16-byte aligned, else -3 and nothing is launched. */
+ * y, sh_act, sh_out as drb_moe_prefill_block. e <= 256, topk <= 32, h == 2048, i == 512 and no pointer but logit_bias NULL, else -1;
+ * x, rows16, act, y, sh_act, sh_out and the weights 16-byte aligned, else -3; nothing is launched then. */
 typedef struct {
   float* x;
   dr_half* rows16;

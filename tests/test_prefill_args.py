@@ -2,6 +2,7 @@
 
 from __future__ import annotations
 
+import ctypes as C
 from types import SimpleNamespace
 
 from drama_rs_b200 import ffi
@@ -53,3 +54,20 @@ def test_replaced_tensors_are_seen_by_the_next_call(monkeypatch):
     p.x, p.logit_bias = FakeBuf(), FakeBuf()
     p.run_device(3)
     assert p.l.b["x"] == p.x.ptr and p.l.b["logit_bias"] == p.logit_bias.ptr
+
+
+def test_the_layer_call_refuses_missing_and_misaligned_buffers():
+    """Refused on the host, before the device is looked at."""
+    w, b = ffi.MoeLayerPtrs(*range(16, 176, 16)), ffi.PrefillBuffers(*range(16, 256, 16))
+    call = lambda: ffi.lib().drb_moe_prefill_layer(C.byref(w), C.byref(b), 4, 16, 8, 2048, 512, 1e-6, None)  # noqa: E731
+    vectors = ("x", "rows16", "y", "sh_out", "act", "sh_act", "router", "gu_q", "gu_sm", "d_q", "d_sm", "sgu_q", "sd_q")
+    for struct in (w, b):
+        for name, _ in struct._fields_:
+            p = getattr(struct, name)
+            if name != "logit_bias":
+                setattr(struct, name, None)
+                assert call() == -1, name
+            if name in vectors:
+                setattr(struct, name, p + 8)
+                assert call() == -3, name
+            setattr(struct, name, p)
