@@ -28,10 +28,9 @@ DRB_DEV float half_round(float v) { return __half2float(__float2half_rn(v)); }
 // A team of eight lanes owns a group: lane j holds inputs j, 8 + j, ..., 56 + j, which are the terms of the converter's
 // running sum j in its order, so a 64-term sum is seven additions in the lane and three exchanges. (With two consecutive
 // inputs per lane, one warp per group, the same order took sixteen exchanges and fourteen additions for two inputs: 6.3 ms
-// for 134 M weights; 1.48 ms so, 0.93 ms with the candidates passed over that cannot win.)
+// for 134 M weights, 1.48 ms so.)
 struct Group {
   unsigned long long v2[4];  // inputs 8 i + j as packed pairs (i = 0, 1), (2, 3), (4, 5), (6, 7)
-  unsigned long long n2[4];  // the same, negated
 };
 
 DRB_DEV unsigned long long mul2(unsigned long long a, unsigned long long b) {
@@ -99,44 +98,77 @@ DRB_DEV void codes8(const Group& g, float lo, float scale, float rcp, unsigned l
 
 // sum of (q * scale + min - v)^2, every operation rounded
 DRB_DEV float error8(const Group& g, const unsigned long long (&q)[4], float scale, float lo) {
-  const unsigned long long s2 = dup2(scale), lo2 = dup2(lo);
+  const unsigned long long s2 = dup2(scale), lo2 = dup2(lo), neg1 = dup2(-1.f);
   unsigned long long t[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const unsigned long long d = add2(add2(mul2(q[i], s2), lo2), g.n2[i]);
+    const unsigned long long d = fma2(g.v2[i], neg1, add2(mul2(q[i], s2), lo2));
     t[i] = mul2(d, d);
   }
   return sum64(t);
 }
 
-// One term of it, for the input v and its code, as the converter computes both.
-DRB_DEV float term(float v, float scale, float lo) {
-  const float n = fminf(fmaxf(rintf(__fdiv_rn(__fsub_rn(v, lo), scale)), 0.f), 15.f);
-  const float d = __fsub_rn(__fadd_rn(__fmul_rn(n, scale), lo), v);
-  return __fmul_rn(d, d);
+// A candidate's error, estimated: in units of its scale and measured from the middle of its range an input is a = |v - min| / scale - 7.5|,
+// its code the nearest of 0.5, 1.5, ..., 7.5. With 32 added a float's last place is 2^-18: cutting off the fraction's 18 bits and
+// setting the highest of them is the rounding. One packed fused operation, two additions, two logic operations, two minima and two more
+// packed operations per two inputs, where the converter's own operations take 22 and a sum across lanes.
+constexpr float EST_BASE = 32.f;
+constexpr uint32_t EST_MASK = 0xFFFC0000u, EST_HALF = 0x00020000u;
+DRB_DEV void estimate2(unsigned long long v2, unsigned long long rcp2, unsigned long long c2, unsigned long long neg1, unsigned long long& sum) {
+  float u0, u1;
+  unpack2(fma2(v2, rcp2, c2), u0, u1);
+  const float r0 = __fadd_rn(fabsf(u0), EST_BASE), r1 = __fadd_rn(fabsf(u1), EST_BASE);
+  const float q0 = fminf(__uint_as_float(lop3_and_or(__float_as_uint(r0), EST_MASK, EST_HALF)), EST_BASE + 7.5f);
+  const float q1 = fminf(__uint_as_float(lop3_and_or(__float_as_uint(r1), EST_MASK, EST_HALF)), EST_BASE + 7.5f);
+  const unsigned long long e = fma2(pack2(q0, q1), neg1, pack2(r0, r1));
+  sum = fma2(e, e, sum);
 }
 
-constexpr int Q4_THREADS = 256, Q4_GROUPS = Q4_THREADS / 8;
-// Six blocks per multiprocessor (40 registers) hide the additions' chains a little better than five: 948 -> 934 us.
-// What bounds it: fp32 issue (24 candidates x 9 fp32 operations and 3 comparisons per weight; the packed forms halve the issue
-// slots), not memory (4.6 bytes per weight). A candidate's scale, min and reciprocal are the same for the whole group:
-// each lane of the team prepares three of the 24 and hands them round.
-// A rounded sum of terms that are not negative is at least the rounded sum of any two of them (rounding keeps the order), so the
-// terms of the group's smallest and largest input, which clipping hits hardest, bound a candidate's error from below. A
-// candidate whose bound is not below the best error so far cannot be taken and is passed over, when that holds for all
-// four groups of the warp. The ends outweigh the other 62 inputs' rounding from a shrink of about 0.8 on, the eleventh of the 24.
-__global__ void __launch_bounds__(Q4_THREADS, 6) k_quant_q4(const float* __restrict__ w, size_t groups, uint8_t* __restrict__ q,
+constexpr int Q4_THREADS = 256, Q4_WARPS = Q4_THREADS / 32, Q4_GROUPS = Q4_THREADS / 8;
+constexpr int Q4_STRIDE = 72;   // floats between a warp's four groups in shared memory: their 16-byte reads share no bank
+constexpr int Q4_LIGHT = 12;    // candidates that are estimated; the others clip a quarter of the range or more
+// What bounds it: fp32 and integer issue, not memory (4.6 bytes per weight). Of the 24 candidates the first twelve are told apart by
+// the estimate, lane j taking candidate j over the group's 64 inputs and candidate 8 + j % 4 over half of them (shared memory, broadcast
+// reads), and only those that the estimate's error leaves in the running are evaluated in the converter's operations and order: 1.02
+// on average on normal weights: 0.56 ms for 134 M weights. Every candidate evaluated that way took 1.48 ms, the half that a bound by the ends
+// leaves 0.93 ms; the estimate for sixteen of them instead of twelve, and with correctly rounded reciprocals and roots, 0.69 ms.
+// How far the estimate is off. In units of the scale, with a below 31 (beyond, and wherever something is not a number, the candidate
+// is evaluated): the estimate's a by 2^-19 for the sum with 32, 39 * 2^-23 for the reciprocal and 39 * 2^-24 for offset and product, the
+// converter's difference by 61 * 2^-24, its choice of code by 2 * 39 * 2^-23 at a boundary; each with 2^-23 |min| / scale for groups far
+// from zero. Together less than eta = 2^-15 + 2^-21 |min| / scale per input, so the sums S of 64 squares differ by less than
+// 16 eta sqrt(S) + 64 eta^2 (Cauchy), and by 2^-16 S for the additions. Two candidates whose estimates differ by more than both bounds are in
+// the right order.
+// The last twelve candidates leave the group's smallest and largest input at least a quarter of half the range outside, less what
+// rounding scale and min to fp16 moves the ends. On most weights those two inputs alone exceed the best error of the others; where
+// they do not, for one of the warp's four groups, all twelve are evaluated.
+template <bool VEC>
+__global__ void __launch_bounds__(Q4_THREADS, 5) k_quant_q4(const float* __restrict__ w, size_t groups, uint8_t* __restrict__ q,
                                                          __half2* __restrict__ sm) {
+  __shared__ __align__(16) float stage[Q4_WARPS][4 * Q4_STRIDE];
   const size_t gi = (size_t)blockIdx.x * Q4_GROUPS + (threadIdx.x >> 3);
-  const int j = threadIdx.x & 7;
-  const size_t gr = gi < groups ? gi : groups - 1;  // teams beyond the end redo the last group and write nothing
+  const int j = threadIdx.x & 7, lane = threadIdx.x & 31, team = lane >> 3;
+  float* const mine = stage[threadIdx.x >> 5] + team * Q4_STRIDE;
+  // teams beyond the end redo the last group and write nothing
+  if (VEC) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const size_t gr = min(gi - team + 2 * h + (lane >> 4), groups - 1);
+      *reinterpret_cast<float4*>(stage[threadIdx.x >> 5] + (2 * h + (lane >> 4)) * Q4_STRIDE + 4 * (lane & 15)) =
+          __ldg(reinterpret_cast<const float4*>(w + gr * 64) + (lane & 15));
+    }
+  } else {
+    const size_t gr = min(gi, groups - 1);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mine[8 * i + j] = __ldg(w + gr * 64 + 8 * i + j);
+  }
+  __syncwarp();
   Group g;
   float gmin = INFINITY, gmax = -INFINITY;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float a = __ldg(w + gr * 64 + 16 * i + j), b = __ldg(w + gr * 64 + 16 * i + 8 + j);
+    const float a = mine[16 * i + j], b = mine[16 * i + 8 + j];
     gmin = fminf(gmin, fminf(a, b)), gmax = fmaxf(gmax, fmaxf(a, b));
-    g.v2[i] = pack2(a, b), g.n2[i] = pack2(-a, -b);
+    g.v2[i] = pack2(a, b);
   }
 #pragma unroll
   for (int o = 1; o < 8; o <<= 1) {
@@ -144,39 +176,104 @@ __global__ void __launch_bounds__(Q4_THREADS, 6) k_quant_q4(const float* __restr
     gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
   }
   const float center = __fmul_rn(__fadd_rn(gmin, gmax), 0.5f);
-  float c_scale[STEPS / 8], c_lo[STEPS / 8], c_rcp[STEPS / 8], c_least[STEPS / 8];  // candidates j, 8 + j, 16 + j
-#pragma unroll
-  for (int t = 0; t < STEPS / 8; ++t) {
-    const float shrink = c_shrink[8 * t + j];
+  const unsigned long long neg1 = dup2(-1.f);
+  struct Candidate {
+    float scale, lo, rcp;
+  };
+  auto candidate = [&](float shrink) {
+    Candidate c;
     const float lo_c = __fadd_rn(center, __fmul_rn(__fsub_rn(gmin, center), shrink));
     const float hi_c = __fadd_rn(center, __fmul_rn(__fsub_rn(gmax, center), shrink));
-    c_scale[t] = fmaxf(half_round(fmaxf(__fdiv_rn(__fsub_rn(hi_c, lo_c), 15.0f), 1e-10f)), 1e-10f);
-    c_lo[t] = half_round(lo_c);
-    c_rcp[t] = __frcp_rn(c_scale[t]);
-    c_least[t] = __fadd_rn(term(gmin, c_scale[t], c_lo[t]), term(gmax, c_scale[t], c_lo[t]));
-  }
-  float best_err = 0.f, best_scale = 0.f, best_lo = 0.f, best_rcp = 0.f;
-  unsigned long long bq[4];
-#pragma unroll
-  for (int t = 0; t < STEPS / 8; ++t)
+    c.scale = fmaxf(half_round(fmaxf(__fdiv_rn(__fsub_rn(hi_c, lo_c), 15.0f), 1e-10f)), 1e-10f);
+    c.lo = half_round(lo_c);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(c.rcp) : "f"(c.scale));
+    return c;
+  };
+  const Candidate ca = candidate(c_shrink[j]), cb = candidate(c_shrink[8 + (j & 3)]);
+  const float mid_a = __fmaf_rn(-ca.lo, ca.rcp, -7.5f), mid_b = __fmaf_rn(-cb.lo, cb.rcp, -7.5f);
+  unsigned long long sum_a = 0ull, sum_b = 0ull;
+  {
+    const unsigned long long ra = dup2(ca.rcp), ma = dup2(mid_a), rb = dup2(cb.rcp), mb = dup2(mid_b);
+    const ulonglong2* chunk = reinterpret_cast<const ulonglong2*>(mine);
 #pragma unroll 2
-    for (int i = 0; i < 8; ++i) {
-      const bool first = t == 0 && i == 0;
-      if (!first && __all_sync(0xffffffffu, __shfl_sync(0xffffffffu, c_least[t], i, 8) >= best_err)) continue;
-      const float scale = __shfl_sync(0xffffffffu, c_scale[t], i, 8), lo = __shfl_sync(0xffffffffu, c_lo[t], i, 8);
-      const float rcp = __shfl_sync(0xffffffffu, c_rcp[t], i, 8);
-      codes8(g, lo, scale, rcp, bq);
-      const float err = error8(g, bq, scale, lo);
-      if (first || err < best_err) best_err = err, best_scale = scale, best_lo = lo, best_rcp = rcp;
+    for (int k = 0; k < 8; ++k) {
+      const ulonglong2 v0 = chunk[2 * k], v1 = chunk[2 * k + 1], u = chunk[2 * k + (j >> 2)];
+      estimate2(v0.x, ra, ma, neg1, sum_a);
+      estimate2(u.x, rb, mb, neg1, sum_b);
+      estimate2(v0.y, ra, ma, neg1, sum_a);
+      estimate2(v1.x, ra, ma, neg1, sum_a);
+      estimate2(u.y, rb, mb, neg1, sum_b);
+      estimate2(v1.y, ra, ma, neg1, sum_a);
     }
-  codes8(g, best_lo, best_scale, best_rcp, bq);
-  // One least-squares refinement of (scale, min) given the codes.
-  const float n = 64.f;
-  unsigned long long t[4];
-  const float sq = sum64(bq);
+  }
+  // an estimate's two sides; NaN where the candidate has to be evaluated whatever the others are
+  auto sides = [&](const Candidate& c, float mid, float s, float& least, float& most) {
+    const float eta = 0x1p-15f + 0x1p-21f * fabsf(c.lo) * c.rcp, s2 = c.scale * c.scale;
+    const float a0 = fabsf(__fmaf_rn(gmin, c.rcp, mid)), a1 = fabsf(__fmaf_rn(gmax, c.rcp, mid));
+    float root;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(root) : "f"(s));
+    const float est = a0 < 31.f && a1 < 31.f ? s2 * s : NAN, off = s2 * (17.f * eta * root + 70.f * eta * eta + 0x1p-16f * s) + 1e-42f;
+    least = est - off, most = est + off;
+  };
+  float lo_s, hi_s, least_a, least_b, most_a, most_b;
+  unpack2(sum_a, lo_s, hi_s);
+  sides(ca, mid_a, lo_s + hi_s, least_a, most_a);
+  unpack2(sum_b, lo_s, hi_s);
+  float s_b = lo_s + hi_s;
+  s_b += __shfl_xor_sync(0xffffffffu, s_b, 4);
+  sides(cb, mid_b, s_b, least_b, most_b);
+  float bound = fminf(most_a, most_b);  // no candidate whose error exceeds it can be the best: fminf passes NaN over
 #pragma unroll
-  for (int i = 0; i < 4; ++i) t[i] = mul2(bq[i], bq[i]);
-  const float sqq = sum64(t);
+  for (int o = 1; o < 8; o <<= 1) bound = fminf(bound, __shfl_xor_sync(0xffffffffu, bound, o));
+  uint32_t open = (__ballot_sync(0xffffffffu, !(least_a > bound)) >> (8 * team)) & 0xffu;  // candidates of this team's group that may be the best
+  open |= ((__ballot_sync(0xffffffffu, !(least_b > bound)) >> (8 * team)) & 0xfu) << 8;
+  const float far = fmaxf(fabsf(gmin), fabsf(gmax)), half = 0.5f * (gmax - gmin);
+  const float clip = 0.2499f * half - 0x1p-10f * (far + half) - 1e-6f;
+  const bool heavy = __any_sync(0xffffffffu, !(clip > 0.f && 1.99f * clip * clip >= bound));
+  float best_err = 0.f, best_scale = 0.f, best_lo = 0.f;
+  unsigned long long bq[4];
+  auto evaluate = [&](const Candidate& c, bool first, bool counts) {
+    unsigned long long cq[4];
+    codes8(g, c.lo, c.scale, c.rcp, cq);
+    const float err = error8(g, cq, c.scale, c.lo);
+    if (first || (counts && err < best_err)) {
+      best_err = err, best_scale = c.scale, best_lo = c.lo;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) bq[i] = cq[i];
+    }
+  };
+  for (bool first = true; __any_sync(0xffffffffu, open != 0u); first = false) {  // the estimate's own least is always open: every team has one
+    const int i = open ? __ffs(open) - 1 : 0;
+    auto of = [&](float a, float b) { return __shfl_sync(0xffffffffu, i < 8 ? a : b, i & 7, 8); };
+    Candidate c;
+    c.scale = of(ca.scale, cb.scale), c.lo = of(ca.lo, cb.lo), c.rcp = of(ca.rcp, cb.rcp);
+    evaluate(c, first, open != 0u);
+    open &= open - 1u;
+    if (best_err == 0.f) open = 0u;  // nothing is less
+  }
+  if (heavy)
+#pragma unroll 1
+    for (int i = Q4_LIGHT; i < STEPS && __any_sync(0xffffffffu, best_err != 0.f); ++i) evaluate(candidate(c_shrink[i]), false, true);
+  // This lane's codes as bytes: inputs 8 i + j in byte i of c0 (i < 4) or c1. With 1.5 * 2^23 added a code is the float's lowest byte.
+  uint32_t c0, c1;
+  {
+    uint32_t n[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float a, b;
+      unpack2(add2(bq[i], dup2(12582912.f)), a, b);
+      n[2 * i] = __float_as_uint(a), n[2 * i + 1] = __float_as_uint(b);
+    }
+    c0 = prmt(prmt(n[0], n[1], 0x0040u), prmt(n[2], n[3], 0x0040u), 0x5410u);
+    c1 = prmt(prmt(n[4], n[5], 0x0040u), prmt(n[6], n[7], 0x0040u), 0x5410u);
+  }
+  // One least-squares refinement of (scale, min) given the codes. Their sums are whole numbers below 2^24, the same in any order.
+  const float n = 64.f;
+  uint32_t isum = __dp4a(c0, 0x01010101u, __dp4a(c1, 0x01010101u, 0u)) | (__dp4a(c0, c0, __dp4a(c1, c1, 0u)) << 12);
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) isum += __shfl_xor_sync(0xffffffffu, isum, o);
+  const float sq = (float)(isum & 0xfffu), sqq = (float)(isum >> 12);
+  unsigned long long t[4];
   const float sw = sum64(g.v2);
 #pragma unroll
   for (int i = 0; i < 4; ++i) t[i] = mul2(bq[i], g.v2[i]);
@@ -189,13 +286,7 @@ __global__ void __launch_bounds__(Q4_THREADS, 6) k_quant_q4(const float* __restr
   const float ls_err = error8(g, bq, ls_scale_h, ls_min_h);
   if (ls_err < best_err && ok && ls_scale_h > 0.f) best_scale = ls_scale_h, best_lo = ls_min_h;
   // Packing: this lane's codes are nibble j of words 0..7; three exchanges transpose that to all nibbles of word j.
-  uint32_t m = 0u;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float a, b;
-    unpack2(bq[i], a, b);
-    m |= ((uint32_t)a << (8 * i)) | ((uint32_t)b << (8 * i + 4));
-  }
+  uint32_t m = prmt(c0 | (c0 >> 4), c1 | (c1 >> 4), 0x6420u);
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) {
     const uint32_t keep = o == 4 ? 0x0000FFFFu : o == 2 ? 0x00FF00FFu : 0x0F0F0F0Fu;  // nibbles whose index lacks bit o
@@ -239,7 +330,8 @@ __global__ void __launch_bounds__(256) k_quant_q8(const float* __restrict__ w, s
 // (its quantiser is the Python converter).
 extern "C" int drb_quant_q4(const float* w, size_t groups, uint8_t* q, __half2* sm, cudaStream_t st) {
   if (groups == 0) return 0;
-  quant::k_quant_q4<<<(unsigned)((groups + quant::Q4_GROUPS - 1) / quant::Q4_GROUPS), quant::Q4_THREADS, 0, st>>>(w, groups, q, sm);
+  const auto kernel = (reinterpret_cast<uintptr_t>(w) & 15) == 0 ? quant::k_quant_q4<true> : quant::k_quant_q4<false>;  // w starts at any float
+  kernel<<<(unsigned)((groups + quant::Q4_GROUPS - 1) / quant::Q4_GROUPS), quant::Q4_THREADS, 0, st>>>(w, groups, q, sm);
   return 0;
 }
 
