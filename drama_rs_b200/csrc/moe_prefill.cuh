@@ -281,40 +281,52 @@ __global__ void __launch_bounds__(64)
 }
 
 // x[r] += sigmoid(sgate[r]) * shared[r] + sum_k w[r,k] * Y[slot_of[r,k]], k ascending (fixed order, so
-// the result does not depend on how slots were handed out). Block (r, c): 1024 columns of row r, one float4 per thread.
+// the result does not depend on how slots were handed out). Block (r, c): 1024 columns of rows r, r + gridDim.x, ..., one float4 per thread.
 // Bound by Y's bytes from L2 or HBM; all of a thread's rows are requested before the first is used (TK = 8: in a loop over a
-// runtime topk every row waited for the one before, 13 us at 300 rows instead of 5).
+// runtime topk every row waited for the one before, 13 us at 300 rows instead of 5). A row's slots, weights and gate lie spread over
+// the lanes of each warp and are fetched a row ahead: behind them its data would wait for two trips instead of one.
+constexpr int CMB_BLOCKS = 4;  // resident blocks per multiprocessor
 template <int TK>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, CMB_BLOCKS)
     k_combine(float* __restrict__ x, const float* __restrict__ Y, const int* __restrict__ slot_of,
-              const float* __restrict__ wts, const float* __restrict__ sgate, const float* __restrict__ shared, int topk,
+              const float* __restrict__ wts, const float* __restrict__ sgate, const float* __restrict__ shared, int rows, int topk,
               int Hd) {
   pdl_wait();
   pdl_launch_dependents();
-  const int r = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
-  if (c >= Hd) return;
-  float4* xo = reinterpret_cast<float4*>(x + (size_t)r * Hd + c);
-  const float gate = __ldcg(sgate + r);
-  const float4 sh = __ldcg(reinterpret_cast<const float4*>(shared + (size_t)r * Hd + c));
-  float4 o = __ldcg(xo), acc;
-  auto add = [&](float w, const float4& v) { acc.x += w * v.x, acc.y += w * v.y, acc.z += w * v.z, acc.w += w * v.w; };
-  auto row = [&](int k) { return __ldcg(reinterpret_cast<const float4*>(Y + (size_t)__ldcg(slot_of + (size_t)r * topk + k) * Hd + c)); };
-  if (TK > 0) {
-    float4 v[TK > 0 ? TK : 1];
-    float w[TK > 0 ? TK : 1];
+  const int lane = threadIdx.x & 31, first = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+  if (first - 4 * lane >= Hd) return;
+  const bool in = first < Hd;
+  const int c = in ? first : Hd - 4;  // whole warps stay for the shuffles
+  auto head = [&](int r) -> int {  // TK > 0: lane k < TK the slot of pair k, TK + k its weight, 2 TK the gate
+    if (lane < TK) return __ldcg(slot_of + (size_t)r * TK + lane);
+    if (lane < 2 * TK) return __float_as_int(__ldcg(wts + (size_t)r * TK + lane - TK));
+    return __float_as_int(__ldcg(sgate + r));
+  };
+  int r = blockIdx.x, next = TK > 0 ? head(r) : 0;
+  for (; r < rows; r += gridDim.x) {
+    const int now = next;
+    if (TK > 0 && r + (int)gridDim.x < rows) next = head(r + gridDim.x);
+    float4* xo = reinterpret_cast<float4*>(x + (size_t)r * Hd + c);
+    const float4 sh = __ldcg(reinterpret_cast<const float4*>(shared + (size_t)r * Hd + c));
+    float4 o = __ldcg(xo), acc;
+    auto add = [&](float w, const float4& v) { acc.x += w * v.x, acc.y += w * v.y, acc.z += w * v.z, acc.w += w * v.w; };
+    auto row = [&](int slot) { return __ldcg(reinterpret_cast<const float4*>(Y + (size_t)slot * Hd + c)); };
+    if (TK > 0) {
+      float4 v[TK > 0 ? TK : 1];
 #pragma unroll
-    for (int k = 0; k < TK; ++k) v[k] = row(k), w[k] = __ldcg(wts + (size_t)r * TK + k);
-    const float sg = sigmoid_f(gate);
-    acc = make_float4(sg * sh.x, sg * sh.y, sg * sh.z, sg * sh.w);
+      for (int k = 0; k < TK; ++k) v[k] = row(__shfl_sync(0xffffffffu, now, k));
+      const float sg = sigmoid_f(__int_as_float(__shfl_sync(0xffffffffu, now, 2 * TK)));
+      acc = make_float4(sg * sh.x, sg * sh.y, sg * sh.z, sg * sh.w);
 #pragma unroll
-    for (int k = 0; k < TK; ++k) add(w[k], v[k]);
-  } else {
-    const float sg = sigmoid_f(gate);
-    acc = make_float4(sg * sh.x, sg * sh.y, sg * sh.z, sg * sh.w);
-    for (int k = 0; k < topk; ++k) add(__ldcg(wts + (size_t)r * topk + k), row(k));
+      for (int k = 0; k < TK; ++k) add(__int_as_float(__shfl_sync(0xffffffffu, now, TK + k)), v[k]);
+    } else {
+      const float sg = sigmoid_f(__ldcg(sgate + r));
+      acc = make_float4(sg * sh.x, sg * sh.y, sg * sh.z, sg * sh.w);
+      for (int k = 0; k < topk; ++k) add(__ldcg(wts + (size_t)r * topk + k), row(__ldcg(slot_of + (size_t)r * topk + k)));
+    }
+    o.x += acc.x, o.y += acc.y, o.z += acc.z, o.w += acc.w;
+    if (in) *xo = o;
   }
-  o.x += acc.x, o.y += acc.y, o.z += acc.z, o.w += acc.w;
-  *xo = o;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -852,8 +864,10 @@ extern "C" int dr_moe_combine(float* x, const float* Y, const int* slot_of, cons
   if (H % 4 != 0) return -1;
   if (rows <= 0 || H <= 0) return 0;
   const DrbDevice& dev = drb_device(st);
-  drb_launch(topk == 8 ? pf::k_combine<8> : pf::k_combine<0>, dim3(rows, (H + 1023) / 1024), dim3(256), 0, st, dev.ready && dev.pdl, x, Y, slot_of,
-             wts, sgate, shared, topk, H);
+  const int gy = (H + 1023) / 1024;
+  const int gx = max(1, pf::CMB_BLOCKS * (dev.ready ? dev.sms : 1) / gy);  // what is resident at once
+  drb_launch(topk == 8 ? pf::k_combine<8> : pf::k_combine<0>, dim3(rows < gx ? rows : gx, gy), dim3(256), 0, st, dev.ready && dev.pdl, x, Y, slot_of,
+             wts, sgate, shared, rows, topk, H);
   return 0;
 }
 
