@@ -191,24 +191,16 @@ __global__ void __launch_bounds__(THREADS, 2)
   const bool writer = (int)threadIdx.x < bo;
   float add = 0.f;
   if (res && writer && u0 + (int)threadIdx.x < u1) add = __ldcg(res + u0 + threadIdx.x);
+  // RMSNorm: the sum is linear in the input, so the rows meet x * nw and the outputs get 1 / rms at the end, where the warps meet
+  // anyway: nothing waits for the sum of squares in front of the conversion (a chain of 33 projections, half of them normed, 129.6 ->
+  // 125.5 us).
+  float ss = 0.f;
   if (nw) {
-    float ss = 0.f;
-#pragma unroll
-    for (int q = 0; q < NSEG; ++q) ss += (xv[q].x * xv[q].x + xv[q].y * xv[q].y) + (xv[q].z * xv[q].z + xv[q].w * xv[q].w);
-    ss = warp_sum(ss);
-    if (lane == 0) ctl.red[warp] = ss;
-    consumer_sync();
-    float tot = 0.f;
-#pragma unroll
-    for (int w = 0; w < KW; w += 4) {  // the warps of tile 0: each input once
-      const float4 v = *reinterpret_cast<const float4*>(&ctl.red[w]);
-      tot += (v.x + v.y) + (v.z + v.w);
-    }
-    const float inv = rsqrtf(tot / K + eps);
 #pragma unroll
     for (int q = 0; q < NSEG; ++q) {
+      ss += (xv[q].x * xv[q].x + xv[q].y * xv[q].y) + (xv[q].z * xv[q].z + xv[q].w * xv[q].w);
       if (!EARLY) wv[q] = __ldcg(reinterpret_cast<const float4*>(nw + q * SEG + kw * GROUP) + lane);
-      xv[q] = make_float4(xv[q].x * inv * wv[q].x, xv[q].y * inv * wv[q].y, xv[q].z * inv * wv[q].z, xv[q].w * inv * wv[q].w);
+      xv[q] = make_float4(xv[q].x * wv[q].x, xv[q].y * wv[q].y, xv[q].z * wv[q].z, xv[q].w * wv[q].w);
     }
   }
   // Limbs. Lane l holds inputs 4 l .. 4 l + 3 of the 128; the operand wants, in lane (g, t4), limb g of inputs 16 t4 + 4 i and
@@ -246,6 +238,11 @@ __global__ void __launch_bounds__(THREADS, 2)
     delta[q] = t4 == 0 ? d : t4 == 1 ? d * 16384.f : 0.f;
   }
   __syncwarp();  // before partial sums overwrite the limbs
+  if (nw) {
+    ss = warp_sum(ss);
+    if (lane == 0) ctl.red[warp] = ss;  // read behind the first batch's barrier
+  }
+  float inv_rms = 1.f;
 
   for (int t = 0; t < ntiles; ++t) {
     float a0 = 0.f, a1 = 0.f;  // rows g and g + 8 of the tile
@@ -285,6 +282,15 @@ __global__ void __launch_bounds__(THREADS, 2)
       consumer_sync();
       const int o = (int)threadIdx.x, first = u0 + t / TB * bo;
       if (writer) {
+        if (nw && t < TB) {
+          float tot = 0.f;
+#pragma unroll
+          for (int w = 0; w < KW; w += 4) {  // the warps of tile 0: each input once
+            const float4 v = *reinterpret_cast<const float4*>(&ctl.red[w]);
+            tot += (v.x + v.y) + (v.z + v.w);
+          }
+          inv_rms = rsqrtf(tot / K + eps);
+        }
         const int tile = o / (16 / U), row = o % (16 / U);  // within the batch
         const float* pp = reinterpret_cast<const float*>(own + (RS > 1 ? tile * KW : 0) * P::WARP_BYTES) + (t / TB & 1) * BATCH + (RS > 1 ? 0 : tile * 16) + row;
         float r0 = 0.f, r1 = 0.f;
@@ -293,7 +299,8 @@ __global__ void __launch_bounds__(THREADS, 2)
           r0 += pp[w * (P::WARP_BYTES / 4)];
           if (U == 2) r1 += pp[w * (P::WARP_BYTES / 4) + 8];
         }
-        if (first + o < u1) y[first + o] = U == 2 ? silu_f(r0) * r1 : r0 + add;
+        r0 *= inv_rms;
+        if (first + o < u1) y[first + o] = U == 2 ? silu_f(r0) * (r1 * inv_rms) : r0 + add;
         add = res && first + bo + o < u1 ? __ldcg(res + first + bo + o) : 0.f;  // the next batch's
       }
     }
@@ -381,23 +388,24 @@ __global__ void __launch_bounds__(THREADS, 2)
     xv[j] = __ldcg(reinterpret_cast<const float4*>(x) + threadIdx.x + j * NT);
     wv[j] = nw ? __ldcg(reinterpret_cast<const float4*>(nw) + threadIdx.x + j * NT) : make_float4(1.f, 1.f, 1.f, 1.f);
   }
-  float inv = 1.f;
-  if (nw) {
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    xs4[swz4(threadIdx.x + j * NT)] = nw ? make_float4(xv[j].x * wv[j].x, xv[j].y * wv[j].y, xv[j].z * wv[j].z, xv[j].w * wv[j].w) : xv[j];
+  if (nw) {  // 1 / rms joins at the end, as in the int8 form
     float ss = 0.f;
 #pragma unroll
     for (int j = 0; j < 2; ++j) ss += xv[j].x * xv[j].x + xv[j].y * xv[j].y + xv[j].z * xv[j].z + xv[j].w * xv[j].w;
     ss = warp_sum(ss);
     if (lane == 0) ctl.red[warp] = ss;
-    consumer_sync();
+  }
+  consumer_sync();
+  float inv = 1.f;
+  if (nw) {
     float t = 0.f;
 #pragma unroll
     for (int w = 0; w < CW; ++w) t += ctl.red[w];
     inv = rsqrtf(t / K + eps);
   }
-#pragma unroll
-  for (int j = 0; j < 2; ++j)
-    xs4[swz4(threadIdx.x + j * NT)] = nw ? make_float4(xv[j].x * inv * wv[j].x, xv[j].y * inv * wv[j].y, xv[j].z * inv * wv[j].z, xv[j].w * inv * wv[j].w) : xv[j];
-  consumer_sync();
   unsigned long long xp[NCH * 4];
 #pragma unroll
   for (int i = 0; i < NCH; ++i)
@@ -426,7 +434,7 @@ __global__ void __launch_bounds__(THREADS, 2)
     unpack2(a0, p0, p1);
     unpack2(a1, p2, p3);
     const float d = warp_sum((p0 + p1) + (p2 + p3));
-    if (lane == 0 && row < u1) y[row] = d;
+    if (lane == 0 && row < u1) y[row] = d * inv;
   }
 }
 
