@@ -940,9 +940,11 @@ static int run_block(const Block& b, const DrbDevice& dev, cudaStream_t st) {
       (b.rows_sh > 0 && (odd(b.sgu_q) || odd(b.sd_q) || odd(b.sh_act))))
     return -3;
   if (prep && !b.prepared) {
+    // Both the preparing launch and the gate/up launch behind it wait for their predecessor themselves, ahead of the first read, and so
+    // may start under it: 20 rows over FP8 experts 54.8 -> 50.4 us, 300 rows 137.0 -> 132.7.
     auto kp = b.x_bf16 ? k_prep_rows<true, FMT == 0> : k_prep_rows<false, FMT == 0>;
     for (int e0 = 0; e0 == 0 || e0 < b.E; e0 += MAX_E)  // the shared expert's rows with the first experts
-      drb_launch(kp, dim3(2 * dev.sms), dim3(PREP_THREADS), 0, st, false, static_cast<const uint4*>(b.x), b.row_of, b.offsets + e0, b.counts + e0,
+      drb_launch(kp, dim3(2 * dev.sms), dim3(PREP_THREADS), 0, st, dev.pdl, static_cast<const uint4*>(b.x), b.row_of, b.offsets + e0, b.counts + e0,
                  b.E - e0 < MAX_E ? b.E - e0 : MAX_E, b.y_row_of, tok, e0 == 0 ? b.rows_sh : 0, shtok);
   }
   // Every gate/up launch before the first down launch: y holds the token rows until then.
@@ -973,7 +975,7 @@ static int run_block(const Block& b, const DrbDevice& dev, cudaStream_t st) {
       a.scales = sc, a.shs = static_cast<const __half*>(gemm == 0 ? b.sgu_s : b.sd_s);
       a.offsets = b.offsets + e0, a.counts = b.counts + e0, a.E = ne > 0 ? ne : 0, a.rows_sh = sh ? b.rows_sh : 0;
       if (gemm == 0)
-        drb_launch(prep ? k_grouped<0, FMT, true> : k_grouped<0, FMT, FMT != 0>, dim3(dev.sms), dim3(Smem<0, FMT>::THREADS), Smem<0, FMT>::BYTES, st, dev.pdl && b.prepared && b.E <= MAX_E, m, a);
+        drb_launch(prep ? k_grouped<0, FMT, true> : k_grouped<0, FMT, FMT != 0>, dim3(dev.sms), dim3(Smem<0, FMT>::THREADS), Smem<0, FMT>::BYTES, st, dev.pdl && prep && b.E <= MAX_E, m, a);
       else  // only the first one follows the gate/up kernel
         drb_launch(k_grouped<1, FMT, true>, dim3(dev.sms), dim3(Smem<1, FMT>::THREADS), Smem<1, FMT>::BYTES, st, dev.pdl && b.E <= MAX_E, m, a);
     }
