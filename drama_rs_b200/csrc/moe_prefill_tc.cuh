@@ -2,7 +2,7 @@
 // the 5th-generation tensor cores, with the dequantised weights handed over in TENSOR memory.
 //
 //   gate/up:  for expert e with its tokens  D[128, nt] = W_tile[128, 2048] . X_e[nt, 2048]^T
-//             (the tile interleaves 64 gate rows with their 64 up rows), epilogue silu(g) * u -> act
+//             (the tile is 64 gate rows and their 64 up rows), epilogue silu(g) * u -> act
 //   down:     D[128, nt] = Wd_tile[128, 512] . act_e[nt, 512]^T -> y
 //
 // The weight rows are the MMA's M = 128 dimension and the tokens its N dimension (16 .. 64): most experts see a handful
@@ -21,9 +21,9 @@
 //                 one row: four (int4) or eight (8-bit) 16-byte pieces out of the swizzled raw stage, two 32-column
 //                 tcgen05.st. Three stages: 128 columns each, with a token tile in shared memory.
 //   MMA warp      sixteen K = 16 instructions per step, one commit that frees the stage
-//   loader warp   tiled TMA: 128 rows x 128 bytes per request with the 128-byte swizzle; a gate/up tile arrives with gate
-//                 row j and up row j interleaved, which a 4-D view of the weight tensor expresses; the item's scales
-//                 ride on its first request
+//   loader warp   tiled TMA: 128 rows x 128 bytes per request with the 128-byte swizzle; a gate/up tile is 64 gate rows and
+//                 their 64 up rows, which a 4-D view of the weight tensor expresses; the item's scales ride on its
+//                 first request
 //   token warp    the tokens' fp16 rows: groups of eight consecutive rows by one TMA request per step (4 KB: eight rows of
 //                 four 128-byte swizzled columns), scattered rows by tile::gather4 (512 bytes per request; it costs the copy
 //                 engine 19 cycles against 49 for the 4 KB box)
@@ -172,9 +172,6 @@ DRB_DEV void dequant8_i8(uint32_t w0, uint32_t w1, __half2 s2, uint32_t* o) {
 DRB_DEV void dequant4_e4m3(uint32_t w, uint32_t* o) {
   asm("{.reg .b16 lo, hi; mov.b32 {lo, hi}, %2; cvt.rn.f16x2.e4m3x2 %0, lo; cvt.rn.f16x2.e4m3x2 %1, hi;}" : "=r"(o[0]), "=r"(o[1]) : "r"(w));
 }
-// Position of input k within its eight in dequant8_perm's order.
-DRB_DEV int perm_pos(int k) { return (k & ~7) | ((k & 3) << 1) | ((k >> 2) & 1); }
-
 // ---- token rows ----------------------------------------------------------------------------------------------------
 // 16-bit rows -> fp16 rows in slot order at a stride of TOKEN_STRIDE bytes: routed slot s from row (row_of ? row_of[s] : s)
 // of x into row (dst_row_of ? dst_row_of[s] : s) of dst, shared row r from row r of x into sh_dst; in the order of dequant8_perm
@@ -270,8 +267,8 @@ __global__ void __launch_bounds__(PREP_THREADS)
 DRB_DEV float silu_fast(float x) { return __fdividef(x, 1.f + expf(-x)); }
 
 // *p = v unless at < 0.
-DRB_DEV void store_valid(__half* p, __half v, int at) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %2, 0;\n\t@p st.global.b16 [%0], %1;\n\t}" ::"l"(p), "h"(__half_as_ushort(v)), "r"(at) : "memory");
+DRB_DEV void store_valid(__half* p, uint32_t two, int at) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %2, 0;\n\t@p st.global.b32 [%0], %1;\n\t}" ::"l"(p), "r"(two), "r"(at) : "memory");
 }
 DRB_DEV void store_valid(float* p, float v, int at) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %2, 0;\n\t@p st.global.f32 [%0], %1;\n\t}" ::"l"(p), "f"(v), "r"(at) : "memory");
@@ -308,6 +305,19 @@ struct Ring {
 template <unsigned ERR, int N>
 DRB_DEV void wait_at(uint64_t* bars, const Ring<N>& r, unsigned& spent) {
   mbar_wait_ring<ERR>(smem_u32(bars) + 8 * r.i, r.par, spent);
+}
+
+// gate/up: unit (0..15) of a quadrant that the i-th lane of its half h holds. The epilogue reads sixteen lanes at a time in the layout of an
+// mma.sync accumulator: thread (i, .) gets lanes i and i + 8, its unit's gate and up values for two tokens each, from either half.
+// The two halves' units lie beside one another in act's order (int4: dequant8_perm's, where unit k + 4 follows unit k; FP8: k, k + 1), so a
+// thread's two results for a token go out as one 32-bit store; the higher unit is in half 0 for i >= 4, which gives the eight lanes of a
+// half eight different row numbers mod 8, and so their reads of the swizzled weights different banks. With gate and up rows in
+// neighbouring lanes every value crossed by a shuffle and two selects, and every result was a store of its own: prefill of 300, 700 and
+// 2048 rows 134.9, 180.7, 310.1 -> 134.0, 179.2, 307.4 us; nothing at 64.
+template <int FMT>
+DRB_DEV int epi_unit(int h, int i) {
+  if (FMT == 0) return i + (h == 0 ? (i < 4 ? 0 : 8) : 4);
+  return 2 * i + ((h == 1) != (i >= 4) ? 1 : 0);
 }
 
 struct Maps {
@@ -427,8 +437,8 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
     it.n0 = (local / MT) * NT;
     return it;
   };
-  // weight row of tile row r: a gate/up tile interleaves gate j (even r) with up j (odd r)
-  auto weight_row = [&](int mt, int r) { return GEMM == 0 ? (r & 1) * I + mt * (TILE_M / 2) + (r >> 1) : mt * TILE_M + r; };
+  // weight row of tile row r: a gate/up tile is 64 gate rows and their 64 up rows
+  auto weight_row = [&](int mt, int r) { return GEMM == 0 ? (r >> 6) * I + mt * (TILE_M / 2) + (r & 63) : mt * TILE_M + r; };
 
   unsigned spent = 0;  // see mbar_wait_ring
 
@@ -439,7 +449,9 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
     // 64 inputs of conversion do, so a thread takes 128 of every other step and not 64 of each (it measured 243 instructions
     // per 64 inputs before, 104 of them conversion).
     const int q4 = warp & 3, half = (warp >> 2) & 1, group = warp >> 3;
-    const int r = q4 * 32 + lane;  // tile row = tensor-memory lane
+    // This thread's tile row; it fills tensor-memory lane 32 q4 + lane. gate/up: lanes 0..7 and 16..23 take gate rows, the eight
+    // behind each the same units' up rows: see epi_unit.
+    const int r = GEMM == 0 ? ((lane >> 3) & 1) * 64 + q4 * 16 + epi_unit<FMT>(lane >> 4, lane & 7) : q4 * 32 + lane;
     const NibbleConst nc;
     const uint32_t acol = tmem + ((uint32_t)(q4 * 32) << 16) + A_COL0 + half * 64;
     const unsigned char* xrow = raw + swz_off(r, 0);  // piece p of the row stands at xrow + piece(p)
@@ -641,11 +653,11 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
           if (FMT == 0 && n == 0 && !it.shared) {
             unsigned char* sp = smbuf + rs.i * SMB;
             mbar_expect_tx(&ctl.smfull[rs.i], SMB);
-            if (GEMM == 0) tma_load_4d(sp, &maps.sm, 0, 0, unit0, e, &ctl.smfull[rs.i]);
+            if (GEMM == 0) tma_load_4d(sp, &maps.sm, 0, unit0, 0, e, &ctl.smfull[rs.i]);
             else bulk_g2s(sp, static_cast<const unsigned char*>(a.scales) + (size_t)row0 * (K / 64) * 4, SMB, &ctl.smfull[rs.i]);
           }
           mbar_expect_tx(bar, RAW_BYTES);
-          if (GEMM == 0) tma_load_4d(raw + (size_t)rr.i * RAW_BYTES, map, n * ROW_BYTES, 0, unit0, e, bar);
+          if (GEMM == 0) tma_load_4d(raw + (size_t)rr.i * RAW_BYTES, map, n * ROW_BYTES, unit0, 0, e, bar);
           else tma_load_2d(raw + (size_t)rr.i * RAW_BYTES, map, n * ROW_BYTES, row0, bar);
         }
         __syncwarp();
@@ -733,8 +745,8 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
     // ================= epilogue warps =================
     if (GEMM == 1) pdl_wait();  // y may still be read as the gate/up kernel's token rows
     const int q4 = warp & 3, set = SETS > 1 ? (warp - CONV_WARPS) / EPI_WARPS : 0;
-    const int r = q4 * 32 + lane;  // tile row
     const int acc0 = set * SET_ACC;
+    const uint32_t quadrant = tmem + ((uint32_t)(q4 * 32) << 16);
     Ring<NTAB> rt;
     Ring<SET_ACC> rc;
     if (SETS > 1) rt.next(set);  // a table slot serves one set only: NTAB is a multiple of SETS
@@ -742,101 +754,106 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
       wait_at<DRB_ERR_FULL_WAIT>(ctl.tabfull, rt, spent);
       const Tab& tab = tabs[rt.i];
       const int cols = FMT == 1 ? tab.cols : tab.used, mt = tab.mt;
-      const bool sh = tab.shared != 0;
-      float sum[FMT == 1 ? NT : 1];  // FP8: the columns' sums over the accumulators
+      const bool sh = tab.shared != 0, peers = GEMM == 1 && a.peer_y && !sh;
+      // gate/up: the place in act of this thread's two units (see epi_unit). down: the column of y of this thread's row.
+      const int i8 = lane >> 2;
+      __half* const act = static_cast<__half*>(sh ? a.sh_dst : a.dst) + mt * (TILE_M / 2) + q4 * 16 + (FMT == 0 ? 8 * (i8 >> 2) + 2 * (i8 & 3) : 2 * i8);
+      float* const y = static_cast<float*>(sh ? a.sh_dst : a.dst) + mt * TILE_M + q4 * 32 + lane;
+      const bool swap = lane & 16;  // half 1 holds the lower unit
+      // The results of eight columns. The stores carry their own predicate: behind a branch on it the arithmetic of one column
+      // waited for the store of the one before (gate/up, 64 columns: 7000 cycles per item).
+      auto units = [&](int c0, const uint32_t* h0, const uint32_t* h1) {  // gate/up: tokens 2 (lane % 4) and the next
+        const int2 d2 = *reinterpret_cast<const int2*>(&tab.dst[c0 + 2 * (lane & 3)]);
+        const float2 f2 = *reinterpret_cast<const float2*>(&tab.fac[c0 + 2 * (lane & 3)]);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const float f = t ? f2.y : f2.x;
+          auto unit = [&](const uint32_t* h) { return silu_fast(__uint_as_float(h[t]) * f) * (__uint_as_float(h[2 + t]) * f); };
+          const float r0 = unit(h0), r1 = unit(h1);
+          const int dt = t ? d2.y : d2.x;
+          store_valid(act + (ptrdiff_t)dt * I, f2h2_sat(swap ? r1 : r0, swap ? r0 : r1), dt);
+        }
+      };
+      auto columns = [&](int c0, const uint32_t(&v)[8]) {  // down
+#pragma unroll
+        for (int i4 = 0; i4 < 8; i4 += 4) {
+          const int4 d4 = *reinterpret_cast<const int4*>(&tab.dst[c0 + i4]);
+          const int dst[4] = {d4.x, d4.y, d4.z, d4.w};
+          if (peers) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              if (dst[i] < 0) continue;
+              const int s = dst[i] / a.peer_cap;
+              a.peer_y[s][((size_t)a.peer_rank * a.peer_cap + (dst[i] - s * a.peer_cap)) * H + mt * TILE_M + q4 * 32 + lane] = __uint_as_float(v[i4 + i]);
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) store_valid(y + (ptrdiff_t)dst[i] * H, __uint_as_float(v[i4 + i]), dst[i]);
+          }
+        }
+      };
       if (FMT == 1) {
+        // FP8: the columns' sums over the accumulators; gate/up: [column block of 16][as tmem_ld_halves16]
+        float sum[FMT == 1 ? NT : 1];
         // Lane l holds a scale: gate/up: input block l % 16 of the gate rows' (l < 16) or the up rows' block row; down: l % 4.
         const Item it = decode(item);
         const float* se = static_cast<const float*>(a.scales) + (size_t)it.e * (R / 128) * (K / 128);
-        const float sv = __ldg(se + (weight_row(mt, lane >> 4) >> 7) * (K / 128) + lane % (K / 128));
+        const float sv = __ldg(se + (weight_row(mt, GEMM == 0 ? 64 * (lane >> 4) : 0) >> 7) * (K / 128) + lane % (K / 128));
 #pragma unroll
         for (int c = 0; c < NT; ++c) sum[c] = 0.f;
 #pragma unroll 1
         for (int kb = 0; kb < K / 128; ++kb) {
-          const float s = __shfl_sync(0xffffffffu, sv, kb + (GEMM == 0 && (r & 1) ? 16 : 0));
+          const float s = __shfl_sync(0xffffffffu, sv, kb), su = GEMM == 0 ? __shfl_sync(0xffffffffu, sv, kb + 16) : s;
           wait_at<DRB_ERR_TMEM>(ctl.accfull + acc0, rc, spent);
           tc_fence_after();
 #pragma unroll
           for (int c0 = 0; c0 < NT; c0 += 16)
             if (c0 < cols) {
+              const uint32_t acc = quadrant + (uint32_t)((acc0 + rc.i) * NT + c0);
               uint32_t v[16];
-              tmem_ld16(tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)((acc0 + rc.i) * NT + c0), v);
+              if (GEMM == 0) tmem_ld_halves16(acc, reinterpret_cast<uint32_t(&)[2][8]>(v));
+              else tmem_ld16(acc, v);
 #pragma unroll
-              for (int i = 0; i < 16; ++i) sum[c0 + i] = fmaf(s, __uint_as_float(v[i]), sum[c0 + i]);
+              for (int i = 0; i < 16; ++i) sum[c0 + i] = fmaf(i & 2 ? su : s, __uint_as_float(v[i]), sum[c0 + i]);
             }
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&ctl.accfree[acc0 + rc.i]);
           rc.next();
         }
-      } else {
-        wait_at<DRB_ERR_TMEM>(ctl.accfull, rc, spent);
-        tc_fence_after();
-      }
-      const uint32_t acc = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(rc.i * NT);
-      // gate/up: unit j of act, in the order in which the down kernel's token rows want it. down: the row's column of y.
-      const int j = mt * (TILE_M / 2) + (r >> 1);
-      __half* const act = static_cast<__half*>(sh ? a.sh_dst : a.dst) + (FMT == 0 ? perm_pos(j) : j);
-      float* const y = static_cast<float*>(sh ? a.sh_dst : a.dst) + mt * TILE_M + r;
-      const bool odd = lane & 1, peers = GEMM == 1 && a.peer_y && !sh;
-      // The results of eight columns. The stores carry their own predicate: behind a branch on it the arithmetic of one column
-      // waited for the store of the one before (gate/up, 64 columns: 7000 cycles per item).
-      auto columns = [&](int c0, const uint32_t(&v)[8]) {
-        if (GEMM == 0) {
-          // even lanes hold gate rows, odd lanes their up rows. Per pair of tokens the lanes swap what the other needs: the
-          // even lane finishes the first token, the odd lane the second.
-          float got[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) got[i] = __shfl_xor_sync(0xffffffffu, __uint_as_float(odd ? v[2 * i] : v[2 * i + 1]), 1);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int2 d2 = *reinterpret_cast<const int2*>(&tab.dst[c0 + 2 * i]);
-            const float2 f2 = *reinterpret_cast<const float2*>(&tab.fac[c0 + 2 * i]);
-            const int dt = odd ? d2.y : d2.x;
-            const float f = odd ? f2.y : f2.x;
-            const float own = __uint_as_float(odd ? v[2 * i + 1] : v[2 * i]);
-            store_valid(act + (ptrdiff_t)dt * I, f2h_sat(silu_fast((odd ? got[i] : own) * f) * ((odd ? own : got[i]) * f)), dt);
-          }
-        } else {
-#pragma unroll
-          for (int i4 = 0; i4 < 8; i4 += 4) {
-            const int4 d4 = *reinterpret_cast<const int4*>(&tab.dst[c0 + i4]);
-            const int dst[4] = {d4.x, d4.y, d4.z, d4.w};
-            if (peers) {
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                if (dst[i] < 0) continue;
-                const int s = dst[i] / a.peer_cap;
-                a.peer_y[s][((size_t)a.peer_rank * a.peer_cap + (dst[i] - s * a.peer_cap)) * H + mt * TILE_M + r] = __uint_as_float(v[i4 + i]);
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 4; ++i) store_valid(y + (ptrdiff_t)dst[i] * H, __uint_as_float(v[i4 + i]), dst[i]);
-            }
-          }
-        }
-      };
-      if (FMT == 1) {
 #pragma unroll
         for (int c0 = 0; c0 < NT; c0 += 8)
           if (c0 < cols) {
             uint32_t v[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = __float_as_uint(sum[FMT == 1 ? c0 + i : 0]);
-            columns(c0, v);
+            for (int i = 0; i < 8; ++i) {
+              // down: columns in order; gate/up: the four of half 0, then the four of half 1
+              const int at = GEMM == 1 ? c0 + i : (c0 & ~15) + 8 * (i >> 2) + ((c0 >> 1) & 4) + (i & 3);
+              v[i] = __float_as_uint(sum[FMT == 1 ? at : 0]);
+            }
+            if (GEMM == 0) units(c0, v, v + 4);
+            else columns(c0, v);
           }
       } else {
+        wait_at<DRB_ERR_TMEM>(ctl.accfull, rc, spent);
+        tc_fence_after();
+        const uint32_t acc = quadrant + (uint32_t)(rc.i * NT);
 #pragma unroll 1
         for (int c0 = 0; c0 < cols; c0 += 16) {
           uint32_t v[2][8];
-          tmem_ld16(acc + (uint32_t)c0, v);
+          if (GEMM == 0) tmem_ld_halves16(acc + (uint32_t)c0, v);
+          else tmem_ld16(acc + (uint32_t)c0, v);
           if (c0 + 16 >= cols) {  // everything is in registers: the accumulator is free
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&ctl.accfree[rc.i]);
           }
-          columns(c0, v[0]);
-          if (c0 + 8 < cols) columns(c0 + 8, v[1]);
+          if (GEMM == 0) units(c0, v[0], v[1]);
+          else columns(c0, v[0]);
+          if (c0 + 8 < cols) {
+            if (GEMM == 0) units(c0 + 8, v[0] + 4, v[1] + 4);
+            else columns(c0 + 8, v[1]);
+          }
         }
         rc.next();
       }
@@ -887,11 +904,11 @@ static int map_rows(CUtensorMap* map, const void* p, uint64_t rows, uint64_t row
   return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, p, dims, strides, box);
 }
 
-// Gate/up: [experts][2 (gate | up)][units][row_bytes] seen as (row byte, gate|up, unit, expert); a box is 128 bytes of
-// 64 units' gate row and up row, interleaved.
+// Gate/up: [experts][2 (gate | up)][units][row_bytes] seen as (row byte, unit, gate|up, expert); a box is 128 bytes of
+// 64 units' gate rows and then of their up rows.
 static int map_gate_up(CUtensorMap* map, const void* p, uint64_t experts, uint64_t units, uint64_t row_bytes) {
-  const cuuint64_t dims[4] = {row_bytes, 2, units, experts}, strides[3] = {units * row_bytes, row_bytes, 2 * units * row_bytes};
-  const cuuint32_t box[4] = {ROW_BYTES, 2, TILE_M / 2, 1};
+  const cuuint64_t dims[4] = {row_bytes, units, 2, experts}, strides[3] = {row_bytes, units * row_bytes, 2 * units * row_bytes};
+  const cuuint32_t box[4] = {ROW_BYTES, TILE_M / 2, 2, 1};
   return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, p, dims, strides, box);
 }
 

@@ -67,6 +67,19 @@ DRB_DEV void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Lanes 0..15 (v[0]) and 16..31 (v[1]) of this warp's 32 x 16 columns, either half in the layout of mma.sync accumulators: thread 4 i + c
+// gets lane i, columns 2 c and 2 c + 1 in v[.][0], v[.][1], lane i + 8 in v[.][2], v[.][3]; the next eight columns in v[.][4..7].
+DRB_DEV void tmem_ld_halves16(uint32_t taddr, uint32_t (&v)[2][8]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%16];\n\t"
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%17];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&r"(v[0][0]), "=&r"(v[0][1]), "=&r"(v[0][2]), "=&r"(v[0][3]), "=&r"(v[0][4]), "=&r"(v[0][5]), "=&r"(v[0][6]), "=&r"(v[0][7]), "=&r"(v[1][0]),
+        "=&r"(v[1][1]), "=&r"(v[1][2]), "=&r"(v[1][3]), "=&r"(v[1][4]), "=&r"(v[1][5]), "=&r"(v[1][6]), "=&r"(v[1][7])
+      : "r"(taddr), "r"(taddr + (16u << 16))
+      : "memory");
+}
+
 DRB_DEV void tmem_ld16(uint32_t taddr, uint32_t (&v)[2][8]) { tmem_ld16(taddr, reinterpret_cast<uint32_t(&)[16]>(v)); }
 
 // Byte offset of 16-byte chunk c (0..7) of row r inside a K-major 128-byte-swizzled tile.
