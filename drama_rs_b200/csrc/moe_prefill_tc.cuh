@@ -627,9 +627,12 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
     }
   } else if (warp == LOAD_WARP) {
     // ================= loader =================
-    // The (scale, min) pairs of an int4 item go to one of NSM slots ahead of its first raw stage. By then the raw stage NRAW
-    // requests back has been read, so every item more than NSM - 1 items back is finished with its slot.
-    static_assert(NSM == 0 || (NSM - 1) * NSTEP >= NRAW, "scale slots");
+    // The (scale, min) pairs of an int4 item go to one of NSM slots. They are requested while the item before still asks for its stages: with
+    // the item's own first stage they came half a thousand cycles after the convert warps (300 rows 134.4 -> 132.8 us, 2048 rows 312.2 ->
+    // 306.6). Behind request SM_AT of that item the raw stage NRAW requests back has been read, so every item more than NSM - 1
+    // items back is finished with its slot.
+    constexpr int SM_AT = NSTEP == 8 ? NRAW - 1 : 1;
+    static_assert(NSM == 0 || (NSM - 2) * NSTEP + SM_AT + 1 >= NRAW, "scale slots");
     // A wait for a raw stage tests one bit of its phase, so it tells "landed" from "in flight" only once the stage's use before
     // this one is known to have landed; boxes land in any order. A group's own uses it has waited for itself. With two groups a
     // stage also passes from one to the other, and there the stage's MMAs vouch: after a_wait() of step s everything up to step s - NST
@@ -639,9 +642,22 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
     Ring<NRAW> rr;
     Ring<(NSM ? NSM : 1)> rs;
     rr.par = 1;  // every raw stage starts free
+    auto scales = [&](const Item& it) {  // one thread
+      unsigned char* sp = smbuf + rs.i * SMB;
+      mbar_expect_tx(&ctl.smfull[rs.i], SMB);
+      if (GEMM == 0) tma_load_4d(sp, &maps.sm, 0, it.mt * (TILE_M / 2), 0, it.e, &ctl.smfull[rs.i]);
+      else bulk_g2s(sp, static_cast<const unsigned char*>(a.scales) + (size_t)(it.e * R + it.mt * TILE_M) * (K / 64) * 4, SMB, &ctl.smfull[rs.i]);
+    };
+    Item next = {};
+    if ((int)blockIdx.x < total_items) next = decode(blockIdx.x);
+    if (FMT == 0 && (int)blockIdx.x < total_items && !next.shared) {
+      if (elect_one()) scales(next);
+      __syncwarp();
+      rs.next();
+    }
     for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
-      const Item it = decode(item);
-      const bool eight = FMT == 1 || it.shared;
+      const Item it = next;
+      const bool eight = FMT == 1 || it.shared, more = item + (int)gridDim.x < total_items;
       const int nraw = NSTEP * (eight ? 2 : 1), unit0 = it.mt * (TILE_M / 2), e = it.shared ? 0 : it.e, row0 = e * R + it.mt * TILE_M;
       const CUtensorMap* map = it.shared ? &maps.sh : &maps.q;
 #pragma unroll 1
@@ -650,20 +666,21 @@ __global__ void __launch_bounds__(Smem<GEMM, FMT>::THREADS, 1) k_grouped(const _
         __syncwarp();
         if (elect_one()) {
           uint64_t* bar = &ctl.rawfull[rr.i];
-          if (FMT == 0 && n == 0 && !it.shared) {
-            unsigned char* sp = smbuf + rs.i * SMB;
-            mbar_expect_tx(&ctl.smfull[rs.i], SMB);
-            if (GEMM == 0) tma_load_4d(sp, &maps.sm, 0, unit0, 0, e, &ctl.smfull[rs.i]);
-            else bulk_g2s(sp, static_cast<const unsigned char*>(a.scales) + (size_t)row0 * (K / 64) * 4, SMB, &ctl.smfull[rs.i]);
-          }
           mbar_expect_tx(bar, RAW_BYTES);
           if (GEMM == 0) tma_load_4d(raw + (size_t)rr.i * RAW_BYTES, map, n * ROW_BYTES, unit0, 0, e, bar);
           else tma_load_2d(raw + (size_t)rr.i * RAW_BYTES, map, n * ROW_BYTES, row0, bar);
         }
         __syncwarp();
         rr.next();
+        if (n == SM_AT) {
+          if (more) next = decode(item + gridDim.x);
+          if (FMT == 0 && more && !next.shared) {
+            if (elect_one()) scales(next);
+            __syncwarp();
+            rs.next();
+          }
+        }
       }
-      if (FMT == 0 && !it.shared) rs.next();
     }
   } else if (warp == TOKEN_WARP) {
     // ================= token warp =================
