@@ -8,6 +8,7 @@
 
 #include "common.cuh"
 #include "moe_prefill_tc.cuh"
+#include "router.cuh"
 
 namespace pf {
 
@@ -662,8 +663,7 @@ __global__ void __launch_bounds__(SC_THREADS)
 
 // router::k_moe_topk and k_scatter_rows in one launch for up to 32 rows, where a launch's way costs more than its work. Block r
 // copies row r; every block forms the routing of all the rows for itself, a warp per row, so nothing crosses blocks: the experts'
-// rows are bit masks, a pair's rank is the number of rows before it in its expert's mask. Weights and order have the same bits as
-// k_moe_topk's (the same sums in the same order; larger probability, then lower index).
+// rows are bit masks, a pair's rank is the number of rows before it in its expert's mask.
 // A whole call: 49.3 -> 46.5 us at 5 rows, 73.6 -> 68.8 at 16, 77.8 -> 75.7 at 20, 91.8 -> 90.6 at 32; the redundant part grows with the
 // rows, and beyond 32 a block has no warp per row.
 constexpr int FEW_ROWS = 32, FEW_MIN_THREADS = 512;  // blocks of 32 threads per row, but at least so many for the copies
@@ -683,47 +683,11 @@ __global__ void __launch_bounds__(FEW_ROWS * 32)
   int mine = 0;  // lane k < topk of warp r: the k-th expert of row r
   if (warp < rows) {
     const float* l = logits + (size_t)warp * (E + 1);
-    float x[8], m = -INFINITY, ws[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      x[j] = lane + 32 * j < E ? __ldcg(l + lane + 32 * j) : -INFINITY;
-    }
-    // the maximum on order-preserving integer keys, as router::softmax_topk takes it
-    unsigned ord = 0u;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const unsigned b = __float_as_uint(x[j]);
-      ord = max(ord, (b & 0x80000000u) ? ~b : (b | 0x80000000u));
-    }
-    m = router::ord_to_float(__reduce_max_sync(0xffffffffu, ord));
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      x[j] = lane + 32 * j < E ? expf(x[j] - m) : 0.f;
-      ws[j] = warp_sum(x[j]);
-    }
-    const float z = ((ws[0] + ws[4]) + (ws[2] + ws[6])) + ((ws[1] + ws[5]) + (ws[3] + ws[7]));
-    unsigned key[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) key[j] = lane + 32 * j < E ? __float_as_uint(x[j] / z) + 1u : 0u;
-    float top = 0.f, total = 0.f;
-    for (int k = 0; k < topk; ++k) {
-      unsigned best = key[0];
-#pragma unroll
-      for (int j = 1; j < 8; ++j) best = max(best, key[j]);
-      best = __reduce_max_sync(0xffffffffu, best);
-      int e = 256;
-#pragma unroll
-      for (int j = 7; j >= 0; --j) e = key[j] == best ? lane + 32 * j : e;
-      e = __reduce_min_sync(0xffffffffu, e);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) key[j] = e == lane + 32 * j ? 0u : key[j];
-      const float p = __uint_as_float(best - 1u);
-      total += p;  // rank order, as the reference accumulates
-      if (lane == k) mine = e, top = p;
-    }
+    float w;
+    mine = router::route_row([&](int e) { return __ldcg(l + e); }, E, topk, lane, w);
     if (lane < topk) {
       atomicOr(&mask[mine], 1u << warp);
-      if (warp == row) idx[row * topk + lane] = mine, wts[row * topk + lane] = top / total;
+      if (warp == row) idx[row * topk + lane] = mine, wts[row * topk + lane] = w;
     }
     if (warp == row && lane == 0) sgate[row] = __ldcg(l + E);
   }
@@ -1075,7 +1039,8 @@ extern "C" int drb_moe_prefill_layer(const drb_moe_layer* w, const drb_prefill_b
   } else {
     // The pairs' ranks: two warps read each, so they do not share slot_of's place; act is free until the gate/up kernel writes it.
     int* rank = reinterpret_cast<int*>(b->act);
-    drb_launch(router::k_moe_topk<true>, dim3(rows), dim3(router::THREADS), 0, st, dev.pdl, (const float*)b->logits, e, topk, e + 1, b->idx, b->wts,
+    drb_launch(router::k_moe_topk<true>, dim3((rows + router::TOPK_ROWS - 1) / router::TOPK_ROWS), dim3(router::TOPK_ROWS * 32), 0, st, dev.pdl,
+               (const float*)b->logits, rows, e, topk, e + 1, b->idx, b->wts,
                b->sgate, b->counts, rank);
     const int blocks = (rows + pf::SC_ROWS - 1) / pf::SC_ROWS;
     drb_launch(pf::k_scatter_rows, dim3(blocks < 8 * dev.sms ? blocks : 8 * dev.sms), dim3(pf::SC_THREADS), 0, st, dev.pdl, (const __half*)b->rows16,
