@@ -168,37 +168,6 @@ class HostRow:
             pass
 
 
-class PinnedPair:
-    """Two arrays of the same size in one pinned allocation, for a small array that a step reads back from the device and another that
-    it sends there: `get` waits for its copy, `put` does not. A copy out of `out` is over by the time the next `get` returns."""
-
-    def __init__(self, count: int, dtype, st: Stream) -> None:
-        self._l, self._st = ffi.lib(), st
-        self.nbytes = count * np.dtype(dtype).itemsize
-        self._p = C.c_void_p()
-        check(self._l.dr_host_alloc(C.byref(self._p), 2 * self.nbytes), "host_alloc")
-        both = np.frombuffer((C.c_char * (2 * self.nbytes)).from_address(self._p.value), dtype=dtype)
-        both[:] = 0
-        self.into, self.out = both[:count], both[count:]
-
-    def get(self, dev) -> np.ndarray:
-        check(self._l.dr_d2h(self._p, dev.ptr, self.nbytes, self._st.raw), "d2h")
-        self._st.sync()
-        return self.into
-
-    def put(self, dev) -> None:
-        check(self._l.dr_h2d(dev.ptr, C.c_void_p(self._p.value + self.nbytes), self.nbytes, self._st.raw), "h2d")
-
-    def __del__(self) -> None:
-        try:
-            if self._p:
-                self._st.sync()  # a copy may be under way
-                self._l.dr_host_free(self._p)
-                self._p = C.c_void_p()
-        except Exception:
-            pass
-
-
 class ExtBuf:
     """Device memory owned by someone else (for example a torch tensor), seen through DevBuf's interface."""
 
