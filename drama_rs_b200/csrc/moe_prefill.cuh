@@ -298,15 +298,16 @@ __global__ void __launch_bounds__(256, CMB_BLOCKS)
   if (first - 4 * lane >= Hd) return;
   const bool in = first < Hd;
   const int c = in ? first : Hd - 4;  // whole warps stay for the shuffles
-  auto head = [&](int r) -> int {  // TK > 0: lane k < TK the slot of pair k, TK + k its weight, 2 TK the gate
+  auto head = [&](unsigned r) -> int {  // TK > 0: lane k < TK the slot of pair k, TK + k its weight, 2 TK the gate
     if (lane < TK) return __ldcg(slot_of + (size_t)r * TK + lane);
     if (lane < 2 * TK) return __float_as_int(__ldcg(wts + (size_t)r * TK + lane - TK));
     return __float_as_int(__ldcg(sgate + r));
   };
-  int r = blockIdx.x, next = TK > 0 ? head(r) : 0;
-  for (; r < rows; r += gridDim.x) {
+  const unsigned n = rows;  // unsigned: a stride past the last row may leave int's range
+  int next = TK > 0 ? head(blockIdx.x) : 0;
+  for (unsigned r = blockIdx.x; r < n; r += gridDim.x) {
     const int now = next;
-    if (TK > 0 && r + (int)gridDim.x < rows) next = head(r + gridDim.x);
+    if (TK > 0 && r + gridDim.x < n) next = head(r + gridDim.x);
     float4* xo = reinterpret_cast<float4*>(x + (size_t)r * Hd + c);
     const float4 sh = __ldcg(reinterpret_cast<const float4*>(shared + (size_t)r * Hd + c));
     float4 o = __ldcg(xo), acc;

@@ -427,7 +427,7 @@ extern "C" int dr_moe_topk(const float* logits, int rows, int E, int topk, int s
   if (rows <= 0) return 0;
   const DrbDevice& dev = drb_device(st);
   if (!dev.ready) return -2;
-  drb_launch(router::k_moe_topk<false>, dim3((rows + router::TOPK_ROWS - 1) / router::TOPK_ROWS), dim3(router::TOPK_ROWS * 32), 0, st, dev.pdl, logits, rows, E,
+  drb_launch(router::k_moe_topk<false>, dim3((rows - 1) / router::TOPK_ROWS + 1), dim3(router::TOPK_ROWS * 32), 0, st, dev.pdl, logits, rows, E,
              topk, stride, idx, wts, sgate, (int*)nullptr, (int*)nullptr);
   return 0;
 }
