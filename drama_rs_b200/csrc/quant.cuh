@@ -23,6 +23,8 @@ __constant__ float c_shrink[STEPS] = {1.0f,        0.97916669f, 0.95833331f, 0.9
                                       0.83333331f, 0.8125f,     0.79166669f, 0.77083331f, 0.75f,       0.72916669f, 0.70833331f, 0.6875f,
                                       0.66666669f, 0.64583331f, 0.625f,      0.60416669f, 0.58333331f, 0.5625f,     0.54166669f, 0.52083331f};
 
+constexpr float FP16_LEAST = 5.9e-8f;  // just below 2^-24: a scale under it sits at the converter's floor
+
 DRB_DEV float half_round(float v) { return __half2float(__float2half_rn(v)); }
 
 // A team of eight lanes owns a group: lane j holds inputs j, 8 + j, ..., 56 + j, which are the terms of the converter's
@@ -33,6 +35,11 @@ struct Group {
   unsigned long long v2[4];  // inputs 8 i + j as packed pairs (i = 0, 1), (2, 3), (4, 5), (6, 7)
 };
 
+DRB_DEV float reciprocal(float v) {  // within one unit in the last place
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
 DRB_DEV unsigned long long mul2(unsigned long long a, unsigned long long b) {
   unsigned long long r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
@@ -64,8 +71,9 @@ DRB_DEV float sum64(const unsigned long long (&t)[4]) {
 // the reciprocal, within 2^-22 of it, clamped before it is rounded. Where it lands within 1e-5 of an inner rounding boundary
 // the candidate n is settled exactly: with d = v - lo (a float, at least scale / 2 here) the remainder d - n scale is exact in
 // one fused operation, and it is compared with scale / 2; d's spacing is too coarse for the rounded quotient to reach a
-// boundary that the exact one misses. Weights on a bf16 grid make such boundaries common (one value in two thousand), nearly
-// all of them exact ties, which go to the even code.
+// boundary that the exact one misses, at a scale that fp16 holds (eleven bits). At the floor of 1e-10, which has 24, it is not, and
+// the division itself decides. Weights on a bf16 grid make such boundaries common (one value in two thousand), nearly all of them
+// exact ties, which go to the even code.
 DRB_DEV void codes8(const Group& g, float lo, float scale, float rcp, unsigned long long (&q)[4]) {
   const unsigned long long nlo = dup2(-lo), r2 = dup2(rcp), magic = dup2(12582912.f), nmagic = dup2(-12582912.f), neg1 = dup2(-1.f);
   float worst = 0.f;
@@ -86,12 +94,14 @@ DRB_DEV void codes8(const Group& g, float lo, float scale, float rcp, unsigned l
       const bool move = fabsf(e) > half || (fabsf(e) == half && odd);
       return fminf(fmaxf(move ? (e > 0.f ? n + 1.f : n - 1.f) : n, 0.f), 15.f);
     };
+    auto divide = [&](float v) { return fminf(fmaxf(rintf(__fdiv_rn(__fadd_rn(v, -lo), scale)), 0.f), 15.f); };
+    const bool floor = scale < FP16_LEAST;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       float v0, v1, n0, n1;
       unpack2(g.v2[i], v0, v1);
       unpack2(q[i], n0, n1);
-      q[i] = pack2(settle(v0, n0), settle(v1, n1));
+      q[i] = floor ? pack2(divide(v0), divide(v1)) : pack2(settle(v0, n0), settle(v1, n1));
     }
   }
 }
@@ -186,7 +196,7 @@ __global__ void __launch_bounds__(Q4_THREADS, 5) k_quant_q4(const float* __restr
     const float hi_c = __fadd_rn(center, __fmul_rn(__fsub_rn(gmax, center), shrink));
     c.scale = fmaxf(half_round(fmaxf(__fdiv_rn(__fsub_rn(hi_c, lo_c), 15.0f), 1e-10f)), 1e-10f);
     c.lo = half_round(lo_c);
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(c.rcp) : "f"(c.scale));
+    c.rcp = reciprocal(c.scale);
     return c;
   };
   const Candidate ca = candidate(c_shrink[j]), cb = candidate(c_shrink[8 + (j & 3)]);
@@ -246,7 +256,8 @@ __global__ void __launch_bounds__(Q4_THREADS, 5) k_quant_q4(const float* __restr
     const int i = open ? __ffs(open) - 1 : 0;
     auto of = [&](float a, float b) { return __shfl_sync(0xffffffffu, i < 8 ? a : b, i & 7, 8); };
     Candidate c;
-    c.scale = of(ca.scale, cb.scale), c.lo = of(ca.lo, cb.lo), c.rcp = of(ca.rcp, cb.rcp);
+    c.scale = of(ca.scale, cb.scale), c.lo = of(ca.lo, cb.lo);
+    c.rcp = reciprocal(c.scale);  // handed round as well, it cost a spilled register and 2 %
     evaluate(c, first, open != 0u);
     open &= open - 1u;
     if (best_err == 0.f) open = 0u;  // nothing is less
@@ -325,15 +336,15 @@ __global__ void __launch_bounds__(Q8_WARPS * 32) k_quant_q8(const float* __restr
     float amax = fmaxf(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))), 0.f);
     amax = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax))), 1e-12f);
     const float scale = fmaxf(half_round(__fdiv_rn(amax, 127.0f)), 1e-12f);
-    float rcp, n[4], worst = 0.f;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rcp) : "f"(scale));
+    const float rcp = reciprocal(scale);
+    float n[4], worst = 0.f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float p = fminf(fmaxf(v[j] * rcp, -127.f), 127.f);
       n[j] = __fadd_rn(__fadd_rn(p, 12582912.f), -12582912.f);  // the nearest integer
       worst = fmaxf(worst, fabsf(p - n[j]));
     }
-    if (scale < 5.9e-8f) {  // below fp16's least, at the floor: a scale of 24 bits, whose products are not exact
+    if (scale < FP16_LEAST) {  // at the floor: a scale of 24 bits, whose products are not exact
 #pragma unroll
       for (int j = 0; j < 4; ++j) n[j] = fminf(fmaxf(rintf(__fdiv_rn(v[j], scale)), -127.f), 127.f);
     } else if (worst >= 0.4999f) {
