@@ -282,53 +282,93 @@ __global__ void __launch_bounds__(64)
 }
 
 // x[r] += sigmoid(sgate[r]) * shared[r] + sum_k w[r,k] * Y[slot_of[r,k]], k ascending (fixed order, so
-// the result does not depend on how slots were handed out). Block (r, c): 1024 columns of rows r, r + gridDim.x, ..., one float4 per thread.
-// Bound by Y's bytes from L2 or HBM; all of a thread's rows are requested before the first is used (TK = 8: in a loop over a
-// runtime topk every row waited for the one before, 13 us at 300 rows instead of 5). A row's slots, weights and gate lie spread over
-// the lanes of each warp and are fetched a row ahead: behind them its data would wait for two trips instead of one.
-constexpr int CMB_BLOCKS = 4;  // resident blocks per multiprocessor
-template <int TK>
+// the result does not depend on how slots were handed out). Two forms, one float4 of 1024 columns per thread.
+//
+// Top-8: block (r, c) takes rows r, r + gridDim.x, ... Bound by Y's bytes from L2 or HBM; all of a thread's rows are requested before the
+// first is used (in a loop over a runtime topk every row waited for the one before, 13 us at 300 rows instead of 5). A row's
+// slots, weights and gate lie spread over the lanes of each warp and are fetched a row ahead: behind them its data would wait for two
+// trips instead of one. 2048 rows 44.5 -> 35.8 us, 300 rows 4.3 -> 3.5, against a block per row.
+constexpr int CMB_TOPK = 8, CMB_BLOCKS = 4;  // resident blocks per multiprocessor
 __global__ void __launch_bounds__(256, CMB_BLOCKS)
-    k_combine(float* __restrict__ x, const float* __restrict__ Y, const int* __restrict__ slot_of,
-              const float* __restrict__ wts, const float* __restrict__ sgate, const float* __restrict__ shared, int rows, int topk,
-              int Hd) {
+    k_combine8(float* __restrict__ x, const float* __restrict__ Y, const int* __restrict__ slot_of,
+               const float* __restrict__ wts, const float* __restrict__ sgate, const float* __restrict__ shared, int rows, int Hd) {
+  constexpr int TK = CMB_TOPK;
   pdl_wait();
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31, first = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
   if (first - 4 * lane >= Hd) return;
   const bool in = first < Hd;
   const int c = in ? first : Hd - 4;  // whole warps stay for the shuffles
-  auto head = [&](unsigned r) -> int {  // TK > 0: lane k < TK the slot of pair k, TK + k its weight, 2 TK the gate
+  auto head = [&](unsigned r) -> int {  // lane k < TK the slot of pair k, TK + k its weight, 2 TK the gate
     if (lane < TK) return __ldcg(slot_of + (size_t)r * TK + lane);
     if (lane < 2 * TK) return __float_as_int(__ldcg(wts + (size_t)r * TK + lane - TK));
     return __float_as_int(__ldcg(sgate + r));
   };
   const unsigned n = rows;  // unsigned: a stride past the last row may leave int's range
-  int next = TK > 0 ? head(blockIdx.x) : 0;
+  int next = head(blockIdx.x);
   for (unsigned r = blockIdx.x; r < n; r += gridDim.x) {
     const int now = next;
-    if (TK > 0 && r + gridDim.x < n) next = head(r + gridDim.x);
+    if (r + gridDim.x < n) next = head(r + gridDim.x);
     float4* xo = reinterpret_cast<float4*>(x + (size_t)r * Hd + c);
     const float4 sh = __ldcg(reinterpret_cast<const float4*>(shared + (size_t)r * Hd + c));
-    float4 o = __ldcg(xo), acc;
-    auto add = [&](float w, const float4& v) { acc.x += w * v.x, acc.y += w * v.y, acc.z += w * v.z, acc.w += w * v.w; };
-    auto row = [&](int slot) { return __ldcg(reinterpret_cast<const float4*>(Y + (size_t)slot * Hd + c)); };
-    if (TK > 0) {
-      float4 v[TK > 0 ? TK : 1];
+    float4 o = __ldcg(xo), v[TK];
 #pragma unroll
-      for (int k = 0; k < TK; ++k) v[k] = row(__shfl_sync(0xffffffffu, now, k));
-      const float sg = sigmoid_f(__int_as_float(__shfl_sync(0xffffffffu, now, 2 * TK)));
-      acc = make_float4(sg * sh.x, sg * sh.y, sg * sh.z, sg * sh.w);
+    for (int k = 0; k < TK; ++k) v[k] = __ldcg(reinterpret_cast<const float4*>(Y + (size_t)__shfl_sync(0xffffffffu, now, k) * Hd + c));
+    const float sg = sigmoid_f(__int_as_float(__shfl_sync(0xffffffffu, now, 2 * TK)));
+    float4 acc = make_float4(sg * sh.x, sg * sh.y, sg * sh.z, sg * sh.w);
 #pragma unroll
-      for (int k = 0; k < TK; ++k) add(__int_as_float(__shfl_sync(0xffffffffu, now, TK + k)), v[k]);
-    } else {
-      const float sg = sigmoid_f(__ldcg(sgate + r));
-      acc = make_float4(sg * sh.x, sg * sh.y, sg * sh.z, sg * sh.w);
-      for (int k = 0; k < topk; ++k) add(__ldcg(wts + (size_t)r * topk + k), row(__ldcg(slot_of + (size_t)r * topk + k)));
+    for (int k = 0; k < TK; ++k) {
+      const float w = __int_as_float(__shfl_sync(0xffffffffu, now, TK + k));
+      acc.x += w * v[k].x, acc.y += w * v[k].y, acc.z += w * v[k].z, acc.w += w * v[k].w;
     }
     o.x += acc.x, o.y += acc.y, o.z += acc.z, o.w += acc.w;
     if (in) *xo = o;
   }
+}
+
+// Any topk: block (r, c) takes row r. With many rows eight resident blocks per multiprocessor cover one another's trips; walking over rows in
+// four of them, as above, lost (H = 2048, 2048 rows of 2, 16, 32 pairs: 8.3, 61, 110 us, and 12.0, 83, 153). FEW: at most three blocks per
+// multiprocessor, where the chain of trips is what there is: four pairs' slots, then four rows (one row of 16, 32 pairs 4.1, 6.6 -> 2.9, 4.2 us;
+// 64 rows of 16 4.3 -> 3.1). With four, 290 rows of 4 to 16
+// took 20 to 30 % longer so.
+template <bool FEW>
+__global__ void __launch_bounds__(256, FEW ? 6 : 8)
+    k_combine(float* __restrict__ x, const float* __restrict__ Y, const int* __restrict__ slot_of, const float* __restrict__ wts,
+              const float* __restrict__ sgate, const float* __restrict__ shared, int topk, int Hd) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int r = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+  if (c >= Hd) return;
+  float4* xo = reinterpret_cast<float4*>(x + (size_t)r * Hd + c);
+  const float gate = __ldcg(sgate + r);
+  const float4 sh = __ldcg(reinterpret_cast<const float4*>(shared + (size_t)r * Hd + c));
+  float4 o = __ldcg(xo);
+  const float sg = sigmoid_f(gate);
+  float4 acc = make_float4(sg * sh.x, sg * sh.y, sg * sh.z, sg * sh.w);
+  const int* slots = slot_of + (size_t)r * topk;
+  const float* weights = wts + (size_t)r * topk;
+  auto row = [&](int slot) { return __ldcg(reinterpret_cast<const float4*>(Y + (size_t)slot * Hd + c)); };
+  auto add = [&](float w, const float4& v) { acc.x += w * v.x, acc.y += w * v.y, acc.z += w * v.z, acc.w += w * v.w; };
+  if (FEW) {
+    int k = 0;
+    for (; k + 4 <= topk; k += 4) {
+      int s[4];
+      float w[4];
+      float4 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[i] = __ldcg(slots + k + i), w[i] = __ldcg(weights + k + i);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = row(s[i]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) add(w[i], v[i]);
+    }
+#pragma unroll 1
+    for (; k < topk; ++k) add(__ldcg(weights + k), row(__ldcg(slots + k)));
+  } else {
+    for (int k = 0; k < topk; ++k) add(__ldcg(wts + (size_t)r * topk + k), row(__ldcg(slot_of + (size_t)r * topk + k)));
+  }
+  o.x += acc.x, o.y += acc.y, o.z += acc.z, o.w += acc.w;
+  *xo = o;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -758,8 +798,9 @@ static cudaError_t configure_all() {
   if ((e = drb_carveout(k_route_few)) != cudaSuccess) return e;
   if ((e = drb_carveout(k_count)) != cudaSuccess) return e;
   if ((e = drb_carveout(k_permute)) != cudaSuccess) return e;
-  if ((e = drb_carveout(k_combine<8>)) != cudaSuccess) return e;
-  if ((e = drb_carveout(k_combine<0>)) != cudaSuccess) return e;
+  if ((e = drb_carveout(k_combine8)) != cudaSuccess) return e;
+  if ((e = drb_carveout(k_combine<true>)) != cudaSuccess) return e;
+  if ((e = drb_carveout(k_combine<false>)) != cudaSuccess) return e;
   if ((e = drb_carveout(k_group)) != cudaSuccess) return e;
   if ((e = drb_carveout(k_ep_plan)) != cudaSuccess) return e;
   if ((e = drb_carveout(k_ep_scatter)) != cudaSuccess) return e;
@@ -830,9 +871,14 @@ extern "C" int dr_moe_combine(float* x, const float* Y, const int* slot_of, cons
   if (rows <= 0 || H <= 0) return 0;
   const DrbDevice& dev = drb_device(st);
   const int gy = (H + 1023) / 1024;
-  const int gx = max(1, pf::CMB_BLOCKS * (dev.ready ? dev.sms : 1) / gy);  // what is resident at once
-  drb_launch(topk == 8 ? pf::k_combine<8> : pf::k_combine<0>, dim3(rows < gx ? rows : gx, gy), dim3(256), 0, st, dev.ready && dev.pdl, x, Y, slot_of,
-             wts, sgate, shared, rows, topk, H);
+  if (topk == pf::CMB_TOPK) {
+    const int gx = max(1, pf::CMB_BLOCKS * (dev.ready ? dev.sms : 1) / gy);  // what is resident at once
+    drb_launch(pf::k_combine8, dim3(rows < gx ? rows : gx, gy), dim3(256), 0, st, dev.ready && dev.pdl, x, Y, slot_of, wts, sgate, shared, rows, H);
+  } else {
+    const bool few = topk >= 4 && (long long)rows * gy <= 3 * dev.sms;
+    drb_launch(few ? pf::k_combine<true> : pf::k_combine<false>, dim3(rows, gy), dim3(256), 0, st, dev.ready && dev.pdl, x, Y, slot_of, wts, sgate,
+               shared, topk, H);
+  }
   return 0;
 }
 
