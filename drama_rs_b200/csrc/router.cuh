@@ -233,6 +233,30 @@ __global__ void __launch_bounds__(TOPK_ROWS * 32)
   if (RANK) rank[p] = atomicAdd(counts + e, 1);
 }
 
+// The same, a block per row, by the decode router's top-k: see topk_by_blocks.
+__global__ void __launch_bounds__(THREADS)
+    k_moe_topk_block(const float* __restrict__ logits, int E, int topk, int stride, int* __restrict__ idx, float* __restrict__ wts,
+                     float* __restrict__ sgate) {
+  __shared__ TopkSmem sm;
+  pdl_launch_dependents();
+  pdl_wait();
+  const size_t r = blockIdx.x;
+  const float* l = logits + r * stride;
+  const float v = (int)threadIdx.x < E ? __ldcg(l + threadIdx.x) : -INFINITY;
+  softmax_topk(v, E, topk, idx + r * topk, wts + r * topk, sm);
+  if (threadIdx.x == 0) sgate[r] = __ldcg(l + E);
+}
+
+// Which form dr_moe_topk takes. A warp's time grows with k, whatever the rows (2.1 us and 0.06 to 0.07 a round up to 600 rows). A block ranks its survivors
+// in one pass, 2.2 us, but where more than 32 survive it counts each against all of them (3.2 to 4 us for 33 to 64 of them, 21 for 256), and its
+// time grows with the rows. So a block wins where all entries fit one pass (E = 32, k = 8, 32: 2.1 against 2.7, 4.2 us; 600 rows 2.8 against 3.0, 5.4), for many
+// rounds over two entries a lane (E = 64, k = 32: 3.6 against 4.2), and where the bound by the warps' maxima, of full warps, leaves few
+// survivors in every row (E = 256, k = 8: one row 2.0 against 3.1, four rows 2.2 to 2.6, 33 rows 4.2).
+inline bool topk_by_blocks(int rows, int E, int topk, int sms) {
+  if (E <= 64) return topk >= (E <= 32 ? 6 : 24) && rows <= 4 * sms;
+  return topk >= 4 && topk <= E / 32 && E % 32 == 0 && rows <= (E <= 128 ? 64 : 4);
+}
+
 constexpr int K = 2048;
 
 // ------------------------------------------------------------------------------------------
@@ -387,6 +411,7 @@ static cudaError_t configure_all() {
   if (e != cudaSuccess) return e;
   if ((e = cudaFuncSetAttribute(cl::k_router_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cl::SMEM_BYTES)) != cudaSuccess) return e;
   if ((e = drb_carveout(k_moe_topk<true>)) != cudaSuccess) return e;
+  if ((e = drb_carveout(k_moe_topk_block)) != cudaSuccess) return e;
   return drb_carveout(k_moe_topk<false>);
 }
 
@@ -427,6 +452,10 @@ extern "C" int dr_moe_topk(const float* logits, int rows, int E, int topk, int s
   if (rows <= 0) return 0;
   const DrbDevice& dev = drb_device(st);
   if (!dev.ready) return -2;
+  if (router::topk_by_blocks(rows, E, topk, dev.sms)) {
+    drb_launch(router::k_moe_topk_block, dim3(rows), dim3(router::THREADS), 0, st, dev.pdl, logits, E, topk, stride, idx, wts, sgate);
+    return 0;
+  }
   drb_launch(router::k_moe_topk<false>, dim3((rows - 1) / router::TOPK_ROWS + 1), dim3(router::TOPK_ROWS * 32), 0, st, dev.pdl, logits, rows, E,
              topk, stride, idx, wts, sgate, (int*)nullptr, (int*)nullptr);
   return 0;
