@@ -180,11 +180,12 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
 
   // ---------------- consumers
-  // The norm weight is a constant: fetch it before the dependency wait. Thread t owns float4 t.
-  const float4 wv = nw ? reinterpret_cast<const float4*>(nw)[threadIdx.x] : make_float4(1.f, 1.f, 1.f, 1.f);
+  // Thread t owns float4 t. The norm weights come as far as L2 before the dependency wait: they may be the work of the launch before.
+  if (nw && (lane & 7) == 0) prefetch_line_l2(nw + 4 * threadIdx.x);
   pdl_wait();               // x is the previous kernel's output
   pdl_launch_dependents();
   const float4 xv = __ldcg(reinterpret_cast<const float4*>(x) + threadIdx.x);
+  const float4 wv = nw ? __ldcg(reinterpret_cast<const float4*>(nw) + threadIdx.x) : make_float4(1.f, 1.f, 1.f, 1.f);
   float inv = 1.f;
   if (nw) {
     const float ss = warp_sum(xv.x * xv.x + xv.y * xv.y + xv.z * xv.z + xv.w * xv.w);

@@ -27,3 +27,16 @@ def test_norm_and_router_weights_are_read_behind_the_wait(file, namespace, kerne
     if kernel == "k_router_logits":
         calls = body[body.index("auto fetch") :]
         assert "fetch(" not in calls[calls.index("};") :]
+
+
+@pytest.mark.parametrize("file,kernel", [("moe_decode.cuh", "k_moe_gate_up"), ("moe_decode_fp8.cuh", "k_moe_gate_up_fp8"), ("router.cuh", "k_router_cluster")])
+def test_decode_reads_norm_weights_behind_the_wait(file, kernel):
+    with open(os.path.join(CSRC, file)) as f:
+        s = f.read()
+    s = s[s.index(f"    {kernel}(") :]
+    s = s[s.index(") {\n") :]
+    at = s.find("- consumers\n")  # their own wait: the producer warp has another
+    s = s[max(at, 0) :]
+    body = s[: s.index("  pdl_wait();")]
+    assert not [line for line in body.splitlines() if "(nw)[" in line or "(nw +" in line and "prefetch" not in line]
+    assert "(nw)" in s  # the read is where this looks for it
