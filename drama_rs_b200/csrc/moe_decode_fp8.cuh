@@ -125,7 +125,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     // The down kernel's rows on their way to L2 while this one still computes: its blocks become resident, and ask for them, only when
     // these are over (the two do not fit a multiprocessor together). This block takes 128 rows of its expert, or of the shared one,
     // and the scales that are read ahead of the down kernel's dependency wait, once its own rows have landed: asked for before,
-    // they would delay what the layer waits for. Eight layers 157.2 -> 154.8 us; on the int4 experts' half as many bytes it gave nothing.
+    // they would delay what the layer waits for. Eight layers 155.5 -> 154.7 us (three comparisons, 0.5 to 0.7 % each); on the int4 experts' half as
+    // many bytes it gave nothing.
     mbar_wait(&ctl.full[QUARTERS - 1], 0, DRB_ERR_FULL_WAIT);
     const int row = b % (I / UNITS) * DOWN_ROWS;
     const size_t ek = shared ? 0 : (size_t)__ldcg(idx + slot);

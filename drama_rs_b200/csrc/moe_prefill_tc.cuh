@@ -22,8 +22,8 @@
 //                 tcgen05.st. Three stages: 128 columns each, with a token tile in shared memory.
 //   MMA warp      sixteen K = 16 instructions per step, one commit that frees the stage
 //   loader warp   tiled TMA: 128 rows x 128 bytes per request with the 128-byte swizzle; a gate/up tile is 64 gate rows and
-//                 their 64 up rows, which a 4-D view of the weight tensor expresses; the item's scales ride on its
-//                 first request
+//                 their 64 up rows, which a 4-D view of the weight tensor expresses; an int4 item's scales are requested while the item before
+//                 still asks for its stages
 //   token warp    the tokens' fp16 rows: groups of eight consecutive rows by one TMA request per step (4 KB: eight rows of
 //                 four 128-byte swizzled columns), scattered rows by tile::gather4 (512 bytes per request; it costs the copy
 //                 engine 19 cycles against 49 for the 4 KB box)

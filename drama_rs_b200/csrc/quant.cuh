@@ -10,7 +10,7 @@
 //
 //   drb_quant_q4: tools/convert.py:44-89 (`quant_q4_groups`: 24-step clipping search, least-squares refit) and
 //                 92-101 (`quant_q4`: packing, low nibble = even k). Eight lanes per group of 64 inputs.
-//   drb_quant_q8: tools/convert.py:33-41 (`quant_q8`). One warp per group of 128 inputs.
+//   drb_quant_q8: tools/convert.py:33-41 (`quant_q8`). A warp takes four groups of 128 inputs.
 #pragma once
 
 #include "common.cuh"
@@ -145,7 +145,9 @@ constexpr int Q4_THREADS = 256, Q4_WARPS = Q4_THREADS / 32, Q4_GROUPS = Q4_THREA
 constexpr int Q4_STRIDE = 72;   // floats between a warp's four groups in shared memory: their 16-byte reads share no bank
 constexpr float Q4_FLAT = 2e-6f;  // a range below it can bring scales to the converter's floor
 constexpr int Q4_LIGHT = 12;    // candidates that are estimated; the others clip a quarter of the range or more
-// What bounds it: fp32 and integer issue, not memory (4.6 bytes per weight). Of the 24 candidates the first twelve are told apart by
+// What bounds it: fp32 and integer issue (an instruction in 0.83 of the cycles, 1030 per warp), not memory (4.6 bytes per weight). Half of
+// the time are the estimates, half what a group costs without them: loads, two candidates a lane, one evaluation, refinement, packing
+// (134 M bf16 weights: 276 us of 560 with the estimates left out). Of the 24 candidates the first twelve are told apart by
 // the estimate, lane j taking candidate j over the group's 64 inputs and candidate 8 + j % 4 over half of them (shared memory, broadcast
 // reads), and only those that the estimate's error leaves in the running are evaluated in the converter's operations and order: 1.02
 // on average on normal weights: 0.56 ms for 134 M weights. Every candidate evaluated that way took 1.48 ms, the half that a bound by the ends
@@ -333,8 +335,10 @@ __global__ void __launch_bounds__(Q4_THREADS, 5) k_quant_q4(const float* __restr
 }
 
 // Lane l holds inputs 4l .. 4l + 3 of a group of 128; a warp takes four groups, all of them requested before the first is used.
-// Bound by the bytes (5 per weight): 134 M weights 162 -> 105 us, 6.4 TB/s, with one group per warp and four divisions per lane before. A quotient is taken as a product with the reciprocal, within 2^-22 of it; where that lands
-// within 1e-4 of a rounding boundary it is settled by the exact remainder, as in codes8 (a code has seven bits and the scale eleven, so their product is exact).
+// Bound by the bytes (5 per weight): 134 M weights take 105 us, 6.4 TB/s; the issue slots stand at 0.74 beside it. (A group per warp, with four
+// divisions per lane, took 162.) A quotient is taken as a product with the reciprocal, within 2^-22 of it; where that lands within 1e-4
+// of a rounding boundary it is settled by the exact remainder, as in codes8 (a code has seven bits and the scale eleven, so their
+// product is exact).
 constexpr int Q8_PER = 4, Q8_WARPS = 8;
 __global__ void __launch_bounds__(Q8_WARPS * 32) k_quant_q8(const float* __restrict__ w, size_t groups, int8_t* __restrict__ q,
                                                   __half* __restrict__ s) {

@@ -85,7 +85,8 @@ int dr_gemv_bf16(const dr_bf16* w, const float* x, float* y, int n, int k, const
 /* Decode router: logits[0..e] = W[e+1, k] . rmsnorm(x); softmax over the first e, top-k in
  * descending probability (ties to the lower index), wts renormalised, sgate = logits[e].
  * counter: one zeroed u32 that is left zero. gu_q != NULL asks for an L2 prefetch of the chosen
- * experts (sizes in bytes per expert). k == 2048, e <= 256, topk <= 32.
+ * experts (sizes in bytes per expert). k == 2048, e <= 256, topk <= 32. w is read ahead of the launch before and must not be that
+ * launch's work; nw may be.
  * drama.cu:371-461; ffi.rs:56-60 */
 int dr_router_topk(const dr_bf16* w, const float* x, const float* nw, float eps, float* logits, int e, int topk,
                    int k, int* idx, float* wts, float* sgate, unsigned* counter, const char* gu_q, const char* gu_sm,
